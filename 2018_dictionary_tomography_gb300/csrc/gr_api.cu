@@ -76,6 +76,17 @@ bool batch_member(const gr_batch_member &m, BatchProb &p) {
 
 }  // namespace
 
+namespace gr {
+// Workspace that gr_radproj cannot do without (0: invalid arguments).
+size_t project_least_bytes(const gr_atoms *atoms, const gr_geometry *geom) {
+  Atoms at;
+  Geom g;
+  int st;
+  if (!to_internal(atoms, geom, at, g, &st)) return 0;
+  return project_min_bytes(g.K, at.n, g.n_angles, g.ax[0].n, g.K == 2 ? g.ax[1].n : 1);
+}
+}  // namespace gr
+
 extern "C" {
 
 size_t gr_batch_workspace_bytes(const gr_batch_member *members, int n) {

@@ -44,6 +44,39 @@ __device__ __forceinline__ float lg2_approx(float v) {
   return y;
 }
 
+// Two FP32 values in one register pair (sm_100 and later): one instruction
+// adds, multiplies or fuses both, each half rounded as the scalar operation.
+struct F2 {
+  unsigned long long v;
+};
+__device__ __forceinline__ F2 f2(float x, float y) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ void f2_get(const F2 &a, float &x, float &y) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v));
+}
+__device__ __forceinline__ F2 f2_add(const F2 &a, const F2 &b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_mul(const F2 &a, const F2 &b) {
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_fma(const F2 &a, const F2 &b, const F2 &c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+// a - b (the product with -1 is exact, so this rounds as a subtraction)
+__device__ __forceinline__ F2 f2_sub(const F2 &a, const F2 &b) {
+  return f2_fma(b, f2(-1.f, -1.f), a);
+}
+
 // Error-free transforms (Knuth TwoSum, FMA TwoProduct) used for the
 // compensated projection centre and compensated accumulators.
 __device__ __forceinline__ void two_sum(float a, float b, float &s, float &e) {
@@ -198,6 +231,7 @@ struct Pair {
   // quantities kept for the derivative assembly
   float Kc[K + 1][K + 1];  // Kc[c][a] = (r B_c)_a, c = 0..K-1 detector axes, K = T
   float Q[K + 1][K + 1];   // Q[c][d] = Kc[c] . Kc[d]
+  float U[K][K + 1];       // projected detector axes, G = U^T U
 };
 
 template <int K>
@@ -234,7 +268,7 @@ __device__ __forceinline__ bool pair_setup(const Atoms &at, int j,
   p.n = rsqrtf(qtt);
   // G = U^T U with U_i = K_i - t (t . K_i), t = K_T / |K_T| (the projected
   // detector axes); this Gram form stays positive semi-definite in FP32.
-  float U[K][D];
+  float (&U)[K][D] = p.U;
 #pragma unroll
   for (int i = 0; i < K; ++i) {
     const float c = p.Q[i][K] * iqtt;
@@ -424,6 +458,21 @@ __device__ __forceinline__ void warp_reduce_scatter32(float (&v)[32], int lane) 
       const float give = up ? v[k] : v[k + m];
       v[k] = keep + __shfl_xor_sync(0xffffffffu, give, m);
     }
+  }
+}
+
+// Sums of FP32 pairs (value and compensation): (s, c) += (t, d).
+__device__ __forceinline__ void pair_add(float &s, float &c, float t, float d) {
+  float h, e;
+  two_sum(s, t, h, e);
+  s = h;
+  c += d + e;
+}
+__device__ __forceinline__ void pair_warp_sum(float &s, float &c) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const float t = __shfl_xor_sync(0xffffffffu, s, o), d = __shfl_xor_sync(0xffffffffu, c, o);
+    pair_add(s, c, t, d);
   }
 }
 

@@ -7,7 +7,7 @@
 namespace gr {
 
 // ---- forward projection tiling -------------------------------------------
-constexpr int kProjWarps = 4;        // independent (angle, tile) warps per CTA
+constexpr int kProjWarps = 4;        // warps per CTA (2D and pixel-integrated)
 constexpr int kTileDim0 = 32;        // 3D tile rows (detector axis 0)
 constexpr int kTileDim1 = 32;        // 3D tile cols (detector axis 1, contiguous)
 constexpr int kTile1D = 32;          // 2D tile length (one cell per lane)
@@ -25,7 +25,19 @@ struct TileCfg {
   int t0, t1;     // tile extent along detector axes 0 and 1
   int nt0, nt1;   // tiles along each axis
   int ntiles;
+  uint32_t inv_ntiles, inv_nt1;   // floor(2^32 / .), for tile_div
 };
+
+// n / d, inv = floor(2^32 / d) (2^32 - 1 for d = 1): the product is at most
+// one too small.
+__host__ __device__ __forceinline__ int tile_div(uint32_t n, uint32_t d, uint32_t inv) {
+#ifdef __CUDA_ARCH__
+  uint32_t q = __umulhi(n, inv);
+#else
+  uint32_t q = (uint32_t)(((unsigned long long)n * inv) >> 32);
+#endif
+  return (int)(n - q * d >= d ? q + 1 : q);
+}
 
 enum Epilogue : int { kEpiNone = 0, kEpiL2 = 1, kEpiKL = 2 };
 
@@ -90,7 +102,7 @@ struct Tuning {
   int deriv_min_angles = 1;         // key 1
   int deriv_atoms_per_warp = 0;     // key 2 (0: automatic)
   int proj_form = 1;                // key 3 (3D 1: 16 x 32 tiles, 2: 32 x 32; 2D 32, 64, 128 cells)
-  int proj_split_cells = 4 << 20;   // key 4
+  int proj_split_cells = 4 << 20;   // key 4 (accepted, without effect: blocks share every tile)
   int deriv_split_lanes = 65536;    // key 6
   int deriv_one_mb = 1024;          // key 7
   int deriv_wide_rows = 0;          // key 8 (1: 3D Hessian rows in 8-cell chunks)
@@ -104,6 +116,8 @@ TileCfg make_tiles(int K, int D0, int D1, int rows);
 // (angle, tile) items of a forward that can skip items no atom meets (the
 // point-sampled 3D projection under t's tiling; 0 for the others)
 size_t project_skip_items(const Geom &g, int psf, const Tuning &t = g_tuning);
+size_t project_min_bytes(int K, int n_atoms, int n_angles, int D0, int D1,
+                         const Tuning &t = g_tuning);
 size_t project_workspace_bytes(int K, int n_atoms, int n_angles, int D0, int D1,
                                const Tuning &t = g_tuning);
 int launch_project(const Atoms &at, const Geom &g, const ProjOut &o,

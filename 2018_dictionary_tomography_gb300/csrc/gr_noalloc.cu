@@ -33,6 +33,10 @@
 #include "gauss_radon.h"
 #include "gr_kernels.cuh"
 
+namespace gr {
+size_t project_least_bytes(const gr_atoms *atoms, const gr_geometry *geom);  // gr_api.cu
+}
+
 namespace {
 
 constexpr size_t kNoAllocScratchBytes = size_t(4) << 20;
@@ -115,7 +119,8 @@ extern "C" int gr_radproj_noalloc(const gr_atoms *atoms, const gr_geometry *geom
                                   float *R, void *stream) {
   using namespace gr;
   if (!atoms || !geom || !R) return GR_ERR_ARG;
-  const size_t need = gr_workspace_bytes(GR_OP_PROJECT, atoms, geom);
+  // (3D pair records use what the scratch has left, if anything)
+  const size_t need = project_least_bytes(atoms, geom);
   if (need == 0) return GR_ERR_ARG;  // invalid atoms or geometry
   if (need > kNoAllocScratchBytes) return GR_ERR_TOO_LARGE;
   void *ws = noalloc_scratch_for_current_device();

@@ -4,98 +4,64 @@
 // (GaussDictCode/bin/NewtonBases2D.py:286-296) and __RadProj_3D/_2p5D
 // (GaussDictCode/bin/NewtonBases.py:731-756), which evaluate every atom at
 // every detector cell.  Here:
-//   1. gr_bin_kernel: per (atom, angle) pair, compute the support box of
-//      m <= 1 and set the atom's bit in the bitmap of every detector tile the
-//      box touches (integer atomicOr, so the bitmap does not depend on the
-//      order in which pairs run).
+//   1. binning (gr_bin_kernel, gr_bin3d_kernel): per (atom, angle) pair,
+//      compute the support box of m <= 1, write the pair's projection data and
+//      set the atom's bit in the bitmap of every detector tile the box touches
+//      (bits only, so the bitmap does not depend on the order in which pairs
+//      run).
 //   2. gr_project3d_kernel (3D / 2.5D detectors) and gr_project1d_kernel
-//      (2D sinograms): one warp per (angle, tile) item.  The warp meets the
-//      tile's atoms in increasing index order and sums every cell over its
-//      atoms in that order with a compensated add and no float atomics, so
-//      results are bitwise reproducible.  The epilogue writes the sinogram
-//      and, fused, the residual or KL weight fields and per-tile loss
-//      partials.  The 3D kernel is persistent: warps take items from a
-//      counter, so tiles of uneven weight do not leave warps idle.
+//      (2D sinograms): a block per (angle, tile) item, the cells' sums in
+//      registers.  Every cell meets the tile's atoms in increasing index order
+//      and adds them with a compensated add and no float atomics, so results
+//      are bitwise reproducible.  The epilogue writes the sinogram and, fused,
+//      the residual or KL weight fields and per-tile loss partials.
 //   3. gr_loss_finalize_kernel: fixed-order FP64 sum of the loss partials.
 #include "gr_kernels.cuh"
 
 namespace gr {
 
-// pairs (2D only, nullable): the pair's projection data as the 2D
-// projection stages it, two float4 per (angle, atom) at [a n + j], written
-// here once instead of being recomputed by every tile the atom touches
-// The body of a 128-thread block of the binning launch: atoms bx * 128 ..,
-// angle a (the launch's block (bx, a); a multi-problem launch maps its
-// blocks to (problem, bx, a)).
-// flag, list, n_list (3D, nullable): the items some atom meets, listed once
-// each (in no fixed order: the order changes no result) for a forward that
-// skips the others.  Only the first bit set in a word can be an item's first,
-// so an item's flag is tested once per word it uses, not once per atom.
-template <int K>
+// 2D binning: the body of a 128-thread block, atoms bx * 128 .., angle a (the
+// launch's block (bx, a); a multi-problem launch maps its blocks to (problem,
+// bx, a)).  pairs (nullable): the pair's projection data as the projection
+// stages it, two float4 per (angle, atom) at [a n + j], written here once
+// instead of being recomputed by every tile the atom touches.
 __device__ __forceinline__ void bin_body(const Atoms &at, const Geom &g, const TileCfg &tc,
-                                         uint32_t *bitmap, int W, float4 *pairs, int bx,
-                                         int a, uint32_t *flag = nullptr, int *list = nullptr,
-                                         int *n_list = nullptr) {
+                                         uint32_t *bitmap, int W, float4 *pairs, int bx, int a) {
   const int j = bx * 128 + (int)threadIdx.x;
   const uint32_t bit = 1u << (j & 31);
   const size_t base = (size_t)a * tc.ntiles;
   const int wj = j >> 5;
-  if constexpr (K == 1) {
-    // a warp holds 32 consecutive atoms: one bitmap word per tile.  Their
-    // bits are merged per tile across the warp (one atomicOr per tile the
-    // warp touches, not one per atom and tile: the 32 atoms of a word would
-    // otherwise all hit the same address)
-    int t_lo = 1 << 30, t_hi = -1;
-    if (j < at.n) {
-      Frame<1> f;
-      load_frame<1>(g.frames, a, f);
-      Pair<1> p;
-      pair_setup<1>(at, j, f, g, p);
-      if (pairs) {
-        float4 *rec = pairs + ((size_t)a * at.n + j) * 2;
-        rec[0] = make_float4(p.qh[0], p.ql[0], p.G[0], p.l2amp);
-        rec[1] = make_float4(__int_as_float(p.lo[0]), __int_as_float(p.hi[0]), p.sgn, 0.f);
-      }
-      if (p.lo[0] <= p.hi[0]) {
-        t_lo = p.lo[0] / tc.t0;
-        t_hi = p.hi[0] / tc.t0;
-      }
+  // a warp holds 32 consecutive atoms: one bitmap word per tile.  Their
+  // bits are merged per tile across the warp (one atomicOr per tile the
+  // warp touches, not one per atom and tile: the 32 atoms of a word would
+  // otherwise all hit the same address)
+  int t_lo = 1 << 30, t_hi = -1;
+  if (j < at.n) {
+    Frame<1> f;
+    load_frame<1>(g.frames, a, f);
+    Pair<1> p;
+    pair_setup<1>(at, j, f, g, p);
+    if (pairs) {
+      float4 *rec = pairs + ((size_t)a * at.n + j) * 2;
+      rec[0] = make_float4(p.qh[0], p.ql[0], p.G[0], p.l2amp);
+      rec[1] = make_float4(__int_as_float(p.lo[0]), __int_as_float(p.hi[0]), p.sgn, 0.f);
     }
-    const int w_lo = __reduce_min_sync(0xffffffffu, t_lo);
-    const int w_hi = __reduce_max_sync(0xffffffffu, t_hi);
-    for (int t = w_lo; t <= w_hi; ++t) {
-      const unsigned bits = __reduce_or_sync(0xffffffffu, (t >= t_lo && t <= t_hi) ? bit : 0u);
-      if ((threadIdx.x & 31) == 0 && bits) atomicOr(bitmap + (base + t) * W + wj, bits);
+    if (p.lo[0] <= p.hi[0]) {
+      t_lo = p.lo[0] / tc.t0;
+      t_hi = p.hi[0] / tc.t0;
     }
-  } else {
-    if (j >= at.n) return;
-    Frame<K> f;
-    load_frame<K>(g.frames, a, f);
-    Pair<K> p;
-    pair_setup<K>(at, j, f, g, p);
-    if (p.lo[0] > p.hi[0]) return;
-    if (p.lo[1] > p.hi[1]) return;
-    const int r_lo = p.lo[0] / tc.t0, r_hi = p.hi[0] / tc.t0;
-    const int c_lo = p.lo[1] / tc.t1, c_hi = p.hi[1] / tc.t1;
-    for (int tr = r_lo; tr <= r_hi; ++tr)
-      for (int tcix = c_lo; tcix <= c_hi; ++tcix) {
-        const size_t item = base + (size_t)tr * tc.nt1 + tcix;
-        if (flag == nullptr) {
-          atomicOr(bitmap + item * W + wj, bit);
-        } else if (atomicOr(bitmap + item * W + wj, bit) == 0u &&
-                   atomicExch(flag + item, 1u) == 0u) {
-          list[atomicAdd(n_list, 1)] = (int)item;
-        }
-      }
+  }
+  const int w_lo = __reduce_min_sync(0xffffffffu, t_lo);
+  const int w_hi = __reduce_max_sync(0xffffffffu, t_hi);
+  for (int t = w_lo; t <= w_hi; ++t) {
+    const unsigned bits = __reduce_or_sync(0xffffffffu, (t >= t_lo && t <= t_hi) ? bit : 0u);
+    if ((threadIdx.x & 31) == 0 && bits) atomicOr(bitmap + (base + t) * W + wj, bits);
   }
 }
 
-template <int K>
-__global__ void __launch_bounds__(128) gr_bin_kernel(Atoms at, Geom g,
-                                                     TileCfg tc, uint32_t *bitmap,
-                                                     int W, float4 *pairs, uint32_t *flag,
-                                                     int *list, int *n_list) {
-  bin_body<K>(at, g, tc, bitmap, W, pairs, blockIdx.x, blockIdx.y, flag, list, n_list);
+__global__ void __launch_bounds__(128) gr_bin_kernel(Atoms at, Geom g, TileCfg tc,
+                                                     uint32_t *bitmap, int W, float4 *pairs) {
+  bin_body(at, g, tc, bitmap, W, pairs, blockIdx.x, blockIdx.y);
 }
 
 // Per-cell KL term f log(f/g) - f + g = g h(u), u = f/g, h(u) = u log u - u + 1,
@@ -116,281 +82,467 @@ __device__ __forceinline__ float kl_term(float f, float g) {
   return g * h;
 }
 
-// 3D detectors: a warp per (angle, tile) item.  Its atoms come from the
-// tile's bitmap in increasing index order; the pair data of each batch of 32
-// atoms is computed in parallel (one atom per lane) and staged in shared
-// memory (three float4 per atom, read as broadcasts, the tile-local clipped
-// box packed in one word); then each atom is evaluated densely over its box,
-// lanes spread over the box cells, into shared-memory cell sums with a
-// compensated (Kahan/Neumaier) add.  Each cell therefore sums its atoms in
-// atom-index order, with no float atomics: results are bitwise reproducible.
-// Sums and compensations use a padded row stride S so that the cells of one
-// box row-block fall in different banks.  Tiles are ROWS x 32 cells.
-template <int ROWS, int S>
-struct Proj3Smem {
-  static constexpr int kAcc = ROWS * S;
-  static constexpr int kRing = 128;     // ring list of atom indices
-  static constexpr int kFloats = 2 * kAcc + 32 * 12 + ROWS + 32 + kRing;
+// 3D detectors: a block of NW warps per (angle, tile) item, tile 4 NW x 32
+// cells.  Each cell's sum lives in the registers of one lane; the atoms come to
+// the cells:
+//   * the tile's atoms (its bitmap, increasing index) are taken in passes of
+//     32 NW; a thread stages one atom's record (Proj3Rec: written once per
+//     (atom, angle) by the binning launch) in shared memory and marks the
+//     4 x 2 subtiles its ellipse meets; a 32 x 32 bit transpose per warp turns
+//     the atoms' subtile bits into the subtiles' atom masks;
+//   * a warp owns 16 x 8 cells, 16 subtiles, one per pair of lanes, 2 x 2
+//     cells a lane; each pair of lanes walks its own subtile's mask, so a warp
+//     step is 16 (subtile, atom) visits.
+// A cell therefore adds its atoms in index order with an exact two-sum and a
+// running compensation, whatever the tiling: results are bitwise reproducible
+// and the same under every tile height.
+// What bounds it: instruction issue (75 % of the slots on 8192 atoms x 2048
+// orientations; DRAM under 10 %).  Per (atom, angle) pair of 22 in-support
+// cells it issues 60 warp instructions: the visits 28, the masks' walk 15, the
+// staging the rest.  One warp walking an atom's whole box over sums in shared
+// memory, the layout before this one, issued 141: index arithmetic and the
+// read-modify-write of the sums for every 32 box cells, two lanes in three
+// active.  Why 2 x 2 cells a lane and 4 x 2 subtiles: of the shapes from
+// 2 x 2 to 8 x 4 cells they gave the fewest warp steps times instructions for
+// footprints of 20 to 140 cells; packed FP32 pairs do both rows at once.
+// 8192 atoms x 20000 x 128^2 cells: binning + projection 23.6 -> 15.1 ms; 1000
+// atoms x 1001 x 95^2: 185 -> 128 us; 2936 atoms x 148 x 493^2: 309 -> 278 us
+// (there 127 us are the 73408 items' own loads and stores: 2.1 us an item and
+// block, latency).  64 registers, 8 blocks an SM; 48 registers: 5 to 10 % slower.
+struct Proj3Rec {
+  float4 a;   // (-qh0, -ql0, -qh1, -ql1): the centre's negative, as a float pair
+  float4 b;   // (u11, u01, +-u00, log2 amplitude)
 };
 
-// NW = 1: persistent warps, each (angle, tile) item walked by one warp.
-// NW = kProjWarps: persistent blocks, each item walked by the whole block,
-// warp w taking the atoms of bitmap words [w wq, (w + 1) wq), wq = ceil(W/NW),
-// into its own cell sums; the block then combines the warps' sums per cell
-// in warp order (compensated).  The word ranges depend on W only, so every
-// tiling still gives the same cell sums.  Used when a problem has too few
-// items to keep the SMs busy: the slowest item, not the total, then sets
-// the kernel time, and splitting its atom list cuts that item's latency.
-// With loss_out, the last block (or warp) to finish sums the items' loss
-// partials in item order (no separate finalize launch).
-// LIST: take only the n_list[0] items of item_list (those some atom meets;
-// the loss partials of the others are already in place).  A template
-// parameter, so that the forward of every item keeps its own registers.
-template <int ROWS, int S, int NW, bool LIST>
-__global__ void __launch_bounds__(kProjWarps * 32)
+// The pair's record: with d = p - q*, 30/ln2 times the form is
+// (u11 d1 + u01 d0)^2 + (u00 d0)^2; u00 comes from the part of U0 orthogonal
+// to U1 (no cancellation of G00 with G01^2 / G11) and carries the sign of I.
+__device__ __forceinline__ Proj3Rec proj3_record(const Pair<2> &p) {
+  const float C = -kNegThirtyLog2e;
+  const float u11 = sqrtf(C * p.G[2]);
+  const float u01 = __fdiv_rn(C * p.G[1], u11);
+  const float t = __fdiv_rn(p.G[1], p.G[2]);
+  float vv = 0.f;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const float v = fmaf(-t, p.U[1][i], p.U[0][i]);
+    vv = fmaf(v, v, vv);
+  }
+  Proj3Rec o;
+  o.a = make_float4(-p.qh[0], -p.ql[0], -p.qh[1], -p.ql[1]);
+  o.b = make_float4(u11, u01, copysignf(sqrtf(C * vv), p.sgn), p.l2amp);
+  return o;
+}
+
+__device__ __forceinline__ float sqrt_approx(float v) {
+  float y;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(v));
+  return y;
+}
+__device__ __forceinline__ float rcp_approx(float v) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(v));
+  return y;
+}
+
+// The subtiles of the tile (rows r0.., columns c0..) that the record's support
+// ellipse meets: bit 16 (b % 2) + c of word b / 2 for rows r0 + 4 b .. + 3,
+// columns c0 + 2 c, + 1.  Over a band of 4 rows the ellipse's column range is
+// reached at the row nearest to its rightmost (leftmost) point; it is widened
+// by 0.02 cells (approximate square roots, FP32 rounding near the ellipse's
+// tips): the cells' own test decides.
+template <int NB>
+__device__ __forceinline__ void proj3_subtiles(const Proj3Rec &q, const Geom &g, int r0, int c0,
+                                               uint32_t (&cols)[NB / 2]) {
+  const float rC = 6.5788183f;                            // sqrt(30 / ln 2)
+  const float h0 = rcp_approx(g.ax[0].inv_step);
+  const float q0 = (-q.a.x - g.ax[0].first) * g.ax[0].inv_step - (float)r0;   // centre in
+  const float q1 = (-q.a.z - g.ax[1].first) * g.ax[1].inv_step - (float)c0;   // tile cells
+  const float k = g.ax[1].inv_step * rcp_approx(q.b.x);
+  const float S = -q.b.y * h0 * k;                        // columns q1 + S d +- hw(d),
+  const float a0 = fabsf(q.b.z) * h0;                     // hw(d) = k sqrt(C - a0^2 d^2)
+  const float ka = k * a0;
+  const float dmax = rC * rcp_approx(a0);                 // rows within dmax
+  const float len = sqrt_approx(fmaf(S, S, ka * ka));
+  const float dx = S * rcp_approx(len) * dmax;            // row of the rightmost point
+  const bool plain = fabsf(dx) < 1e8f && dmax < 1e8f;     // else every subtile
+  const float top = q0 - dmax - 0.02f, bot = q0 + dmax + 0.02f;
+#pragma unroll
+  for (int w = 0; w < NB / 2; ++w) cols[w] = 0u;
+#pragma unroll
+  for (int b = 0; b < NB; ++b) {
+    const float ra = fmaxf(top, (float)(4 * b)), rb = fminf(bot, (float)(4 * b + 3));
+    const float da = ra - q0, db = rb - q0;
+    const float dr = fminf(fmaxf(dx, da), db), dl = fminf(fmaxf(-dx, da), db);
+    const float hr = k * sqrt_approx(fmaxf(fmaf(-a0 * dr, a0 * dr, rC * rC), 0.f));
+    const float hl = k * sqrt_approx(fmaxf(fmaf(-a0 * dl, a0 * dl, rC * rC), 0.f));
+    const float xr = fminf(fmaf(S, dr, q1) + fmaf(hr, 1.0001f, 0.02f), 31.f);
+    const float xl = fmaxf(fmaf(S, dl, q1) - fmaf(hl, 1.0001f, 0.02f), 0.f);
+    const int xa = (int)ceilf(xl), xb = (int)floorf(xr);
+    uint32_t m = xa <= xb && ra <= rb ? (2u << (xb >> 1)) - (1u << (xa >> 1)) : 0u;
+    if (!plain) m = 0xffffu;
+    cols[b / 2] |= m << (16 * (b % 2));
+  }
+}
+
+// Bit transpose over the warp: bit i of lane l becomes bit l of lane i.
+__device__ __forceinline__ uint32_t warp_transpose32(uint32_t x, int lane) {
+#pragma unroll
+  for (int j = 16; j >= 1; j >>= 1) {
+    const uint32_t lo = j == 16 ? 0x0000ffffu : j == 8 ? 0x00ff00ffu
+                        : j == 4 ? 0x0f0f0f0fu : j == 2 ? 0x33333333u : 0x55555555u;
+    const uint32_t y = __shfl_xor_sync(0xffffffffu, x, j);
+    const bool up = (lane & j) != 0;
+    const uint32_t rot = __funnelshift_l(y, y, up ? 32 - j : j);
+    const uint32_t keep = up ? ~lo : lo;
+    x = (x & keep) | (rot & ~keep);
+  }
+  return x;
+}
+
+// One visit: the record's values at a lane's 2 x 2 cells, added to their sums.
+// row, col: the cells' coordinates; s, c: sums and compensations of the two
+// cells of each column.
+__device__ __forceinline__ void proj3_visit(const Proj3Rec &q, const float (&row)[2],
+                                            const float (&col)[2], F2 (&s)[2], F2 (&c)[2]) {
+  float bb[2], cc[2];
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const float d0 = (row[r] + q.a.x) + q.a.y;
+    const float b = q.b.z * d0;
+    bb[r] = b * b;
+    cc[r] = q.b.y * d0;
+  }
+  const float sg = copysignf(1.f, q.b.z);
+  const F2 S = f2(sg, sg), bbp = f2(bb[0], bb[1]);
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const float d1 = (col[k] + q.a.z) + q.a.w;
+    const F2 a = f2(fmaf(q.b.x, d1, cc[0]), fmaf(q.b.x, d1, cc[1]));
+    float m0, m1;
+    f2_get(f2_fma(a, a, bbp), m0, m1);               // 30/ln2 times the form
+    const float e0 = ex2_approx(q.b.w - m0), e1 = ex2_approx(q.b.w - m1);
+    const F2 v = f2(m0 <= -kNegThirtyLog2e ? e0 : 0.f, m1 <= -kNegThirtyLog2e ? e1 : 0.f);
+    // two-sum of s and S v, both cells at once
+    const F2 tt = f2_fma(v, S, s[k]);
+    const F2 nb = f2_sub(s[k], tt);
+    const F2 w = f2_sub(s[k], f2_add(tt, nb));
+    c[k] = f2_add(c[k], f2_add(w, f2_fma(v, S, nb)));
+    s[k] = tt;
+  }
+}
+
+// With loss_out, the last block to finish sums the items' loss partials in
+// item order (no separate finalize launch).
+// LIST: only the n_list[0] items of item_list are taken (those some atom
+// meets; the loss partials of the others are already in place).
+// rec (nullable): the (angle, atom) records; without it a thread sets its
+// pairs up itself.
+template <int NW, bool LIST>
+__global__ void __launch_bounds__(NW * 32, 32 / NW)
     gr_project3d_kernel(Atoms at, Geom g, TileCfg tc, const uint32_t *bitmap, int W,
-                        ProjOut out, int *next_item, double *loss_out,
-                        const int *item_list, const int *n_list) {
-  static_assert(NW == 1 || NW == kProjWarps, "a split item takes the whole block");
-  using L = Proj3Smem<ROWS, S>;
-  constexpr int kRing = L::kRing;
-  static_assert((kRing & (kRing - 1)) == 0 && kRing >= 64, "ring");
-  extern __shared__ float smem[];
+                        const Proj3Rec *__restrict__ rec, ProjOut out, int *next_item,
+                        double *loss_out, const int *item_list, const int *n_list) {
+  constexpr int T = NW * 32;            // threads
+  constexpr int kWords = 2 * NW;        // 32-atom words per pass
+  constexpr int kSub = 16 * NW;         // subtiles of the tile
+  constexpr int kList = 1024;           // atoms listed at a time
+  constexpr int kPitch = 36;
+  // slot 33 k + 1 + l: the record of bit l of word k; slot 33 k adds nothing
+  // (where a mask runs dry)
+  __shared__ float4 sA[33 * kWords], sB[33 * kWords];
+  __shared__ uint32_t sMask[kWords][kSub];
+  __shared__ int list[kList];
+  __shared__ int s_count[NW];
+  __shared__ float sV[4 * NW][kPitch];
   __shared__ int s_item;
-  __shared__ double s_loss[NW];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  __shared__ float2 s_loss[T];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n_items = g.n_angles * tc.ntiles;
-  const int n_take = LIST ? *n_list : n_items;
-  float *acc = smem + (size_t)warp * L::kFloats;
-  float *cmp = acc + L::kAcc;
-  float4 *prm = reinterpret_cast<float4 *>(cmp + L::kAcc);  // 16-byte aligned
-  float *pc0 = reinterpret_cast<float *>(prm + 32 * 3);
-  float *pc1 = pc0 + ROWS;
-  int *list = reinterpret_cast<int *>(pc1 + 32);
-  const int wq = (W + NW - 1) / NW;
-  const int w_lo = min(W, warp * wq * (NW > 1)), w_hi = NW > 1 ? min(W, w_lo + wq) : W;
-
-  // persistent warps (blocks): each takes the next (angle, tile) item from a
-  // counter, so heavy tiles do not hold the others idle; what an item
-  // computes does not depend on which warp (block) takes it
-  for (;;) {
-  int item = 0;
-  if constexpr (NW == 1) {
-    if (lane == 0) item = atomicAdd(next_item, 1);
-    item = __shfl_sync(0xffffffffu, item, 0);
-    if (item >= n_take) break;  // whole warp leaves together
-    __syncwarp();  // the previous item's epilogue reads are done
-  } else {
-    if (threadIdx.x == 0) s_item = atomicAdd(next_item, 1);
-    __syncthreads();
-    item = s_item;
-    if (item >= n_take) break;  // whole block leaves together
-  }
-  if constexpr (LIST) item = item_list[item];
-  const int a = item / tc.ntiles, t = item - a * tc.ntiles;
-  const int tr = t / tc.nt1, tcix = t - tr * tc.nt1;
-  const int r0 = tr * ROWS, c0 = tcix * 32;
   const int D0 = g.ax[0].n, D1 = g.ax[1].n;
-
-  for (int e = lane; e < L::kAcc; e += 32) {
-    acc[e] = 0.f;
-    cmp[e] = 0.f;
+  // the lane's subtile and cells
+  const int grp = lane >> 1;
+  const int band = 4 * (warp >> 2) + (grp >> 2), cpair = 4 * (warp & 3) + (grp & 3);
+  const int row_in = 4 * band + 2 * (lane & 1), col_in = 2 * cpair;
+  const int n_take = LIST ? *n_list : n_items;
+  if (tid < kWords) {
+    sA[33 * tid] = make_float4(0.f, 0.f, 0.f, 0.f);
+    sB[33 * tid] = make_float4(0.f, 0.f, 0.f, __int_as_float(0xff800000));
   }
-  for (int e = lane; e < ROWS; e += 32)
-    pc0[e] = (r0 + e < D0) ? g.ax[0].coords[r0 + e] : 0.f;
-  pc1[lane] = (c0 + lane < D1) ? g.ax[1].coords[c0 + lane] : 0.f;
-  Frame<2> f;
-  load_frame<2>(g.frames, a, f);
-  __syncwarp();
 
-  // The warp's atoms of the tile, in index order, pass through a ring list:
-  // a refill reads 32 bitmap words (one per lane) and appends the atoms of as
-  // many whole words as fit, so every batch but the last holds 32 atoms
-  // however sparse the bitmap is.
-  const uint32_t *words = bitmap + (size_t)item * W;
-  int head = 0, count = 0, wb = w_lo;
-  while (true) {
-    while (count < 32 && wb < w_hi) {
-      const int wi = wb + lane;
-      uint32_t wd = wi < w_hi ? words[wi] : 0u;
-      const int cnt = __popc(wd);
-      int incl = cnt;
+  // persistent blocks: the first item is the block's own, the others come from
+  // a counter (asked for an item ahead), so heavy tiles do not hold the others
+  // idle; what an item computes does not depend on which block takes it
+  int take = blockIdx.x;
+  while (take < n_take) {
+    int ahead = 0;
+    if (tid == 0) ahead = (int)gridDim.x + atomicAdd(next_item, 1);
+    const int item = LIST ? item_list[take] : take;
+    const int a = tile_div(item, tc.ntiles, tc.inv_ntiles), t = item - a * tc.ntiles;
+    const int tr = tile_div(t, tc.nt1, tc.inv_nt1), tcix = t - tr * tc.nt1;
+    const int r0 = tr * (4 * NW), c0 = tcix * 32;
+    // the tile's atoms: warp w counts the words [w per, (w + 1) per)
+    const uint32_t *words = bitmap + (size_t)item * W;
+    int per = (W + NW - 1) / NW;
+    int wlo = min(W, warp * per), whi = min(W, wlo + per);
+    uint32_t wd0 = wlo + lane < whi ? __ldg(words + wlo + lane) : 0u;
+    int mine = __popc(wd0);
+    for (int wb = wlo + 32 + lane; wb < whi; wb += 32) mine += __popc(__ldg(words + wb));
+    // the epilogue's cells of this thread: rows 4 warp .. + 3, column lane;
+    // their data is read before the atoms so that the epilogue does not wait
+    const bool want_data = out.epilogue == kEpiL2 || out.epilogue == kEpiKL;
+    const int er = r0 + 4 * warp, ec = c0 + lane;
+    const int nr = ec < D1 ? min(4, D0 - er) : 0;   // its cells inside the detector
+    const size_t gi0 = ((size_t)a * D0 + er) * D1 + ec;
+    float dv[4] = {0.f, 0.f, 0.f, 0.f};
+    if (want_data) {
+      const float *src = out.data + gi0;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
-      }
-      // incl never decreases along the lanes, so the lanes that fit are a
-      // prefix; at least one word fits (count < 32, a word adds <= 32)
-      const bool take = incl <= kRing - count;
-      const unsigned tmask = __ballot_sync(0xffffffffu, take);
-      const int ntake = __popc(tmask);
-      if (take) {
-        int pos = head + count + incl - cnt;
-        while (wd) {
-          const int b = __ffs(wd) - 1;
-          list[(pos++) & (kRing - 1)] = (wi << 5) + b;
-          wd &= wd - 1;
-        }
-      }
-      count += __shfl_sync(0xffffffffu, incl, ntake - 1);
-      wb += ntake;
-      __syncwarp();
+      for (int r = 0; r < 4; ++r, src += D1)
+        if (r < nr) dv[r] = __ldg(src);
     }
-    if (count == 0) break;
-    {
-      __syncwarp();  // every lane is done with the previous batch's data
-      const int nb = min(32, count);
-      // C.y: the tile-local clipped box as first row | first column << 8 |
-      // width << 16 | rows << 24 (0: empty), C.z: 1 / width; both formed
-      // here, one atom per lane, rather than by the whole warp per atom
-      float4 A = make_float4(0.f, 0.f, 0.f, 0.f), B = A, C = A;
-      if (lane < nb) {
-        Pair<2> p;
-        pair_setup<2>(at, list[(head + lane) & (kRing - 1)], f, g, p);
-        const int lr0 = max(p.lo[0], r0) - r0, lr1 = min(p.hi[0], r0 + ROWS - 1) - r0;
-        const int lc0 = max(p.lo[1], c0) - c0, lc1 = min(p.hi[1], c0 + 31) - c0;
-        const bool empty = lr0 > lr1 || lc0 > lc1;
-        A = make_float4(p.qh[0], p.ql[0], p.qh[1], p.ql[1]);
-        B = make_float4(p.G[0], 2.f * p.G[1], p.G[2], p.l2amp);
-        C.x = p.sgn;
-        const int bw = lc1 - lc0 + 1;
-        C.y = __uint_as_float(empty ? 0u
-                                    : (unsigned)(lr0 | (lc0 << 8) | (bw << 16) |
-                                                 ((lr1 - lr0 + 1) << 24)));
-        C.z = empty ? 0.f : __frcp_rn((float)bw);
+    float v[4] = {0.f, 0.f, 0.f, 0.f};
+    mine = __reduce_add_sync(0xffffffffu, mine);
+    if (lane == 0) s_count[warp] = mine;
+    __syncthreads();
+    int total = 0;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) total += s_count[w];
+
+    if (total > 0) {
+      float row[2], col[2];
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        row[k] = r0 + row_in + k < D0 ? __ldg(g.ax[0].coords + r0 + row_in + k) : 0.f;
+        col[k] = c0 + col_in + k < D1 ? __ldg(g.ax[1].coords + c0 + col_in + k) : 0.f;
       }
-      head += nb;
-      count -= nb;
-      prm[lane * 3 + 0] = A;
-      prm[lane * 3 + 1] = B;
-      prm[lane * 3 + 2] = C;
-      __syncwarp();
-      for (int sI = 0; sI < nb; ++sI) {
-        const float4 qC = prm[sI * 3 + 2];
-        const unsigned box = __float_as_uint(qC.y);
-        if (box == 0u) continue;  // warp-uniform
-        const int lr0 = box & 0xff, lc0 = (box >> 8) & 0xff, bw = (box >> 16) & 0xff;
-        const int ncell = (int)(box >> 24) * bw;
-        const float inv_bw = qC.z;
-        const float4 qA = prm[sI * 3 + 0], qB = prm[sI * 3 + 1];
-        for (int e = lane; e < ncell; e += 32) {
-          // (e + 1/2) / bw is at least 1/(2 bw) from an integer, far more
-          // than the rounding of the product: the row index is exact
-          const int rr = (int)(((float)e + 0.5f) * inv_bw);
-          const int lr = lr0 + rr;
-          const int lc = lc0 + (e - rr * bw);
-          const float d0 = (pc0[lr] - qA.x) - qA.y;
-          const float d1 = (pc1[lc] - qA.z) - qA.w;
-          const float m = fmaf(d0, fmaf(qB.x, d0, qB.y * d1), qB.z * d1 * d1);
-          if (m <= 1.f) {
-            const float v = qC.x * ex2_approx(fmaf(m, kNegThirtyLog2e, qB.w));
-            const int ci = lr * S + lc;
-            const float s0 = acc[ci];
-            const float tt = s0 + v;
-            cmp[ci] += (fabsf(s0) >= fabsf(v)) ? ((s0 - tt) + v) : ((v - tt) + s0);
-            acc[ci] = tt;
+      F2 acc[2], cmp[2];
+#pragma unroll
+      for (int k = 0; k < 2; ++k) acc[k] = cmp[k] = f2(0.f, 0.f);
+      // all words at once where the list holds their atoms, else 32 words at
+      // a time
+      const int step = total <= kList ? W : 32;
+      for (int wbase = 0; wbase < W; wbase += step) {
+        int n_listed = total;
+        if (step < W) {
+          __syncthreads();              // s_count is read
+          const int wi = wbase + lane;
+          per = 32;
+          wlo = warp == 0 ? wbase : W;  // the first warp lists them
+          whi = warp == 0 ? min(W, wbase + 32) : W;
+          wd0 = wi < W ? __ldg(words + wi) : 0u;
+          n_listed = __reduce_add_sync(0xffffffffu, __popc(wd0));
+          if (warp != 0) wd0 = 0u;
+          if (lane == 0) s_count[warp] = warp == 0 ? n_listed : 0;
+          __syncthreads();
+          if (n_listed == 0) continue;
+        }
+        int at_pos = 0;
+#pragma unroll
+        for (int w = 0; w < NW; ++w)
+          if (w < warp) at_pos += s_count[w];
+        for (int wb = wlo; wb < whi; wb += 32) {
+          uint32_t wd = wb == wlo ? wd0 : (wb + lane < whi ? __ldg(words + wb + lane) : 0u);
+          const int cnt = __popc(wd);
+          int incl = cnt;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += u;
           }
+          int pos = at_pos + incl - cnt;
+          while (wd) {
+            list[pos++] = ((wb + lane) << 5) + (__ffs(wd) - 1);
+            wd &= wd - 1;
+          }
+          at_pos += __shfl_sync(0xffffffffu, incl, 31);
         }
-        __syncwarp();
+        __syncthreads();
+        for (int first = 0; first < n_listed; first += 32 * kWords) {
+          const int nwords = min(kWords, (n_listed - first + 31) >> 5);
+          // bit l of a word is the (31 - l)-th of its atoms: a mask's highest
+          // bit is its first atom
+#pragma unroll
+          for (int k0 = 0; k0 < kWords; k0 += NW) {
+            const int k = k0 + warp;
+            if (k >= nwords) break;     // (the warp leaves together)
+            const int e = first + 32 * k + 31 - lane;
+            uint32_t cols[NW / 2];
+#pragma unroll
+            for (int u = 0; u < NW / 2; ++u) cols[u] = 0u;
+            if (e < n_listed) {
+              const int j = list[e];
+              Proj3Rec q;
+              if (rec) {
+                const Proj3Rec *p = rec + (size_t)a * at.n + j;
+                q.a = __ldg(&p->a);
+                q.b = __ldg(&p->b);
+              } else {
+                Frame<2> f;
+                load_frame<2>(g.frames, a, f);
+                Pair<2> p;
+                pair_setup<2>(at, j, f, g, p);
+                q = proj3_record(p);
+              }
+              sA[33 * k + 1 + lane] = q.a;
+              sB[33 * k + 1 + lane] = q.b;
+              proj3_subtiles<NW>(q, g, r0, c0, cols);
+            }
+#pragma unroll
+            for (int u = 0; u < NW / 2; ++u)
+              sMask[k][32 * u + lane] = warp_transpose32(cols[u], lane);
+          }
+          __syncthreads();
+          // walk the subtile's masks; a step takes the next atom of the word,
+          // or the first one of the next word (nothing if that one is empty)
+          const char *pa = reinterpret_cast<const char *>(sA);
+          const char *pb = reinterpret_cast<const char *>(sB);
+          const uint32_t *pm = &sMask[0][16 * band + cpair];
+          uint32_t m = *pm;
+          int left = nwords - 1;
+          int base = 16;
+          while (m != 0u || left > 0) {
+            if (m == 0u) {
+              pm += kSub;
+              m = *pm;
+              base += 33 * 16;
+              --left;
+            }
+            const int i = 31 - __clz(m);              // -1: the empty slot
+            m &= ~(1u << (i & 31));
+            const int o = base + 16 * i;
+            Proj3Rec q;
+            q.a = *reinterpret_cast<const float4 *>(pa + o);
+            q.b = *reinterpret_cast<const float4 *>(pb + o);
+            proj3_visit(q, row, col, acc, cmp);
+          }
+          __syncthreads();  // the pass's staged records are done with
+        }
       }
-    }
-  }
-  if constexpr (NW == 1) __syncwarp();
-  else __syncthreads();
-
-  // epilogue: write the tile, fused fit fields and loss partial; a split
-  // item's cells combine the warps' sums in warp order
-  // The data values of a batch of a thread's cells are loaded before any of
-  // them is written (the output fields may alias nothing, but the compiler
-  // cannot know that), so a batch costs one memory latency, not one per cell.
-  constexpr int kPer = ROWS / NW;                 // cells per thread
-  constexpr int kBatch = kPer < (NW == 1 ? 8 : 4) ? kPer : (NW == 1 ? 8 : 4);
-  static_assert(kPer % kBatch == 0, "batch");
-  const bool want_data = out.epilogue == kEpiL2 || out.epilogue == kEpiKL;
-  const int e0 = NW == 1 ? lane : (int)threadIdx.x;
-  const int col = c0 + lane;
-  float lsum = 0.f, lcmp = 0.f;
-  for (int eb = 0; eb < kPer; eb += kBatch) {
-    float dv[kBatch];
 #pragma unroll
-    for (int i = 0; i < kBatch; ++i) {
-      const int row = r0 + ((e0 + (eb + i) * NW * 32) >> 5);
-      dv[i] = (want_data && row < D0 && col < D1)
-                  ? __ldg(out.data + ((size_t)a * D0 + row) * D1 + col)
-                  : 0.f;
-    }
-#pragma unroll
-    for (int i = 0; i < kBatch; ++i) {
-    const int lr = (e0 + (eb + i) * NW * 32) >> 5;
-    const int row = r0 + lr;
-    if (row >= D0 || col >= D1) continue;
-    const int ci = lr * S + lane;
-    float v;
-    if constexpr (NW == 1) {
-      v = acc[ci] + cmp[ci];
-    } else {
-      float s0 = 0.f, c0s = 0.f;
-#pragma unroll
-      for (int w = 0; w < NW; ++w) {
-        const float *aw = smem + (size_t)w * L::kFloats;
-        const float x = aw[ci] + aw[L::kAcc + ci];
-        const float tt = s0 + x;
-        c0s += (fabsf(s0) >= fabsf(x)) ? ((s0 - tt) + x) : ((x - tt) + s0);
-        s0 = tt;
+      for (int k = 0; k < 2; ++k) {
+        float s0, s1, e0, e1;
+        f2_get(acc[k], s0, s1);
+        f2_get(cmp[k], e0, e1);
+        sV[row_in][col_in + k] = __fadd_rn(s0, e0);
+        sV[row_in + 1][col_in + k] = __fadd_rn(s1, e1);
       }
-      v = s0 + c0s;
-    }
-    const size_t gi = ((size_t)a * D0 + row) * D1 + col;
-    if (out.R) out.R[gi] = v;
-    float l = 0.f;
-    if (out.epilogue == kEpiL2) {
-      const float res = v - dv[i];
-      if (out.alpha) out.alpha[gi] = res;
-      l = 0.5f * res * res;
-    } else if (out.epilogue == kEpiKL) {
-      const float fo = dv[i];
-      const float gg = v + out.bg;
-      const float ig = 1.f / gg;
-      if (out.alpha) out.alpha[gi] = 1.f - fo * ig;
-      if (out.beta) out.beta[gi] = fo * ig * ig;
-      l = kl_term(fo, gg);
-    }
-    const float tt = lsum + l;
-    lcmp += (fabsf(lsum) >= fabsf(l)) ? ((lsum - tt) + l) : ((l - tt) + lsum);
-    lsum = tt;
-    }
-  }
-  if (out.loss_part) {
-    double d = warp_sum_d((double)lsum + (double)lcmp);
-    if constexpr (NW == 1) {
-      if (lane == 0) out.loss_part[item] = d;
-    } else {
-      if (lane == 0) s_loss[warp] = d;
       __syncthreads();
-      if (threadIdx.x == 0) {
-        double tl = 0.0;
 #pragma unroll
-        for (int w = 0; w < NW; ++w) tl += s_loss[w];
-        out.loss_part[item] = tl;
+      for (int r = 0; r < 4; ++r) v[r] = sV[4 * warp + r][lane];
+    }
+
+    // write the cells, fused fit fields and loss partial (rounding spelled
+    // out, so that both forms of the kernel give the same bits)
+    float lsum = 0.f, lcmp = 0.f;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      if (r >= nr) break;
+      const size_t gi = gi0 + (size_t)(r * D1);
+      if (out.R) out.R[gi] = v[r];
+      float l = 0.f;
+      if (out.epilogue == kEpiL2) {
+        const float res = v[r] - dv[r];
+        if (out.alpha) out.alpha[gi] = res;
+        l = __fmul_rn(__fmul_rn(0.5f, res), res);
+      } else if (out.epilogue == kEpiKL) {
+        const float fo = dv[r];
+        const float gg = v[r] + out.bg;
+        const float ig = 1.f / gg;
+        if (out.alpha) out.alpha[gi] = fmaf(-fo, ig, 1.f);
+        if (out.beta) out.beta[gi] = __fmul_rn(__fmul_rn(fo, ig), ig);
+        l = kl_term(fo, gg);
+      }
+      const float tt = lsum + l;
+      lcmp += (fabsf(lsum) >= fabsf(l)) ? ((lsum - tt) + l) : ((l - tt) + lsum);
+      lsum = tt;
+    }
+    if (out.loss_part) {
+      // the block's sum as an FP32 pair (exact two-sums, about 46 bits), FP64
+      // from the item's partial on: 12 conversions and adds an item would
+      // hold the SM's FP64 pipe, at 16 cycles each, longer than its memory
+      s_loss[tid] = make_float2(lsum, lcmp);
+      __syncthreads();
+      if (warp == 0) {
+#pragma unroll
+        for (int w = 1; w < NW; ++w)
+          pair_add(lsum, lcmp, s_loss[32 * w + lane].x, s_loss[32 * w + lane].y);
+        pair_warp_sum(lsum, lcmp);
+        if (lane == 0) out.loss_part[item] = (double)lsum + (double)lcmp;
       }
     }
-  }
-  if constexpr (NW > 1) __syncthreads();  // cell sums and s_item are reused
+    if (tid == 0) s_item = ahead;
+    __syncthreads();  // sV, s_count and s_loss are reused
+    take = s_item;
   }
 
   if (loss_out && out.loss_part) {
-    // the last warp (block) to finish sums the items' partials in item order
-    const int units = NW == 1 ? (int)gridDim.x * kProjWarps : (int)gridDim.x;
-    if (NW > 1 && warp != 0) return;
-    int last = 0;
-    if (lane == 0) {
+    // the last block to finish sums the items' partials in item order
+    if (tid == 0) {
       __threadfence();
-      last = atomicAdd(next_item + 1, 1) == units - 1;
+      s_item = atomicAdd(next_item + 1, 1) == (int)gridDim.x - 1;
     }
-    if (__shfl_sync(0xffffffffu, last, 0)) {
+    __syncthreads();
+    if (s_item) {
       __threadfence();
-      sum_partials_warp(out.loss_part, n_items, loss_out, lane);
+      sum_partials_block<NW>(out.loss_part, n_items, loss_out);
+    }
+  }
+}
+
+// Binning of a 3D forward: a block takes 256 atoms (8 bitmap words) of one
+// angle, writes their records (rec, nullable) and gathers the tiles' words in
+// shared memory, a range of kBinTiles tiles at a time, so that every word of
+// the bitmap is written once: no clear, and no global atomics (whose latency
+// and contention bounded the launch before).
+// counters (nullable): zeroed, for the projection that follows.
+constexpr int kBinTiles = 512;
+__global__ void __launch_bounds__(256)
+    gr_bin3d_kernel(Atoms at, Geom g, TileCfg tc, uint32_t *bitmap, int W, Proj3Rec *rec,
+                    int *counters, uint32_t *flag, int *list, int *n_list) {
+  __shared__ uint32_t sw[kBinTiles][8];
+  const int tid = threadIdx.x, a = blockIdx.y, w0 = 8 * blockIdx.x;
+  const int j = 32 * w0 + tid;
+  if (counters && blockIdx.x == 0 && a == 0 && tid < 4) counters[tid] = 0;
+  int r_lo = 1, r_hi = 0, c_lo = 1, c_hi = 0;
+  if (j < at.n) {
+    Frame<2> f;
+    load_frame<2>(g.frames, a, f);
+    Pair<2> p;
+    pair_setup<2>(at, j, f, g, p);
+    if (p.lo[0] <= p.hi[0] && p.lo[1] <= p.hi[1]) {
+      r_lo = p.lo[0] / tc.t0;
+      r_hi = p.hi[0] / tc.t0;
+      c_lo = p.lo[1] / tc.t1;
+      c_hi = p.hi[1] / tc.t1;
+      if (rec) rec[(size_t)a * at.n + j] = proj3_record(p);
+    }
+  }
+  const uint32_t bit = 1u << (j & 31);
+  const int nw = min(8, W - w0);
+  for (int t0 = 0; t0 < tc.ntiles; t0 += kBinTiles) {
+    const int nt = min(kBinTiles, tc.ntiles - t0);
+    if (t0 > 0) __syncthreads();
+    for (int e = tid; e < nt * 8; e += 256) (&sw[0][0])[e] = 0u;
+    __syncthreads();
+    for (int r = r_lo; r <= r_hi; ++r)
+      for (int c = c_lo; c <= c_hi; ++c) {
+        const int t = r * tc.nt1 + c - t0;
+        if (t >= 0 && t < nt) atomicOr(&sw[t][tid >> 5], bit);
+      }
+    __syncthreads();
+    const size_t base = (size_t)a * tc.ntiles + t0;
+    for (int e0 = 0; e0 < nt * 8; e0 += 256) {
+      const int e = e0 + tid;
+      const uint32_t wd = e < nt * 8 ? (&sw[0][0])[e] : 0u;
+      const int t = e >> 3, w = e & 7;
+      if (e < nt * 8 && w < nw) bitmap[(base + t) * W + w0 + w] = wd;
+      if (flag) {
+        // an item is listed by the first block that meets it
+        const uint32_t any = __ballot_sync(0xffffffffu, wd != 0u) >> (tid & 24);
+        if (w == 0 && (any & 0xffu) && atomicExch(flag + base + t, 1u) == 0u)
+          list[atomicAdd(n_list, 1)] = (int)(base + t);
+      }
     }
   }
 }
@@ -841,20 +993,12 @@ static int proj_rows(int form) { return form == 2 ? kTileDim0 : 16; }
 // above it the 1024-thread gr_loss_finalize_kernel does it.
 constexpr size_t kFusedLossItems = 8192;
 
-// 3D problems of fewer detector cells (all angles) than
-// Tuning::proj_split_cells (key 4; 0: never) split every tile's atoms over a
-// block's warps.
-
-template <int ROWS, int S, int NW>
+template <int NW>
 static void launch_project3d(size_t items, const Atoms &at, const Geom &g, const TileCfg &tc,
-                             const uint32_t *bitmap, int W, const ProjOut &o, int *next_item,
-                             double *loss_out, const int *item_list, cudaStream_t stream) {
-  constexpr size_t smem = kProjWarps * Proj3Smem<ROWS, S>::kFloats * sizeof(float);
-  // with the few static bytes, below the 48 KB that needs no opt-in, so no
-  // function attribute is set (safe under stream capture)
-  static_assert(smem + 64 <= 48 * 1024, "smem");
-  // persistent grid: the resident blocks of every SM, at most the blocks
-  // that have an item to take
+                             const uint32_t *bitmap, int W, const Proj3Rec *rec, const ProjOut &o,
+                             int *next_item, double *loss_out, const int *item_list,
+                             cudaStream_t stream) {
+  // persistent grid: the resident blocks of every SM, at most one per item
   static int resident[64] = {0};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -862,18 +1006,17 @@ static void launch_project3d(size_t items, const Atoms &at, const Geom &g, const
   if (resident[dev] == 0) {
     int sms = 0, per_sm = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gr_project3d_kernel<ROWS, S, NW, false>,
-                                                  kProjWarps * 32, smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gr_project3d_kernel<NW, true>,
+                                                  NW * 32, 0);
     resident[dev] = (sms > 0 ? sms : 1) * (per_sm > 0 ? per_sm : 1);
   }
-  const size_t want = NW == 1 ? (items + kProjWarps - 1) / kProjWarps : items;
-  const int grid = (int)(want < (size_t)resident[dev] ? want : (size_t)resident[dev]);
+  const int grid = (int)(items < (size_t)resident[dev] ? items : (size_t)resident[dev]);
   if (item_list)
-    gr_project3d_kernel<ROWS, S, NW, true><<<grid, kProjWarps * 32, smem, stream>>>(
-        at, g, tc, bitmap, W, o, next_item, loss_out, item_list, next_item + 2);
+    gr_project3d_kernel<NW, true><<<grid, NW * 32, 0, stream>>>(
+        at, g, tc, bitmap, W, rec, o, next_item, loss_out, item_list, next_item + 2);
   else
-    gr_project3d_kernel<ROWS, S, NW, false><<<grid, kProjWarps * 32, smem, stream>>>(
-        at, g, tc, bitmap, W, o, next_item, loss_out, nullptr, nullptr);
+    gr_project3d_kernel<NW, false><<<grid, NW * 32, 0, stream>>>(
+        at, g, tc, bitmap, W, rec, o, next_item, loss_out, nullptr, nullptr);
 }
 
 // rows: the tile's rows (3D) or cells (2D)
@@ -891,6 +1034,9 @@ TileCfg make_tiles(int K, int D0, int D1, int rows) {
     tc.nt1 = (D1 + tc.t1 - 1) / tc.t1;
   }
   tc.ntiles = tc.nt0 * tc.nt1;
+  auto inv = [](int d) { return d > 1 ? (uint32_t)((1ull << 32) / (unsigned)d) : 0xffffffffu; };
+  tc.inv_ntiles = inv(tc.ntiles);
+  tc.inv_nt1 = inv(tc.nt1);
   return tc;
 }
 
@@ -900,8 +1046,9 @@ size_t project_skip_items(const Geom &g, int psf, const Tuning &t) {
   return (size_t)g.n_angles * tc.ntiles;
 }
 
-size_t project_workspace_bytes(int K, int n_atoms, int n_angles, int D0, int D1,
-                               const Tuning &t) {
+// Workspace of a projection without the 3D pair records: the least a launch
+// takes.
+size_t project_min_bytes(int K, int n_atoms, int n_angles, int D0, int D1, const Tuning &t) {
   // sized for the smaller of the point-sampled and pixel-integrated tilings
   const int rows = K == 1 ? kTile1D
                           : (proj_rows(t.proj_form) < kTileDim0 ? proj_rows(t.proj_form)
@@ -912,8 +1059,8 @@ size_t project_workspace_bytes(int K, int n_atoms, int n_angles, int D0, int D1,
   // item counter of the persistent 3D kernel, finished-block counter, count
   // of listed items
   size_t bytes = align_up(4 * sizeof(int));
-  // 3D: the bitmap is followed by a flag per item (cleared with it) and the
-  // list of items some atom meets (a forward that skips the others)
+  // 3D: a flag per item (cleared with the counters) before the bitmap, and
+  // the list of items some atom meets (a forward that skips the others)
   bytes += align_up(items * W * sizeof(uint32_t) + (K == 2 ? items * sizeof(uint32_t) : 0));
   bytes += align_up(items * sizeof(double));
   bytes += align_up(kLossMaxBlocks * sizeof(double));  // block sums of the loss finalize
@@ -921,6 +1068,22 @@ size_t project_workspace_bytes(int K, int n_atoms, int n_angles, int D0, int D1,
     bytes += align_up((size_t)n_angles * (size_t)n_atoms * 2 * sizeof(float4));
   else
     bytes += align_up(items * sizeof(int));
+  return bytes;
+}
+
+// 3D pair records: setting a pair up again in each of the 1.3 to 2.5 tiles it
+// touches took 40 % of the projection (8.4 of 20.9 ms on 8192 atoms x 20000
+// orientations), so the binning writes each pair's 32-byte record once.  Problems whose records pass
+// kRecBytes run in ranges of angles, each binned and projected in turn.
+constexpr size_t kRecBytes = (size_t)512 << 20;
+
+size_t project_workspace_bytes(int K, int n_atoms, int n_angles, int D0, int D1,
+                               const Tuning &t) {
+  size_t bytes = project_min_bytes(K, n_atoms, n_angles, D0, D1, t);
+  if (K == 2) {
+    const size_t row = (size_t)n_atoms * sizeof(Proj3Rec), all = row * (size_t)n_angles;
+    bytes += align_up(all <= kRecBytes ? all : (row <= kRecBytes ? kRecBytes / row * row : row));
+  }
   return bytes;
 }
 
@@ -939,7 +1102,7 @@ int launch_project(const Atoms &at, const Geom &g, const ProjOut &o_in,
                                  : (!o_in.psf ? proj_rows(form) : kTileDim0));
   const int W = (at.n + 31) / 32;
   const size_t items = (size_t)g.n_angles * tc.ntiles;
-  const size_t need = project_workspace_bytes(K, at.n, g.n_angles, D0, D1, t);
+  const size_t need = project_min_bytes(K, at.n, g.n_angles, D0, D1, t);
   // items no atom meets: point-sampled 3D only, fields only
   const int emode = o_in.empty_mode;
   if (emode != kEmptyNone &&
@@ -947,23 +1110,28 @@ int launch_project(const Atoms &at, const Geom &g, const ProjOut &o_in,
     return kErrArg;
   const bool record = emode == kEmptyRecord;
   if (ws_bytes < need || (ws == nullptr && need > 0)) return kErrWorkspace;
+  // (the binning grid's y extent; a forward without atoms has no such limit)
+  if (W > 0 && !record && g.n_angles > 65535) return kErrLaunch;
+  const bool skip = emode == kEmptySkip;
+  const bool point3 = K == 2 && !o_in.psf;
   char *wp = static_cast<char *>(ws);
   int *next_item = reinterpret_cast<int *>(wp);
   wp += align_up(4 * sizeof(int));
-  uint32_t *bitmap = reinterpret_cast<uint32_t *>(wp);
-  uint32_t *flag = bitmap + items * W;  // 3D: one per item
+  uint32_t *flag = reinterpret_cast<uint32_t *>(wp);  // 3D: one per item
+  uint32_t *bitmap = flag + (K == 2 ? items : 0);
   wp += align_up(items * W * sizeof(uint32_t) + (K == 2 ? items * sizeof(uint32_t) : 0));
   double *loss_part = reinterpret_cast<double *>(wp);
   wp += align_up(items * sizeof(double)) + align_up(kLossMaxBlocks * sizeof(double));
   float4 *pairs = K == 1 ? reinterpret_cast<float4 *>(wp) : nullptr;
   int *item_list = K == 2 ? reinterpret_cast<int *>(wp) : nullptr;
-  const bool skip = emode == kEmptySkip;
-  // one clear covers the counters and the bitmap (and the item flags)
-  if (cudaMemsetAsync(ws, 0,
-                      align_up(4 * sizeof(int)) + items * W * sizeof(uint32_t) +
-                          (skip ? items * sizeof(uint32_t) : 0),
-                      stream) != cudaSuccess)
-    return kErrLaunch;
+  // the 3D binning writes every word of the bitmap and clears the counters;
+  // the others want the counters and the bitmap cleared, a skipping forward
+  // the counters and the item flags
+  size_t clear = align_up(4 * sizeof(int));
+  if (!point3) clear += (K == 2 ? items * sizeof(uint32_t) : 0) + items * W * sizeof(uint32_t);
+  else if (skip) clear += items * sizeof(uint32_t);
+  else if (W > 0 && !record) clear = 0;
+  if (clear && cudaMemsetAsync(ws, 0, clear, stream) != cudaSuccess) return kErrLaunch;
   ProjOut o = o_in;
   o.loss_part = loss_out ? loss_part : nullptr;
   // skipping: the items no atom meets take their recorded loss partials
@@ -974,26 +1142,21 @@ int launch_project(const Atoms &at, const Geom &g, const ProjOut &o_in,
     return kErrLaunch;
   if (record) {
     // every item as if no atom met it: its loss partial goes to empty_loss,
-    // under the schedule (split, tiling) of a forward of these atoms, so it
-    // equals bitwise what that forward computes for an empty item
+    // under the tiling of a forward of these atoms, so it equals bitwise what
+    // that forward computes for an empty item
     o.alpha = o.beta = nullptr;
     o.loss_part = o_in.empty_loss;
     loss_out = nullptr;
   }
   // half-width of the (square) cells of the pixel-integrated operator
   const float psf_s = 0.5f / g.ax[0].inv_step;
-  if (W > 0 && !record) {
+  if (W > 0 && !point3) {
     dim3 bgrid((at.n + 127) / 128, g.n_angles);
     if (o.psf) {
       if (K == 1) gr_psf_bin_kernel<1><<<bgrid, 128, 0, stream>>>(at, g, tc, bitmap, W, psf_s);
       else gr_psf_bin_kernel<2><<<bgrid, 128, 0, stream>>>(at, g, tc, bitmap, W, psf_s);
-    } else if (K == 1) {
-      gr_bin_kernel<1><<<bgrid, 128, 0, stream>>>(at, g, tc, bitmap, W, pairs, nullptr, nullptr,
-                                                  nullptr);
     } else {
-      gr_bin_kernel<2><<<bgrid, 128, 0, stream>>>(at, g, tc, bitmap, W, nullptr,
-                                                  skip ? flag : nullptr, item_list,
-                                                  next_item + 2);
+      gr_bin_kernel<<<bgrid, 128, 0, stream>>>(at, g, tc, bitmap, W, pairs);
     }
     note_launches(1);
   }
@@ -1003,58 +1166,87 @@ int launch_project(const Atoms &at, const Geom &g, const ProjOut &o_in,
   // needs no opt-in, so no function attribute is set (safe under capture)
   static_assert(kProjWarps * kProjWarpFloats * sizeof(float) <= 48 * 1024, "smem");
   bool fused_loss = false;
-  timer_mark(1, 0, stream);
-  if (o.psf) {
-    if (K == 1)
-      gr_psf_project_kernel<1><<<blocks, kProjWarps * 32, smem, stream>>>(at, g, tc, bitmap, W, psf_s, o);
-    else
-      gr_psf_project_kernel<2><<<blocks, kProjWarps * 32, smem, stream>>>(at, g, tc, bitmap, W, psf_s, o);
-  } else if (K == 1) {
-    // one block per (angle, tile) item; for up to kFusedLossItems tiles the
-    // last block also sums the loss partials (no separate finalize launch)
-    fused_loss = loss_out != nullptr && items <= kFusedLossItems;
-    double *lo = fused_loss ? loss_out : nullptr;
-    if (wide4 && W >= 8)
-      gr_project1d_kernel<true, 8, 4, 2><<<(unsigned)items, 8 * 32, 0, stream>>>(
-          at, g, tc, bitmap, W, o, lo, next_item + 1, pairs);
-    else if (wide4)
-      gr_project1d_kernel<true, kProjWarps, 4><<<(unsigned)items, kProjWarps * 32, 0, stream>>>(
-          at, g, tc, bitmap, W, o, lo, next_item + 1, pairs);
-    else if (wide2d && W >= 8)
-      gr_project1d_kernel<true, 8, 2, 2><<<(unsigned)items, 8 * 32, 0, stream>>>(
-          at, g, tc, bitmap, W, o, lo, next_item + 1, pairs);
-    else if (wide2d)
-      gr_project1d_kernel<true, kProjWarps, 2><<<(unsigned)items, kProjWarps * 32, 0, stream>>>(
-          at, g, tc, bitmap, W, o, lo, next_item + 1, pairs);
-    else if (W >= 32)  // 1024 atoms up: four list entries per thread
-      gr_project1d_kernel<true, 8, 1, 4><<<(unsigned)items, 8 * 32, 0, stream>>>(
-          at, g, tc, bitmap, W, o, lo, next_item + 1, pairs);
-    else if (W >= 8)  // 8 warps share a tile's atoms from 8 bitmap words (256 atoms) up
-      gr_project1d_kernel<true, 8, 1, 2><<<(unsigned)items, 8 * 32, 0, stream>>>(
-          at, g, tc, bitmap, W, o, lo, next_item + 1, pairs);
-    else
-      gr_project1d_kernel<true, kProjWarps><<<(unsigned)items, kProjWarps * 32, 0, stream>>>(
-          at, g, tc, bitmap, W, o, lo, next_item + 1, pairs);
-  } else {
-    // the split is chosen from the problem's size alone (not from the
-    // tiling), so both tilings keep giving the same cell sums
-    const bool split = t.proj_split_cells > 0 && W >= kProjWarps &&
-                       (size_t)g.n_angles * D0 * D1 < (size_t)t.proj_split_cells;
-    fused_loss = loss_out != nullptr && items <= kFusedLossItems;
-    double *lo = fused_loss ? loss_out : nullptr;
-    const int Wk = record ? 0 : W;  // recording: no atom in any item
-    // skipping: only the listed items (none without atoms)
-    const int *il = skip ? item_list : nullptr;
-    if (form == 2) {
-      if (split) launch_project3d<32, 34, kProjWarps>(items, at, g, tc, bitmap, Wk, o, next_item, lo, il, stream);
-      else launch_project3d<32, 34, 1>(items, at, g, tc, bitmap, Wk, o, next_item, lo, il, stream);
-    } else {
-      if (split) launch_project3d<16, 37, kProjWarps>(items, at, g, tc, bitmap, Wk, o, next_item, lo, il, stream);
-      else launch_project3d<16, 37, 1>(items, at, g, tc, bitmap, Wk, o, next_item, lo, il, stream);
+  if (point3) {
+    // records: as many angles at a time as the workspace holds; a skipping
+    // forward (one list of items) takes all angles at once or none
+    const size_t row = (size_t)at.n * sizeof(Proj3Rec);
+    const size_t base = align_up(need);
+    Proj3Rec *rec = reinterpret_cast<Proj3Rec *>(static_cast<char *>(ws) + base);
+    size_t range = row > 0 && ws_bytes > base ? (ws_bytes - base) / row : 0;
+    if (range > (size_t)g.n_angles) range = g.n_angles;
+    if (range == 0 || record || (skip && range < (size_t)g.n_angles)) {
+      rec = nullptr;
+      range = g.n_angles;
     }
+    const size_t cells = (size_t)D0 * D1;
+    fused_loss = loss_out != nullptr && items <= kFusedLossItems && range == (size_t)g.n_angles;
+    double *lo = fused_loss ? loss_out : nullptr;
+    for (size_t a0 = 0; a0 < (size_t)g.n_angles; a0 += range) {
+      Geom gr = g;
+      gr.n_angles = (int)(g.n_angles - a0 < range ? g.n_angles - a0 : range);
+      gr.frames = g.frames + a0 * kFrameStride3D;
+      const size_t i0 = a0 * tc.ntiles, ni = (size_t)gr.n_angles * tc.ntiles;
+      ProjOut oc = o;
+      if (oc.R) oc.R += a0 * cells;
+      if (oc.data) oc.data += a0 * cells;
+      if (oc.alpha) oc.alpha += a0 * cells;
+      if (oc.beta) oc.beta += a0 * cells;
+      if (oc.loss_part) oc.loss_part += i0;
+      uint32_t *bm = bitmap + i0 * W;
+      if (W > 0 && !record) {
+        gr_bin3d_kernel<<<dim3((W + 7) / 8, gr.n_angles), 256, 0, stream>>>(
+            at, gr, tc, bm, W, rec, skip ? nullptr : next_item,
+            skip ? flag : nullptr, item_list, next_item + 2);
+        note_launches(1);
+      }
+      const int Wk = record ? 0 : W;  // recording: no atom in any item
+      // skipping: only the listed items (none without atoms)
+      const int *il = skip ? item_list : nullptr;
+      timer_mark(1, 0, stream);
+      if (form == 2)
+        launch_project3d<8>(ni, at, gr, tc, bm, Wk, rec, oc, next_item, lo, il, stream);
+      else
+        launch_project3d<4>(ni, at, gr, tc, bm, Wk, rec, oc, next_item, lo, il, stream);
+      timer_mark(1, 1, stream);
+      note_launches(1);
+    }
+  } else {
+    timer_mark(1, 0, stream);
+    if (o.psf) {
+      if (K == 1)
+        gr_psf_project_kernel<1><<<blocks, kProjWarps * 32, smem, stream>>>(at, g, tc, bitmap, W, psf_s, o);
+      else
+        gr_psf_project_kernel<2><<<blocks, kProjWarps * 32, smem, stream>>>(at, g, tc, bitmap, W, psf_s, o);
+    } else {
+      // one block per (angle, tile) item; for up to kFusedLossItems tiles the
+      // last block also sums the loss partials (no separate finalize launch)
+      fused_loss = loss_out != nullptr && items <= kFusedLossItems;
+      double *lo = fused_loss ? loss_out : nullptr;
+      if (wide4 && W >= 8)
+        gr_project1d_kernel<true, 8, 4, 2><<<(unsigned)items, 8 * 32, 0, stream>>>(
+            at, g, tc, bitmap, W, o, lo, next_item + 1, pairs);
+      else if (wide4)
+        gr_project1d_kernel<true, kProjWarps, 4><<<(unsigned)items, kProjWarps * 32, 0, stream>>>(
+            at, g, tc, bitmap, W, o, lo, next_item + 1, pairs);
+      else if (wide2d && W >= 8)
+        gr_project1d_kernel<true, 8, 2, 2><<<(unsigned)items, 8 * 32, 0, stream>>>(
+            at, g, tc, bitmap, W, o, lo, next_item + 1, pairs);
+      else if (wide2d)
+        gr_project1d_kernel<true, kProjWarps, 2><<<(unsigned)items, kProjWarps * 32, 0, stream>>>(
+            at, g, tc, bitmap, W, o, lo, next_item + 1, pairs);
+      else if (W >= 32)  // 1024 atoms up: four list entries per thread
+        gr_project1d_kernel<true, 8, 1, 4><<<(unsigned)items, 8 * 32, 0, stream>>>(
+            at, g, tc, bitmap, W, o, lo, next_item + 1, pairs);
+      else if (W >= 8)  // 8 warps share a tile's atoms from 8 bitmap words (256 atoms) up
+        gr_project1d_kernel<true, 8, 1, 2><<<(unsigned)items, 8 * 32, 0, stream>>>(
+            at, g, tc, bitmap, W, o, lo, next_item + 1, pairs);
+      else
+        gr_project1d_kernel<true, kProjWarps><<<(unsigned)items, kProjWarps * 32, 0, stream>>>(
+            at, g, tc, bitmap, W, o, lo, next_item + 1, pairs);
+    }
+    timer_mark(1, 1, stream);
+    note_launches(1);
   }
-  timer_mark(1, 1, stream);
-  note_launches(1);
   if (loss_out && !fused_loss) {
     // about 8 partials per thread, at most kLossMaxBlocks blocks; the
     // finished-block counter (next_item + 1) is unused when the loss is not
@@ -1080,7 +1272,7 @@ __global__ void __launch_bounds__(128)
   const BatchProb &B = probs[p];
   const int lb = blockIdx.x - off[p];
   const int bxn = (B.cur.n + 127) / 128;
-  bin_body<1>(use_trial ? B.trial : B.cur, B.g, B.tc, B.bitmap, B.W, B.pairs, lb % bxn,
+  bin_body(use_trial ? B.trial : B.cur, B.g, B.tc, B.bitmap, B.W, B.pairs, lb % bxn,
               lb / bxn);
 }
 
@@ -1112,16 +1304,10 @@ int launch_batch_project(const BatchLaunch &b, int use_trial, cudaStream_t strea
 }
 
 int preload_project() {
-  return preload_fn(gr_bin_kernel<1>) + preload_fn(gr_bin_kernel<2>) +
+  return preload_fn(gr_bin_kernel) + preload_fn(gr_bin3d_kernel) +
          preload_fn(gr_psf_bin_kernel<1>) + preload_fn(gr_psf_bin_kernel<2>) +
-         preload_fn(gr_project3d_kernel<16, 37, 1, false>) +
-         preload_fn(gr_project3d_kernel<16, 37, kProjWarps, false>) +
-         preload_fn(gr_project3d_kernel<32, 34, 1, false>) +
-         preload_fn(gr_project3d_kernel<32, 34, kProjWarps, false>) +
-         preload_fn(gr_project3d_kernel<16, 37, 1, true>) +
-         preload_fn(gr_project3d_kernel<16, 37, kProjWarps, true>) +
-         preload_fn(gr_project3d_kernel<32, 34, 1, true>) +
-         preload_fn(gr_project3d_kernel<32, 34, kProjWarps, true>) +
+         preload_fn(gr_project3d_kernel<4, false>) + preload_fn(gr_project3d_kernel<4, true>) +
+         preload_fn(gr_project3d_kernel<8, false>) + preload_fn(gr_project3d_kernel<8, true>) +
          preload_fn(gr_project1d_kernel<true, 8, 1, 4>) +
          preload_fn(gr_project1d_kernel<true, 8, 1, 2>) +
          preload_fn(gr_project1d_kernel<true, kProjWarps>) +

@@ -768,7 +768,8 @@ class GaussFitServer:
         qn = 1 + P + P * (P + 1) // 2
         deriv = 4096 * 32 * qn * 4 + qn * n * 8 + n * qn * 4 * 256
         per_atom = n * (P * P + 4 * P + 16) * 8
-        return int(1.3 * (sino + bitmap + deriv + per_atom)) + (8 << 20)
+        records = min(n * len(req.orientations) * 32, max(512 << 20, n * 32)) if dim == 3 else 0
+        return int(1.3 * (sino + bitmap + deriv + per_atom + records)) + (8 << 20)
 
     def submit(self, req):
         """Queue a request.  Malformed requests are refused here

@@ -39,8 +39,8 @@ def set_projection_tiling(form):
 
 
 def set_projection_split(cells):
-    """3D problems with fewer detector cells (all angles) than ``cells``
-    split each tile's atoms over a block's warps (0: never)."""
+    """Accepted for callers of earlier versions; without effect (a block
+    takes every 3D tile)."""
     _lib.check(_lib.load().gr_set_tuning(4, int(cells)), "gr_set_tuning")
 
 
@@ -146,9 +146,8 @@ _req_plans = {}
 # alone on an idle GPU but lost among concurrent fits, 1.655 s against 1.624 s
 # untuned on the 512-request stream)
 DERIV_CANDIDATES = ((131072, 1, 1, 0), (131072, 1, 1, 1))
-PROJ_CANDIDATES = ((1, 4 << 20), (1, 0), (2, 4 << 20), (2, 0))
-# 2D: the block split does not apply; tiles of 32, 64 or 128 cells
-PROJ_CANDIDATES_2D = ((1, 0), (2, 0), (3, 0))
+PROJ_CANDIDATES = (1, 2)          # 3D: tiles of 16 or 32 rows
+PROJ_CANDIDATES_2D = (1, 2, 3)    # 2D: tiles of 32, 64 or 128 cells
 
 
 def request_key(req, order=2):
@@ -166,8 +165,8 @@ def plans_for_request(req, order=2):
 
 def tune_request_classes(requests, device, reps=3, order=2):
     """Tune each shape class among ``requests`` once, on its first request:
-    the projection's tiling and block split and the derivative split, each
-    timed under a plan of its own.  Returns the number of classes tuned."""
+    the projection's tiling and the derivative split, each timed under a plan
+    of its own.  Returns the number of classes tuned."""
     from .geometry import DeviceGeometry
     done = 0
     for req in requests:
@@ -180,13 +179,13 @@ def tune_request_classes(requests, device, reps=3, order=2):
         data = req.device_data(geom, device, stream)
         pp = engine.Plan(_lib.GR_OP_PROJECT, atoms, geom)
         best_p = None
-        for form, split in (PROJ_CANDIDATES_2D if len(req.detector) == 1 else PROJ_CANDIDATES):
-            pp.set(3, form).set(4, split)
+        for form in (PROJ_CANDIDATES_2D if len(req.detector) == 1 else PROJ_CANDIDATES):
+            pp.set(3, form)
             ms = _time(lambda: engine.fit_forward(atoms, geom, data, req.fit, req.background,
                                                   plan=pp), reps)
-            if best_p is None or ms < best_p[2] * (1.0 - MARGIN):
-                best_p = (form, split, ms)
-        pp.set(3, best_p[0]).set(4, best_p[1])
+            if best_p is None or ms < best_p[1] * (1.0 - MARGIN):
+                best_p = (form, ms)
+        pp.set(3, best_p[0])
         fw = engine.fit_forward(atoms, geom, data, req.fit, req.background, plan=pp)
         autotune_derivs(atoms, geom, fw["alpha"], fw["beta"],
                         1.0 if req.fit == "l2" else 0.0, order=order, reps=reps,

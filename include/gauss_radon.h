@@ -101,7 +101,9 @@ const char *gr_status_string(int status);
 
 /*
  * Device workspace (bytes) an operation needs; the caller allocates it
- * (256-byte aligned) and may reuse it across calls on the same stream.
+ * (256-byte aligned) and may reuse it across calls on the same stream.  For a
+ * 3D projection it includes up to 512 MB of 32-byte (atom, angle) records; a
+ * launch given less works through the angles in ranges, or without records.
  */
 size_t gr_workspace_bytes(int op, const gr_atoms *atoms, const gr_geometry *geom);
 
@@ -279,14 +281,13 @@ unsigned long long gr_launch_count(void);
  * power of two up to 32, the other lanes taking further angles of the same
  * atoms (default 0: automatic, one atom per warp for Hessians and for series
  * of 1024 or more angles, else four).  GR_TUNE_PROJ_TILING: tiles of the
- * point-sampled 3D projection, 1 = 16 x 32 cells (default, more resident
- * warps), 2 = 32 x 32 (fewer atoms cut by tile edges), 3 = as 1; of the 2D
+ * point-sampled 3D projection, 1 = 16 x 32 cells (default), 2 = 32 x 32
+ * (fewer atoms cut by tile edges), 3 = as 1; of the 2D
  * projection, 32, 64 and 128 cells (one, two or four per lane: wide
  * footprints are listed and staged for fewer tiles).
- * GR_TUNE_PROJ_SPLIT_CELLS: 3D problems with fewer detector cells over all
- * angles than this (default 4194304; 0 = never) split each tile's atoms over
- * the four warps of a block, which shortens the slowest tile when there are
- * too few tiles to fill the GPU.  GR_TUNE_DERIV_SPLIT_LANES: problems with
+ * GR_TUNE_PROJ_SPLIT_CELLS: accepted and without effect (it once chose
+ * whether a block or a warp takes a 3D tile; a block always does).
+ * GR_TUNE_DERIV_SPLIT_LANES: problems with
  * fewer (atom, angle) pairs than this split each pair's cells over 2, 4 or 8
  * lanes of the point-sampled derivative kernel (the largest split with
  * pairs x lanes <= value; default 65536; 0 = never).  GR_TUNE_DERIV_ONE_MB:
@@ -304,8 +305,8 @@ unsigned long long gr_launch_count(void);
  * bitwise the same).  Set them before
  * gr_workspace_bytes and keep them fixed while launches that used the old
  * values are in flight.  Results do not depend on them beyond FP rounding of
- * the derivative chunk and lane sums and of a split tile's combined cell sums (the
- * tiling leaves projections bitwise equal).  gr_set_tuning returns
+ * the derivative chunk and lane sums (the tiling leaves 3D projections bitwise
+ * equal).  gr_set_tuning returns
  * GR_ERR_ARG for an unknown key or out-of-range value; gr_get_tuning returns
  * the current value (-1 for an unknown key).
  */
@@ -583,8 +584,9 @@ int gr_kernel_timer_read(int which, double *total_ms, int *launches);
  * allocator, or a loop that must avoid cudaMalloc/cudaFree because they
  * synchronise the device.  The scratch is a 4 MiB array compiled into the
  * library; every GPU that loads the library keeps it until the process exits.
- * Problems whose projection workspace (gr_workspace_bytes(GR_OP_PROJECT, ..))
- * exceeds 4 MiB are rejected with GR_ERR_TOO_LARGE.  The call allocates
+ * Problems whose projection workspace (gr_workspace_bytes(GR_OP_PROJECT, ..)
+ * without 3D pair records: bitmaps, loss partials and item lists) exceeds
+ * 4 MiB are rejected with GR_ERR_TOO_LARGE.  The call allocates
  * nothing.  The first call on a device looks up the scratch address on that
  * device (make it before any stream capture there); the address is kept per
  * CUDA context, so a call under another context of the device (one the
