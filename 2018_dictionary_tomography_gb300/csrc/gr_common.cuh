@@ -231,7 +231,6 @@ struct Pair {
   // quantities kept for the derivative assembly
   float Kc[K + 1][K + 1];  // Kc[c][a] = (r B_c)_a, c = 0..K-1 detector axes, K = T
   float Q[K + 1][K + 1];   // Q[c][d] = Kc[c] . Kc[d]
-  float U[K][K + 1];       // projected detector axes, G = U^T U
 };
 
 template <int K>
@@ -268,7 +267,7 @@ __device__ __forceinline__ bool pair_setup(const Atoms &at, int j,
   p.n = rsqrtf(qtt);
   // G = U^T U with U_i = K_i - t (t . K_i), t = K_T / |K_T| (the projected
   // detector axes); this Gram form stays positive semi-definite in FP32.
-  float (&U)[K][D] = p.U;
+  float U[K][D];
 #pragma unroll
   for (int i = 0; i < K; ++i) {
     const float c = p.Q[i][K] * iqtt;

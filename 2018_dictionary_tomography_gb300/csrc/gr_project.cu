@@ -111,26 +111,15 @@ __device__ __forceinline__ float kl_term(float f, float g) {
 // block, latency).  64 registers, 8 blocks an SM; 48 registers: 5 to 10 % slower.
 struct Proj3Rec {
   float4 a;   // (-qh0, -ql0, -qh1, -ql1): the centre's negative, as a float pair
-  float4 b;   // (u11, u01, +-u00, log2 amplitude)
+  float4 b;   // (G00, 2 G01, G11, log2 amplitude)
 };
 
-// The pair's record: with d = p - q*, 30/ln2 times the form is
-// (u11 d1 + u01 d0)^2 + (u00 d0)^2; u00 comes from the part of U0 orthogonal
-// to U1 (no cancellation of G00 with G01^2 / G11) and carries the sign of I.
+// The pair's record.  The sign of I rides on G00's (>= 0 where a record is
+// written).
 __device__ __forceinline__ Proj3Rec proj3_record(const Pair<2> &p) {
-  const float C = -kNegThirtyLog2e;
-  const float u11 = sqrtf(C * p.G[2]);
-  const float u01 = __fdiv_rn(C * p.G[1], u11);
-  const float t = __fdiv_rn(p.G[1], p.G[2]);
-  float vv = 0.f;
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    const float v = fmaf(-t, p.U[1][i], p.U[0][i]);
-    vv = fmaf(v, v, vv);
-  }
   Proj3Rec o;
   o.a = make_float4(-p.qh[0], -p.ql[0], -p.qh[1], -p.ql[1]);
-  o.b = make_float4(u11, u01, copysignf(sqrtf(C * vv), p.sgn), p.l2amp);
+  o.b = make_float4(copysignf(p.G[0], p.sgn), 2.f * p.G[1], p.G[2], p.l2amp);
   return o;
 }
 
@@ -154,17 +143,16 @@ __device__ __forceinline__ float rcp_approx(float v) {
 template <int NB>
 __device__ __forceinline__ void proj3_subtiles(const Proj3Rec &q, const Geom &g, int r0, int c0,
                                                uint32_t (&cols)[NB / 2]) {
-  const float rC = 6.5788183f;                            // sqrt(30 / ln 2)
-  const float h0 = rcp_approx(g.ax[0].inv_step);
+  const float g00 = fabsf(q.b.x), g01 = 0.5f * q.b.y, g11 = q.b.z;
+  const float det = fmaf(g00, g11, -g01 * g01);
+  const float h0 = rcp_approx(g.ax[0].inv_step), i1 = g.ax[1].inv_step, i11 = rcp_approx(g11);
   const float q0 = (-q.a.x - g.ax[0].first) * g.ax[0].inv_step - (float)r0;   // centre in
-  const float q1 = (-q.a.z - g.ax[1].first) * g.ax[1].inv_step - (float)c0;   // tile cells
-  const float k = g.ax[1].inv_step * rcp_approx(q.b.x);
-  const float S = -q.b.y * h0 * k;                        // columns q1 + S d +- hw(d),
-  const float a0 = fabsf(q.b.z) * h0;                     // hw(d) = k sqrt(C - a0^2 d^2)
-  const float ka = k * a0;
-  const float dmax = rC * rcp_approx(a0);                 // rows within dmax
-  const float len = sqrt_approx(fmaf(S, S, ka * ka));
-  const float dx = S * rcp_approx(len) * dmax;            // row of the rightmost point
+  const float q1 = (-q.a.z - g.ax[1].first) * i1 - (float)c0;                 // tile cells
+  const float S = -g01 * i11 * h0 * i1;                   // columns q1 + S d +- hw(d),
+  const float k = i1 * sqrt_approx(i11);                  // hw(d) = k sqrt(1 - a2 d^2)
+  const float a2 = det * i11 * h0 * h0;
+  const float dmax = rcp_approx(sqrt_approx(a2));         // rows within dmax
+  const float dx = S * dmax * rcp_approx(sqrt_approx(fmaf(S, S, k * k * a2)));  // of the rightmost
   const bool plain = fabsf(dx) < 1e8f && dmax < 1e8f;     // else every subtile
   const float top = q0 - dmax - 0.02f, bot = q0 + dmax + 0.02f;
 #pragma unroll
@@ -174,8 +162,8 @@ __device__ __forceinline__ void proj3_subtiles(const Proj3Rec &q, const Geom &g,
     const float ra = fmaxf(top, (float)(4 * b)), rb = fminf(bot, (float)(4 * b + 3));
     const float da = ra - q0, db = rb - q0;
     const float dr = fminf(fmaxf(dx, da), db), dl = fminf(fmaxf(-dx, da), db);
-    const float hr = k * sqrt_approx(fmaxf(fmaf(-a0 * dr, a0 * dr, rC * rC), 0.f));
-    const float hl = k * sqrt_approx(fmaxf(fmaf(-a0 * dl, a0 * dl, rC * rC), 0.f));
+    const float hr = k * sqrt_approx(fmaxf(fmaf(-a2 * dr, dr, 1.f), 0.f));
+    const float hl = k * sqrt_approx(fmaxf(fmaf(-a2 * dl, dl, 1.f), 0.f));
     const float xr = fminf(fmaf(S, dr, q1) + fmaf(hr, 1.0001f, 0.02f), 31.f);
     const float xl = fmaxf(fmaf(S, dl, q1) - fmaf(hl, 1.0001f, 0.02f), 0.f);
     const int xa = (int)ceilf(xl), xb = (int)floorf(xr);
@@ -205,24 +193,27 @@ __device__ __forceinline__ uint32_t warp_transpose32(uint32_t x, int lane) {
 // cells of each column.
 __device__ __forceinline__ void proj3_visit(const Proj3Rec &q, const float (&row)[2],
                                             const float (&col)[2], F2 (&s)[2], F2 (&c)[2]) {
-  float bb[2], cc[2];
+  const float g00 = fabsf(q.b.x);
+  float t[2], u[2];
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
     const float d0 = (row[r] + q.a.x) + q.a.y;
-    const float b = q.b.z * d0;
-    bb[r] = b * b;
-    cc[r] = q.b.y * d0;
+    t[r] = g00 * d0 * d0;
+    u[r] = q.b.y * d0;
   }
-  const float sg = copysignf(1.f, q.b.z);
-  const F2 S = f2(sg, sg), bbp = f2(bb[0], bb[1]);
+  const float sg = copysignf(1.f, q.b.x);
+  const F2 S = f2(sg, sg), tp = f2(t[0], t[1]);
+  const F2 K2 = f2(kNegThirtyLog2e, kNegThirtyLog2e), amp = f2(q.b.w, q.b.w);
 #pragma unroll
   for (int k = 0; k < 2; ++k) {
     const float d1 = (col[k] + q.a.z) + q.a.w;
-    const F2 a = f2(fmaf(q.b.x, d1, cc[0]), fmaf(q.b.x, d1, cc[1]));
-    float m0, m1;
-    f2_get(f2_fma(a, a, bbp), m0, m1);               // 30/ln2 times the form
-    const float e0 = ex2_approx(q.b.w - m0), e1 = ex2_approx(q.b.w - m1);
-    const F2 v = f2(m0 <= -kNegThirtyLog2e ? e0 : 0.f, m1 <= -kNegThirtyLog2e ? e1 : 0.f);
+    const F2 m = f2_fma(f2(d1, d1), f2(fmaf(q.b.z, d1, u[0]), fmaf(q.b.z, d1, u[1])), tp);
+    float m0, m1, e0, e1;
+    f2_get(m, m0, m1);
+    f2_get(f2_fma(m, K2, amp), e0, e1);
+    e0 = ex2_approx(e0);
+    e1 = ex2_approx(e1);
+    const F2 v = f2(m0 <= 1.f ? e0 : 0.f, m1 <= 1.f ? e1 : 0.f);
     // two-sum of s and S v, both cells at once
     const F2 tt = f2_fma(v, S, s[k]);
     const F2 nb = f2_sub(s[k], tt);
