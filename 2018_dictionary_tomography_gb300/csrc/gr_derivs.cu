@@ -18,13 +18,15 @@
 // Per cell the kernel evaluates one exp2 and a handful of FMAs; moments are
 // accumulated per detector row and folded with powers of d0 at row end.
 //
-// Work layout: lane = atom, a warp holds 32 atoms (or fewer atoms with the
-// angles of each atom split over several lanes), and loops over a chunk of
-// angles.  Gradients are accumulated per lane with compensated FP32 sums,
-// Hessians in FP32; lanes sharing an atom are combined by a fixed-order
-// butterfly; chunk partials are summed in FP64 in chunk order by
-// gr_deriv_finalize_kernel, which also applies the isotropic chain rule.
-// No float atomics anywhere: results are bitwise reproducible.
+// Work layout: a warp's lanes are the (atom, angle) pairs of one atom (or a
+// few) and a chunk of angles.  A lane sets its pair up and does its chain-rule
+// assembly; in between, for Hessians, groups of lanes walk the pairs' cells
+// together (gr_hess_kernel); for gradients (gr_grad_kernel) a lane walks alone.  Gradients are
+// accumulated per lane with compensated FP32 sums, Hessians in FP32; lanes
+// sharing an atom are combined by a fixed-order butterfly; chunk partials are
+// summed in FP64 in chunk order by gr_deriv_finalize_kernel, which also applies
+// the isotropic chain rule.  No float atomics anywhere: results are bitwise
+// reproducible.
 #include "gr_assembly.cuh"
 
 namespace gr {
@@ -35,23 +37,10 @@ inline int next_pow2(int v) {
   return p;
 }
 
-constexpr int kRowChunk = 8;
-// cells per chunk of a 3D box row, and resident blocks per SM asked of the
-// gradient (order 1) kernels; compile-time, for sweeps
-// (4 and 8 measured best on 8192 atoms x 5000 orientations: 4.59 ms against
-// 5.73 ms for 8-cell chunks at 5 blocks; 64 registers, with a few spills,
-// give the gradient kernels 32 resident warps per SM instead of 20)
-#ifndef GR_ROW_CHUNK_3D
-#define GR_ROW_CHUNK_3D 4
-#endif
-#ifndef GR_GRAD_MIN_BLOCKS
-#define GR_GRAD_MIN_BLOCKS 8
-#endif
-// resident blocks per SM asked of the 2D Hessian kernel with one angle per lane
-#ifndef GR_HESS2D_MIN_BLOCKS
-#define GR_HESS2D_MIN_BLOCKS 3
-#endif
-constexpr int kRowChunk3 = GR_ROW_CHUNK_3D;
+// resident warps per SM asked of the Hessian kernels
+__host__ __device__ constexpr int hess_min_warps(int K, bool one) {
+  return one ? (K == 1 ? 24 : 16) : 4;
+}
 
 // Work split of the derivative kernels (Tuning, gr_set_tuning / gr_plan_set):
 // about deriv_target_warps warps in total, each angle chunk holding at least
@@ -61,13 +50,10 @@ constexpr int kRowChunk3 = GR_ROW_CHUNK_3D;
 // support boxes are of similar size, so fewer lanes idle.  Automatic: one
 // atom per warp for Hessians and for long angle series, else four (so each
 // lane still has a few angles to amortise the warp's closing reduction).
-// deriv_split_lanes: problems with few (atom, angle) pairs split each pair's
-// cells over rs lanes (rows of a 3D box, chunks of kRowChunk cells of a 2D
-// one), rs the largest power of two up to 8 with pairs * rs <=
-// deriv_split_lanes; the lanes' moment sums are combined before one of them
-// does the chain-rule assembly.  A pair's cell walk is otherwise one lane's
-// serial loop, which sets the kernel time when there are too few pairs to
-// fill the GPU and their boxes are large.  0: never split.
+// deriv_split_lanes: problems with few (atom, angle) pairs give a warp 32 / rs
+// of them, rs the largest power of two up to 8 with pairs * rs <=
+// deriv_split_lanes, so that the pairs spread over more warps (a 3D gradient's
+// pair then has its rows split over rs lanes).  0: never split.
 // deriv_one_mb: take as many angle chunks as give every lane at most one
 // angle (the ONE kernel variant: fewer registers, no spills) whenever the
 // chunk partials then fit in this many MB; 0: keep the target-warps split.
@@ -106,203 +92,285 @@ DerivCfg deriv_cfg(int K, int n_atoms, int n_angles, int order, const Tuning &t,
   return c;
 }
 
-// Cell moments of one pair.
-template <int K, int DEG, bool GN>
-struct PairMoments {
-  float Ma[n_mom<K, DEG>()];
-  float Mb[GN ? n_mom<K, DEG>() : 1];
-  float X0, Y0;  // sum E*C and sum E^2 (per-atom L2 value)
+// ---- the cell walk -----------------------------------------------------------
+// A warp's pairs are set up one per lane and staged in shared memory; groups of
+// GL lanes then walk one pair each, lane l the cells of columns l, l + GL, ..
+// of its support (3D) or the cells l, l + GL, .. (2D), so that a load of the
+// weight field covers GL neighbouring cells, and the lanes' moment sums are
+// combined and handed back to the pair's lane, which does the chain-rule
+// assembly.  The groups walk rows (3D) in step, so that their loads share
+// sectors, and two cells at a time in packed FP32 pairs.
+// What bounds it: issue (58 % of the slots) and the 128 registers of the 3D
+// assembly (16 warps an SM; 168 registers and 12 warps: 363 against 301 us, 96
+// registers 310 us with four rows a lane).  A lane walking its pair alone, as
+// before, waited on 32 lines of the field per load with 12 warps an SM and 124
+// registers of moment sums; a group's lane keeps 20.  2936 atoms x 148 x 493^2
+// (3D, 120 cells a pair): 401 -> 277 us; 146 x 61 x 301 x 275: 18.7 -> 15.5 us;
+// 2150 x 153 x 467 (2D): 85.5 -> 58.6 us; 512 x 180 x 256 (9 cells a pair): 10.6
+// -> 11.8 us.  Cells a lane loads together: 2D, 2 lanes: 4, 6, 8: 60.0, 58.6,
+// 56.8 us there, 11.5, 11.8, 11.8 us on the small one; 3D, 4 lanes: 2, 4, 6, 8:
+// 397, 301, 277, 290 us.  4 lanes in 2D: 61.9 and 11.2 us.
+// cells of a lane loaded together (even)
+template <int K>
+__host__ __device__ constexpr int walk_cells_of() { return 6; }
+// lanes of a group (8 where a warp has four pairs)
+template <int K>
+__host__ __device__ constexpr int walk_lanes_of() { return K == 1 ? 2 : 4; }
+template <int K>
+__host__ __device__ constexpr int n_sums() {   // moments (alpha, beta), sum E C, sum E^2
+  return (2 * n_mom<K, 4>() + 2 + 7) / 8 * 8;   // (up to 8 lanes share them out)
+}
+
+// What the weight fields are: a kernel of its own for each (a test in the cell
+// loop cost the Hessian kernels 10 to 20 %), one for all where a lane takes
+// several angles.
+enum FieldKind : int { kFieldPlain = 0, kFieldBeta = 1, kFieldL2Atom = 2, kFieldAny = 3 };
+
+struct WalkPair {
+  float4 q;      // -qh0, -ql0, -qh1, -ql1
+  float4 v;      // G00, 2 G01, G11, log2 n
+  float4 r;      // centre row, its drift per unit of d1, half-height per unit, I (walk_stage)
+  float4 e;      // det G, d1 of the support's lowest row
+  int4 box;      // first and last cell along each axis
 };
 
-// CH: cells per chunk of the row walk (loaded together before any is used)
-template <int K, int DEG, bool GN, int CH>
-__device__ __forceinline__ void pair_moments(const Pair<K> &p, const Geom &g,
-                                             const DerivIn &in, int a, float I,
-                                             PairMoments<K, DEG, GN> &mo, int phase = 0,
-                                             int rs = 1) {
+template <int K>
+struct WalkSmem {
+  static constexpr int NV = n_sums<K>();
+  WalkPair pair[32];
+  float sum[32][NV + 1];
+};
+
+template <int K>
+__device__ __forceinline__ void walk_stage(const Pair<K> &p, const Geom &g, float I, bool live,
+                                           WalkPair &w) {
+  w.q = make_float4(-p.qh[0], -p.ql[0], K == 2 ? -p.qh[K - 1] : 0.f, K == 2 ? -p.ql[K - 1] : 0.f);
+  w.v = make_float4(p.G[0], 2.f * p.G[1], p.G[2], lg2_approx(p.n));
+  const DetAxis &x0 = g.ax[0];
+  // 3D: at column offset d1 the support's rows are r.x - r.y d1 -+ r.z
+  // sqrt(G00 - e.x d1^2); its lowest row is at d1 = e.y, its highest at -e.y
+  const float iG0 = 1.f / p.G[0], det = p.G[0] * p.G[2] - p.G[1] * p.G[1];
+  w.r = make_float4((p.qh[0] - x0.first) * x0.inv_step, p.G[1] * iG0 * x0.inv_step,
+                    iG0 * x0.inv_step, I);
+  w.e = make_float4(det, K == 2 && p.G[1] != 0.f ? p.G[1] * rsqrtf(p.G[2] * det) : 0.f,
+                    0.f, 0.f);
+  w.box = live ? make_int4(p.lo[0], p.hi[0], K == 2 ? p.lo[K - 1] : 0, K == 2 ? p.hi[K - 1] : 0)
+               : make_int4(1, 0, 1, 0);
+}
+
+__device__ __forceinline__ F2 f2_keep(const F2 &v, bool k0, bool k1) {
+  float x, y;
+  f2_get(v, x, y);
+  return f2(k0 ? x : 0.f, k1 ? y : 0.f);
+}
+
+// Two cells' terms: m their form, d0 their offsets along axis 0, c and b their
+// field values.
+// Sa, Sb: sums over alpha E and beta E^2 times powers of d0.
+__device__ __forceinline__ void walk_cells(F2 m, F2 d0, bool in0, bool in1, F2 c, F2 b, float l2n,
+                                           float I, const bool l2atom, const bool bfield,
+                                           F2 (&Sa)[5], F2 (&Sb)[5], F2 &X0, F2 &Y0) {
+  constexpr int DEG = 4;
+  float m0, m1;
+  f2_get(m, m0, m1);
+  in0 = in0 && m0 <= 1.f;
+  in1 = in1 && m1 <= 1.f;
+  float e0, e1;
+  f2_get(f2_fma(m, f2(kNegThirtyLog2e, kNegThirtyLog2e), f2(l2n, l2n)), e0, e1);
+  const F2 E = f2(ex2_approx(e0), ex2_approx(e1));
+  F2 al = c;
+  if (l2atom) al = f2_fma(f2(I, I), E, f2_mul(c, f2(-1.f, -1.f)));
+  // the products, not their factors, are cut off: a field value beyond the
+  // cut-off counts for nothing, also one that is not finite
+  const F2 w = f2_keep(f2_mul(al, E), in0, in1);
+  F2 pw[DEG + 1];
+  pw[1] = d0;
+#pragma unroll
+  for (int q = 2; q <= DEG; ++q) pw[q] = f2_mul(pw[q - 1], d0);
+  Sa[0] = f2_add(Sa[0], w);
+#pragma unroll
+  for (int q = 1; q <= DEG; ++q) Sa[q] = f2_fma(w, pw[q], Sa[q]);
+  // a constant beta scales the moments once per pair instead
+  F2 wb = f2_mul(E, E);
+  if (bfield) wb = f2_mul(wb, b);
+  wb = f2_keep(wb, in0, in1);
+  Sb[0] = f2_add(Sb[0], wb);
+#pragma unroll
+  for (int q = 1; q <= DEG; ++q) Sb[q] = f2_fma(wb, pw[q], Sb[q]);
+  if (l2atom) {
+    X0 = f2_add(X0, f2_keep(f2_mul(E, c), in0, in1));
+    Y0 = f2_add(Y0, f2_keep(f2_mul(E, E), in0, in1));
+  }
+}
+
+__device__ __forceinline__ float f2_sum(const F2 &a) {
+  float x, y;
+  f2_get(a, x, y);
+  return x + y;
+}
+
+// The sums of one pair over this lane's share of its cells (v: moments of
+// alpha, of beta, then sum E C and sum E^2).  R: cells of a column loaded
+// together before any is used (even); they may lie past the support's end
+// (their terms are cut off), not past the detector's.
+template <int K, int GL, int R, int FK>
+__device__ __forceinline__ void walk_pair(const WalkPair &w, const Geom &g, const DerivIn &in, int a,
+                                          int sub, float (&v)[n_sums<K>()]) {
+  constexpr int DEG = 4;
   constexpr int NM = n_mom<K, DEG>();
+  constexpr int NV = n_sums<K>();
 #pragma unroll
-  for (int i = 0; i < NM; ++i) {
-    mo.Ma[i] = 0.f;
-    if (GN) mo.Mb[i] = 0.f;
-  }
-  mo.X0 = 0.f;
-  mo.Y0 = 0.f;
-  if (p.lo[0] > p.hi[0]) return;
-  if constexpr (K == 2)
-    if (p.lo[1] > p.hi[1]) return;
-  const float l2n = lg2_approx(p.n);
-  const int D0 = g.ax[0].n;
-  const int D1 = K == 2 ? g.ax[1].n : 1;
-  const float *__restrict__ field = in.alpha;
-  const float *__restrict__ bfield = in.beta;
-  const size_t abase = (size_t)a * D0 * D1;
-  // per row, m <= 1 holds for d1 within hw(d0) = sqrt(G2 - d0^2 det)/G2 of
-  // -G1 d0/G2: the row loop visits that range (widened like the support box)
-  // instead of the whole box; the m <= 1 test still decides every cell
-  float det = 0.f, iG2 = 0.f;
-  if constexpr (K == 2) {
-    det = p.G[0] * p.G[2] - p.G[1] * p.G[1];
-    iG2 = 1.f / p.G[2];
-  }
+  for (int q = 0; q < NV; ++q) v[q] = 0.f;
+  const float4 q = w.q, u = w.v;
+  const int4 box = w.box;
+  const float I = w.r.w;
+  const bool l2atom = FK == kFieldAny ? in.mode == kModeL2Atom : FK == kFieldL2Atom;
+  const bool bfield = FK == kFieldAny ? in.beta != nullptr : FK == kFieldBeta;
+  const int D0 = g.ax[0].n, D1 = K == 2 ? g.ax[1].n : 1;
+  const float *__restrict__ x0 = g.ax[0].coords;
+  const F2 nqh = f2(q.x, q.x), nql = f2(q.y, q.y), g00 = f2(u.x, u.x);
+  F2 X0 = f2(0.f, 0.f), Y0 = X0;
   if constexpr (K == 1) {
-    // the detector row is walked in chunks of kRowChunk cells whose field
-    // values and coordinates are loaded together first (one cell per load
-    // round trip would leave the lane waiting on every cell)
-    const int c_hi = p.hi[0];
-    for (int kb = p.lo[0] + phase * CH; kb <= c_hi; kb += rs * CH) {
-      float cv[CH], pv[CH], bv[GN ? CH : 1];
+    const float *__restrict__ fa = in.alpha + (size_t)a * D0;
+    const float *__restrict__ fb = bfield ? in.beta + (size_t)a * D0 : fa;
+    F2 Sa[DEG + 1], Sb[DEG + 1];
 #pragma unroll
-      for (int i = 0; i < CH; ++i) {
-        const int k0 = min(kb + i, c_hi);
-        cv[i] = __ldg(field + abase + k0);
-        pv[i] = __ldg(g.ax[0].coords + k0);
-        if (GN) bv[i] = bfield ? __ldg(bfield + abase + k0) : 0.f;
-      }
+    for (int e = 0; e <= DEG; ++e) {
+      Sa[e] = f2(0.f, 0.f);
+      Sb[e] = f2(0.f, 0.f);
+    }
+    auto cells = [&](float xa, float xb, float ca, float cb, float ba, float bb, bool two) {
+      const F2 d0 = f2_add(f2_add(f2(xa, xb), nqh), nql);
+      walk_cells(f2_mul(f2_mul(g00, d0), d0), d0, true, two, f2(ca, cb), f2(ba, bb), u.w, I, l2atom,
+                          bfield, Sa, Sb, X0, Y0);
+    };
+    for (int k = box.x + sub; k <= box.y; k += GL * R) {
+      if (k + (R - 1) * GL < D0) {
+        float c[R], b[R], x[R];
 #pragma unroll
-      for (int i = 0; i < CH; ++i) {
-        if (kb + i > c_hi) break;
-        const float d0 = (pv[i] - p.qh[0]) - p.ql[0];
-        const float m = p.G[0] * d0 * d0;
-        if (m <= 1.f) {
-          const float E = ex2_approx(fmaf(m, kNegThirtyLog2e, l2n));
-          const float c = cv[i];
-          const float al = (in.mode == kModeL2Atom) ? fmaf(I, E, -c) : c;
-          // powers of d0, shared by both moment sets: one FMA per moment
-          float pw[NM];
-          pw[0] = 1.f;
+        for (int i = 0; i < R; ++i) {
+          c[i] = __ldg(fa + k + i * GL);
+          x[i] = __ldg(x0 + k + i * GL);
+          b[i] = bfield ? __ldg(fb + k + i * GL) : 0.f;
+        }
 #pragma unroll
-          for (int q = 1; q < NM; ++q) pw[q] = pw[q - 1] * d0;
-          const float w = al * E;
-          mo.Ma[0] += w;
-#pragma unroll
-          for (int q = 1; q < NM; ++q) mo.Ma[q] = fmaf(w, pw[q], mo.Ma[q]);
-          if (GN) {
-            // a constant beta scales the moments once per pair instead
-            const float wb = bfield ? bv[i] * (E * E) : E * E;
-            mo.Mb[0] += wb;
-#pragma unroll
-            for (int q = 1; q < NM; ++q) mo.Mb[q] = fmaf(wb, pw[q], mo.Mb[q]);
-          }
-          if (in.mode == kModeL2Atom) {
-            mo.X0 = fmaf(E, c, mo.X0);
-            mo.Y0 = fmaf(E, E, mo.Y0);
-          }
+        for (int i = 0; i < R; i += 2)
+          cells(x[i], x[i + 1], c[i], c[i + 1], b[i], b[i + 1], true);
+      } else {
+        for (int kk = k; kk <= box.y; kk += GL) {
+          const float c = __ldg(fa + kk), x = __ldg(x0 + kk), b = bfield ? __ldg(fb + kk) : 0.f;
+          cells(x, x, c, c, b, b, false);
         }
       }
+    }
+#pragma unroll
+    for (int e = 0; e <= DEG; ++e) {
+      v[e] = f2_sum(Sa[e]);
+      v[NM + e] = f2_sum(Sb[e]);
     }
   } else {
-    for (int k0 = p.lo[0] + phase; k0 <= p.hi[0]; k0 += rs) {
-      const float d0 = (__ldg(g.ax[0].coords + k0) - p.qh[0]) - p.ql[0];
-      {
-        const float t0 = p.G[0] * d0 * d0;
-        const float u = 2.f * p.G[1] * d0;
-        float Sa[DEG + 1], Sb[GN ? DEG + 1 : 1];
+    const size_t abase = (size_t)a * D0 * D1;
+    for (int c0 = box.z; c0 <= box.w; c0 += GL) {
+      // rows that the ellipse reaches in columns c0 .. c0 + GL - 1, the same
+      // for every lane of the group so that its loads share sectors: the
+      // row range at the column nearest to the ellipse's lowest (highest)
+      // point, widened like the support box
+      const int cz = min(c0 + GL - 1, box.w), col = min(c0 + sub, box.w);
+      const float da = (__ldg(g.ax[1].coords + c0) + q.z) + q.w;
+      const float db = (__ldg(g.ax[1].coords + cz) + q.z) + q.w;
+      const float d1 = (__ldg(g.ax[1].coords + col) + q.z) + q.w;
+      const float low = w.e.y;
+      const float dh = fminf(fmaxf(-low, da), db), dl = fminf(fmaxf(low, da), db);
+      const float hh = sqrtf(fmaxf(fmaf(-w.e.x * dh, dh, u.x), 0.f));
+      const float hl = sqrtf(fmaxf(fmaf(-w.e.x * dl, dl, u.x), 0.f));
+      const float rhi = fmaf(hh * w.r.z, 1.0001f, fmaf(-w.r.y, dh, w.r.x)) + 0.02f;
+      const float rlo = fmaf(hl * w.r.z, -1.0001f, fmaf(-w.r.y, dl, w.r.x)) - 0.02f;
+      const int r_lo = (int)fminf(fmaxf(ceilf(rlo), (float)box.x), (float)box.y + 1.f);
+      const int r_hi = (int)fmaxf(fminf(floorf(rhi), (float)box.y), (float)box.x - 1.f);
+      const bool mine = c0 + sub <= box.w;
+      // (a lane past the last column repeats it, cut off)
+      const float c1 = u.y * d1, b1 = mine ? u.z * d1 * d1 : 4.f + u.z * d1 * d1 + c1 * c1 / u.x;
+      const F2 c1p = f2(c1, c1), b1p = f2(b1, b1);
+      const float *__restrict__ fa = in.alpha + abase + (size_t)r_lo * D1 + col;
+      const float *__restrict__ fb = bfield ? in.beta + abase + (size_t)r_lo * D1 + col : fa;
+      F2 Sa[DEG + 1], Sb[DEG + 1];
 #pragma unroll
-        for (int q = 0; q <= DEG; ++q) {
-          Sa[q] = 0.f;
-          if (GN) Sb[q] = 0.f;
-        }
-        const size_t rbase = abase + (size_t)k0 * D1;
-        const float rem = fmaf(-d0 * d0, det, p.G[2]);
-        const float rc = (p.qh[1] - p.G[1] * d0 * iG2 - g.ax[1].first) * g.ax[1].inv_step;
-        const float rh = sqrtf(fmaxf(rem, 0.f)) * iG2 * g.ax[1].inv_step * 1.0001f + 1e-3f;
-        const float rlo = ceilf(rc - rh), rhi = floorf(rc + rh);
-        const int c_lo = (int)fminf(fmaxf(rlo, (float)p.lo[1]), (float)p.hi[1] + 1.f);
-        const int c_hi = (int)fmaxf(fminf(rhi, (float)p.hi[1]), (float)p.lo[1] - 1.f);
-        // the row is walked in chunks of CH cells whose field values and
-        // coordinates are loaded together first, so the loads overlap
-        // instead of each cell waiting for its own
-        for (int kb = c_lo; kb <= c_hi; kb += CH) {
-          float cv[CH], pv[CH], bv[GN ? CH : 1];
+      for (int e = 0; e <= DEG; ++e) {
+        Sa[e] = f2(0.f, 0.f);
+        Sb[e] = f2(0.f, 0.f);
+      }
+      auto cells = [&](float xa, float xb, float ca, float cb, float ba, float bb, bool two) {
+        const F2 d0 = f2_add(f2_add(f2(xa, xb), nqh), nql);
+        walk_cells(f2_fma(d0, f2_fma(g00, d0, c1p), b1p), d0, true, two, f2(ca, cb), f2(ba, bb), u.w, I, l2atom,
+                            bfield, Sa, Sb, X0, Y0);
+      };
+      for (int k = r_lo; k <= r_hi; k += R) {
+        if (k + R <= D0) {
+          float c[R], b[R], x[R];
 #pragma unroll
-          for (int i = 0; i < CH; ++i) {
-            const int k1 = min(kb + i, c_hi);
-            cv[i] = __ldg(field + rbase + k1);
-            pv[i] = __ldg(g.ax[1].coords + k1);
-            if (GN) bv[i] = bfield ? __ldg(bfield + rbase + k1) : 0.f;
+          for (int i = 0; i < R; ++i) {
+            c[i] = __ldg(fa);
+            b[i] = bfield ? __ldg(fb) : 0.f;
+            x[i] = __ldg(x0 + k + i);
+            fa += D1;
+            if (bfield) fb += D1;
           }
 #pragma unroll
-          for (int i = 0; i < CH; ++i) {
-            if (kb + i > c_hi) break;
-            const float d1 = (pv[i] - p.qh[1]) - p.ql[1];
-            const float m = fmaf(d1, fmaf(p.G[2], d1, u), t0);
-            if (m <= 1.f) {
-              const float E = ex2_approx(fmaf(m, kNegThirtyLog2e, l2n));
-              const float c = cv[i];
-              const float al = (in.mode == kModeL2Atom) ? fmaf(I, E, -c) : c;
-              float pw[DEG + 1];
-              pw[0] = 1.f;
-#pragma unroll
-              for (int q = 1; q <= DEG; ++q) pw[q] = pw[q - 1] * d1;
-              const float w = al * E;
-              Sa[0] += w;
-#pragma unroll
-              for (int q = 1; q <= DEG; ++q) Sa[q] = fmaf(w, pw[q], Sa[q]);
-              if (GN) {
-                const float wb = bfield ? bv[i] * (E * E) : E * E;
-                Sb[0] += wb;
-#pragma unroll
-                for (int q = 1; q <= DEG; ++q) Sb[q] = fmaf(wb, pw[q], Sb[q]);
-              }
-              if (in.mode == kModeL2Atom) {
-                mo.X0 = fmaf(E, c, mo.X0);
-                mo.Y0 = fmaf(E, E, mo.Y0);
-              }
-            }
+          for (int i = 0; i < R; i += 2)
+            cells(x[i], x[i + 1], c[i], c[i + 1], b[i], b[i + 1], true);
+        } else {
+          for (int kk = k; kk <= r_hi; ++kk) {
+            const float c = __ldg(fa), x = __ldg(x0 + kk), b = bfield ? __ldg(fb) : 0.f;
+            cells(x, x, c, c, b, b, false);
+            fa += D1;
+            if (bfield) fb += D1;
           }
         }
-        float pw = 1.f;
+      }
+      // fold the column's sums with powers of d1
+      float pw = 1.f;
 #pragma unroll
-        for (int i = 0; i <= DEG; ++i) {
+      for (int e = 0; e <= DEG; ++e) {
 #pragma unroll
-          for (int j = 0; j <= DEG - i; ++j) {
-            mo.Ma[mi(i, j)] = fmaf(pw, Sa[j], mo.Ma[mi(i, j)]);
-            if (GN) mo.Mb[mi(i, j)] = fmaf(pw, Sb[j], mo.Mb[mi(i, j)]);
-          }
-          pw *= d0;
+        for (int i = 0; i <= DEG - e; ++i) {
+          v[mi(i, e)] = fmaf(pw, f2_sum(Sa[i]), v[mi(i, e)]);
+          v[NM + mi(i, e)] = fmaf(pw, f2_sum(Sb[i]), v[NM + mi(i, e)]);
         }
+        pw *= d1;
       }
     }
   }
-  if (GN && !bfield) {
-#pragma unroll
-    for (int q = 0; q < NM; ++q) mo.Mb[q] *= in.beta_const;
-  }
+  v[NV - 2] = f2_sum(X0);
+  v[NV - 1] = f2_sum(Y0);
 }
 
 // ONE: the work split gives every lane at most one angle of its atom (every
 // Hessian split of up to ~32 angles per chunk, which covers the tilt series
 // and the served fits): the angle loop runs at most once, so the per-lane
-// accumulators need not live across the whole pair computation, which cuts
-// the Hessian kernel from 255 to 168 registers (3 resident blocks per SM
-// instead of 2).
-// WIDE (3D Hessians): rows walked in chunks of 8 cells instead of 4, which
-// keeps more field loads in flight when supports are many cells wide and
-// costs idle lanes on narrow ones (Tuning key 8; measured: 2936 atoms x 148
-// angles of 493^2 cells 460 -> 408 us, config 2's atoms 192 -> 200 us; 16
-// instead of 8 cells slowed every 2D Hessian measured, by up to 25 %)
+// accumulators need not live across the whole pair computation.
 // The body of one block whose first warp is warp0 of the launch's warps
 // (warp w takes the w-th (atom group, angle chunk); a multi-problem launch
 // maps its blocks to (problem, first warp)).  What a warp computes depends on
 // its warp index only, so the block size changes no result.
-template <int K, int ORDER, bool ONE, bool WIDE = false>
-__device__ __forceinline__ void deriv_body(const Atoms &at, const Geom &g, const DerivIn &in,
-                                           const DerivCfg &cfg, float *part, int warp0) {
-  constexpr int D = K + 1;
+// smem: the warp's own staging area.
+template <int K, bool ONE, int GL, int R, int FK>
+__device__ __forceinline__ void hess_body(const Atoms &at, const Geom &g, const DerivIn &in,
+                                           const DerivCfg &cfg, float *part, int warp0,
+                                           WalkSmem<K> &sm) {
   constexpr int PR = n_rparam<K>();
   constexpr int P = n_par<K>();
   constexpr int NPSI = n_psi<K>();
-  constexpr int NG = K * (K + 1) / 2;
-  constexpr int DEG = ORDER == 1 ? 2 : 4;
+  constexpr int DEG = 4;
+  constexpr int NM = n_mom<K, DEG>();
+  constexpr int NV = n_sums<K>();
   constexpr int NH = P * (P + 1) / 2;
-  constexpr bool GN = ORDER > 1;
+  constexpr int NG = 32 / GL;                    // groups of a warp
   const int gw = warp0 + ((int)threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   const int warps_atoms = (at.n + cfg.ag - 1) / cfg.ag;
   if (gw >= warps_atoms * cfg.nchunks) return;
   const int chunk = gw / warps_atoms, wa = gw - chunk * warps_atoms;
-  const int j = wa * cfg.ag + (lane % cfg.ag);   // slot
+  const int j = wa * cfg.ag + (lane & (cfg.ag - 1));   // slot
   const int sub = lane / cfg.ag;
   const bool valid = j < at.n;
   const int jj = valid ? (at.order ? at.order[j] : j) : 0;  // atom of the slot
@@ -312,52 +380,72 @@ __device__ __forceinline__ void deriv_body(const Atoms &at, const Geom &g, const
 
   float f = 0.f;
   CAcc gacc[P];
-  float hacc[ORDER > 1 ? NH : 1];
+  float hacc[NH];
 #pragma unroll
   for (int i = 0; i < P; ++i) gacc[i].zero();
 #pragma unroll
-  for (int i = 0; i < (ORDER > 1 ? NH : 1); ++i) hacc[i] = 0.f;
+  for (int i = 0; i < NH; ++i) hacc[i] = 0.f;
 
-  // lanes sharing a pair (cfg.rs of them, sub = s rs + phase) walk its rows
-  // phase, phase + rs, ... and combine their moment sums
-  const int phase = sub & (cfg.rs - 1);
-  unsigned gmask = 0u;
-  for (int o = 0; o < cfg.rs; ++o) gmask |= 1u << (lane + (o - phase) * cfg.ag);
-  for (int a = a_lo + sub / cfg.rs; a < a_hi && valid; a += cfg.sg / cfg.rs) {
+  // the warp's first 32 / rs lanes have a pair each (atom lane % ag, angle
+  // a0 + lane / ag); small problems give a warp fewer pairs than lanes
+  const int npairs = 32 / cfg.rs, astep = cfg.sg / cfg.rs;
+  for (int a0 = a_lo; a0 < a_hi; a0 += astep) {
+    const int a = a0 + sub;
+    const bool mine = valid && lane < npairs && a < a_hi;
     Frame<K> fr;
-    load_frame<K>(g.frames, a, fr);
     Pair<K> p;
-    pair_setup<K>(at, jj, fr, g, p);
-    PairMoments<K, DEG, GN> mo;
-    static_assert(!WIDE || K == 2, "wide rows: 3D Hessians only");
-    constexpr int CH = K == 1 ? kRowChunk : (WIDE ? 2 * kRowChunk3 : kRowChunk3);
-    pair_moments<K, DEG, GN, CH>(p, g, in, a, I, mo, phase, cfg.rs);
-    for (int o = 1; o < cfg.rs; o <<= 1) {
-#pragma unroll
-      for (int q = 0; q < n_mom<K, DEG>(); ++q) {
-        mo.Ma[q] += __shfl_xor_sync(gmask, mo.Ma[q], o * cfg.ag);
-        if (GN) mo.Mb[q] += __shfl_xor_sync(gmask, mo.Mb[q], o * cfg.ag);
-      }
-      mo.X0 += __shfl_xor_sync(gmask, mo.X0, o * cfg.ag);
-      mo.Y0 += __shfl_xor_sync(gmask, mo.Y0, o * cfg.ag);
+    if (mine) {
+      load_frame<K>(g.frames, a, fr);
+      pair_setup<K>(at, jj, fr, g, p);
+      walk_stage<K>(p, g, I, true, sm.pair[lane]);
+    } else {
+      sm.pair[lane].box = make_int4(1, 0, 1, 0);
     }
-    if (phase == 0) {
-      float Aa[NPSI];
-      first_psi<K, n_mom<K, DEG>()>(mo.Ma, p.G, Aa);
-      // value
-      if (in.mode == kModeInner) f += I * mo.Ma[0];
-      else if (in.mode == kModeL2Atom) f += I * (0.5f * I * mo.Y0 - mo.X0);
-      if constexpr (ORDER > 1) {
-        float Ba[NPSI][NPSI], Bb[NPSI][NPSI];
-        psi_gram<K, true>(mo.Ma, p.G, Ba);
-        psi_gram<K, false>(mo.Mb, p.G, Bb);
-        accumulate_pair<K, ORDER>(p, fr, I, Aa, Ba, Bb, gacc, hacc);
-      } else {
-        float Z[NPSI][NPSI];
-        accumulate_pair<K, ORDER>(p, fr, I, Aa, Z, Z, gacc, hacc);
+    __syncwarp();
+    for (int s0 = 0; s0 < npairs; s0 += NG) {
+      const int s = s0 + lane / GL, gl = lane % GL;
+      float v[NV];
+      walk_pair<K, GL, R, FK>(sm.pair[s < 32 ? s : 31], g, in, a0 + s / cfg.ag, gl, v);
+      __syncwarp();
+      // the group's lanes: each ends with the sums of NV / GL of the values
+      int n = NV, first = 0;
+#pragma unroll
+      for (int m = GL / 2; m >= 1; m >>= 1) {
+        n /= 2;
+        const bool up = (gl & m) != 0;
+        if (up) first += n;
+#pragma unroll
+        for (int k = 0; k < NV / 2; ++k)
+          if (k < n) {
+            const float keep = up ? v[k + n] : v[k];
+            const float give = up ? v[k] : v[k + n];
+            v[k] = keep + __shfl_xor_sync(0xffffffffu, give, m);
+          }
       }
+#pragma unroll
+      for (int k = 0; k < NV / GL; ++k) sm.sum[s < 32 ? s : 31][first + k] = v[k];
+    }
+    __syncwarp();
+    if (mine) {
+      float Ma[NM], Mb[NM];
+#pragma unroll
+      for (int q = 0; q < NM; ++q) {
+        Ma[q] = sm.sum[lane][q];
+        Mb[q] = in.beta ? sm.sum[lane][NM + q] : in.beta_const * sm.sum[lane][NM + q];
+      }
+      float Aa[NPSI];
+      first_psi<K, NM>(Ma, p.G, Aa);
+      // value
+      if (in.mode == kModeInner) f += I * Ma[0];
+      else if (in.mode == kModeL2Atom)
+        f += I * (0.5f * I * sm.sum[lane][NV - 1] - sm.sum[lane][NV - 2]);
+      float Ba[NPSI][NPSI], Bb[NPSI][NPSI];
+      psi_gram<K, true>(Ma, p.G, Ba);
+      psi_gram<K, false>(Mb, p.G, Bb);
+      accumulate_pair<K, 2>(p, fr, I, Aa, Ba, Bb, gacc, hacc);
     }
     if constexpr (ONE) break;
+    __syncwarp();
   }
 
   // combine lanes sharing an atom, then write
@@ -365,12 +453,12 @@ __device__ __forceinline__ void deriv_body(const Atoms &at, const Geom &g, const
   float gv[P];
 #pragma unroll
   for (int i = 0; i < P; ++i) gv[i] = gacc[i].get();
-  if (ORDER > 1 && cfg.ag == 1) {
+  if (cfg.ag == 1) {
     // one atom per warp: a reduce-scatter leaves the warp sum of value
     // 32 c + lane of the atom's qn values in lane `lane` (chunk c), so every
     // lane stores one value; a full butterfly of every value on every lane
     // would cost qn * 5 shuffles per lane instead of 31 per 32 values
-    constexpr int QN = 1 + P + (ORDER > 1 ? NH : 0);
+    constexpr int QN = 1 + P + NH;
     constexpr int NC = (QN + 31) / 32;
     float *dst = part + (size_t)chunk * cfg.qn * at.n + j;
 #pragma unroll
@@ -391,10 +479,8 @@ __device__ __forceinline__ void deriv_body(const Atoms &at, const Geom &g, const
     vals_f += __shfl_xor_sync(0xffffffffu, vals_f, off);
 #pragma unroll
     for (int i = 0; i < P; ++i) gv[i] += __shfl_xor_sync(0xffffffffu, gv[i], off);
-    if constexpr (ORDER > 1) {
 #pragma unroll
-      for (int i = 0; i < NH; ++i) hacc[i] += __shfl_xor_sync(0xffffffffu, hacc[i], off);
-    }
+    for (int i = 0; i < NH; ++i) hacc[i] += __shfl_xor_sync(0xffffffffu, hacc[i], off);
   }
   if (!valid || sub != 0) return;
   const size_t N = at.n;
@@ -402,23 +488,183 @@ __device__ __forceinline__ void deriv_body(const Atoms &at, const Geom &g, const
   dst[0] = vals_f;
 #pragma unroll
   for (int i = 0; i < P; ++i) dst[(1 + i) * N] = gv[i];
-  if constexpr (ORDER > 1) {
 #pragma unroll
-    for (int i = 0; i < NH; ++i) dst[(1 + P + i) * N] = hacc[i];
+  for (int i = 0; i < NH; ++i) dst[(1 + P + i) * N] = hacc[i];
+}
+
+// One-warp blocks: a warp that finishes frees its slot at once; with four, a
+// block holds its slot until its slowest warp (the one with the widest
+// supports) is done, which lowers the resident warps of the register-limited
+// Hessian kernels.
+template <int K, bool ONE, int GL, int R, int FK>
+__global__ void __launch_bounds__(32, hess_min_warps(K, ONE))
+    gr_hess_kernel(Atoms at, Geom g, DerivIn in, DerivCfg cfg, float *part) {
+  __shared__ WalkSmem<K> sm;
+  hess_body<K, ONE, GL, R, FK>(at, g, in, cfg, part, (int)blockIdx.x, sm);
+}
+
+// ---- gradients: a lane per pair ------------------------------------------------
+// A lane walks its pair's support alone: in 2D its cells, in 3D the rows of its
+// ellipse, in chunks of CH cells whose field values are loaded together.  A 3D
+// pair holds 20 to 40 cells, which groups of 2, 4 or 8 lanes per pair, as the
+// Hessians use, pad to 56 to 87 lane steps: 21.4, 21.2 and 24.5 against 17.4 ms
+// on 8192 atoms x 20000 orientations.  The loads bound it: 32 lanes touch 32
+// lines of the field, one L1 tag each.
+template <int K, int CH>
+__device__ __forceinline__ void lane_moments(const Pair<K> &p, const Geom &g, const DerivIn &in, int a,
+                                             float I, float (&Ma)[n_mom<K, 2>()], float &X0,
+                                             float &Y0, int phase, int rs) {
+  constexpr int NM = n_mom<K, 2>();
+#pragma unroll
+  for (int i = 0; i < NM; ++i) Ma[i] = 0.f;
+  X0 = 0.f;
+  Y0 = 0.f;
+  if (p.lo[0] > p.hi[0]) return;
+  if constexpr (K == 2)
+    if (p.lo[1] > p.hi[1]) return;
+  const float l2n = lg2_approx(p.n);
+  const int D0 = g.ax[0].n, D1 = K == 2 ? g.ax[1].n : 1;
+  const float *__restrict__ field = in.alpha;
+  const size_t abase = (size_t)a * D0 * D1;
+  // a cell's term: m its form, d its offset along the walk, c its field value
+  auto cell = [&](float m, float d, float c, float *S) {
+    if (m <= 1.f) {
+      const float E = ex2_approx(fmaf(m, kNegThirtyLog2e, l2n));
+      const float al = (in.mode == kModeL2Atom) ? fmaf(I, E, -c) : c;
+      const float w = al * E;
+      S[0] += w;
+      S[1] = fmaf(w, d, S[1]);
+      S[2] = fmaf(w, d * d, S[2]);
+      if (in.mode == kModeL2Atom) {
+        X0 = fmaf(E, c, X0);
+        Y0 = fmaf(E, E, Y0);
+      }
+    }
+  };
+  if constexpr (K == 1) {
+    const int c_hi = p.hi[0];
+    for (int kb = p.lo[0] + phase * CH; kb <= c_hi; kb += rs * CH) {
+      float cv[CH], pv[CH];
+#pragma unroll
+      for (int i = 0; i < CH; ++i) {
+        const int k0 = min(kb + i, c_hi);
+        cv[i] = __ldg(field + abase + k0);
+        pv[i] = __ldg(g.ax[0].coords + k0);
+      }
+#pragma unroll
+      for (int i = 0; i < CH; ++i) {
+        if (kb + i > c_hi) break;
+        const float d0 = (pv[i] - p.qh[0]) - p.ql[0];
+        cell(p.G[0] * d0 * d0, d0, cv[i], Ma);
+      }
+    }
+  } else {
+    // per row, m <= 1 holds for d1 within hw(d0) = sqrt(G2 - d0^2 det)/G2 of
+    // -G1 d0/G2: the row loop visits that range (widened like the support box)
+    // instead of the whole box; the m <= 1 test still decides every cell
+    const float det = p.G[0] * p.G[2] - p.G[1] * p.G[1];
+    const float iG2 = 1.f / p.G[2];
+    for (int k0 = p.lo[0] + phase; k0 <= p.hi[0]; k0 += rs) {
+      const float d0 = (__ldg(g.ax[0].coords + k0) - p.qh[0]) - p.ql[0];
+      const float t0 = p.G[0] * d0 * d0;
+      const float u = 2.f * p.G[1] * d0;
+      float Sa[3] = {0.f, 0.f, 0.f};
+      const size_t rbase = abase + (size_t)k0 * D1;
+      const float rem = fmaf(-d0 * d0, det, p.G[2]);
+      const float rc = (p.qh[1] - p.G[1] * d0 * iG2 - g.ax[1].first) * g.ax[1].inv_step;
+      const float rh = sqrtf(fmaxf(rem, 0.f)) * iG2 * g.ax[1].inv_step * 1.0001f + 1e-3f;
+      const float rlo = ceilf(rc - rh), rhi = floorf(rc + rh);
+      const int c_lo = (int)fminf(fmaxf(rlo, (float)p.lo[1]), (float)p.hi[1] + 1.f);
+      const int c_hi = (int)fmaxf(fminf(rhi, (float)p.hi[1]), (float)p.lo[1] - 1.f);
+      for (int kb = c_lo; kb <= c_hi; kb += CH) {
+        float cv[CH], pv[CH];
+#pragma unroll
+        for (int i = 0; i < CH; ++i) {
+          const int k1 = min(kb + i, c_hi);
+          cv[i] = __ldg(field + rbase + k1);
+          pv[i] = __ldg(g.ax[1].coords + k1);
+        }
+#pragma unroll
+        for (int i = 0; i < CH; ++i) {
+          if (kb + i > c_hi) break;
+          const float d1 = (pv[i] - p.qh[1]) - p.ql[1];
+          cell(fmaf(d1, fmaf(p.G[2], d1, u), t0), d1, cv[i], Sa);
+        }
+      }
+      float pw = 1.f;
+#pragma unroll
+      for (int i = 0; i <= 2; ++i) {
+#pragma unroll
+        for (int j = 0; j <= 2 - i; ++j) Ma[mi(i, j)] = fmaf(pw, Sa[j], Ma[mi(i, j)]);
+        pw *= d0;
+      }
+    }
   }
 }
 
-// BW warps per block.  With one-warp blocks a warp that finishes frees its
-// slot at once; with four, a block holds its slot until its slowest warp
-// (the one with the widest supports) is done, which lowers the resident
-// warps of the register-limited Hessian kernels (Tuning key 9).
-template <int K, int ORDER, bool ONE, bool WIDE = false, int BW = 4>
-__global__ void __launch_bounds__(BW * 32,
-                                  (ORDER == 1 ? GR_GRAD_MIN_BLOCKS
-                                              : (ONE ? (K == 1 ? GR_HESS2D_MIN_BLOCKS : 3) : 1)) *
-                                      4 / BW)
-    gr_deriv_kernel(Atoms at, Geom g, DerivIn in, DerivCfg cfg, float *part) {
-  deriv_body<K, ORDER, ONE, WIDE>(at, g, in, cfg, part, (int)blockIdx.x * BW);
+// ONE, one-warp blocks: as gr_hess_kernel.
+template <int K, bool ONE>
+__global__ void __launch_bounds__(32, 32)
+    gr_grad_kernel(Atoms at, Geom g, DerivIn in, DerivCfg cfg, float *part) {
+  constexpr int P = n_par<K>();
+  constexpr int NM = n_mom<K, 2>();
+  constexpr int NPSI = n_psi<K>();
+  const int gw = blockIdx.x, lane = threadIdx.x;
+  const int warps_atoms = (at.n + cfg.ag - 1) / cfg.ag;
+  const int chunk = gw / warps_atoms, wa = gw - chunk * warps_atoms;
+  const int j = wa * cfg.ag + (lane % cfg.ag);   // slot
+  const int sub = lane / cfg.ag;
+  const bool valid = j < at.n;
+  const int jj = valid ? (at.order ? at.order[j] : j) : 0;  // atom of the slot
+  const float I = at.I[jj];
+  const int a_lo = chunk * cfg.ch;
+  const int a_hi = min(g.n_angles, a_lo + cfg.ch);
+  float f = 0.f, none[1];
+  CAcc gacc[P];
+#pragma unroll
+  for (int i = 0; i < P; ++i) gacc[i].zero();
+  // lanes sharing a pair (cfg.rs of them, sub = s rs + phase) walk its rows
+  // (2D: chunks) phase, phase + rs, ... and combine their moment sums
+  const int phase = sub & (cfg.rs - 1);
+  unsigned gmask = 0u;
+  for (int o = 0; o < cfg.rs; ++o) gmask |= 1u << (lane + (o - phase) * cfg.ag);
+  for (int a = a_lo + sub / cfg.rs; a < a_hi && valid; a += cfg.sg / cfg.rs) {
+    Frame<K> fr;
+    load_frame<K>(g.frames, a, fr);
+    Pair<K> p;
+    pair_setup<K>(at, jj, fr, g, p);
+    float Ma[NM], X0, Y0;
+    lane_moments<K, K == 1 ? 8 : 4>(p, g, in, a, I, Ma, X0, Y0, phase, cfg.rs);
+    for (int o = 1; o < cfg.rs; o <<= 1) {
+#pragma unroll
+      for (int q = 0; q < NM; ++q) Ma[q] += __shfl_xor_sync(gmask, Ma[q], o * cfg.ag);
+      X0 += __shfl_xor_sync(gmask, X0, o * cfg.ag);
+      Y0 += __shfl_xor_sync(gmask, Y0, o * cfg.ag);
+    }
+    if (phase == 0) {
+      float Aa[NPSI], Z[NPSI][NPSI];
+      first_psi<K, NM>(Ma, p.G, Aa);
+      if (in.mode == kModeInner) f += I * Ma[0];
+      else if (in.mode == kModeL2Atom) f += I * (0.5f * I * Y0 - X0);
+      accumulate_pair<K, 1>(p, fr, I, Aa, Z, Z, gacc, none);
+    }
+    if constexpr (ONE) break;
+  }
+  // combine lanes sharing an atom, then write
+  float gv[P];
+#pragma unroll
+  for (int i = 0; i < P; ++i) gv[i] = gacc[i].get();
+  for (int off = cfg.ag; off < 32; off <<= 1) {
+    f += __shfl_xor_sync(0xffffffffu, f, off);
+#pragma unroll
+    for (int i = 0; i < P; ++i) gv[i] += __shfl_xor_sync(0xffffffffu, gv[i], off);
+  }
+  if (!valid || sub != 0) return;
+  const size_t N = at.n;
+  float *dst = part + (size_t)chunk * cfg.qn * N + j;
+  dst[0] = f;
+#pragma unroll
+  for (int i = 0; i < P; ++i) dst[(1 + i) * N] = gv[i];
 }
 
 // Pixel-integrated operator: per cell, the quadrature points' moments give
@@ -431,7 +677,6 @@ __global__ void __launch_bounds__(BW * 32,
 template <int K, int ORDER>
 __global__ void __launch_bounds__(128)
     gr_psf_deriv_kernel(Atoms at, Geom g, DerivIn in, DerivCfg cfg, float *part, float s) {
-  constexpr int D = K + 1;
   constexpr int P = n_par<K>();
   constexpr int NPSI = n_psi<K>();
   constexpr int DEG = ORDER == 1 ? 2 : 4;
@@ -794,6 +1039,48 @@ size_t derivs_workspace_bytes(int K, int n_atoms, int n_angles, int order, const
   return b;
 }
 
+struct DerivArgs {
+  const Atoms &at;
+  const Geom &g;
+  const DerivIn &in;
+  const DerivCfg &cfg;
+  float *part;
+  int warps;
+  bool one;
+  cudaStream_t stream;
+};
+
+template <int K>
+static void start_grad(const DerivArgs &d) {
+  if (d.one) gr_grad_kernel<K, true><<<d.warps, 32, 0, d.stream>>>(d.at, d.g, d.in, d.cfg, d.part);
+  else gr_grad_kernel<K, false><<<d.warps, 32, 0, d.stream>>>(d.at, d.g, d.in, d.cfg, d.part);
+}
+
+template <int K, int GL, int FK>
+static void start_one(const DerivArgs &d) {
+  gr_hess_kernel<K, true, GL, walk_cells_of<K>(), FK><<<d.warps, 32, 0, d.stream>>>(
+      d.at, d.g, d.in, d.cfg, d.part);
+}
+
+template <int K>
+static void start_hess(const DerivArgs &d) {
+  const bool beta = d.in.beta != nullptr, l2atom = d.in.mode == kModeL2Atom;
+  if (!d.one || (beta && l2atom)) {
+    gr_hess_kernel<K, false, walk_lanes_of<K>(), walk_cells_of<K>(), kFieldAny>
+        <<<d.warps, 32, 0, d.stream>>>(d.at, d.g, d.in, d.cfg, d.part);
+  } else if (d.cfg.rs == 8) {
+    // a warp with four pairs has eight lanes walk each
+    if (l2atom) start_one<K, 8, kFieldL2Atom>(d);
+    else if (beta) start_one<K, 8, kFieldBeta>(d);
+    else start_one<K, 8, kFieldPlain>(d);
+  } else {
+    constexpr int GL = walk_lanes_of<K>();
+    if (l2atom) start_one<K, GL, kFieldL2Atom>(d);
+    else if (beta) start_one<K, GL, kFieldBeta>(d);
+    else start_one<K, GL, kFieldPlain>(d);
+  }
+}
+
 int launch_derivs(const Atoms &at, const Geom &g, const DerivIn &in,
                   const DerivOut &out, void *ws, size_t ws_bytes,
                   cudaStream_t stream, const Tuning &t) {
@@ -820,11 +1107,8 @@ int launch_derivs(const Atoms &at, const Geom &g, const DerivIn &in,
     fe = f_extra;
   }
   const int warps = ((at.n + c.ag - 1) / c.ag) * c.nchunks;
-  const int blocks = (warps + 3) / 4;
-  const float s = 0.5f / g.ax[0].inv_step;  // cell half-width (pixel-integrated operator)
-  // one-warp blocks (Tuning key 9) for the kernels with one angle per lane
-  const bool bw1 = t.deriv_block_warps == 1;
-  const int blocks1 = warps;
+  const int blocks = (warps + 3) / 4;       // (pixel-integrated operator)
+  const float s = 0.5f / g.ax[0].inv_step;  // its cell half-width
   timer_mark(2, 0, stream);
   if (in.psf) {
     if (K == 1) {
@@ -838,36 +1122,10 @@ int launch_derivs(const Atoms &at, const Geom &g, const DerivIn &in,
     // at most one angle per lane: a lane's angles a_lo + sub + k sg lie
     // below a_lo + ch
     const bool one = c.ch <= c.sg / c.rs;
-    const bool wide = t.deriv_wide_rows != 0;
-    if (K == 1) {
-      if (in.order == 1) {
-        if (one) gr_deriv_kernel<1, 1, true><<<blocks, 128, 0, stream>>>(at, g, in, c, part);
-        else gr_deriv_kernel<1, 1, false><<<blocks, 128, 0, stream>>>(at, g, in, c, part);
-      } else {
-        if (one && bw1)
-          gr_deriv_kernel<1, 2, true, false, 1><<<blocks1, 32, 0, stream>>>(at, g, in, c, part);
-        else if (one) gr_deriv_kernel<1, 2, true><<<blocks, 128, 0, stream>>>(at, g, in, c, part);
-        else gr_deriv_kernel<1, 2, false><<<blocks, 128, 0, stream>>>(at, g, in, c, part);
-      }
-    } else {
-      if (in.order == 1) {
-        if (one && bw1)
-          gr_deriv_kernel<2, 1, true, false, 1><<<blocks1, 32, 0, stream>>>(at, g, in, c, part);
-        else if (one) gr_deriv_kernel<2, 1, true><<<blocks, 128, 0, stream>>>(at, g, in, c, part);
-        else gr_deriv_kernel<2, 1, false><<<blocks, 128, 0, stream>>>(at, g, in, c, part);
-      } else if (wide) {
-        if (one && bw1)
-          gr_deriv_kernel<2, 2, true, true, 1><<<blocks1, 32, 0, stream>>>(at, g, in, c, part);
-        else if (one)
-          gr_deriv_kernel<2, 2, true, true><<<blocks, 128, 0, stream>>>(at, g, in, c, part);
-        else gr_deriv_kernel<2, 2, false, true><<<blocks, 128, 0, stream>>>(at, g, in, c, part);
-      } else {
-        if (one && bw1)
-          gr_deriv_kernel<2, 2, true, false, 1><<<blocks1, 32, 0, stream>>>(at, g, in, c, part);
-        else if (one) gr_deriv_kernel<2, 2, true><<<blocks, 128, 0, stream>>>(at, g, in, c, part);
-        else gr_deriv_kernel<2, 2, false><<<blocks, 128, 0, stream>>>(at, g, in, c, part);
-      }
-    }
+    const DerivArgs d{at, g, in, c, part, warps, one, stream};
+    if (in.order == 2) K == 1 ? start_hess<1>(d) : start_hess<2>(d);
+    else if (K == 1) start_grad<1>(d);
+    else start_grad<2>(d);
   }
   timer_mark(2, 1, stream);
   const int fblocks = (at.n + kFinAtoms - 1) / kFinAtoms;
@@ -891,13 +1149,21 @@ __device__ __forceinline__ bool batch_derivs_wanted(const BatchProb &B, int acti
   return !(c > 0 && c <= B.hist_len && !B.hist_acc[c - 1]);
 }
 
-__global__ void __launch_bounds__(128, GR_HESS2D_MIN_BLOCKS)
+__global__ void __launch_bounds__(128, hess_min_warps(1, true) / 4)
     gr_batch_deriv_kernel(const BatchProb *__restrict__ probs, const int *__restrict__ off,
                           int n, const int *__restrict__ active) {
+  __shared__ WalkSmem<1> sm[4];
   const int p = batch_find(off, n, blockIdx.x);
   const BatchProb &B = probs[p];
   if (!batch_derivs_wanted(B, active[p])) return;
-  deriv_body<1, 2, true>(B.cur, B.g, B.din, B.cfg, B.part, ((int)blockIdx.x - off[p]) * 4);
+  const int warp0 = ((int)blockIdx.x - off[p]) * 4;
+  WalkSmem<1> &w = sm[threadIdx.x >> 5];
+  if (B.cfg.rs == 8)
+    hess_body<1, true, 8, walk_cells_of<1>(), kFieldPlain>(
+        B.cur, B.g, B.din, B.cfg, B.part, warp0, w);
+  else
+    hess_body<1, true, walk_lanes_of<1>(), walk_cells_of<1>(), kFieldPlain>(
+        B.cur, B.g, B.din, B.cfg, B.part, warp0, w);
 }
 
 __global__ void __launch_bounds__(kFinThreads)
@@ -921,17 +1187,21 @@ int launch_batch_derivs(const BatchLaunch &b, cudaStream_t stream) {
   return cudaGetLastError() == cudaSuccess ? kOk : kErrLaunch;
 }
 
+template <int K, int GL>
+static int preload_one() {
+  return preload_fn(gr_hess_kernel<K, true, GL, walk_cells_of<K>(), kFieldPlain>) +
+         preload_fn(gr_hess_kernel<K, true, GL, walk_cells_of<K>(), kFieldBeta>) +
+         preload_fn(gr_hess_kernel<K, true, GL, walk_cells_of<K>(), kFieldL2Atom>);
+}
+template <int K>
+static int preload_walk() {
+  return preload_one<K, walk_lanes_of<K>()>() + preload_one<K, 8>() +
+         preload_fn(gr_hess_kernel<K, false, walk_lanes_of<K>(), walk_cells_of<K>(), kFieldAny>) +
+         preload_fn(gr_grad_kernel<K, true>) + preload_fn(gr_grad_kernel<K, false>);
+}
+
 int preload_derivs() {
-  return preload_fn(gr_deriv_kernel<1, 1, false>) + preload_fn(gr_deriv_kernel<1, 2, false>) +
-         preload_fn(gr_deriv_kernel<2, 1, false>) + preload_fn(gr_deriv_kernel<2, 2, false>) +
-         preload_fn(gr_deriv_kernel<1, 1, true>) + preload_fn(gr_deriv_kernel<1, 2, true>) +
-         preload_fn(gr_deriv_kernel<2, 1, true>) + preload_fn(gr_deriv_kernel<2, 2, true>) +
-         preload_fn(gr_deriv_kernel<2, 2, false, true>) +
-         preload_fn(gr_deriv_kernel<2, 2, true, true>) +
-         preload_fn(gr_deriv_kernel<1, 2, true, false, 1>) +
-         preload_fn(gr_deriv_kernel<2, 1, true, false, 1>) +
-         preload_fn(gr_deriv_kernel<2, 2, true, false, 1>) +
-         preload_fn(gr_deriv_kernel<2, 2, true, true, 1>) +
+  return preload_walk<1>() + preload_walk<2>() +
          preload_fn(gr_psf_deriv_kernel<1, 1>) + preload_fn(gr_psf_deriv_kernel<1, 2>) +
          preload_fn(gr_psf_deriv_kernel<2, 1>) + preload_fn(gr_psf_deriv_kernel<2, 2>) +
          preload_fn(gr_deriv_finalize_kernel<1>) + preload_fn(gr_deriv_finalize_kernel<2>) +

@@ -88,7 +88,7 @@ struct DerivCfg {
   int ch;       // angles per chunk
   int nchunks;
   int qn;       // partial values per atom
-  int rs;       // lanes sharing one (atom, angle) pair's cells (power of two)
+  int rs;       // 32 / (atom, angle) pairs of a warp (power of two)
 };
 
 inline size_t align_up(size_t b) { return (b + 255) & ~(size_t)255; }
@@ -105,8 +105,8 @@ struct Tuning {
   int proj_split_cells = 4 << 20;   // key 4 (accepted, without effect: blocks share every tile)
   int deriv_split_lanes = 65536;    // key 6
   int deriv_one_mb = 1024;          // key 7
-  int deriv_wide_rows = 0;          // key 8 (1: 3D Hessian rows in 8-cell chunks)
-  int deriv_block_warps = 1;        // key 9 (warps per block, one-angle-per-lane kernels)
+  int deriv_wide_rows = 0;          // key 8 (accepted, without effect)
+  int deriv_block_warps = 1;        // key 9 (accepted, without effect: one-warp blocks)
 };
 extern Tuning g_tuning;
 int tuning_set(Tuning &t, int key, int value);

@@ -45,8 +45,8 @@ def set_projection_split(cells):
 
 
 def set_derivative_split(lanes):
-    """Problems with fewer (atom, angle) pairs than ``lanes`` split each
-    pair's cells over 2, 4 or 8 lanes of the derivative kernel (0: never)."""
+    """Problems with fewer (atom, angle) pairs than ``lanes`` spread them over
+    more warps: 16, 8 or 4 pairs a warp instead of 32 (0: never)."""
     _lib.check(_lib.load().gr_set_tuning(6, int(lanes)), "gr_set_tuning")
 
 
@@ -142,10 +142,10 @@ def apply_for(atoms, geom, order, psf=False):
 _req_plans = {}
 # small candidate sets: a server tunes each new class once, on its first
 # request, and the fits of the class then run under the winners
-# (only the row-walk switch for the derivatives: splits into fewer warps won
-# alone on an idle GPU but lost among concurrent fits, 1.655 s against 1.624 s
-# untuned on the 512-request stream)
-DERIV_CANDIDATES = ((131072, 1, 1, 0), (131072, 1, 1, 1))
+# (the derivatives keep the default split: splits into fewer warps won alone on
+# an idle GPU but lost among concurrent fits, 1.655 s against 1.624 s untuned on
+# the 512-request stream)
+DERIV_CANDIDATES = ((131072, 1, 1),)
 PROJ_CANDIDATES = (1, 2)          # 3D: tiles of 16 or 32 rows
 PROJ_CANDIDATES_2D = (1, 2, 3)    # 2D: tiles of 32, 64 or 128 cells
 

@@ -288,21 +288,14 @@ unsigned long long gr_launch_count(void);
  * GR_TUNE_PROJ_SPLIT_CELLS: accepted and without effect (it once chose
  * whether a block or a warp takes a 3D tile; a block always does).
  * GR_TUNE_DERIV_SPLIT_LANES: problems with
- * fewer (atom, angle) pairs than this split each pair's cells over 2, 4 or 8
- * lanes of the point-sampled derivative kernel (the largest split with
- * pairs x lanes <= value; default 65536; 0 = never).  GR_TUNE_DERIV_ONE_MB:
+ * fewer (atom, angle) pairs than this give a warp of the point-sampled
+ * derivative kernels 16, 8 or 4 pairs instead of 32 (the fewest with pairs x
+ * 32 / that <= value; default 65536; 0 = never).  GR_TUNE_DERIV_ONE_MB:
  * take enough angle chunks that every lane has at most one angle whenever the
  * chunk partials then fit in this many MB of workspace (default 1024; 0 =
- * keep GR_TUNE_DERIV_WARPS).  GR_TUNE_DERIV_WIDE_ROWS: 1 walks the rows of
- * the 3D Hessian (order 2) kernels in chunks of 8 cells instead of 4, which
- * keeps more field loads in flight when supports are many cells wide and
- * idles lanes when they are narrow (default 0; the serving tuner picks it
- * per class of requests).  GR_TUNE_DERIV_BLOCK_WARPS: warps per block of
- * the derivative kernels that give each lane at most one angle, 1 (default)
- * or 4; with one-warp blocks a finished warp frees its slot at once instead
- * of waiting for the slowest warp of its block (3D Hessians of the largest
- * served requests 458 -> 415 us, config 4's gradient 5 % faster; results are
- * bitwise the same).  Set them before
+ * keep GR_TUNE_DERIV_WARPS).  GR_TUNE_DERIV_WIDE_ROWS and
+ * GR_TUNE_DERIV_BLOCK_WARPS: accepted and without effect (they chose the row
+ * walk and block size of earlier kernels).  Set them before
  * gr_workspace_bytes and keep them fixed while launches that used the old
  * values are in flight.  Results do not depend on them beyond FP rounding of
  * the derivative chunk and lane sums (the tiling leaves 3D projections bitwise
