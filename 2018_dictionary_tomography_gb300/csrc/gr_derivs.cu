@@ -142,8 +142,7 @@ struct WalkSmem {
 };
 
 template <int K>
-__device__ __forceinline__ void walk_stage(const Pair<K> &p, const Geom &g, float I, bool live,
-                                           WalkPair &w) {
+__device__ __forceinline__ void walk_stage(const Pair<K> &p, const Geom &g, float I, WalkPair &w) {
   w.q = make_float4(-p.qh[0], -p.ql[0], K == 2 ? -p.qh[K - 1] : 0.f, K == 2 ? -p.ql[K - 1] : 0.f);
   w.v = make_float4(p.G[0], 2.f * p.G[1], p.G[2], lg2_approx(p.n));
   const DetAxis &x0 = g.ax[0];
@@ -154,8 +153,10 @@ __device__ __forceinline__ void walk_stage(const Pair<K> &p, const Geom &g, floa
                     iG0 * x0.inv_step, I);
   w.e = make_float4(det, K == 2 && p.G[1] != 0.f ? p.G[1] * rsqrtf(p.G[2] * det) : 0.f,
                     0.f, 0.f);
-  w.box = live ? make_int4(p.lo[0], p.hi[0], K == 2 ? p.lo[K - 1] : 0, K == 2 ? p.hi[K - 1] : 0)
-               : make_int4(1, 0, 1, 0);
+  // a support off the detector along either axis has no cells (the walk's rows
+  // and columns are clipped to the box, not to the detector)
+  const bool live = p.lo[0] <= p.hi[0] && p.lo[K - 1] <= p.hi[K - 1];
+  w.box = live ? make_int4(p.lo[0], p.hi[0], p.lo[K - 1], p.hi[K - 1]) : make_int4(1, 0, 1, 0);
 }
 
 __device__ __forceinline__ F2 f2_keep(const F2 &v, bool k0, bool k1) {
@@ -397,7 +398,7 @@ __device__ __forceinline__ void hess_body(const Atoms &at, const Geom &g, const 
     if (mine) {
       load_frame<K>(g.frames, a, fr);
       pair_setup<K>(at, jj, fr, g, p);
-      walk_stage<K>(p, g, I, true, sm.pair[lane]);
+      walk_stage<K>(p, g, I, sm.pair[lane]);
     } else {
       sm.pair[lane].box = make_int4(1, 0, 1, 0);
     }

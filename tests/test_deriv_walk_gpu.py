@@ -79,3 +79,36 @@ def test_fields_beyond_the_cut_off_count_for_nothing(eng, cuda_ready, kind, orde
         assert torch.equal(o[1], res[0][1])
         if order == 2:
             assert torch.equal(o[2], res[0][2])
+
+
+@pytest.mark.parametrize("kind", ["2d", "2p5d", "3d"])
+def test_supports_off_the_detector(eng, cuda_ready, kind):
+    """Atoms beyond each edge of a small detector, supports reaching over it or
+    not, some along one axis only: what the oracle counts, and exactly nothing
+    where no support meets the detector."""
+    dim = 2 if kind == "2d" else 3
+    g = make_geometry(kind, 8, 20, 16, det_box=0.5)
+    rng = np.random.default_rng(4)
+    x = []
+    for r0 in (0.45, 0.55, 0.8, 1.5, 3.0):
+        for v in list(np.eye(dim)) + list(-np.eye(dim)) + [np.ones(dim), -np.ones(dim)]:
+            x.append(r0 * v + 0.05 * rng.normal(size=dim))
+    x = np.array(x).astype(np.float32).astype(np.float64)
+    N = len(x)
+    I, _x, r = make_atoms(dim, N, 5, rdiag=(2.0, 8.0), roff=1.0)
+    al = rng.normal(size=g.shape).astype(np.float32).astype(np.float64)
+    for order in (1, 2):
+        _f, G, H = eng.atom_derivs(engine_atoms(I, x, r), engine_geometry(g), "field",
+                                   torch.from_numpy(al).float().cuda(), order=order)
+        G = G.cpu().numpy()
+        ref = [go.atom_derivs("field", I[j], x[j], r[j], g, al, 2, beta=np.ones_like(al))
+               for j in range(N)]
+        assert entry_relerr(G, np.array([o[1] for o in ref])) < TOL
+        off = np.array([not np.any(go.radproj(I[j:j + 1], x[j:j + 1], r[j:j + 1] * 0.99, g))
+                        for j in range(N)])
+        # (in 2D every atom here meets the detector at some angle)
+        assert off.sum() == 0 if kind == "2d" else 0 < off.sum() < N
+        assert not np.any(G[off])
+    H = H.cpu().numpy()
+    Ho = np.array([o[2] for o in ref])
+    assert np.max(np.abs(H - Ho)) <= TOL * np.max(np.abs(Ho)) and not np.any(H[off])
