@@ -77,7 +77,7 @@ EXPORTS = ("gr_version", "gr_preload", "gr_status_string", "gr_workspace_bytes",
            "gr_plan_workspace_bytes", "gr_radproj_plan", "gr_fit_forward_plan",
            "gr_atom_derivs_plan", "gr_batch_workspace_bytes", "gr_batch_create",
            "gr_batch_prologue", "gr_batch_iterate", "gr_fit_loop_end_open", "gr_batch_destroy",
-           "gr_fit_items", "gr_fit_empty_loss", "gr_fit_forward_skip")
+           "gr_fit_items", "gr_fit_empty_loss", "gr_fit_forward_skip", "gr_atom_grads")
 
 _lock = threading.Lock()
 _lib = None
@@ -90,6 +90,8 @@ def library_path():
 def load(build_if_missing=True):
     """Load libgauss_radon.so (building it first when allowed)."""
     global _lib
+    if _lib is not None:
+        return _lib
     with _lock:
         if _lib is not None:
             return _lib
@@ -155,6 +157,10 @@ def load(build_if_missing=True):
         lib.gr_psf_radproj.argtypes = lib.gr_radproj.argtypes
         lib.gr_psf_fit_forward.restype = ctypes.c_int
         lib.gr_psf_fit_forward.argtypes = lib.gr_fit_forward.argtypes
+        lib.gr_atom_grads.restype = ctypes.c_int
+        lib.gr_atom_grads.argtypes = [P(GrAtoms), P(GrGeometry), ctypes.c_void_p, ctypes.c_void_p,
+                                      ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,
+                                      ctypes.c_size_t, ctypes.c_void_p]
         lib.gr_psf_atom_derivs.restype = ctypes.c_int
         lib.gr_psf_atom_derivs.argtypes = lib.gr_atom_derivs.argtypes
         lib.gr_psf_volproj.restype = ctypes.c_int

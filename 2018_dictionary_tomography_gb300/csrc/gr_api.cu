@@ -58,7 +58,7 @@ bool batch_member(const gr_batch_member &m, BatchProb &p) {
   p.out = ProjOut{nullptr, kEpiL2, m.data, 0.f, m.fields, nullptr, nullptr, 0};
   p.loss_cur = m.loss_cur;
   p.loss_trial = m.loss_trial;
-  p.dout = DerivOut{m.f, m.g, m.H};
+  p.dout = DerivOut{m.f, m.g, m.H, nullptr, nullptr, nullptr};
   p.theta = m.theta;
   p.theta_trial = m.theta_trial;
   p.lam = m.lam;
@@ -242,7 +242,7 @@ static int atom_derivs_impl(const gr_atoms *atoms, const gr_geometry *geom, int 
   in.beta = mode == GR_MODE_FIELD ? beta_field : nullptr;
   in.beta_const = mode == GR_MODE_FIELD ? beta_const : (mode == GR_MODE_L2_ATOM ? 1.f : 0.f);
   in.psf = psf;
-  DerivOut out{f, g_out, H};
+  DerivOut out{f, g_out, H, nullptr, nullptr, nullptr};
   return launch_derivs(at, g, in, out, workspace, workspace_bytes,
                        static_cast<cudaStream_t>(stream), t);
 }
@@ -253,6 +253,22 @@ int gr_atom_derivs(const gr_atoms *atoms, const gr_geometry *geom, int mode,
                    size_t workspace_bytes, void *stream) {
   return atom_derivs_impl(atoms, geom, mode, field, beta_field, beta_const, order, f, g_out,
                           H, workspace, workspace_bytes, stream, 0);
+}
+
+int gr_atom_grads(const gr_atoms *atoms, const gr_geometry *geom, const float *field, float *gI,
+                  float *gx, float *gr, void *workspace, size_t workspace_bytes, void *stream) {
+  Atoms at;
+  Geom g;
+  int st;
+  if (!to_internal(atoms, geom, at, g, &st)) return st;
+  if (!field || !gI || !gx || !gr) return GR_ERR_ARG;
+  DerivIn in{};
+  in.mode = GR_MODE_INNER;
+  in.order = 1;
+  in.alpha = field;
+  DerivOut out{nullptr, nullptr, nullptr, gI, gx, gr};
+  return launch_derivs(at, g, in, out, workspace, workspace_bytes,
+                       static_cast<cudaStream_t>(stream));
 }
 
 int gr_psf_atom_derivs(const gr_atoms *atoms, const gr_geometry *geom, int mode,

@@ -79,6 +79,8 @@ struct DerivOut {
   double *f;   // (N)
   double *g;   // (N, P_out)
   double *H;   // (N, P_out, P_out), order 2
+  // gradients as float32 arrays instead of f and g (order 1; null: none)
+  float *gI, *gx, *gr;
 };
 
 // Work split of a derivative launch (gr_derivs.cu, deriv_cfg).

@@ -979,10 +979,10 @@ __global__ void __launch_bounds__(kLossThreads)
 // by tile edges).
 static int proj_rows(int form) { return form == 2 ? kTileDim0 : 16; }
 
-// Loss partials of up to this many items are summed by the projection's
-// last warp or block (sum_partials_warp: a chain of n / 256 FP64 adds);
-// above it the 1024-thread gr_loss_finalize_kernel does it.
-constexpr size_t kFusedLossItems = 8192;
+// Loss partials of up to this many items are summed by the projection's last
+// block (sum_partials_block: a chain of n / 512 FP64 adds, 2 us for 16384);
+// above it gr_loss_finalize_kernel does it (6 to 9 us and a launch).
+constexpr size_t kFusedLossItems = 16384;
 
 template <int NW>
 static void launch_project3d(size_t items, const Atoms &at, const Geom &g, const TileCfg &tc,

@@ -154,6 +154,15 @@ int gr_atom_derivs(const gr_atoms *atoms, const gr_geometry *geom, int mode,
                    size_t workspace_bytes, void *stream);
 
 /*
+ * The adjoint alone, as float32 arrays like the atoms' own: gI (N), gx (N, d)
+ * and gr (N, P_r) (isotropic: N) of <R, field>, the gradients of
+ * GR_MODE_INNER rounded once (the vector-Jacobian product of an automatic
+ * differentiation).  Workspace: GR_OP_DERIVS_1.
+ */
+int gr_atom_grads(const gr_atoms *atoms, const gr_geometry *geom, const float *field, float *gI,
+                  float *gx, float *gr, void *workspace, size_t workspace_bytes, void *stream);
+
+/*
  * Render atoms on a voxel grid: u[i0, i1(, i2)] = sum_j I_j sqrt(30/pi)
  * exp(-30 |r_j (y - x_j)|^2) where |r_j (y - x_j)| <= 1, y = (coords[0][i0],
  * coords[1][i1](, coords[2][i2])).  Replaces VolProj / __VolProj
