@@ -46,7 +46,7 @@ def _atoms(atom, first_only=False):
     I, x, r = atom.I, atom.x, atom.r
     if first_only:
         I, x, r = I[:1], x[:1], r[:1]
-    return engine.DeviceAtoms(_tensor(I), _tensor(x), _tensor(r))
+    return engine.DeviceAtoms(I, x, r)
 
 
 def _tensor(a):
@@ -87,11 +87,10 @@ def _derivs(atom, Rad, C, order, mode, dim, psf=False):
     atoms = _atoms(atom, first_only=True)
     C = _tensor(_data(C))
     o = 2 if order > 1 else 1
-    f, g, H = engine.atom_derivs(atoms, geom, mode, C.reshape(geom.shape), order=o, psf=psf)
-    f = float(f[0].item())
-    Df = g[0].cpu().numpy()
-    DDf = H[0].cpu().numpy() if H is not None else np.zeros((Df.size, Df.size))
-    return f, Df, DDf
+    f, g, H = engine.atom_derivs_host(atoms, geom, mode, C.reshape(geom.shape), order=o, psf=psf)
+    Df = g[0]
+    DDf = H[0] if H is not None else np.zeros((Df.size, Df.size))
+    return float(f[0]), Df, DDf
 
 
 def l2derivs(atom, Rad, C, order, dim, psf=False):

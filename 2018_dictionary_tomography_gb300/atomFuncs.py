@@ -54,7 +54,7 @@ class GaussTomo:
         return self._geom
 
     def device_atoms(self, atoms):
-        return engine.DeviceAtoms(_t(atoms.I), _t(atoms.x), _t(atoms.r))
+        return engine.DeviceAtoms(atoms.I, atoms.x, atoms.r)
 
     # ---- reference operator API ------------------------------------------
     def __call__(self, atoms, out=None):
@@ -76,14 +76,13 @@ class GaussTomo:
         C = C.asarray() if hasattr(C, "asarray") else C
         field = C if isinstance(C, torch.Tensor) else torch.from_numpy(
             np.ascontiguousarray(C, dtype=np.float32))
-        f, g, H = engine.atom_derivs(self.device_atoms(atoms), self.geometry, mode,
-                                     field.reshape(self.geometry.shape),
-                                     order=2 if order > 1 else 1, psf=self._psf)
-        f = f.cpu().numpy().reshape(-1, 1)
-        df = g.cpu().numpy()
+        f, df, ddf = engine.atom_derivs_host(self.device_atoms(atoms), self.geometry, mode,
+                                             field.reshape(self.geometry.shape),
+                                             order=2 if order > 1 else 1, psf=self._psf)
+        f = f.reshape(-1, 1)
         if order == 1:
             return f, df
-        return f, df, H.cpu().numpy()
+        return f, df, ddf
 
     def derivs(self, atoms, C, order=2):
         """Per atom: <R(a), C>, <dR(a), C>, <d2R(a), C> (atomFuncs.py:130)."""
@@ -116,12 +115,6 @@ class SingleParticleGaussTomo(GaussTomo):
         pkg = __name__.rsplit(".", 1)[0]
         mod = importlib.import_module(pkg + ".point_spread_functions")
         return mod.RadProj, mod.derivs_RadProj, mod.L2derivs_RadProj, mod.VolProj
-
-
-def _t(a):
-    if isinstance(a, torch.Tensor):
-        return a
-    return torch.from_numpy(np.ascontiguousarray(a, dtype=np.float32))
 
 
 def theta_to_vec(theta):

@@ -16,7 +16,7 @@ from . import engine
 class GaussRadonFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, I, x, r, geom):
-        atoms = engine.DeviceAtoms(I.detach(), x.detach(), r.detach(), geom.device)
+        atoms = engine.DeviceAtoms(I, x, r, geom.device)
         R = engine.radproj(atoms, geom)
         ctx.geom = geom
         ctx.save_for_backward(I, x, r)
@@ -27,9 +27,13 @@ class GaussRadonFunction(torch.autograd.Function):
     def backward(ctx, grad_R):
         I, x, r = ctx.saved_tensors
         geom = ctx.geom
-        atoms = engine.DeviceAtoms(I.detach(), x.detach(), r.detach(), geom.device)
-        _f, g, _H = engine.atom_derivs(atoms, geom, "inner",
-                                       grad_R.float().contiguous(), order=1)
+        atoms = engine.DeviceAtoms(I, x, r, geom.device)
+        field = grad_R.float().contiguous()
+        if I.dtype == x.dtype == r.dtype == torch.float32:
+            # float32 gradients in their own arrays, straight from the FP64 sums
+            gI, gx, gr = engine.atom_grads(atoms, geom, field)
+            return gI.reshape(I.shape), gx.reshape(x.shape), gr.reshape(r.shape), None
+        _f, g, _H = engine.atom_derivs(atoms, geom, "inner", field, order=1)
         d = atoms.dim
         gI = g[:, 0].to(I.dtype).reshape(I.shape)
         gx = g[:, 1:1 + d].to(x.dtype).reshape(x.shape)

@@ -30,10 +30,16 @@ def _require_cuda(device):
         raise _lib.EngineError("engine tensors must live on a CUDA device, got %s" % device)
 
 
+def _raw_stream(device):
+    """The current torch stream's handle (``torch.cuda.current_stream`` builds
+    a Stream object for it, 3.5 us on the host)."""
+    i = device.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if i is None else i)
+
+
 def workspace(nbytes, device):
     """Per-(device, stream) scratch buffer, grown on demand and reused."""
-    stream = torch.cuda.current_stream(device)
-    key = (device.index, stream.cuda_stream)
+    key = (device.index, _raw_stream(device))
     with _ws_lock:
         buf = _workspaces.get(key)
         if buf is None or buf.numel() < nbytes:
@@ -43,7 +49,30 @@ def workspace(nbytes, device):
 
 
 def _stream_handle(device):
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+    return ctypes.c_void_p(_raw_stream(device))
+
+
+def _host_f32(a):
+    """A host array or CPU tensor as a flat float32 numpy array."""
+    if isinstance(a, torch.Tensor):
+        a = a.detach().to(torch.float32).numpy()
+    return np.asarray(a, dtype=np.float32).reshape(-1)
+
+
+def to_device_packed(arrays, device):
+    """Float32 device copies of host arrays of any shape, moved with one copy
+    (a small host-to-device copy costs 17 us whatever its size): flat views of
+    one buffer, each starting at a multiple of 16 bytes."""
+    flat = [_host_f32(a) for a in arrays]
+    off, n = [], 0
+    for t in flat:
+        off.append(n)
+        n += (t.size + 3) // 4 * 4
+    host = np.zeros(n, dtype=np.float32)
+    for o, t in zip(off, flat):
+        host[o:o + t.size] = t
+    buf = torch.from_numpy(host).to(device)
+    return [buf[o:o + t.size] for o, t in zip(off, flat)]
 
 
 def morton_order(x):
@@ -72,19 +101,32 @@ class DeviceAtoms:
     def __init__(self, I, x, r, device=None, order=None):
         device = torch.device(device or "cuda")
         _require_cuda(device)
-        I = torch.as_tensor(I).to(device=device, dtype=torch.float32).reshape(-1).contiguous()
+        on_host = not any(isinstance(a, torch.Tensor) and a.is_cuda for a in (I, x, r))
+        if on_host:
+            # host arrays travel together
+            xs, rs = np.shape(x), np.shape(r)
+            I, x, r = to_device_packed((I, x, r), device)
+            if x.shape != xs:
+                x = x.reshape(xs)
+            if r.shape != rs:
+                r = r.reshape(rs)
+        else:
+            I, x, r = (torch.as_tensor(a).to(device=device, dtype=torch.float32)
+                       for a in (I, x, r))
         n = I.numel()
-        x = torch.as_tensor(x).to(device=device, dtype=torch.float32)
-        r = torch.as_tensor(r).to(device=device, dtype=torch.float32)
+        if I.dim() != 1:
+            I = I.reshape(-1)
         if n > 0:
-            x = x.reshape(n, -1).contiguous()
-            r = r.reshape(n, -1).contiguous()
+            if x.dim() != 2 or x.shape[0] != n:
+                x = x.reshape(n, -1)
+            if r.dim() != 2 or r.shape[0] != n:
+                r = r.reshape(n, -1)
         else:
             x = x.reshape(0, x.shape[-1] if x.dim() > 1 else 0)
             r = r.reshape(0, r.shape[-1] if r.dim() > 1 else 1)
         if r.shape[1] == 1:
-            r = r.reshape(n).contiguous()
-        self._bind(I, x, r, device, order)
+            r = r.reshape(n)
+        self._bind(I.contiguous(), x.contiguous(), r.contiguous(), device, order)
 
     @classmethod
     def wrap(cls, I, x, r):
@@ -282,21 +324,58 @@ def atom_derivs(atoms, geom, mode, field, beta_field=None, beta_const=1.0, order
     return f, g, H
 
 
+def atom_derivs_host(atoms, geom, mode, field, order=2, psf=False):
+    """``atom_derivs`` with its results as host arrays (f (N,), g (N, P), H
+    (N, P, P) or None), brought back with one copy."""
+    _check_dims(atoms, geom)
+    dev = geom.device
+    field = torch.as_tensor(field, device=dev, dtype=torch.float32).contiguous()
+    if tuple(field.shape) != tuple(geom.shape):
+        raise ValueError("field shape %s does not match geometry %s" % (tuple(field.shape), geom.shape))
+    N, P = atoms.n, atoms.n_params()
+    if N == 0:
+        f, g, H = atom_derivs(atoms, geom, mode, field, order=order, psf=psf)
+        return tuple(None if t is None else t.cpu().numpy() for t in (f, g, H))
+    nf, ng = N, N * P
+    buf = torch.empty(nf + ng + (N * P * P if order == 2 else 0), dtype=torch.float64, device=dev)
+    f, g = buf[:nf], buf[nf:nf + ng]
+    H = buf[nf + ng:] if order == 2 else None
+    ws, n = _ws_for(_lib.GR_OP_DERIVS_1 if order == 1 else _lib.GR_OP_DERIVS_2, atoms, geom)
+    atom_derivs_into(atoms, geom, mode, field, None, 1.0, order, f, g, H, ws, psf=psf)
+    h = buf.cpu().numpy()
+    return (h[:nf], h[nf:nf + ng].reshape(N, P),
+            h[nf + ng:].reshape(N, P, P) if order == 2 else None)
+
+
+def atom_grads(atoms, geom, field):
+    """Gradients of <R, field> as float32 device tensors like the atoms' own
+    (I (N,), x (N, d), r (N, P_r) or (N,)); see gr_atom_grads."""
+    _check_dims(atoms, geom)
+    dev = geom.device
+    gI, gx, gr = (torch.empty_like(t) for t in (atoms.I, atoms.x, atoms.r))
+    if atoms.n == 0:
+        return gI, gx, gr
+    ws, n = _ws_for(_lib.GR_OP_DERIVS_1, atoms, geom)
+    st = _lib.load().gr_atom_grads(
+        ctypes.byref(atoms.struct), ctypes.byref(geom.struct), field.data_ptr(), gI.data_ptr(),
+        gx.data_ptr(), gr.data_ptr(), ws.data_ptr(), n, _stream_handle(dev))
+    _lib.check(st, "gr_atom_grads")
+    return gI, gx, gr
+
+
 def l2_fit_derivs(atoms, geom, data, order=2):
     """Loss 1/2|R - data|^2 and, for every atom j, the gradient and Hessian of
     the reference's L2derivs_RadProj(atom_j, data + R_j - R) (the Newton-loop
     call, NewtonGaussian.py:59-60).  f_j equals the loss for every j."""
     fw = fit_forward(atoms, geom, data, "l2")
-    f, g, H = atom_derivs(atoms, geom, "field", fw["alpha"], None, 1.0, order)
-    f.copy_(fw["loss"].expand_as(f))
+    _f, g, H = atom_derivs(atoms, geom, "field", fw["alpha"], None, 1.0, order)
     return fw["loss"], g, H
 
 
 def kl_fit_derivs(atoms, geom, data, background, order=2):
     """KL(data || R + b) with its per-atom gradient and Hessian."""
     fw = fit_forward(atoms, geom, data, "kl", background)
-    f, g, H = atom_derivs(atoms, geom, "field", fw["alpha"], fw["beta"], 0.0, order)
-    f.copy_(fw["loss"].expand_as(f))
+    _f, g, H = atom_derivs(atoms, geom, "field", fw["alpha"], fw["beta"], 0.0, order)
     return fw["loss"], g, H
 
 

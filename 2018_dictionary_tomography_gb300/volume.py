@@ -16,8 +16,11 @@ def volproj(atoms, coords, device=None, psf=False):
     dim = len(coords)
     if atoms.n and atoms.dim != dim:
         raise ValueError("atoms are %dD, grid is %dD" % (atoms.dim, dim))
-    ys = [torch.as_tensor(np.asarray(c, dtype=np.float32).reshape(-1) if not isinstance(c, torch.Tensor)
-                          else c.float().reshape(-1)).to(dev).contiguous() for c in coords]
+    if any(isinstance(c, torch.Tensor) for c in coords):
+        ys = [torch.as_tensor(np.asarray(c, dtype=np.float32).reshape(-1) if not isinstance(c, torch.Tensor)
+                              else c.float().reshape(-1)).to(dev).contiguous() for c in coords]
+    else:
+        ys = engine.to_device_packed([np.asarray(c, dtype=np.float32) for c in coords], dev)
     shape = tuple(int(y.numel()) for y in ys)
     u = torch.empty(shape, dtype=torch.float32, device=dev)
     n = (ctypes.c_int * 3)(*(list(shape) + [1] * (3 - dim)))

@@ -81,6 +81,52 @@ def test_fields_beyond_the_cut_off_count_for_nothing(eng, cuda_ready, kind, orde
             assert torch.equal(o[2], res[0][2])
 
 
+@pytest.mark.parametrize("kind", ["2d", "2p5d"])
+@pytest.mark.parametrize("A", [1, 7, 8, 9, 65, 300])
+def test_chunk_sums(eng, cuda_ready, kind, A):
+    """Chunk counts around the batches and shared ranges of the finalize sum,
+    and the float32 gradients written straight from it."""
+    g = make_geometry(kind, A, 40, 30)
+    I, x, r = make_atoms(2 if kind == "2d" else 3, 5, A, rdiag=(3.0, 8.0))
+    atoms, geom = engine_atoms(I, x, r), engine_geometry(g)
+    C = np.random.default_rng(A).normal(size=g.shape).astype(np.float32).astype(np.float64)
+    Ct = torch.from_numpy(C).float().cuda()
+    ref = [go.atom_derivs("ip", I[j], x[j], r[j], g, C, 2) for j in range(5)]
+    for order in (1, 2):
+        _f, G, H = eng.atom_derivs(atoms, geom, "inner", Ct, order=order)
+        assert entry_relerr(G.cpu().numpy(), np.array([o[1] for o in ref])) < TOL
+    assert atom_normwise_relerr(H.cpu().numpy(), np.array([o[2] for o in ref])) < TOL
+    _f, G, _H = eng.atom_derivs(atoms, geom, "inner", Ct, order=1)
+    gI, gx, gr_ = eng.atom_grads(atoms, geom, Ct)
+    d = 2 if kind == "2d" else 3
+    assert torch.equal(gI, G[:, 0].float()) and torch.equal(gx, G[:, 1:1 + d].float())
+    assert torch.equal(gr_, G[:, 1 + d:].float())
+
+
+@pytest.mark.parametrize("iso", [False, True])
+def test_atoms_from_host_and_float32_gradients(eng, cuda_ready, iso):
+    """Atoms from lists, numpy arrays and tensors are the same, and the adjoint
+    of float32 parameters is the rounded adjoint of float64 ones."""
+    import importlib
+    ag = importlib.import_module("2018_dictionary_tomography_gb300.autograd")
+    g = make_geometry("2p5d", 9, 30, 26)
+    I, x, r = make_atoms(3, 7, 3, iso=iso)
+    geom = engine_geometry(g)
+    ref = eng.radproj(engine_atoms(I, x, r), geom)
+    dev = lambda a, t: torch.tensor(a, dtype=t, device="cuda")
+    for v in ((I.tolist(), x.tolist(), r.tolist()), tuple(torch.from_numpy(a) for a in (I, x, r)),
+              tuple(dev(a, torch.float64) for a in (I, x, r)),
+              tuple(dev(a, torch.float32) for a in (I, x, r))):
+        assert torch.equal(eng.radproj(eng.DeviceAtoms(*v), geom), ref)
+    G = torch.randn(geom.shape, device="cuda")
+    grads = []
+    for t in (torch.float32, torch.float64):
+        p = [dev(a, t).requires_grad_(True) for a in (I, x, r)]
+        grads.append(torch.autograd.grad(ag.project(*p, geom), p, G))
+    for a, b in zip(*grads):
+        assert a.shape == b.shape and a.dtype == torch.float32 and torch.equal(a, b.float())
+
+
 @pytest.mark.parametrize("kind", ["2d", "2p5d", "3d"])
 def test_supports_off_the_detector(eng, cuda_ready, kind):
     """Atoms beyond each edge of a small detector, supports reaching over it or
