@@ -675,27 +675,49 @@ __global__ void __launch_bounds__(32, 32)
 // "total mass" cells zero derivatives).  The pair's sums
 //   Sa = sum alpha A_cell, Ta = sum alpha BC_cell, Ub = sum beta A_cell A_cell^T
 // feed the same chain-rule assembly as the point-sampled kernel.
-template <int K, int ORDER>
-__global__ void __launch_bounds__(128)
-    gr_psf_deriv_kernel(Atoms at, Geom g, DerivIn in, DerivCfg cfg, float *part, float s) {
+// A block's 32 pairs: the sums over an atom's pairs, in angle order.
+template <int QN>
+__device__ __forceinline__ void psf_close(const float (*vals)[QN + 1], int n_atoms,
+                                          const DerivCfg &cfg, int chunk, int wa, float *part) {
+  for (int e = threadIdx.x; e < cfg.ag * QN; e += blockDim.x) {
+    const int t = e / QN, q = e - t * QN;
+    if (wa * cfg.ag + t >= n_atoms) continue;
+    double v = 0.0;
+    for (int k = 0; k < cfg.sg; ++k) v += (double)vals[t + k * cfg.ag][q];
+    part[((size_t)chunk * cfg.qn + q) * n_atoms + wa * cfg.ag + t] = (float)v;
+  }
+}
+
+// 2D: a block takes 32 (atom, angle) pairs at a time (as a warp of the other
+// kernels does), four lanes each, which share the pair's few cells (11 points
+// each); a pair's first lane assembles, and the block adds its pairs' values per
+// atom.
+constexpr int kPsfLanes = 4;
+template <int ORDER>
+__global__ void __launch_bounds__(32 * kPsfLanes)
+    gr_psf_deriv1d_kernel(Atoms at, Geom g, DerivIn in, DerivCfg cfg, float *part, float s) {
+  constexpr int K = 1;
   constexpr int P = n_par<K>();
   constexpr int NPSI = n_psi<K>();
   constexpr int DEG = ORDER == 1 ? 2 : 4;
   constexpr int NM = n_mom<K, DEG>();
   constexpr int NH = P * (P + 1) / 2;
-  const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
+  constexpr int QN = 1 + P + (ORDER > 1 ? NH : 0);
+  constexpr int NT = ORDER > 1 ? NPSI * (NPSI + 1) / 2 : 1;   // upper triangles
+  __shared__ float vals[32][QN + 1];
+  const int gw = blockIdx.x;
+  const int pr = threadIdx.x / kPsfLanes, gl = threadIdx.x % kPsfLanes;
+  const unsigned gmask = ((1u << kPsfLanes) - 1u) << ((threadIdx.x & 31) & ~(kPsfLanes - 1));
   const int warps_atoms = (at.n + cfg.ag - 1) / cfg.ag;
-  if (gw >= warps_atoms * cfg.nchunks) return;
   const int chunk = gw / warps_atoms, wa = gw - chunk * warps_atoms;
-  const int j = wa * cfg.ag + (lane % cfg.ag);   // slot
-  const int sub = lane / cfg.ag;
+  const int j = wa * cfg.ag + (pr % cfg.ag);   // slot
+  const int sub = pr / cfg.ag;
   const bool valid = j < at.n;
   const int jj = valid ? (at.order ? at.order[j] : j) : 0;  // atom of the slot
   const float I = at.I[jj];
   const int a_lo = chunk * cfg.ch;
   const int a_hi = min(g.n_angles, a_lo + cfg.ch);
-  const int D0 = g.ax[0].n, D1 = K == 2 ? g.ax[1].n : 1;
+  const int D0 = g.ax[0].n;
 
   float f = 0.f;
   CAcc gacc[P];
@@ -713,85 +735,254 @@ __global__ void __launch_bounds__(128)
     PsfPair<K> q;
     psf_setup<K>(at, jj, g, p, ok, s, q);
     const float l2n = lg2_approx(p.n);
-    float Sa[NPSI], Ta[NPSI][NPSI], Ub[NPSI][NPSI];
+    float Sa[NPSI], Tt[NT], Ut[NT], fa = 0.f;
 #pragma unroll
-    for (int k = 0; k < NPSI; ++k) {
-      Sa[k] = 0.f;
+    for (int k = 0; k < NPSI; ++k) Sa[k] = 0.f;
 #pragma unroll
-      for (int l = 0; l < NPSI; ++l) {
-        Ta[k][l] = 0.f;
-        Ub[k][l] = 0.f;
+    for (int k = 0; k < NT; ++k) Tt[k] = Ut[k] = 0.f;
+    for (int k0 = q.lo[0] + gl; k0 <= q.hi[0]; k0 += kPsfLanes) {
+      float dc[K], base[K], step[K];
+      dc[0] = (__ldg(g.ax[0].coords + k0) - p.qh[0]) - p.ql[0];
+      const int kind = psf_cell_kind<K>(q, dc, s, base, step);
+      if (kind == 0) continue;
+      const size_t gi = (size_t)a * D0 + k0;
+      const float c = __ldg(in.alpha + gi);
+      if (kind == 1) {
+        const float R = q.total;
+        if (in.mode == kModeInner) fa = fmaf(c, R, fa);
+        else if (in.mode == kModeL2Atom) fa += R * (0.5f * R - c);
+        continue;
+      }
+      float M[NM];
+#pragma unroll
+      for (int i = 0; i < NM; ++i) M[i] = 0.f;
+#pragma unroll
+      for (int t = 1; t <= 11; ++t) {
+        const float d = fmaf((float)t, step[0], base[0]);
+        float w = ex2_approx(fmaf(p.G[0] * d * d, kNegThirtyLog2e, l2n));
+#pragma unroll
+        for (int i = 0; i < NM; ++i) {
+          M[i] += w;
+          w *= d;
+        }
+      }
+      const float scale = 10.f * step[0] / 11.f;
+      const float R = I * scale * M[0];
+      float al, be;
+      if (in.mode == kModeInner) {
+        al = c;
+        be = 0.f;
+        fa = fmaf(c, R, fa);
+      } else if (in.mode == kModeL2Atom) {
+        al = R - c;
+        be = 1.f;
+        fa += R * (0.5f * R - c);
+      } else {
+        al = c;
+        be = in.beta ? __ldg(in.beta + gi) : in.beta_const;
+      }
+      float A[NPSI];
+      first_psi<K, NM>(M, p.G, A);
+#pragma unroll
+      for (int k = 0; k < NPSI; ++k) {
+        A[k] *= scale;
+        Sa[k] = fmaf(al, A[k], Sa[k]);
+      }
+      if constexpr (ORDER > 1) {
+        float BC[NPSI][NPSI];
+        psi_gram<K, true>(M, p.G, BC);
+        const float as = al * scale;
+        int o = 0;
+#pragma unroll
+        for (int k = 0; k < NPSI; ++k)
+#pragma unroll
+          for (int l = k; l < NPSI; ++l, ++o) {
+            Tt[o] = fmaf(as, BC[k][l], Tt[o]);
+            Ut[o] = fmaf(be * A[k], A[l], Ut[o]);
+          }
       }
     }
-    const int lo1 = K == 2 ? q.lo[K - 1] : 0, hi1 = K == 2 ? q.hi[K - 1] : 0;
-    for (int k0 = q.lo[0]; k0 <= q.hi[0]; ++k0) {
-      for (int k1 = lo1; k1 <= hi1; ++k1) {
-        float dc[K], base[K], step[K];
-        dc[0] = (__ldg(g.ax[0].coords + k0) - p.qh[0]) - p.ql[0];
-        if constexpr (K == 2) dc[1] = (__ldg(g.ax[1].coords + k1) - p.qh[1]) - p.ql[1];
-        const int kind = psf_cell_kind<K>(q, dc, s, base, step);
-        if (kind == 0) continue;
-        const size_t gi = ((size_t)a * D0 + k0) * D1 + k1;
-        const float c = __ldg(in.alpha + gi);
-        if (kind == 1) {
-          const float R = q.total;
-          if (in.mode == kModeInner) f = fmaf(c, R, f);
-          else if (in.mode == kModeL2Atom) f += R * (0.5f * R - c);
-          continue;
+    __syncwarp(gmask);
+#pragma unroll
+    for (int o = kPsfLanes / 2; o > 0; o >>= 1) {
+      fa += __shfl_xor_sync(gmask, fa, o);
+#pragma unroll
+      for (int k = 0; k < NPSI; ++k) Sa[k] += __shfl_xor_sync(gmask, Sa[k], o);
+      if constexpr (ORDER > 1) {
+#pragma unroll
+        for (int k = 0; k < NT; ++k) {
+          Tt[k] += __shfl_xor_sync(gmask, Tt[k], o);
+          Ut[k] += __shfl_xor_sync(gmask, Ut[k], o);
         }
+      }
+    }
+    if (gl == 0) {
+      f += fa;
+      float Ta[NPSI][NPSI], Ub[NPSI][NPSI];
+      if constexpr (ORDER > 1) {
+        int o = 0;
+#pragma unroll
+        for (int k = 0; k < NPSI; ++k)
+#pragma unroll
+          for (int l = k; l < NPSI; ++l, ++o) {
+            Ta[k][l] = Ta[l][k] = Tt[o];
+            Ub[k][l] = Ub[l][k] = Ut[o];
+          }
+      }
+      accumulate_pair<K, ORDER>(p, fr, I, Sa, Ta, Ub, gacc, hacc);
+    }
+  }
+
+  if (gl == 0) {
+    vals[pr][0] = f;
+#pragma unroll
+    for (int i = 0; i < P; ++i) vals[pr][1 + i] = gacc[i].get();
+    if constexpr (ORDER > 1) {
+#pragma unroll
+      for (int i = 0; i < NH; ++i) vals[pr][1 + P + i] = hacc[i];
+    }
+  }
+  __syncthreads();
+  psf_close<QN>(vals, at.n, cfg, chunk, wa, part);
+}
+
+// 3D: a block takes 32 (atom, angle) pairs at a time, a warp eight of them.  The
+// warp's lanes look over a pair's cell box and queue the cells it reaches; 32
+// queued cells at a time, of as many pairs as that takes, are summed over their
+// 121 points, two to a register pair (this bounds it), and reduced pair by pair
+// into shared memory.  A lane per pair then assembles, and the block adds its
+// pairs' values per atom.  128 atoms x 401 x 64^2, gradient: 163 us with a lane
+// per pair, which walked some 40 cells in series on 10 warps an SM; 143 us with
+// eight lanes a pair, 12 of 32 lanes at work; with the queue 66 us.
+constexpr int kPsfWarps = 4, kPsfPairs = 8;
+
+struct PsfWalk {
+  float4 a, b;        // qh0 ql0 qh1 ql1; G00 G01 G11 log2 n
+  float rr, total, I;
+  int angle;
+  int lo0, lo1, bw, ncell;
+};
+
+template <int ORDER>
+__global__ void __launch_bounds__(32 * kPsfWarps, ORDER == 1 ? 4 : 2)
+    gr_psf_deriv_kernel(Atoms at, Geom g, DerivIn in, DerivCfg cfg, float *part, float s) {
+  constexpr int K = 2;
+  constexpr int P = n_par<K>();
+  constexpr int NPSI = n_psi<K>();
+  constexpr int DEG = ORDER == 1 ? 2 : 4;
+  constexpr int NM = n_mom<K, DEG>();
+  constexpr int NH = P * (P + 1) / 2;
+  constexpr int QN = 1 + P + (ORDER > 1 ? NH : 0);
+  constexpr int NT = ORDER > 1 ? NPSI * (NPSI + 1) / 2 : 0;   // upper triangles
+  // a cell's sums: f, first order, second order against alpha and against beta
+  constexpr int NV = (1 + NPSI + 2 * NT + 7) / 8 * 8;
+  __shared__ PsfWalk s_walk[kPsfWarps][kPsfPairs];
+  __shared__ int2 s_queue[kPsfWarps][64];
+  __shared__ float s_sum[kPsfWarps][kPsfPairs][NV + 1];
+  __shared__ float vals[kPsfWarps * kPsfPairs][QN + 1];
+  const int gw = blockIdx.x;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  PsfWalk *walk = s_walk[warp];
+  int2 *queue = s_queue[warp];
+  float(*sum)[NV + 1] = s_sum[warp];
+  const int pr = warp * kPsfPairs + (lane & (kPsfPairs - 1));
+  const int warps_atoms = (at.n + cfg.ag - 1) / cfg.ag;
+  const int chunk = gw / warps_atoms, wa = gw - chunk * warps_atoms;
+  const int j = wa * cfg.ag + (pr % cfg.ag);   // slot
+  const int sub = pr / cfg.ag;
+  const bool valid = lane < kPsfPairs && j < at.n;
+  const int jj = valid ? (at.order ? at.order[j] : j) : 0;  // atom of the slot
+  const float I = at.I[jj];
+  const int a_lo = chunk * cfg.ch;
+  const int a_hi = min(g.n_angles, a_lo + cfg.ch);
+  const int D0 = g.ax[0].n, D1 = g.ax[1].n;
+
+  float f = 0.f;
+  CAcc gacc[P];
+  float hacc[ORDER > 1 ? NH : 1];
+#pragma unroll
+  for (int i = 0; i < P; ++i) gacc[i].zero();
+#pragma unroll
+  for (int i = 0; i < (ORDER > 1 ? NH : 1); ++i) hacc[i] = 0.f;
+
+  // the first n queued cells
+  auto add_cells = [&](int n) {
+    const bool on = lane < n;
+    const int2 it = queue[on ? lane : n - 1];
+    const int slot = it.x & (kPsfPairs - 1), k0 = it.x >> 3, k1 = it.y;
+    const float4 wa4 = walk[slot].a, wb4 = walk[slot].b;
+    const float Ij = walk[slot].I;
+    float V[NV];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) V[i] = 0.f;
+    if (on) {
+      Pair<K> p;
+      p.G[0] = wb4.x;
+      p.G[1] = wb4.y;
+      p.G[2] = wb4.z;
+      const float l2n = wb4.w;
+      PsfPair<K> q;
+      q.rr = walk[slot].rr;
+      float dc[K], base[K], step[K];
+      dc[0] = (__ldg(g.ax[0].coords + k0) - wa4.x) - wa4.y;
+      dc[1] = (__ldg(g.ax[1].coords + k1) - wa4.z) - wa4.w;
+      const int kind = psf_cell_kind<K>(q, dc, s, base, step);
+      const size_t gi = ((size_t)walk[slot].angle * D0 + k0) * D1 + k1;
+      const float c = __ldg(in.alpha + gi);
+      if (kind == 1) {
+        const float R = walk[slot].total;
+        if (in.mode == kModeInner) V[0] = c * R;
+        else if (in.mode == kModeL2Atom) V[0] = R * (0.5f * R - c);
+      } else {
+        // a row's points two at a time (packed FP32)
         float M[NM];
 #pragma unroll
         for (int i = 0; i < NM; ++i) M[i] = 0.f;
-        float scale;
-        if constexpr (K == 1) {
+        const PsfRow row(base[1], step[1], p.G[2]);
+        const float g0 = p.G[0] * kNegThirtyLog2e, g1 = 2.f * p.G[1] * kNegThirtyLog2e;
+#pragma unroll 1
+        for (int t = 1; t <= 11; ++t) {
+          const float d0 = fmaf((float)t, step[0], base[0]);
+          const float c0 = fmaf(g0 * d0, d0, l2n), u = g1 * d0;
+          const F2 cp = f2(c0, c0), up = f2(u, u);
+          F2 S2[DEG + 1];
 #pragma unroll
-          for (int t = 1; t <= 11; ++t) {
-            const float d = fmaf((float)t, step[0], base[0]);
-            float w = ex2_approx(fmaf(p.G[0] * d * d, kNegThirtyLog2e, l2n));
-#pragma unroll
-            for (int e = 0; e < NM; ++e) {
-              M[e] += w;
-              w *= d;
-            }
-          }
-          scale = 10.f * step[0] / 11.f;
-        } else {
-          for (int t = 1; t <= 11; ++t) {
-            const float d0 = fmaf((float)t, step[0], base[0]);
-            const float t0 = p.G[0] * d0 * d0, u = 2.f * p.G[1] * d0;
-            float S[DEG + 1];
-#pragma unroll
-            for (int e = 0; e <= DEG; ++e) S[e] = 0.f;
-            for (int v = 1; v <= 11; ++v) {
-              const float d1 = fmaf((float)v, step[1], base[1]);
-              const float m = fmaf(d1, fmaf(p.G[2], d1, u), t0);
-              float w = ex2_approx(fmaf(m, kNegThirtyLog2e, l2n));
-#pragma unroll
-              for (int e = 0; e <= DEG; ++e) {
-                S[e] += w;
-                w *= d1;
-              }
-            }
-            float pw = 1.f;
+          for (int v = 0; v < 5; ++v) {
+            F2 w = row.pair(v, up, cp);
 #pragma unroll
             for (int i = 0; i <= DEG; ++i) {
-#pragma unroll
-              for (int jx = 0; jx <= DEG - i; ++jx) M[mi(i, jx)] = fmaf(pw, S[jx], M[mi(i, jx)]);
-              pw *= d0;
+              S2[i] = v == 0 ? w : f2_add(S2[i], w);
+              if (i < DEG) w = f2_mul(w, row.d[v]);
             }
           }
-          scale = 100.f * step[0] * step[1] / 121.f;
+          float w = row.end(u, c0);
+          float S[DEG + 1];
+#pragma unroll
+          for (int i = 0; i <= DEG; ++i) {
+            float x, y;
+            f2_get(S2[i], x, y);
+            S[i] = (x + y) + w;
+            w *= row.last;
+          }
+          float pw = 1.f;
+#pragma unroll
+          for (int i = 0; i <= DEG; ++i) {
+#pragma unroll
+            for (int jx = 0; jx <= DEG - i; ++jx) M[mi(i, jx)] = fmaf(pw, S[jx], M[mi(i, jx)]);
+            pw *= d0;
+          }
         }
-        const float R = I * scale * M[0];
+        const float scale = 100.f * step[0] * step[1] / 121.f;
+        const float R = Ij * scale * M[0];
         float al, be;
         if (in.mode == kModeInner) {
           al = c;
           be = 0.f;
-          f = fmaf(c, R, f);
+          V[0] = c * R;
         } else if (in.mode == kModeL2Atom) {
           al = R - c;
           be = 1.f;
-          f += R * (0.5f * R - c);
+          V[0] = R * (0.5f * R - c);
         } else {
           al = c;
           be = in.beta ? __ldg(in.beta + gi) : in.beta_const;
@@ -801,48 +992,147 @@ __global__ void __launch_bounds__(128)
 #pragma unroll
         for (int k = 0; k < NPSI; ++k) {
           A[k] *= scale;
-          Sa[k] = fmaf(al, A[k], Sa[k]);
+          V[1 + k] = al * A[k];
         }
         if constexpr (ORDER > 1) {
           float BC[NPSI][NPSI];
           psi_gram<K, true>(M, p.G, BC);
           const float as = al * scale;
+          int o = 1 + NPSI;
 #pragma unroll
           for (int k = 0; k < NPSI; ++k)
 #pragma unroll
-            for (int l = 0; l < NPSI; ++l) {
-              Ta[k][l] = fmaf(as, BC[k][l], Ta[k][l]);
-              Ub[k][l] = fmaf(be * A[k], A[l], Ub[k][l]);
+            for (int l = k; l < NPSI; ++l, ++o) {
+              V[o] = as * BC[k][l];
+              V[NT + o] = be * A[k] * A[l];
             }
         }
       }
     }
-    accumulate_pair<K, ORDER>(p, fr, I, Sa, Ta, Ub, gacc, hacc);
+    // pair by pair, eight values at a time: halve the values held over three
+    // exchanges, then sum the four lanes that hold the same one
+    const int first = __shfl_sync(0xffffffffu, slot, 0), last = __shfl_sync(0xffffffffu, slot, 31);
+    for (int sl = first; sl <= last; ++sl) {
+      const bool mine = on && slot == sl;
+      if (!__any_sync(0xffffffffu, mine)) continue;
+#pragma unroll
+      for (int v0 = 0; v0 < NV; v0 += 8) {
+        float h[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) h[i] = mine ? V[v0 + i] : 0.f;
+#pragma unroll
+        for (int w = 4; w > 0; w >>= 1) {
+          const bool up = lane & (4 * w);
+#pragma unroll
+          for (int i = 0; i < w; ++i) {
+            const float keep = up ? h[w + i] : h[i], give = up ? h[i] : h[w + i];
+            h[i] = keep + __shfl_xor_sync(0xffffffffu, give, 4 * w);
+          }
+        }
+        h[0] += __shfl_xor_sync(0xffffffffu, h[0], 2);
+        h[0] += __shfl_xor_sync(0xffffffffu, h[0], 1);
+        if ((lane & 3) == 0) sum[sl][v0 + (lane >> 2)] += h[0];
+      }
+    }
+    __syncwarp();
+  };
+
+  const int steps = (a_hi - a_lo + cfg.sg - 1) / cfg.sg;
+  for (int st = 0; st < steps; ++st) {
+    const int a = a_lo + sub + st * cfg.sg;
+    const bool on = valid && a < a_hi;
+    Frame<K> fr;
+    Pair<K> p;
+    int ncell = 0;
+    for (int i = lane; i < kPsfPairs * (NV + 1); i += 32) (&sum[0][0])[i] = 0.f;
+    if (on) {
+      load_frame<K>(g.frames, a, fr);
+      const bool ok = pair_setup<K>(at, jj, fr, g, p);
+      PsfPair<K> q;
+      psf_setup<K>(at, jj, g, p, ok, s, q);
+      PsfWalk w;
+      w.a = make_float4(p.qh[0], p.ql[0], p.qh[1], p.ql[1]);
+      w.b = make_float4(p.G[0], p.G[1], p.G[2], lg2_approx(p.n));
+      w.rr = q.rr;
+      w.total = q.total;
+      w.I = I;
+      w.angle = a;
+      w.lo0 = q.lo[0];
+      w.lo1 = q.lo[1];
+      w.bw = max(q.hi[1] - q.lo[1] + 1, 0);
+      w.ncell = ncell = max(q.hi[0] - q.lo[0] + 1, 0) * w.bw;
+      walk[lane] = w;
+    }
+    __syncwarp();
+    int queued = 0;
+    for (int sl = 0; sl < kPsfPairs; ++sl) {
+      const int nc = __shfl_sync(0xffffffffu, ncell, sl);
+      if (nc == 0) continue;
+      const PsfWalk w = walk[sl];
+      PsfPair<K> q;
+      q.rr = w.rr;
+      const float inv_bw = 1.f / (float)w.bw;
+      for (int e0 = 0; e0 < nc; e0 += 32) {
+        const int e = e0 + lane;
+        // (the estimate is within one for boxes below 2^23 cells a row)
+        int row = (int)(((float)e + 0.5f) * inv_bw);
+        if (row * w.bw > e) --row;
+        if ((row + 1) * w.bw <= e) ++row;
+        const int k0 = w.lo0 + row, k1 = w.lo1 + (e - row * w.bw);
+        bool hit = false;
+        if (e < nc) {
+          float dc[K], base[K], step[K];
+          dc[0] = (__ldg(g.ax[0].coords + k0) - w.a.x) - w.a.y;
+          dc[1] = (__ldg(g.ax[1].coords + k1) - w.a.z) - w.a.w;
+          hit = psf_cell_kind<K>(q, dc, s, base, step) != 0;
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, hit);
+        if (hit) queue[queued + __popc(m & ((1u << lane) - 1u))] = make_int2(k0 << 3 | sl, k1);
+        queued += __popc(m);
+        __syncwarp();
+        if (queued >= 32) {
+          add_cells(32);
+          queued -= 32;
+          const int2 left = queue[32 + lane];
+          __syncwarp();
+          if (lane < queued) queue[lane] = left;
+          __syncwarp();
+        }
+      }
+    }
+    if (queued) add_cells(queued);
+    if (on) {
+      const float *v = sum[lane];
+      f += v[0];
+      float Sa[NPSI], Ta[NPSI][NPSI], Ub[NPSI][NPSI];
+#pragma unroll
+      for (int k = 0; k < NPSI; ++k) Sa[k] = v[1 + k];
+      if constexpr (ORDER > 1) {
+        int o = 1 + NPSI;
+#pragma unroll
+        for (int k = 0; k < NPSI; ++k)
+#pragma unroll
+          for (int l = k; l < NPSI; ++l, ++o) {
+            Ta[k][l] = Ta[l][k] = v[o];
+            Ub[k][l] = Ub[l][k] = v[NT + o];
+          }
+      }
+      accumulate_pair<K, ORDER>(p, fr, I, Sa, Ta, Ub, gacc, hacc);
+    }
+    __syncwarp();
   }
 
-  float vals_f = f;
-  float gv[P];
+  if (lane < kPsfPairs) {
+    vals[pr][0] = f;
 #pragma unroll
-  for (int i = 0; i < P; ++i) gv[i] = gacc[i].get();
-  for (int off = cfg.ag; off < 32; off <<= 1) {
-    vals_f += __shfl_xor_sync(0xffffffffu, vals_f, off);
-#pragma unroll
-    for (int i = 0; i < P; ++i) gv[i] += __shfl_xor_sync(0xffffffffu, gv[i], off);
+    for (int i = 0; i < P; ++i) vals[pr][1 + i] = gacc[i].get();
     if constexpr (ORDER > 1) {
 #pragma unroll
-      for (int i = 0; i < NH; ++i) hacc[i] += __shfl_xor_sync(0xffffffffu, hacc[i], off);
+      for (int i = 0; i < NH; ++i) vals[pr][1 + P + i] = hacc[i];
     }
   }
-  if (!valid || sub != 0) return;
-  const size_t N = at.n;
-  float *dst = part + (size_t)chunk * cfg.qn * N + j;
-  dst[0] = vals_f;
-#pragma unroll
-  for (int i = 0; i < P; ++i) dst[(1 + i) * N] = gv[i];
-  if constexpr (ORDER > 1) {
-#pragma unroll
-    for (int i = 0; i < NH; ++i) dst[(1 + P + i) * N] = hacc[i];
-  }
+  __syncthreads();
+  psf_close<QN>(vals, at.n, cfg, chunk, wa, part);
 }
 
 // Sum chunk partials (FP64), expand the packed Hessian and apply the isotropic
@@ -1156,16 +1446,16 @@ int launch_derivs(const Atoms &at, const Geom &g, const DerivIn &in,
     fe = f_extra;
   }
   const int warps = ((at.n + c.ag - 1) / c.ag) * c.nchunks;
-  const int blocks = (warps + 3) / 4;       // (pixel-integrated operator)
-  const float s = 0.5f / g.ax[0].inv_step;  // its cell half-width
+  const float s = 0.5f / g.ax[0].inv_step;  // cell half-width (pixel-integrated operator)
   timer_mark(2, 0, stream);
   if (in.psf) {
+    constexpr int T1 = 32 * kPsfLanes, T2 = 32 * kPsfWarps;
     if (K == 1) {
-      if (in.order == 1) gr_psf_deriv_kernel<1, 1><<<blocks, 128, 0, stream>>>(at, g, in, c, part, s);
-      else gr_psf_deriv_kernel<1, 2><<<blocks, 128, 0, stream>>>(at, g, in, c, part, s);
+      if (in.order == 1) gr_psf_deriv1d_kernel<1><<<warps, T1, 0, stream>>>(at, g, in, c, part, s);
+      else gr_psf_deriv1d_kernel<2><<<warps, T1, 0, stream>>>(at, g, in, c, part, s);
     } else {
-      if (in.order == 1) gr_psf_deriv_kernel<2, 1><<<blocks, 128, 0, stream>>>(at, g, in, c, part, s);
-      else gr_psf_deriv_kernel<2, 2><<<blocks, 128, 0, stream>>>(at, g, in, c, part, s);
+      if (in.order == 1) gr_psf_deriv_kernel<1><<<warps, T2, 0, stream>>>(at, g, in, c, part, s);
+      else gr_psf_deriv_kernel<2><<<warps, T2, 0, stream>>>(at, g, in, c, part, s);
     }
   } else {
     // at most one angle per lane: a lane's angles a_lo + sub + k sg lie
@@ -1251,8 +1541,8 @@ static int preload_walk() {
 
 int preload_derivs() {
   return preload_walk<1>() + preload_walk<2>() +
-         preload_fn(gr_psf_deriv_kernel<1, 1>) + preload_fn(gr_psf_deriv_kernel<1, 2>) +
-         preload_fn(gr_psf_deriv_kernel<2, 1>) + preload_fn(gr_psf_deriv_kernel<2, 2>) +
+         preload_fn(gr_psf_deriv1d_kernel<1>) + preload_fn(gr_psf_deriv1d_kernel<2>) +
+         preload_fn(gr_psf_deriv_kernel<1>) + preload_fn(gr_psf_deriv_kernel<2>) +
          preload_fn(gr_deriv_finalize_kernel<1>) + preload_fn(gr_deriv_finalize_kernel<2>) +
          preload_fn(gr_sumsq_kernel) + preload_fn(gr_sumsq_finalize_kernel) +
          preload_fn(gr_batch_deriv_kernel) + preload_fn(gr_batch_finalize_kernel);

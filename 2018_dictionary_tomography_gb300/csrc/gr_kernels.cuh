@@ -11,11 +11,6 @@ constexpr int kProjWarps = 4;        // warps per CTA (2D and pixel-integrated)
 constexpr int kTileDim0 = 32;        // 3D tile rows (detector axis 0)
 constexpr int kTileDim1 = 32;        // 3D tile cols (detector axis 1, contiguous)
 constexpr int kTile1D = 32;          // 2D tile length (one cell per lane)
-constexpr int kTileCells = 1024;     // shared-memory cell sums per warp
-constexpr int kListWords = 16;       // bitmap words compacted per pass
-constexpr int kProjWarpFloats =
-    2 * kTileCells + 64 + kTileDim1 + kListWords * 32;
-
 // Parameters of a per-atom regulariser (gr_reg.cu).
 struct RegParams {
   double p[8];

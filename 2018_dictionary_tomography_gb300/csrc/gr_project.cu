@@ -749,166 +749,184 @@ __global__ void __launch_bounds__(128) gr_psf_bin_kernel(Atoms at, Geom g, TileC
   }
 }
 
-struct PsfLite {
-  float qh0, ql0, qh1, ql1, G0, G1, G2, l2amp, sgn, rr, total;
-  int lo0, hi0, lo1, hi1;
+// A block per (angle, tile): its atoms, in index order, go round its four
+// warps.  A warp's lanes look over an atom's cell box clipped to the tile and
+// queue the cells it reaches; 32 queued cells at a time, of as many atoms as
+// that takes, get their value by the quadrature rule (121 exponentials, what
+// bounds it) and go into the warp's own compensated sums in shared memory,
+// those of one cell in atom order; a cell then adds the four sums in warp order
+// (deterministic).  128 atoms x 401 x 64^2: 138 us with a warp per tile of 32 x
+// 32 cells, 109 us with four, 15 of 32 lanes at work; with the queue 65 us.
+struct PsfStage {
+  float4 a, b;   // qh0 ql0 qh1 ql1; G00 G01 G11 log2 amplitude
+  float4 c;      // sign of I, rr, total mass
+  int4 box;      // first and last cell along each axis, clipped to the tile
 };
+constexpr int kPsfTileWarps = 4;
+constexpr int kPsfList = 256;  // atoms listed at a time (8 bitmap words)
+static_assert(kTileDim0 <= 32 && kTileDim1 <= 32, "a queued cell's row and column: 5 bits each");
 
-__device__ __forceinline__ PsfLite shfl_psf(const PsfLite &v, int src) {
-  PsfLite o;
-  const unsigned m = 0xffffffffu;
-  o.qh0 = __shfl_sync(m, v.qh0, src);
-  o.ql0 = __shfl_sync(m, v.ql0, src);
-  o.qh1 = __shfl_sync(m, v.qh1, src);
-  o.ql1 = __shfl_sync(m, v.ql1, src);
-  o.G0 = __shfl_sync(m, v.G0, src);
-  o.G1 = __shfl_sync(m, v.G1, src);
-  o.G2 = __shfl_sync(m, v.G2, src);
-  o.l2amp = __shfl_sync(m, v.l2amp, src);
-  o.sgn = __shfl_sync(m, v.sgn, src);
-  o.rr = __shfl_sync(m, v.rr, src);
-  o.total = __shfl_sync(m, v.total, src);
-  o.lo0 = __shfl_sync(m, v.lo0, src);
-  o.hi0 = __shfl_sync(m, v.hi0, src);
-  o.lo1 = __shfl_sync(m, v.lo1, src);
-  o.hi1 = __shfl_sync(m, v.hi1, src);
-  return o;
-}
+// words a warp's staging and sums take (rows x cols cells)
+__host__ __device__ constexpr int psf_warp_words(int cells) { return 2 * cells + 32 * 16; }
 
-// Warp per (angle, tile), atoms in index order from the bitmap, lanes spread
-// over each atom's cell box clipped to the tile, each cell's value by the
-// quadrature rule; compensated shared-memory cell sums (deterministic).
 template <int K>
-__global__ void __launch_bounds__(kProjWarps * 32)
+__global__ void __launch_bounds__(kPsfTileWarps * 32, 8)
     gr_psf_project_kernel(Atoms at, Geom g, TileCfg tc, const uint32_t *bitmap, int W,
-                          float s, ProjOut out) {
-  extern __shared__ float smem[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int item = blockIdx.x * kProjWarps + warp;
-  if (item >= g.n_angles * tc.ntiles) return;
+                          float s, ProjOut out, double *loss_out, int *done) {
+  extern __shared__ __align__(16) float smem[];
+  __shared__ int list[kPsfList];
+  __shared__ float pc0[kTileDim0], pc1[kTileDim1];
+  __shared__ float2 s_loss[kPsfTileWarps * 32];
+  __shared__ uint32_t s_queue[kPsfTileWarps][64];
+  __shared__ int s_last;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  uint32_t *queue = s_queue[warp];
+  const int item = blockIdx.x, n_items = g.n_angles * tc.ntiles;
   const int cells = tc.t0 * tc.t1;
-  float *acc = smem + (size_t)warp * kProjWarpFloats;
-  float *cmp = acc + kTileCells;
-  float *pc0 = cmp + kTileCells;
-  float *pc1 = pc0 + 64;
-  int *list = reinterpret_cast<int *>(pc1 + kTileDim1);
-  const int a = item / tc.ntiles, t = item - a * tc.ntiles;
-  const int tr = t / tc.nt1, tcix = t - tr * tc.nt1;
+  float *acc = smem + (size_t)warp * psf_warp_words(cells);
+  float *cmp = acc + cells;
+  PsfStage *stage = reinterpret_cast<PsfStage *>(cmp + cells);  // (cells: a multiple of 4)
+  const int a = tile_div(item, tc.ntiles, tc.inv_ntiles), t = item - a * tc.ntiles;
+  const int tr = tile_div(t, tc.nt1, tc.inv_nt1), tcix = t - tr * tc.nt1;
   const int r0 = tr * tc.t0, c0 = tcix * tc.t1;
   const int D0 = g.ax[0].n, D1 = (K == 1) ? 1 : g.ax[1].n;
-  for (int e = lane; e < cells; e += 32) {
-    acc[e] = 0.f;
-    cmp[e] = 0.f;
-  }
-  for (int e = lane; e < tc.t0; e += 32)
-    pc0[e] = (r0 + e < D0) ? g.ax[0].coords[r0 + e] : 0.f;
+  for (int e = lane; e < 2 * cells; e += 32) acc[e] = 0.f;
+  if (tid < tc.t0) pc0[tid] = (r0 + tid < D0) ? g.ax[0].coords[r0 + tid] : 0.f;
   if constexpr (K == 2)
-    for (int e = lane; e < tc.t1; e += 32)
-      pc1[e] = (c0 + e < D1) ? g.ax[1].coords[c0 + e] : 0.f;
-  Frame<K> f;
-  load_frame<K>(g.frames, a, f);
-  __syncwarp();
+    if (tid < tc.t1) pc1[tid] = (c0 + tid < D1) ? g.ax[1].coords[c0 + tid] : 0.f;
   const uint32_t *words = bitmap + (size_t)item * W;
-  for (int wb = 0; wb < W; wb += kListWords) {
-    const int wi = wb + (lane < kListWords ? lane : 0);
-    uint32_t wd = (lane < kListWords && wi < W) ? words[wi] : 0u;
-    int cnt = __popc(wd), incl = cnt;
+  for (int wb = 0; wb < W; wb += 8) {
+    // list 8 words' atoms (the first warp), then deal them out
+    __syncthreads();
+    int total = 0;
+    {
+      uint32_t wd = lane < 8 && wb + lane < W ? words[wb + lane] : 0u;
+      const int cnt = __popc(wd);
+      int incl = cnt;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      int v = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += v;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+      }
+      total = __shfl_sync(0xffffffffu, incl, 31);
+      if (warp == 0) {
+        int pos = incl - cnt;
+        while (wd) {
+          list[pos++] = ((wb + lane) << 5) + (__ffs(wd) - 1);
+          wd &= wd - 1;
+        }
+      }
     }
-    const int total = __shfl_sync(0xffffffffu, incl, 31);
-    int pos = incl - cnt;
-    while (wd) {
-      const int b = __ffs(wd) - 1;
-      list[pos++] = (wi << 5) + b;
-      wd &= wd - 1;
-    }
-    __syncwarp();
-    for (int bs = 0; bs < total; bs += 32) {
-      const int idx = bs + lane;
-      PsfLite mine{};
-      mine.lo0 = 1;
-      mine.hi0 = 0;
-      mine.lo1 = 1;
-      mine.hi1 = 0;
-      if (idx < total) {
-        const int j = list[idx];
+    __syncthreads();
+    const int mine = (total - warp + kPsfTileWarps - 1) / kPsfTileWarps;   // entries warp, warp + 4, ..
+    for (int bs = 0; bs < mine; bs += 32) {
+      const int nb = min(32, mine - bs);
+      if (lane < nb) {
+        const int j = list[warp + kPsfTileWarps * (bs + lane)];
+        Frame<K> f;
+        load_frame<K>(g.frames, a, f);
         Pair<K> p;
         const bool ok = pair_setup<K>(at, j, f, g, p);
         PsfPair<K> q;
         psf_setup<K>(at, j, g, p, ok, s, q);
-        mine.qh0 = p.qh[0];
-        mine.ql0 = p.ql[0];
-        mine.G0 = p.G[0];
-        mine.G1 = p.G[1];
-        mine.G2 = p.G[2];
-        mine.l2amp = p.l2amp;
-        mine.sgn = p.sgn;
-        mine.rr = q.rr;
-        mine.total = q.total;
-        mine.lo0 = max(q.lo[0], r0);
-        mine.hi0 = min(q.hi[0], r0 + tc.t0 - 1);
-        if constexpr (K == 2) {
-          mine.qh1 = p.qh[1];
-          mine.ql1 = p.ql[1];
-          mine.lo1 = max(q.lo[1], c0);
-          mine.hi1 = min(q.hi[1], c0 + tc.t1 - 1);
-        } else {
-          mine.lo1 = 0;
-          mine.hi1 = 0;
-        }
+        PsfStage st;
+        st.a = make_float4(p.qh[0], p.ql[0], K == 2 ? p.qh[K - 1] : 0.f, K == 2 ? p.ql[K - 1] : 0.f);
+        st.b = make_float4(p.G[0], p.G[1], p.G[2], p.l2amp);
+        st.c = make_float4(p.sgn, q.rr, q.total, 0.f);
+        st.box = make_int4(max(q.lo[0], r0), min(q.hi[0], r0 + tc.t0 - 1),
+                           K == 2 ? max(q.lo[K - 1], c0) : 0,
+                           K == 2 ? min(q.hi[K - 1], c0 + tc.t1 - 1) : 0);
+        stage[lane] = st;
       }
-      const int nb = min(32, total - bs);
-      for (int s2 = 0; s2 < nb; ++s2) {
-        const PsfLite qq = shfl_psf(mine, s2);
-        if (qq.lo0 > qq.hi0 || qq.lo1 > qq.hi1) continue;
+      __syncwarp();
+      // the values of the first n queued cells, into the sums
+      auto add_cells = [&](int n) {
+        const bool on = lane < n;
+        const uint32_t it = queue[on ? lane : 0];
+        const int slot = it & 31, lr = (it >> 5) & 31, lc = it >> 10;
+        const float4 qa = stage[slot].a, qb = stage[slot].b, qc = stage[slot].c;
         Pair<K> p;
-        p.qh[0] = qq.qh0;
-        p.ql[0] = qq.ql0;
-        p.G[0] = qq.G0;
-        p.G[1] = qq.G1;
-        p.G[2] = qq.G2;
-        p.l2amp = qq.l2amp;
-        if constexpr (K == 2) {
-          p.qh[1] = qq.qh1;
-          p.ql[1] = qq.ql1;
-        }
+        p.G[0] = qb.x;
+        p.G[1] = qb.y;
+        p.G[2] = qb.z;
+        p.l2amp = qb.w;
         PsfPair<K> q;
-        q.rr = qq.rr;
-        q.total = qq.total;
-        const int bw = qq.hi1 - qq.lo1 + 1;
-        const int ncell = (qq.hi0 - qq.lo0 + 1) * bw;
-        const float inv_bw = 1.f / (float)bw;
-        for (int e = lane; e < ncell; e += 32) {
-          const int rr_ = (int)(((float)e + 0.5f) * inv_bw);
-          const int cc = e - rr_ * bw;
-          const int lr = qq.lo0 - r0 + rr_;
-          const int lc = (K == 2) ? (qq.lo1 - c0 + cc) : 0;
-          float dc[K], base[K], step[K];
-          dc[0] = (pc0[lr] - qq.qh0) - qq.ql0;
-          if constexpr (K == 2) dc[1] = (pc1[lc] - qq.qh1) - qq.ql1;
-          const int kind = psf_cell_kind<K>(q, dc, s, base, step);
-          if (kind == 0) continue;
-          const float v = kind == 1 ? qq.total : qq.sgn * psf_quadrature<K>(p, base, step);
-          const int ci = lr * tc.t1 + lc;
-          const float s0 = acc[ci];
-          const float tt = s0 + v;
-          cmp[ci] += (fabsf(s0) >= fabsf(v)) ? ((s0 - tt) + v) : ((v - tt) + s0);
-          acc[ci] = tt;
+        q.rr = qc.y;
+        float dc[K], base[K], step[K];
+        dc[0] = (pc0[lr] - qa.x) - qa.y;
+        if constexpr (K == 2) dc[1] = (pc1[lc] - qa.z) - qa.w;
+        const int kind = psf_cell_kind<K>(q, dc, s, base, step);
+        float v = qc.z;
+        if (kind == 2) v = qc.x * psf_quadrature<K>(p, base, step);
+        const int ci = lr * tc.t1 + lc;
+        const unsigned same = __match_any_sync(0xffffffffu, on ? ci : -1 - lane);
+        const int rank = __popc(same & ((1u << lane) - 1u));
+        const int ranks = __reduce_max_sync(0xffffffffu, rank);
+        for (int k = 0; k <= ranks; ++k) {
+          if (on && rank == k) {
+            const float s0 = acc[ci];
+            const float tt = s0 + v;
+            cmp[ci] += (fabsf(s0) >= fabsf(v)) ? ((s0 - tt) + v) : ((v - tt) + s0);
+            acc[ci] = tt;
+          }
+          __syncwarp();
         }
-        __syncwarp();
+      };
+      int queued = 0;
+      for (int s2 = 0; s2 < nb; ++s2) {
+        const int4 box = stage[s2].box;
+        if (box.x > box.y || box.z > box.w) continue;
+        const float4 qa = stage[s2].a;
+        PsfPair<K> q;
+        q.rr = stage[s2].c.y;
+        const int bw = box.w - box.z + 1;
+        const int ncell = (box.y - box.x + 1) * bw;
+        const float inv_bw = 1.f / (float)bw;
+        for (int e0 = 0; e0 < ncell; e0 += 32) {
+          const int e = e0 + lane;
+          const int rr_ = (int)(((float)e + 0.5f) * inv_bw);
+          const int lr = box.x - r0 + rr_;
+          const int lc = (K == 2) ? (box.z - c0 + (e - rr_ * bw)) : 0;
+          bool hit = false;
+          if (e < ncell) {
+            float dc[K], base[K], step[K];
+            dc[0] = (pc0[lr] - qa.x) - qa.y;
+            if constexpr (K == 2) dc[1] = (pc1[lc] - qa.z) - qa.w;
+            hit = psf_cell_kind<K>(q, dc, s, base, step) != 0;
+          }
+          const unsigned m = __ballot_sync(0xffffffffu, hit);
+          if (hit)
+            queue[queued + __popc(m & ((1u << lane) - 1u))] =
+                (uint32_t)s2 | (uint32_t)lr << 5 | (uint32_t)lc << 10;
+          queued += __popc(m);
+          __syncwarp();
+          if (queued >= 32) {
+            add_cells(32);
+            queued -= 32;
+            const uint32_t left = queue[32 + lane];
+            __syncwarp();
+            if (lane < queued) queue[lane] = left;
+            __syncwarp();
+          }
+        }
       }
+      if (queued) add_cells(queued);
     }
   }
-  __syncwarp();
+  __syncthreads();
   float lsum = 0.f, lcmp = 0.f;
-  for (int e = lane; e < cells; e += 32) {
+  for (int e = tid; e < cells; e += kPsfTileWarps * 32) {
     const int lr = e / tc.t1, lc = e - lr * tc.t1;
     const int row = r0 + lr, col = c0 + lc;
     if (row >= D0 || col >= D1) continue;
-    const float v = acc[e] + cmp[e];
+    // the warps' sums in warp order
+    float sv = 0.f, cv = 0.f;
+#pragma unroll
+    for (int w = 0; w < kPsfTileWarps; ++w) {
+      const float *aw = smem + (size_t)w * psf_warp_words(cells);
+      pair_add(sv, cv, aw[e], aw[cells + e]);
+    }
+    const float v = sv + cv;
     const size_t gi = ((size_t)a * D0 + row) * D1 + col;
     if (out.R) out.R[gi] = v;
     float l = 0.f;
@@ -928,10 +946,28 @@ __global__ void __launch_bounds__(kProjWarps * 32)
     lcmp += (fabsf(lsum) >= fabsf(l)) ? ((lsum - tt) + l) : ((l - tt) + lsum);
     lsum = tt;
   }
-  if (out.loss_part) {
-    double d = warp_sum_d((double)lsum + (double)lcmp);
-    if (lane == 0) out.loss_part[item] = d;
+  if (!out.loss_part) return;
+  s_loss[tid] = make_float2(lsum, lcmp);
+  __syncthreads();
+  if (warp == 0) {
+#pragma unroll
+    for (int w = 1; w < kPsfTileWarps; ++w)
+      pair_add(lsum, lcmp, s_loss[32 * w + lane].x, s_loss[32 * w + lane].y);
+    pair_warp_sum(lsum, lcmp);
+    if (lane == 0) {
+      out.loss_part[item] = (double)lsum + (double)lcmp;
+      if (loss_out) {
+        __threadfence();
+        s_last = atomicAdd(done, 1) == n_items - 1;
+      }
+    }
   }
+  if (!loss_out) return;
+  __syncthreads();
+  if (!s_last) return;
+  // the last block to finish sums the items' partials in item order
+  __threadfence();
+  sum_partials_block<kPsfTileWarps>(out.loss_part, n_items, loss_out);
 }
 
 // Fixed-order FP64 sum of n loss partials over many blocks (one block's FP64
@@ -1090,7 +1126,7 @@ int launch_project(const Atoms &at, const Geom &g, const ProjOut &o_in,
   const bool wide4 = K == 1 && !o_in.psf && form == 3;
   TileCfg tc = make_tiles(K, D0, D1,
                           K == 1 ? (wide4 ? 4 * kTile1D : wide2d ? 2 * kTile1D : kTile1D)
-                                 : (!o_in.psf ? proj_rows(form) : kTileDim0));
+                                 : proj_rows(form));
   const int W = (at.n + 31) / 32;
   const size_t items = (size_t)g.n_angles * tc.ntiles;
   const size_t need = project_min_bytes(K, at.n, g.n_angles, D0, D1, t);
@@ -1151,11 +1187,11 @@ int launch_project(const Atoms &at, const Geom &g, const ProjOut &o_in,
     }
     note_launches(1);
   }
-  const int blocks = (int)((items + kProjWarps - 1) / kProjWarps);
-  const size_t smem = (size_t)kProjWarps * kProjWarpFloats * sizeof(float);
-  // smem (kProjWarps * kProjWarpFloats floats) stays below the 48 KB that
-  // needs no opt-in, so no function attribute is set (safe under capture)
-  static_assert(kProjWarps * kProjWarpFloats * sizeof(float) <= 48 * 1024, "smem");
+  // below the 48 KB that needs no opt-in, so no function attribute is set (safe
+  // under capture)
+  const size_t smem = (size_t)kPsfTileWarps * psf_warp_words(tc.t0 * tc.t1) * sizeof(float);
+  static_assert(kPsfTileWarps * psf_warp_words(kTileDim0 * kTileDim1) * sizeof(float) <= 42 * 1024,
+                "smem");
   bool fused_loss = false;
   if (point3) {
     // records: as many angles at a time as the workspace holds; a skipping
@@ -1204,10 +1240,14 @@ int launch_project(const Atoms &at, const Geom &g, const ProjOut &o_in,
   } else {
     timer_mark(1, 0, stream);
     if (o.psf) {
+      fused_loss = loss_out != nullptr && items <= kFusedLossItems;
+      double *lo = fused_loss ? loss_out : nullptr;
       if (K == 1)
-        gr_psf_project_kernel<1><<<blocks, kProjWarps * 32, smem, stream>>>(at, g, tc, bitmap, W, psf_s, o);
+        gr_psf_project_kernel<1><<<(unsigned)items, kPsfTileWarps * 32, smem, stream>>>(
+            at, g, tc, bitmap, W, psf_s, o, lo, next_item + 1);
       else
-        gr_psf_project_kernel<2><<<blocks, kProjWarps * 32, smem, stream>>>(at, g, tc, bitmap, W, psf_s, o);
+        gr_psf_project_kernel<2><<<(unsigned)items, kPsfTileWarps * 32, smem, stream>>>(
+            at, g, tc, bitmap, W, psf_s, o, lo, next_item + 1);
     } else {
       // one block per (angle, tile) item; for up to kFusedLossItems tiles the
       // last block also sums the loss partials (no separate finalize launch)
