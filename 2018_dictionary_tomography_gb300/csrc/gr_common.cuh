@@ -38,6 +38,12 @@ __device__ __forceinline__ float ex2_approx(float v) {
   return y;
 }
 
+__device__ __forceinline__ float sqrt_approx(float v) {
+  float y;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(v));
+  return y;
+}
+
 __device__ __forceinline__ float lg2_approx(float v) {
   float y;
   asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(v));
@@ -176,6 +182,37 @@ __device__ __forceinline__ void load_frame(const float *frames, int a,
   f.wl = p + D * (1 + 2 * K);
 }
 
+// A warp's 3D frames in shared memory: lanes of a warp take different angles, and
+// a lane's own 24 loads, 96 bytes from its neighbour's, touch 24 lines each; the
+// records are one run of memory, so the warp copies them 16 bytes a lane.
+struct FrameSmem {
+  static constexpr int kStride = kFrameStride3D + 4;  // 8 lanes' 16-byte reads: all banks
+  float4 v[32][kStride / 4];
+};
+
+// the n <= 32 records from `frames` on (the caller synchronises the warp)
+__device__ __forceinline__ void stage_frames(FrameSmem &sm, const float *frames, int n) {
+  constexpr int Q = kFrameStride3D / 4;
+  const int lane = threadIdx.x & 31;
+  if ((reinterpret_cast<size_t>(frames) & 15) == 0) {
+    for (int i = lane; i < n * Q; i += 32)
+      sm.v[i / Q][i % Q] = __ldg(reinterpret_cast<const float4 *>(frames) + i);
+  } else {
+    for (int i = lane; i < n * kFrameStride3D; i += 32)
+      reinterpret_cast<float *>(sm.v[i / kFrameStride3D])[i % kFrameStride3D] = __ldg(frames + i);
+  }
+}
+
+__device__ __forceinline__ void load_frame(const FrameSmem &sm, int i, Frame<2> &f) {
+  const float4 a = sm.v[i][0], b = sm.v[i][1], c = sm.v[i][2], d = sm.v[i][3];
+  f.T[0] = a.x, f.T[1] = a.y, f.T[2] = a.z;
+  f.w[0][0] = a.w, f.w[0][1] = b.x, f.w[0][2] = b.y;
+  f.w[1][0] = b.z, f.w[1][1] = b.w, f.w[1][2] = c.x;
+  f.wt[0][0] = c.y, f.wt[0][1] = c.z, f.wt[0][2] = c.w;
+  f.wt[1][0] = d.x, f.wt[1][1] = d.y, f.wt[1][2] = d.z;
+  f.wl = reinterpret_cast<const float *>(sm.v[i]) + 15;
+}
+
 // Upper-triangular r as a dense (K+1)x(K+1) matrix.
 template <int K>
 __device__ __forceinline__ void load_r(const Atoms &at, int j,
@@ -233,7 +270,8 @@ struct Pair {
   float Q[K + 1][K + 1];   // Q[c][d] = Kc[c] . Kc[d]
 };
 
-template <int K>
+// STAGED: the frame was read from shared memory (load_frame of a FrameSmem).
+template <int K, bool STAGED = false>
 __device__ __forceinline__ bool pair_setup(const Atoms &at, int j,
                                            const Frame<K> &f, const Geom &g,
                                            Pair<K> &p) {
@@ -305,7 +343,13 @@ __device__ __forceinline__ bool pair_setup(const Atoms &at, int j,
     float hi, lo;
     dot2<D>(f.wt[k], xv, hi, lo);
 #pragma unroll
-    for (int a = 0; a < D; ++a) lo = fmaf(__ldg(f.wl + k * D + a), xv[a], lo);
+    for (int a = 0; a < D; ++a) {
+      // (a staged frame's residues lie in shared memory: no read-only load)
+      float w;
+      if constexpr (STAGED) w = f.wl[k * D + a];
+      else w = __ldg(f.wl + k * D + a);
+      lo = fmaf(w, xv[a], lo);
+    }
     two_sum(hi, lo, p.qh[k], p.ql[k]);
   }
 

@@ -49,7 +49,12 @@ __host__ __device__ constexpr int hess_min_warps(int K, bool one) {
 // atoms per warp the lanes of a warp take different angles of one atom, whose
 // support boxes are of similar size, so fewer lanes idle.  Automatic: one
 // atom per warp for Hessians and for long angle series, else four (so each
-// lane still has a few angles to amortise the warp's closing reduction).
+// lane still has a few angles to amortise the warp's closing reduction).  A 3D
+// gradient has a cheap closing reduction for one atom, so there a series is long
+// from two angles per lane on (fewer would leave lanes idle): 4096 atoms x 121 x
+// 256^2: 63.7 us and 4.1 to sum the chunks, against 71.8 and 6.6 with four; 1000
+// x 1001 x 95^2: 89.4 + 4.5 against 98.0 + 13.7.  (The pixel-integrated kernel
+// keeps the longer line: 66 us with four, 76 with one at 128 x 401 x 64^2.)
 // deriv_split_lanes: problems with few (atom, angle) pairs give a warp 32 / rs
 // of them, rs the largest power of two up to 8 with pairs * rs <=
 // deriv_split_lanes, so that the pairs spread over more warps (a 3D gradient's
@@ -64,7 +69,7 @@ DerivCfg deriv_cfg(int K, int n_atoms, int n_angles, int order, const Tuning &t,
   DerivCfg c;
   c.ag = next_pow2(n_atoms < 1 ? 1 : n_atoms);
   const int ag_cap = t.deriv_atoms_per_warp > 0 ? t.deriv_atoms_per_warp
-                     : (order > 1 || n_angles >= 1024) ? 1 : 4;
+                     : (order > 1 || n_angles >= (K == 2 && split ? 64 : 1024)) ? 1 : 4;
   if (c.ag > ag_cap) c.ag = ag_cap;
   c.sg = 32 / c.ag;
   const long long pairs = (long long)(n_atoms < 1 ? 1 : n_atoms) * (n_angles < 1 ? 1 : n_angles);
@@ -506,110 +511,180 @@ __global__ void __launch_bounds__(32, hess_min_warps(K, ONE))
 
 // ---- gradients: a lane per pair ------------------------------------------------
 // A lane walks its pair's support alone: in 2D its cells, in 3D the rows of its
-// ellipse, in chunks of CH cells whose field values are loaded together.  A 3D
-// pair holds 20 to 40 cells, which groups of 2, 4 or 8 lanes per pair, as the
-// Hessians use, pad to 56 to 87 lane steps: 21.4, 21.2 and 24.5 against 17.4 ms
-// on 8192 atoms x 20000 orientations.  The loads bound it: 32 lanes touch 32
-// lines of the field, one L1 tag each.
-template <int K, int CH>
-__device__ __forceinline__ void lane_moments(const Pair<K> &p, const Geom &g, const DerivIn &in, int a,
-                                             float I, float (&Ma)[n_mom<K, 2>()], float &X0,
-                                             float &Y0, int phase, int rs) {
-  constexpr int NM = n_mom<K, 2>();
+// ellipse.  A 3D pair holds 20 to 40 cells, which groups of 2, 4 or 8 lanes per
+// pair, as the Hessians use, pad to 56 to 87 lane steps: 21.4, 21.2 and 24.5
+// against 17.4 ms on 8192 atoms x 20000 orientations of 128^2.
+//
+// 2D: cells in chunks of CH, whose field values are loaded together.
+template <int CH>
+__device__ __forceinline__ void lane_cells(const Pair<1> &p, const Geom &g, const DerivIn &in, int a,
+                                           float I, float (&Ma)[n_mom<1, 2>()], float &X0,
+                                           float &Y0, int phase, int rs) {
+  constexpr int NM = n_mom<1, 2>();
 #pragma unroll
   for (int i = 0; i < NM; ++i) Ma[i] = 0.f;
   X0 = 0.f;
   Y0 = 0.f;
   if (p.lo[0] > p.hi[0]) return;
-  if constexpr (K == 2)
-    if (p.lo[1] > p.hi[1]) return;
   const float l2n = lg2_approx(p.n);
-  const int D0 = g.ax[0].n, D1 = K == 2 ? g.ax[1].n : 1;
-  const float *__restrict__ field = in.alpha;
-  const size_t abase = (size_t)a * D0 * D1;
-  // a cell's term: m its form, d its offset along the walk, c its field value
-  auto cell = [&](float m, float d, float c, float *S) {
+  const float *__restrict__ field = in.alpha + (size_t)a * g.ax[0].n;
+  // a cell's term: m its form, d its offset, c its field value
+  auto cell = [&](float m, float d, float c) {
     if (m <= 1.f) {
       const float E = ex2_approx(fmaf(m, kNegThirtyLog2e, l2n));
       const float al = (in.mode == kModeL2Atom) ? fmaf(I, E, -c) : c;
       const float w = al * E;
-      S[0] += w;
-      S[1] = fmaf(w, d, S[1]);
-      S[2] = fmaf(w, d * d, S[2]);
+      Ma[0] += w;
+      Ma[1] = fmaf(w, d, Ma[1]);
+      Ma[2] = fmaf(w, d * d, Ma[2]);
       if (in.mode == kModeL2Atom) {
         X0 = fmaf(E, c, X0);
         Y0 = fmaf(E, E, Y0);
       }
     }
   };
-  if constexpr (K == 1) {
-    const int c_hi = p.hi[0];
-    for (int kb = p.lo[0] + phase * CH; kb <= c_hi; kb += rs * CH) {
-      float cv[CH], pv[CH];
+  const int c_hi = p.hi[0];
+  for (int kb = p.lo[0] + phase * CH; kb <= c_hi; kb += rs * CH) {
+    float cv[CH], pv[CH];
 #pragma unroll
-      for (int i = 0; i < CH; ++i) {
-        const int k0 = min(kb + i, c_hi);
-        cv[i] = __ldg(field + abase + k0);
-        pv[i] = __ldg(g.ax[0].coords + k0);
-      }
-#pragma unroll
-      for (int i = 0; i < CH; ++i) {
-        if (kb + i > c_hi) break;
-        const float d0 = (pv[i] - p.qh[0]) - p.ql[0];
-        cell(p.G[0] * d0 * d0, d0, cv[i], Ma);
-      }
+    for (int i = 0; i < CH; ++i) {
+      const int k0 = min(kb + i, c_hi);
+      cv[i] = __ldg(field + k0);
+      pv[i] = __ldg(g.ax[0].coords + k0);
     }
-  } else {
-    // per row, m <= 1 holds for d1 within hw(d0) = sqrt(G2 - d0^2 det)/G2 of
-    // -G1 d0/G2: the row loop visits that range (widened like the support box)
-    // instead of the whole box; the m <= 1 test still decides every cell
-    const float det = p.G[0] * p.G[2] - p.G[1] * p.G[1];
-    const float iG2 = 1.f / p.G[2];
-    for (int k0 = p.lo[0] + phase; k0 <= p.hi[0]; k0 += rs) {
-      const float d0 = (__ldg(g.ax[0].coords + k0) - p.qh[0]) - p.ql[0];
-      const float t0 = p.G[0] * d0 * d0;
-      const float u = 2.f * p.G[1] * d0;
-      float Sa[3] = {0.f, 0.f, 0.f};
-      const size_t rbase = abase + (size_t)k0 * D1;
-      const float rem = fmaf(-d0 * d0, det, p.G[2]);
-      const float rc = (p.qh[1] - p.G[1] * d0 * iG2 - g.ax[1].first) * g.ax[1].inv_step;
-      const float rh = sqrtf(fmaxf(rem, 0.f)) * iG2 * g.ax[1].inv_step * 1.0001f + 1e-3f;
-      const float rlo = ceilf(rc - rh), rhi = floorf(rc + rh);
-      const int c_lo = (int)fminf(fmaxf(rlo, (float)p.lo[1]), (float)p.hi[1] + 1.f);
-      const int c_hi = (int)fmaxf(fminf(rhi, (float)p.hi[1]), (float)p.lo[1] - 1.f);
-      for (int kb = c_lo; kb <= c_hi; kb += CH) {
-        float cv[CH], pv[CH];
 #pragma unroll
-        for (int i = 0; i < CH; ++i) {
-          const int k1 = min(kb + i, c_hi);
-          cv[i] = __ldg(field + rbase + k1);
-          pv[i] = __ldg(g.ax[1].coords + k1);
-        }
-#pragma unroll
-        for (int i = 0; i < CH; ++i) {
-          if (kb + i > c_hi) break;
-          const float d1 = (pv[i] - p.qh[1]) - p.ql[1];
-          cell(fmaf(d1, fmaf(p.G[2], d1, u), t0), d1, cv[i], Sa);
-        }
-      }
-      float pw = 1.f;
-#pragma unroll
-      for (int i = 0; i <= 2; ++i) {
-#pragma unroll
-        for (int j = 0; j <= 2 - i; ++j) Ma[mi(i, j)] = fmaf(pw, Sa[j], Ma[mi(i, j)]);
-        pw *= d0;
-      }
+    for (int i = 0; i < CH; ++i) {
+      if (kb + i > c_hi) break;
+      const float d0 = (pv[i] - p.qh[0]) - p.ql[0];
+      cell(p.G[0] * d0 * d0, d0, cv[i]);
     }
   }
 }
 
-// ONE, one-warp blocks: as gr_hess_kernel.
-template <int K, bool ONE>
+// 3D: a row's cells in aligned fours of the field, two at a time in packed FP32
+// pairs.  The loads bound it: 32 lanes touch 32 lines of the field, one L1 tag
+// each, so a load takes 16 bytes a lane (a four of 4-byte loads took four times
+// the tags: 17.4 ms where this takes 13.5; a row's first four loaded a row ahead
+// costs registers: 15.4 to 16.3).  The m <= 1 test decides every
+// cell of a four; QUAD: rows begin on fours (D1 a multiple of four, both arrays
+// on 16 bytes), so a four lies in one row and its coordinates are one load too.
+// Otherwise fours are aligned in the whole field, and one that crosses an end of
+// its row loads the row's cells one by one.
+template <bool QUAD, bool L2ATOM>
+__device__ __forceinline__ void lane_rows(const Pair<2> &p, const Geom &g, const DerivIn &in, int a,
+                                          float I, float (&Ma)[n_mom<2, 2>()], float &X0,
+                                          float &Y0, int phase, int rs) {
+  constexpr int NM = n_mom<2, 2>();
+#pragma unroll
+  for (int i = 0; i < NM; ++i) Ma[i] = 0.f;
+  X0 = 0.f;
+  Y0 = 0.f;
+  if (p.lo[0] > p.hi[0] || p.lo[1] > p.hi[1]) return;
+  const float l2n = lg2_approx(p.n);
+  const int D0 = g.ax[0].n, D1 = g.ax[1].n;
+  const float *__restrict__ x0 = g.ax[0].coords, *__restrict__ x1 = g.ax[1].coords;
+  const float *__restrict__ field = in.alpha + (size_t)a * D0 * D1;
+  const F2 nqh = f2(-p.qh[1], -p.qh[1]), nql = f2(-p.ql[1], -p.ql[1]);
+  const F2 g2 = f2(p.G[2], p.G[2]), amp = f2(l2n, l2n);
+  // per row, m <= 1 holds for d1 within hw(d0) = sqrt(G2 - d0^2 det)/G2 of
+  // -G1 d0/G2: the walk visits that range (widened like the support box)
+  // instead of the whole box; the m <= 1 test still decides every cell
+  const float det = p.G[0] * p.G[2] - p.G[1] * p.G[1];
+  const float iG2 = 1.f / p.G[2];
+  const float rc0 = (p.qh[1] - g.ax[1].first) * g.ax[1].inv_step;
+  const float rcd = p.G[1] * iG2 * g.ax[1].inv_step;
+  const float rhs = iG2 * g.ax[1].inv_step * 1.0001f;
+  for (int k0 = p.lo[0] + phase; k0 <= p.hi[0]; k0 += rs) {
+    const float d0 = (__ldg(x0 + k0) - p.qh[0]) - p.ql[0];
+    const float t0 = p.G[0] * d0 * d0, u = 2.f * p.G[1] * d0;
+    const float rc = fmaf(-rcd, d0, rc0);
+    const float rh = fmaf(sqrt_approx(fmaxf(fmaf(-d0 * d0, det, p.G[2]), 0.f)), rhs, 1e-3f);
+    const int c_lo = (int)fminf(fmaxf(ceilf(rc - rh), (float)p.lo[1]), (float)p.hi[1] + 1.f);
+    const int c_hi = (int)fmaxf(fminf(floorf(rc + rh), (float)p.hi[1]), (float)p.lo[1] - 1.f);
+    if (c_lo > c_hi) continue;
+    const float *__restrict__ row = field + (size_t)k0 * D1;
+    const F2 t0p = f2(t0, t0), up = f2(u, u);
+    F2 S0 = f2(0.f, 0.f), S1 = S0, S2 = S0, X = S0, Y = S0;
+    // two cells: coordinates, field values, whether they are cells of the row
+    auto cells = [&](F2 x, F2 c, bool in0, bool in1) {
+      const F2 d = f2_add(f2_add(x, nqh), nql);
+      const F2 m = f2_fma(d, f2_fma(g2, d, up), t0p);
+      float m0, m1, e0, e1;
+      f2_get(m, m0, m1);
+      in0 = in0 && m0 <= 1.f;
+      in1 = in1 && m1 <= 1.f;
+      f2_get(f2_fma(m, f2(kNegThirtyLog2e, kNegThirtyLog2e), amp), e0, e1);
+      const F2 E = f2(ex2_approx(e0), ex2_approx(e1));
+      F2 al = c;
+      if (L2ATOM) al = f2_fma(f2(I, I), E, f2_mul(c, f2(-1.f, -1.f)));
+      // the product is cut off: a field value beyond the cut-off counts for
+      // nothing, also one that is not finite
+      const F2 w = f2_keep(f2_mul(al, E), in0, in1);
+      S0 = f2_add(S0, w);
+      const F2 wd = f2_mul(w, d);
+      S1 = f2_add(S1, wd);
+      S2 = f2_fma(wd, d, S2);
+      if (L2ATOM) {
+        X = f2_add(X, f2_keep(f2_mul(E, c), in0, in1));
+        Y = f2_add(Y, f2_keep(f2_mul(E, E), in0, in1));
+      }
+    };
+    if constexpr (QUAD) {
+      for (int kb = c_lo & ~3; kb <= c_hi; kb += 4) {
+        const float4 c = __ldg(reinterpret_cast<const float4 *>(row + kb));
+        const float4 x = __ldg(reinterpret_cast<const float4 *>(x1 + kb));
+        cells(f2(x.x, x.y), f2(c.x, c.y), true, true);
+        cells(f2(x.z, x.w), f2(c.z, c.w), true, true);
+      }
+    } else {
+      // cells before c_lo down to a 16-byte boundary
+      const int back = (int)((reinterpret_cast<size_t>(row + c_lo) >> 2) & 3);
+      for (int kb = c_lo - back; kb <= c_hi; kb += 4) {
+        if (kb >= 0 && kb + 4 <= D1) {
+          const float4 c = __ldg(reinterpret_cast<const float4 *>(row + kb));
+          const float *x = x1 + kb;
+          cells(f2(__ldg(x), __ldg(x + 1)), f2(c.x, c.y), true, true);
+          cells(f2(__ldg(x + 2), __ldg(x + 3)), f2(c.z, c.w), true, true);
+        } else {
+          // a four that crosses an end of the row: the row's cells only
+#pragma unroll
+          for (int i = 0; i < 4; i += 2) {
+            const int ka = kb + i, ia = min(max(ka, 0), D1 - 1), ib = min(max(ka + 1, 0), D1 - 1);
+            cells(f2(__ldg(x1 + ia), __ldg(x1 + ib)), f2(__ldg(row + ia), __ldg(row + ib)),
+                  ka == ia, ka + 1 == ib);
+          }
+        }
+      }
+    }
+    const float S[3] = {f2_sum(S0), f2_sum(S1), f2_sum(S2)};
+    if (L2ATOM) {
+      X0 += f2_sum(X);
+      Y0 += f2_sum(Y);
+    }
+    float pw = 1.f;
+#pragma unroll
+    for (int i = 0; i <= 2; ++i) {
+#pragma unroll
+      for (int j = 0; j <= 2 - i; ++j) Ma[mi(i, j)] = fmaf(pw, S[j], Ma[mi(i, j)]);
+      pw *= d0;
+    }
+  }
+}
+
+template <int K>
+struct FramesOf { using type = FrameSmem; };
+template <>
+struct FramesOf<1> { using type = int; };  // (2D: not used)
+
+// ONE, one-warp blocks: as gr_hess_kernel.  QUAD, L2ATOM: 3D only (2D reads the
+// mode from `in`).
+template <int K, bool ONE, bool QUAD, bool L2ATOM>
 __global__ void __launch_bounds__(32, 32)
     gr_grad_kernel(Atoms at, Geom g, DerivIn in, DerivCfg cfg, float *part) {
   constexpr int P = n_par<K>();
   constexpr int NM = n_mom<K, 2>();
   constexpr int NPSI = n_psi<K>();
+  __shared__ typename FramesOf<K>::type s_frames;
   const int gw = blockIdx.x, lane = threadIdx.x;
   const int warps_atoms = (at.n + cfg.ag - 1) / cfg.ag;
   const int chunk = gw / warps_atoms, wa = gw - chunk * warps_atoms;
@@ -629,13 +704,16 @@ __global__ void __launch_bounds__(32, 32)
   const int phase = sub & (cfg.rs - 1);
   unsigned gmask = 0u;
   for (int o = 0; o < cfg.rs; ++o) gmask |= 1u << (lane + (o - phase) * cfg.ag);
-  for (int a = a_lo + sub / cfg.rs; a < a_hi && valid; a += cfg.sg / cfg.rs) {
+  // angle a (3D: frame i of the staged)
+  auto add_pair = [&](int a, int i) {
     Frame<K> fr;
-    load_frame<K>(g.frames, a, fr);
+    if constexpr (K == 2) load_frame(s_frames, i, fr);
+    else load_frame<K>(g.frames, a, fr);
     Pair<K> p;
-    pair_setup<K>(at, jj, fr, g, p);
+    pair_setup<K, K == 2>(at, jj, fr, g, p);
     float Ma[NM], X0, Y0;
-    lane_moments<K, K == 1 ? 8 : 4>(p, g, in, a, I, Ma, X0, Y0, phase, cfg.rs);
+    if constexpr (K == 1) lane_cells<8>(p, g, in, a, I, Ma, X0, Y0, phase, cfg.rs);
+    else lane_rows<QUAD, L2ATOM>(p, g, in, a, I, Ma, X0, Y0, phase, cfg.rs);
     for (int o = 1; o < cfg.rs; o <<= 1) {
 #pragma unroll
       for (int q = 0; q < NM; ++q) Ma[q] += __shfl_xor_sync(gmask, Ma[q], o * cfg.ag);
@@ -643,18 +721,59 @@ __global__ void __launch_bounds__(32, 32)
       Y0 += __shfl_xor_sync(gmask, Y0, o * cfg.ag);
     }
     if (phase == 0) {
+      if constexpr (K == 2) {  // (read again rather than held over the walk)
+        asm volatile("" ::: "memory");
+        load_frame(s_frames, i, fr);
+      }
       float Aa[NPSI], Z[NPSI][NPSI];
       first_psi<K, NM>(Ma, p.G, Aa);
       if (in.mode == kModeInner) f += I * Ma[0];
       else if (in.mode == kModeL2Atom) f += I * (0.5f * I * Y0 - X0);
       accumulate_pair<K, 1>(p, fr, I, Aa, Z, Z, gacc, none);
     }
-    if constexpr (ONE) break;
+  };
+  const int astep = cfg.sg / cfg.rs;
+  if constexpr (K == 1) {
+    for (int a = a_lo + sub / cfg.rs; a < a_hi && valid; a += astep) {
+      add_pair(a, 0);
+      if constexpr (ONE) break;
+    }
+  } else {
+    for (int a0 = a_lo; a0 < a_hi; a0 += astep) {
+      stage_frames(s_frames, g.frames + (size_t)a0 * kFrameStride3D, min(astep, a_hi - a0));
+      __syncwarp();
+      const int i = sub / cfg.rs;
+      if (valid && a0 + i < a_hi) add_pair(a0 + i, i);
+      if constexpr (ONE) break;
+      __syncwarp();
+    }
   }
   // combine lanes sharing an atom, then write
   float gv[P];
 #pragma unroll
   for (int i = 0; i < P; ++i) gv[i] = gacc[i].get();
+  if constexpr (K == 2) {
+    if (cfg.ag == 1) {
+      // one atom per warp: halve the 16 values held over four exchanges, then one
+      // more sums each (16 shuffles, not five for each of the 11 values)
+      float v[16];
+#pragma unroll
+      for (int k = 0; k < 16; ++k) v[k] = k == 0 ? f : (k <= P ? gv[k - 1] : 0.f);
+#pragma unroll
+      for (int w = 8; w > 0; w >>= 1) {
+        const bool up = lane & (2 * w);
+#pragma unroll
+        for (int k = 0; k < w; ++k) {
+          const float keep = up ? v[w + k] : v[k], give = up ? v[k] : v[w + k];
+          v[k] = keep + __shfl_xor_sync(0xffffffffu, give, 2 * w);
+        }
+      }
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+      const int q = lane >> 1;
+      if (valid && (lane & 1) == 0 && q <= P) part[((size_t)chunk * cfg.qn + q) * at.n + j] = v[0];
+      return;
+    }
+  }
   for (int off = cfg.ag; off < 32; off <<= 1) {
     f += __shfl_xor_sync(0xffffffffu, f, off);
 #pragma unroll
@@ -1389,10 +1508,21 @@ struct DerivArgs {
   cudaStream_t stream;
 };
 
-template <int K>
+template <int K, bool QUAD, bool L2ATOM>
 static void start_grad(const DerivArgs &d) {
-  if (d.one) gr_grad_kernel<K, true><<<d.warps, 32, 0, d.stream>>>(d.at, d.g, d.in, d.cfg, d.part);
-  else gr_grad_kernel<K, false><<<d.warps, 32, 0, d.stream>>>(d.at, d.g, d.in, d.cfg, d.part);
+  if (d.one)
+    gr_grad_kernel<K, true, QUAD, L2ATOM><<<d.warps, 32, 0, d.stream>>>(d.at, d.g, d.in, d.cfg, d.part);
+  else
+    gr_grad_kernel<K, false, QUAD, L2ATOM><<<d.warps, 32, 0, d.stream>>>(d.at, d.g, d.in, d.cfg, d.part);
+}
+
+static void start_grad3(const DerivArgs &d) {
+  const bool l2atom = d.in.mode == kModeL2Atom;
+  const size_t at16 = reinterpret_cast<size_t>(d.in.alpha) | reinterpret_cast<size_t>(d.g.ax[1].coords);
+  if (d.g.ax[1].n % 4 == 0 && at16 % 16 == 0)
+    l2atom ? start_grad<2, true, true>(d) : start_grad<2, true, false>(d);
+  else
+    l2atom ? start_grad<2, false, true>(d) : start_grad<2, false, false>(d);
 }
 
 template <int K, int GL, int FK>
@@ -1463,8 +1593,8 @@ int launch_derivs(const Atoms &at, const Geom &g, const DerivIn &in,
     const bool one = c.ch <= c.sg / c.rs;
     const DerivArgs d{at, g, in, c, part, warps, one, stream};
     if (in.order == 2) K == 1 ? start_hess<1>(d) : start_hess<2>(d);
-    else if (K == 1) start_grad<1>(d);
-    else start_grad<2>(d);
+    else if (K == 1) start_grad<1, false, false>(d);
+    else start_grad3(d);
   }
   timer_mark(2, 1, stream);
   const int fblocks = (at.n + kFinAtoms - 1) / kFinAtoms;
@@ -1536,11 +1666,15 @@ template <int K>
 static int preload_walk() {
   return preload_one<K, walk_lanes_of<K>()>() + preload_one<K, 8>() +
          preload_fn(gr_hess_kernel<K, false, walk_lanes_of<K>(), walk_cells_of<K>(), kFieldAny>) +
-         preload_fn(gr_grad_kernel<K, true>) + preload_fn(gr_grad_kernel<K, false>);
+         preload_fn(gr_grad_kernel<K, true, false, false>) +
+         preload_fn(gr_grad_kernel<K, false, false, false>);
 }
 
 int preload_derivs() {
   return preload_walk<1>() + preload_walk<2>() +
+         preload_fn(gr_grad_kernel<2, true, true, false>) + preload_fn(gr_grad_kernel<2, false, true, false>) +
+         preload_fn(gr_grad_kernel<2, true, true, true>) + preload_fn(gr_grad_kernel<2, false, true, true>) +
+         preload_fn(gr_grad_kernel<2, true, false, true>) + preload_fn(gr_grad_kernel<2, false, false, true>) +
          preload_fn(gr_psf_deriv1d_kernel<1>) + preload_fn(gr_psf_deriv1d_kernel<2>) +
          preload_fn(gr_psf_deriv_kernel<1>) + preload_fn(gr_psf_deriv_kernel<2>) +
          preload_fn(gr_deriv_finalize_kernel<1>) + preload_fn(gr_deriv_finalize_kernel<2>) +

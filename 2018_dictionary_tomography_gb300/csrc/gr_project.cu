@@ -123,11 +123,6 @@ __device__ __forceinline__ Proj3Rec proj3_record(const Pair<2> &p) {
   return o;
 }
 
-__device__ __forceinline__ float sqrt_approx(float v) {
-  float y;
-  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(v));
-  return y;
-}
 __device__ __forceinline__ float rcp_approx(float v) {
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(v));
