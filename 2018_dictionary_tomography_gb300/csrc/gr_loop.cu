@@ -358,7 +358,7 @@ bool batch_shape(const BatchProb &p, BatchShape &s) {
   if (s.cfg.ch > s.cfg.sg / s.cfg.rs) return false;     // one angle per lane
   s.bitmap_bytes = align_up((size_t)s.items * s.W * sizeof(uint32_t));
   s.loss_bytes = align_up((size_t)s.items * sizeof(double));
-  s.pair_bytes = align_up((size_t)A * n * 2 * sizeof(float4));
+  s.pair_bytes = align_up((size_t)A * n * sizeof(float4));
   s.part_bytes = align_up((size_t)s.cfg.nchunks * s.cfg.qn * n * sizeof(float));
   const int P = p.cur.r_iso ? 4 : 6;
   const long long warps = (long long)((n + s.cfg.ag - 1) / s.cfg.ag) * s.cfg.nchunks;

@@ -42,9 +42,9 @@ __device__ __forceinline__ void bin_body(const Atoms &at, const Geom &g, const T
     Pair<1> p;
     pair_setup<1>(at, j, f, g, p);
     if (pairs) {
-      float4 *rec = pairs + ((size_t)a * at.n + j) * 2;
-      rec[0] = make_float4(p.qh[0], p.ql[0], p.G[0], p.l2amp);
-      rec[1] = make_float4(__int_as_float(p.lo[0]), __int_as_float(p.hi[0]), p.sgn, 0.f);
+      // (the sign of I rides on G's, which is >= 0)
+      pairs[(size_t)a * at.n + j] =
+          make_float4(p.qh[0], p.ql[0], copysignf(p.G[0], p.sgn), p.l2amp);
     }
     if (p.lo[0] <= p.hi[0]) {
       t_lo = p.lo[0] / tc.t0;
@@ -549,7 +549,12 @@ __global__ void __launch_bounds__(256)
 // LM: a pass lists up to LM * NW * 32 atoms (each thread stages LM of them),
 // so tiles crossed by many atoms take fewer passes and barriers (2150 atoms x
 // 153 angles: 87.9 us with one atom per thread, 82.6 with two, 79.5 with
-// four; 512 atoms: 20.6, 20.7, 21.1 us)
+// four; 512 atoms: 20.6, 20.7, 21.1 us).
+// What bounds it: issue (78 % of the slots), some 17 instructions a cell and
+// atom: one 16-byte record, the form, the exponential and the compensated sum,
+// without a branch (with the support box in a second record and tests of it and
+// of the form: 75 us where this takes 51.1; with the form's test alone as a
+// branch 57.7; 64 cells a tile 68.8).
 // The body of one block of the 2D projection: (angle, tile) item of n_items
 // (the launch's block; a multi-problem launch maps its blocks to (problem,
 // item)).
@@ -561,7 +566,7 @@ __device__ __forceinline__ void project1d_body(const Atoms &at, const Geom &g, c
                                                int n_items) {
   constexpr int T = NW * 32;
   constexpr int LT = LM * T;
-  __shared__ float4 prm[LT][2];
+  __shared__ float4 prm[LT];
   __shared__ int list[LT];
   __shared__ int wsum[NW];
   __shared__ float parts[NW][2][32 * CPL];
@@ -577,7 +582,7 @@ __device__ __forceinline__ void project1d_body(const Atoms &at, const Geom &g, c
     acc[k] = 0.f;
     cmp[k] = 0.f;
   }
-  const float4 *apairs = pairs + (size_t)a * at.n * 2;
+  const float4 *apairs = pairs + (size_t)a * at.n;
 
   const uint32_t *words = bitmap + (size_t)item * W;
   for (int wb = 0; wb < W;) {
@@ -614,34 +619,27 @@ __device__ __forceinline__ void project1d_body(const Atoms &at, const Geom &g, c
     wb += ntake > 0 ? ntake : W;   // ntake = 0 only past the last word
     // pair data of the listed atoms (set up once per pair by the binning
     // launch), up to LM per thread
-    for (int e = threadIdx.x; e < total; e += T) {
-      const float4 *rec = apairs + (size_t)list[e] * 2;
-      prm[e][0] = __ldg(rec);
-      prm[e][1] = __ldg(rec + 1);
-    }
+    for (int e = threadIdx.x; e < total; e += T) prm[e] = __ldg(apairs + list[e]);
     __syncthreads();
     // warp w: slice [w total / NW, (w + 1) total / NW) in list order
     const int s_lo = (warp * total) / NW, s_hi = ((warp + 1) * total) / NW;
 #pragma unroll 4
     for (int s2 = s_lo; s2 < s_hi; ++s2) {
-      const float4 q0 = prm[s2][0];
-      const float4 q1 = prm[s2][1];
-      const int lo = __float_as_int(q1.x), hi = __float_as_int(q1.y);
+      const float4 q = prm[s2];
 #pragma unroll
       for (int k = 0; k < CPL; ++k) {
-        if (cell[k] >= lo && cell[k] <= hi) {
-          const float d = (pc[k] - q0.x) - q0.y;
-          const float m = q0.z * d * d;
-          if (m <= 1.f) {
-            const float v = q1.z * ex2_approx(fmaf(m, kNegThirtyLog2e, q0.w));
-            if (KAHAN) {
-              const float tt = acc[k] + v;
-              cmp[k] += (fabsf(acc[k]) >= fabsf(v)) ? ((acc[k] - tt) + v) : ((v - tt) + acc[k]);
-              acc[k] = tt;
-            } else {
-              acc[k] += v;
-            }
-          }
+        const float d = (pc[k] - q.x) - q.y;
+        const float m = fabsf(q.z) * d * d;
+        // (a cell that the atom misses adds zero, which leaves both sums as they
+        // are)
+        const float E = ex2_approx(fmaf(m, kNegThirtyLog2e, q.w));
+        const float v = m <= 1.f ? copysignf(E, q.z) : 0.f;
+        if (KAHAN) {
+          const float tt = acc[k] + v;
+          cmp[k] += (fabsf(acc[k]) >= fabsf(v)) ? ((acc[k] - tt) + v) : ((v - tt) + acc[k]);
+          acc[k] = tt;
+        } else {
+          acc[k] += v;
         }
       }
     }
@@ -707,13 +705,26 @@ __device__ __forceinline__ void project1d_body(const Atoms &at, const Geom &g, c
   sum_partials_block<NW>(out.loss_part, n_items, loss_out);
 }
 
+// The item (angle a, tile t: a ntiles + t) of block b, in launches of a block per
+// item: the tiles at the detector's middle first, of every angle, those at its
+// ends last.  Atoms sit about the middle, so the blocks that start last are the
+// short ones (in angle order, the SMs idled for a third of the launch on 2150
+// atoms x 153 angles x 15 tiles: 51.1 us, 41.1 us; pixel-integrated, 128
+// x 401 x 8 tiles: 64.8 and 62.5 us).
+__device__ __forceinline__ int centre_out(int b, int n_angles, const TileCfg &tc) {
+  const int rank = b / n_angles, a = b - rank * n_angles;
+  const int k0 = rank / tc.nt1, k1 = rank - k0 * tc.nt1;
+  auto at = [](int k, int n) { return (k & 1) ? n / 2 - (k + 1) / 2 : n / 2 + k / 2; };
+  return a * tc.ntiles + at(k0, tc.nt0) * tc.nt1 + at(k1, tc.nt1);
+}
+
 template <bool KAHAN, int NW, int CPL = 1, int LM = 1>
 __global__ void __launch_bounds__(NW * 32)
     gr_project1d_kernel(Atoms at, Geom g, TileCfg tc, const uint32_t *bitmap,
                         int W, ProjOut out, double *loss_out, int *done,
                         const float4 *__restrict__ pairs) {
   project1d_body<KAHAN, NW, CPL, LM>(at, g, tc, bitmap, W, out, loss_out, done, pairs,
-                                     blockIdx.x, gridDim.x);
+                                     centre_out(blockIdx.x, g.n_angles, tc), gridDim.x);
 }
 
 // ---- pixel-integrated operator: binning and projection -------------------
@@ -776,7 +787,7 @@ __global__ void __launch_bounds__(kPsfTileWarps * 32, 8)
   __shared__ int s_last;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   uint32_t *queue = s_queue[warp];
-  const int item = blockIdx.x, n_items = g.n_angles * tc.ntiles;
+  const int item = centre_out(blockIdx.x, g.n_angles, tc), n_items = g.n_angles * tc.ntiles;
   const int cells = tc.t0 * tc.t1;
   float *acc = smem + (size_t)warp * psf_warp_words(cells);
   float *cmp = acc + cells;
@@ -1087,7 +1098,7 @@ size_t project_min_bytes(int K, int n_atoms, int n_angles, int D0, int D1, const
   bytes += align_up(items * sizeof(double));
   bytes += align_up(kLossMaxBlocks * sizeof(double));  // block sums of the loss finalize
   if (K == 1)  // per-(angle, atom) pair records of the 2D projection
-    bytes += align_up((size_t)n_angles * (size_t)n_atoms * 2 * sizeof(float4));
+    bytes += align_up((size_t)n_angles * (size_t)n_atoms * sizeof(float4));
   else
     bytes += align_up(items * sizeof(int));
   return bytes;
