@@ -480,7 +480,9 @@ __global__ void __launch_bounds__(NW * 32, 32 / NW)
 // angle, writes their records (rec, nullable) and gathers the tiles' words in
 // shared memory, a range of kBinTiles tiles at a time, so that every word of
 // the bitmap is written once: no clear, and no global atomics (whose latency
-// and contention bounded the launch before).
+// and contention bounded the launch before).  Instruction issue bounds it (89 % of
+// the slots, 500 a warp of pairs): four divisions by the tile's sides were a
+// fifth of them (8192 atoms x 20000: 3.05 ms, 2.46 with shifts).
 // counters (nullable): zeroed, for the projection that follows.
 constexpr int kBinTiles = 512;
 __global__ void __launch_bounds__(256)
@@ -497,10 +499,11 @@ __global__ void __launch_bounds__(256)
     Pair<2> p;
     pair_setup<2>(at, j, f, g, p);
     if (p.lo[0] <= p.hi[0] && p.lo[1] <= p.hi[1]) {
-      r_lo = p.lo[0] / tc.t0;
-      r_hi = p.hi[0] / tc.t0;
-      c_lo = p.lo[1] / tc.t1;
-      c_hi = p.hi[1] / tc.t1;
+      const int sh = 31 - __clz(tc.t0);  // (16 or 32 rows a tile, 32 columns)
+      r_lo = p.lo[0] >> sh;
+      r_hi = p.hi[0] >> sh;
+      c_lo = p.lo[1] / kTileDim1;
+      c_hi = p.hi[1] / kTileDim1;
       if (rec) rec[(size_t)a * at.n + j] = proj3_record(p);
     }
   }
