@@ -608,11 +608,15 @@ class FitStep:
     (when given), replays and waits; its results are views of the pinned
     output buffers, overwritten by the next run.
 
-    Large sinograms are fitted in ``chunks`` ranges of angles (default: one
-    per 128 MB of data, at most 8): a side stream copies range i+1 in while
-    the projection of range i runs, so the copy of the data overlaps the
-    projection instead of preceding it; the loss is the FP64 sum of the
-    ranges' losses, and the derivatives run once over all angles.
+    Sinograms of 16 MB and more are fitted in ``chunks`` ranges of angles
+    (default: one per 8 MB of data up to 4, one per 48 MB up to 8): a side
+    stream copies range i+1 in while the projection of range i runs, so the
+    copy of the data overlaps the projection instead of preceding it; the loss
+    is the FP64 sum of the ranges' losses, and the derivatives run once over all
+    angles.  A range costs some 10 us of launches.  1, 2, 4, 6, 8 ranges: 36 MB
+    (1000 atoms) 430, 389, 373, 394, 419 us; 24 MB (500 atoms, order 2) 315, 294,
+    293, 316, 338; 307 MB (4000 atoms) 4314, 3629, 3339, 3283, 3288; 4.9 MB 118,
+    122, 143, 171, 196.
     """
 
     def __init__(self, geom, n_atoms, iso=False, fit="l2", background=0.0, order=2,
@@ -665,7 +669,8 @@ class FitStep:
         A = geom.n_angles
         data_bytes = int(self.data_d.numel()) * 4
         if chunks is None:
-            chunks = min(8, (data_bytes + (128 << 20) - 1) >> 27) if data_bytes >= (128 << 20) else 1
+            mb = data_bytes >> 20
+            chunks = max(min(4, mb // 8), min(8, mb // 48)) if mb >= 16 else 1
         chunks = max(1, min(int(chunks), A))
         bounds = [(i * A) // chunks for i in range(chunks + 1)]
         self.ranges = [(a0, a1, geom.angle_range(a0, a1) if chunks > 1 else geom)
