@@ -561,16 +561,16 @@ __device__ __forceinline__ void lane_cells(const Pair<1> &p, const Geom &g, cons
   }
 }
 
-// 3D: a row's cells in aligned fours of the field, two at a time in packed FP32
-// pairs.  The loads bound it: 32 lanes touch 32 lines of the field, one L1 tag
-// each, so a load takes 16 bytes a lane (a four of 4-byte loads took four times
-// the tags: 17.4 ms where this takes 13.5; a row's first four loaded a row ahead
-// costs registers: 15.4 to 16.3).  The m <= 1 test decides every
-// cell of a four; QUAD: rows begin on fours (D1 a multiple of four, both arrays
-// on 16 bytes), so a four lies in one row and its coordinates are one load too.
-// Otherwise fours are aligned in the whole field, and one that crosses an end of
-// its row loads the row's cells one by one.
-template <bool QUAD, bool L2ATOM>
+// 3D: a row's cells in aligned fours of the field, in packed FP32 pairs.  The
+// loads bound it: 32 lanes touch 32 lines of the field, one L1 tag each, so a load
+// takes 16 bytes a lane (a four of 4-byte loads took four times the tags: 17.4 ms
+// where this takes 12.7; a row's first four loaded a row ahead costs registers:
+// 15.4 to 16.3).  The m <= 1 test decides every cell of a four.
+//
+// Rows that begin anywhere: fours are aligned in the whole field, two cells of a
+// four at a time; a four that crosses an end of its row loads the row's cells one
+// by one.
+template <bool L2ATOM>
 __device__ __forceinline__ void lane_rows(const Pair<2> &p, const Geom &g, const DerivIn &in, int a,
                                           float I, float (&Ma)[n_mom<2, 2>()], float &X0,
                                           float &Y0, int phase, int rs) {
@@ -629,30 +629,21 @@ __device__ __forceinline__ void lane_rows(const Pair<2> &p, const Geom &g, const
         Y = f2_add(Y, f2_keep(f2_mul(E, E), in0, in1));
       }
     };
-    if constexpr (QUAD) {
-      for (int kb = c_lo & ~3; kb <= c_hi; kb += 4) {
+    // cells before c_lo down to a 16-byte boundary
+    const int back = (int)((reinterpret_cast<size_t>(row + c_lo) >> 2) & 3);
+    for (int kb = c_lo - back; kb <= c_hi; kb += 4) {
+      if (kb >= 0 && kb + 4 <= D1) {
         const float4 c = __ldg(reinterpret_cast<const float4 *>(row + kb));
-        const float4 x = __ldg(reinterpret_cast<const float4 *>(x1 + kb));
-        cells(f2(x.x, x.y), f2(c.x, c.y), true, true);
-        cells(f2(x.z, x.w), f2(c.z, c.w), true, true);
-      }
-    } else {
-      // cells before c_lo down to a 16-byte boundary
-      const int back = (int)((reinterpret_cast<size_t>(row + c_lo) >> 2) & 3);
-      for (int kb = c_lo - back; kb <= c_hi; kb += 4) {
-        if (kb >= 0 && kb + 4 <= D1) {
-          const float4 c = __ldg(reinterpret_cast<const float4 *>(row + kb));
-          const float *x = x1 + kb;
-          cells(f2(__ldg(x), __ldg(x + 1)), f2(c.x, c.y), true, true);
-          cells(f2(__ldg(x + 2), __ldg(x + 3)), f2(c.z, c.w), true, true);
-        } else {
-          // a four that crosses an end of the row: the row's cells only
+        const float *x = x1 + kb;
+        cells(f2(__ldg(x), __ldg(x + 1)), f2(c.x, c.y), true, true);
+        cells(f2(__ldg(x + 2), __ldg(x + 3)), f2(c.z, c.w), true, true);
+      } else {
+        // a four that crosses an end of the row: the row's cells only
 #pragma unroll
-          for (int i = 0; i < 4; i += 2) {
-            const int ka = kb + i, ia = min(max(ka, 0), D1 - 1), ib = min(max(ka + 1, 0), D1 - 1);
-            cells(f2(__ldg(x1 + ia), __ldg(x1 + ib)), f2(__ldg(row + ia), __ldg(row + ib)),
-                  ka == ia, ka + 1 == ib);
-          }
+        for (int i = 0; i < 4; i += 2) {
+          const int ka = kb + i, ia = min(max(ka, 0), D1 - 1), ib = min(max(ka + 1, 0), D1 - 1);
+          cells(f2(__ldg(x1 + ia), __ldg(x1 + ib)), f2(__ldg(row + ia), __ldg(row + ib)),
+                ka == ia, ka + 1 == ib);
         }
       }
     }
@@ -671,15 +662,107 @@ __device__ __forceinline__ void lane_rows(const Pair<2> &p, const Geom &g, const
   }
 }
 
+// Rows that begin on fours (D1 a multiple of four, field and coordinates on 16
+// bytes): two rows at a time, a row per half of a register pair, over the union of
+// their ranges, so that coordinates and a load's latency are shared by two (8192
+// atoms x 20000 x 128^2: 12.7 ms, 13.5 a row at a time; 4096 x 121 x 256^2: 59 and
+// 64 us).
+template <bool L2ATOM>
+__device__ __forceinline__ void lane_row_pairs(const Pair<2> &p, const Geom &g, const DerivIn &in,
+                                               int a, float I, float (&Ma)[n_mom<2, 2>()],
+                                               float &X0, float &Y0, int phase, int rs) {
+  constexpr int NM = n_mom<2, 2>();
+#pragma unroll
+  for (int i = 0; i < NM; ++i) Ma[i] = 0.f;
+  X0 = 0.f;
+  Y0 = 0.f;
+  if (p.lo[0] > p.hi[0] || p.lo[1] > p.hi[1]) return;
+  const float l2n = lg2_approx(p.n);
+  const int D1 = g.ax[1].n;
+  const float *__restrict__ x0 = g.ax[0].coords, *__restrict__ x1 = g.ax[1].coords;
+  const float *__restrict__ field = in.alpha + (size_t)a * g.ax[0].n * D1;
+  const F2 K2 = f2(kNegThirtyLog2e, kNegThirtyLog2e), amp = f2(l2n, l2n);
+  // (the rows' ranges as in lane_rows)
+  const float det = p.G[0] * p.G[2] - p.G[1] * p.G[1];
+  const float iG2 = 1.f / p.G[2];
+  const float rc0 = (p.qh[1] - g.ax[1].first) * g.ax[1].inv_step;
+  const float rcd = p.G[1] * iG2 * g.ax[1].inv_step;
+  const float rhs = iG2 * g.ax[1].inv_step * 1.0001f;
+  const float c_min = (float)p.lo[1], c_max = (float)p.hi[1];
+  for (int k0 = p.lo[0] + 2 * phase; k0 <= p.hi[0]; k0 += 2 * rs) {
+    const bool two = k0 < p.hi[0];
+    const float da = (__ldg(x0 + k0) - p.qh[0]) - p.ql[0];
+    const float db = (__ldg(x0 + k0 + (two ? 1 : 0)) - p.qh[0]) - p.ql[0];
+    const float ra = fmaf(-rcd, da, rc0), rb = fmaf(-rcd, db, rc0);
+    const float ha = fmaf(sqrt_approx(fmaxf(fmaf(-da * da, det, p.G[2]), 0.f)), rhs, 1e-3f);
+    const float hb = fmaf(sqrt_approx(fmaxf(fmaf(-db * db, det, p.G[2]), 0.f)), rhs, 1e-3f);
+    const int c_lo = (int)fmaxf(ceilf(fminf(ra - ha, rb - hb)), c_min);
+    const int c_hi = (int)fminf(floorf(fmaxf(ra + ha, rb + hb)), c_max);
+    // (a row past the support: no cell of it is within)
+    const F2 t0 = f2(p.G[0] * da * da, two ? p.G[0] * db * db : 4.f);
+    const F2 u = f2(2.f * p.G[1] * da, two ? 2.f * p.G[1] * db : 0.f);
+    const float *__restrict__ row = field + (size_t)k0 * D1;
+    const int to_b = two ? D1 : 0;
+    F2 S0 = f2(0.f, 0.f), S1 = S0, S2 = S0, X = S0, Y = S0;
+    for (int kb = c_lo & ~3; kb <= c_hi; kb += 4) {
+      const float4 ca = __ldg(reinterpret_cast<const float4 *>(row + kb));
+      const float4 cb = __ldg(reinterpret_cast<const float4 *>(row + kb + to_b));
+      const float4 xv = __ldg(reinterpret_cast<const float4 *>(x1 + kb));
+      auto column = [&](float x, float fa, float fb) {
+        const float d = (x - p.qh[1]) - p.ql[1];
+        const float gd = p.G[2] * d;
+        const F2 D = f2(d, d);
+        const F2 m = f2_fma(D, f2_add(f2(gd, gd), u), t0);
+        float m0, m1, e0, e1;
+        f2_get(m, m0, m1);
+        f2_get(f2_fma(m, K2, amp), e0, e1);
+        const F2 E = f2(ex2_approx(e0), ex2_approx(e1)), c = f2(fa, fb);
+        const bool in0 = m0 <= 1.f, in1 = m1 <= 1.f;
+        F2 al = c;
+        if (L2ATOM) al = f2_fma(f2(I, I), E, f2_mul(c, f2(-1.f, -1.f)));
+        const F2 w = f2_keep(f2_mul(al, E), in0, in1);
+        S0 = f2_add(S0, w);
+        const F2 wd = f2_mul(w, D);
+        S1 = f2_add(S1, wd);
+        S2 = f2_fma(wd, D, S2);
+        if (L2ATOM) {
+          X = f2_add(X, f2_keep(f2_mul(E, c), in0, in1));
+          Y = f2_add(Y, f2_keep(f2_mul(E, E), in0, in1));
+        }
+      };
+      column(xv.x, ca.x, cb.x);
+      column(xv.y, ca.y, cb.y);
+      column(xv.z, ca.z, cb.z);
+      column(xv.w, ca.w, cb.w);
+    }
+    if (L2ATOM) {
+      X0 += f2_sum(X);
+      Y0 += f2_sum(Y);
+    }
+    float s0a, s0b, s1a, s1b;
+    f2_get(S0, s0a, s0b);
+    f2_get(S1, s1a, s1b);
+    Ma[mi(0, 0)] += s0a + s0b;
+    Ma[mi(0, 1)] += s1a + s1b;
+    Ma[mi(0, 2)] += f2_sum(S2);
+    Ma[mi(1, 1)] += fmaf(da, s1a, db * s1b);
+    const float w0a = da * s0a, w0b = db * s0b;
+    Ma[mi(1, 0)] += w0a + w0b;
+    Ma[mi(2, 0)] += fmaf(da, w0a, db * w0b);
+  }
+}
+
 template <int K>
 struct FramesOf { using type = FrameSmem; };
 template <>
 struct FramesOf<1> { using type = int; };  // (2D: not used)
 
 // ONE, one-warp blocks: as gr_hess_kernel.  QUAD, L2ATOM: 3D only (2D reads the
-// mode from `in`).
+// mode from `in`).  Row pairs take 28 warps an SM (72 registers: tilt series of 4096
+// x 121 x 256^2 59.3 us, 63.0 with 32 warps), single rows 32 (1000 x 1001 x 95^2:
+// 88.4 us, 91.0 with 28).
 template <int K, bool ONE, bool QUAD, bool L2ATOM>
-__global__ void __launch_bounds__(32, 32)
+__global__ void __launch_bounds__(32, QUAD ? 28 : 32)
     gr_grad_kernel(Atoms at, Geom g, DerivIn in, DerivCfg cfg, float *part) {
   constexpr int P = n_par<K>();
   constexpr int NM = n_mom<K, 2>();
@@ -713,7 +796,8 @@ __global__ void __launch_bounds__(32, 32)
     pair_setup<K, K == 2>(at, jj, fr, g, p);
     float Ma[NM], X0, Y0;
     if constexpr (K == 1) lane_cells<8>(p, g, in, a, I, Ma, X0, Y0, phase, cfg.rs);
-    else lane_rows<QUAD, L2ATOM>(p, g, in, a, I, Ma, X0, Y0, phase, cfg.rs);
+    else if constexpr (QUAD) lane_row_pairs<L2ATOM>(p, g, in, a, I, Ma, X0, Y0, phase, cfg.rs);
+    else lane_rows<L2ATOM>(p, g, in, a, I, Ma, X0, Y0, phase, cfg.rs);
     for (int o = 1; o < cfg.rs; o <<= 1) {
 #pragma unroll
       for (int q = 0; q < NM; ++q) Ma[q] += __shfl_xor_sync(gmask, Ma[q], o * cfg.ag);
