@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(NW * 32, 32 / NW)
   __shared__ int list[kList];
   __shared__ int s_count[NW];
   __shared__ float sV[4 * NW][kPitch];
-  __shared__ int s_item;
+  __shared__ int s_item, s_last;
   __shared__ float2 s_loss[T];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n_items = g.n_angles * tc.ntiles;
@@ -463,13 +463,14 @@ __global__ void __launch_bounds__(NW * 32, 32 / NW)
   }
 
   if (loss_out && out.loss_part) {
-    // the last block to finish sums the items' partials in item order
+    // the last block to finish sums the items' partials in item order (a flag of
+    // its own: a slower warp may still have the last s_item to read)
     if (tid == 0) {
       __threadfence();
-      s_item = atomicAdd(next_item + 1, 1) == (int)gridDim.x - 1;
+      s_last = atomicAdd(next_item + 1, 1) == (int)gridDim.x - 1;
     }
     __syncthreads();
-    if (s_item) {
+    if (s_last) {
       __threadfence();
       sum_partials_block<NW>(out.loss_part, n_items, loss_out);
     }
