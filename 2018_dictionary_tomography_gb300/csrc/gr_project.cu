@@ -921,6 +921,7 @@ __global__ void __launch_bounds__(kPsfTileWarps * 32, 8)
         }
       }
       if (queued) add_cells(queued);
+      __syncwarp();  // the staged atoms are done with
     }
   }
   __syncthreads();
