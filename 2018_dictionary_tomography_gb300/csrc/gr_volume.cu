@@ -219,8 +219,8 @@ __global__ void __launch_bounds__(kVolThreads)
 }
 
 // ---- 3D, point values -------------------------------------------------------
-// A block of 256 threads owns 8 x 16 x 16 voxels, a warp 8 x 4 x 8 of them: a
-// lane a column of 8 voxels along axis 0, its sums in registers.  The block
+// A block of 256 threads owns V0 x 16 x 16 voxels (V0 = 8 on large grids), a warp
+// V0 x 4 x 8 of them: a lane a column of V0 voxels along axis 0, its sums in registers.  The block
 // finds the atoms that meet its voxels, kAtoms at a time (a thread each, so an
 // atom is set up once per 2048 voxels), and stages them in index order; each
 // warp ballots them against its own voxels, 32 at a time, and adds those left.
@@ -228,7 +228,8 @@ __global__ void __launch_bounds__(kVolThreads)
 // What bounds it: the scan of all atoms by every block (1000 atoms on 128 x 124
 // x 120 voxels: 13.2 us; with 256 voxels a block, one per thread, 65.7 us: eight
 // times the scans, and every listed atom evaluated at every voxel of the tile).
-constexpr int kVol0 = 8, kVol1 = 16, kVol2 = 16;
+constexpr int kVol1 = 16, kVol2 = 16;
+template <int V0>
 __global__ void __launch_bounds__(kVolThreads)
     gr_volproj3_kernel(Atoms at, VolGrid vg, float *u) {
   constexpr int kAtoms = kVolThreads;
@@ -243,15 +244,15 @@ __global__ void __launch_bounds__(kVolThreads)
   const int b2 = b % nt2;
   b /= nt2;
   const int b1 = b % nt1, b0 = b / nt1;
-  const int o0 = b0 * kVol0, o1 = b1 * kVol1, o2 = b2 * kVol2;
+  const int o0 = b0 * V0, o1 = b1 * kVol1, o2 = b2 * kVol2;
   // the warp's voxels: 4 x 8 columns of the tile's 16 x 16
   const int w1 = o1 + 4 * (warp >> 1), w2 = o2 + 8 * (warp & 1);
   const int i1 = w1 + (lane >> 3), i2 = w2 + (lane & 7);
   const bool inside = i1 < vg.n[1] && i2 < vg.n[2];
-  const int n0 = min(kVol0, vg.n[0] - o0);
-  float y0[kVol0], acc[kVol0];
+  const int n0 = min(V0, vg.n[0] - o0);
+  float y0[V0], acc[V0];
 #pragma unroll
-  for (int k = 0; k < kVol0; ++k) {
+  for (int k = 0; k < V0; ++k) {
     y0[k] = vg.y[0][min(o0 + k, vg.n[0] - 1)];
     acc[k] = 0.f;
   }
@@ -264,7 +265,7 @@ __global__ void __launch_bounds__(kVolThreads)
     hi = fmaxf(p, q);
   };
   float blo[3], bhi[3], wlo[3], whi[3];
-  box(0, o0, kVol0, blo[0], bhi[0]);
+  box(0, o0, V0, blo[0], bhi[0]);
   box(1, o1, kVol1, blo[1], bhi[1]);
   box(2, o2, kVol2, blo[2], bhi[2]);
   box(1, w1, 4, wlo[1], whi[1]);
@@ -330,7 +331,7 @@ __global__ void __launch_bounds__(kVolThreads)
         const float c = fmaf(Q.x, Y1, Q.y * Y2), d = Q.z * Y2;
         const float cd = fmaf(c, c, d * d);
 #pragma unroll
-        for (int k2 = 0; k2 < kVol0; ++k2) {
+        for (int k2 = 0; k2 < V0; ++k2) {
           const float a = fmaf(R.x, y0[k2] - X.x, t);
           const float nn = fmaf(a, a, cd);
           if (nn <= 1.f) acc[k2] = fmaf(X.w, ex2_approx(nn * kNegThirtyLog2e), acc[k2]);
@@ -341,10 +342,14 @@ __global__ void __launch_bounds__(kVolThreads)
   }
   if (inside)
 #pragma unroll
-    for (int k = 0; k < kVol0; ++k)
+    for (int k = 0; k < V0; ++k)
       if (k < n0) u[((size_t)(o0 + k) * vg.n[1] + i1) * vg.n[2] + i2] = acc[k];
 }
 
+// 3D point values: the most voxels a lane (of 8, 4, 2, 1 along axis 0) that still
+// gives two blocks an SM: a block scans all atoms, so few blocks of many voxels
+// leave the SMs idle (16 blocks for 32^3 voxels).
+constexpr int kVolBlocks = 304;
 int launch_volproj(const Atoms &at, int dim, const int *n, const float *const *y,
                    float *u, int psf, float s, cudaStream_t stream) {
   VolGrid vg;
@@ -359,9 +364,12 @@ int launch_volproj(const Atoms &at, int dim, const int *n, const float *const *y
     else gr_volproj_kernel<2, false><<<blocks, kVolThreads, 0, stream>>>(at, vg, t0, t1, 1, s, u);
   } else {
     if (!psf) {
-      const int nb = ((vg.n[0] + kVol0 - 1) / kVol0) * ((vg.n[1] + kVol1 - 1) / kVol1) *
-                     ((vg.n[2] + kVol2 - 1) / kVol2);
-      gr_volproj3_kernel<<<nb, kVolThreads, 0, stream>>>(at, vg, u);
+      const int nb12 = ((vg.n[1] + kVol1 - 1) / kVol1) * ((vg.n[2] + kVol2 - 1) / kVol2);
+      auto nb = [&](int v) { return ((vg.n[0] + v - 1) / v) * nb12; };
+      if (nb(8) >= kVolBlocks) gr_volproj3_kernel<8><<<nb(8), kVolThreads, 0, stream>>>(at, vg, u);
+      else if (nb(4) >= kVolBlocks) gr_volproj3_kernel<4><<<nb(4), kVolThreads, 0, stream>>>(at, vg, u);
+      else if (nb(2) >= kVolBlocks) gr_volproj3_kernel<2><<<nb(2), kVolThreads, 0, stream>>>(at, vg, u);
+      else gr_volproj3_kernel<1><<<nb(1), kVolThreads, 0, stream>>>(at, vg, u);
       note_launches(1);
       return cudaGetLastError() == cudaSuccess ? kOk : kErrLaunch;
     }
@@ -375,7 +383,9 @@ int launch_volproj(const Atoms &at, int dim, const int *n, const float *const *y
 }
 
 int preload_volume() {
-  return preload_fn(gr_volproj_kernel<2, false>) + preload_fn(gr_volproj3_kernel) +
+  return preload_fn(gr_volproj_kernel<2, false>) + preload_fn(gr_volproj3_kernel<8>) +
+         preload_fn(gr_volproj3_kernel<4>) + preload_fn(gr_volproj3_kernel<2>) +
+         preload_fn(gr_volproj3_kernel<1>) +
          preload_fn(gr_volproj_kernel<2, true>) + preload_fn(gr_volproj_kernel<3, true>);
 }
 

@@ -15,7 +15,9 @@ vol = importlib.import_module("2018_dictionary_tomography_gb300.volume")
 
 
 @pytest.mark.parametrize("n,N", [((1, 1, 1), 40), ((8, 16, 16), 256), ((7, 15, 17), 257),
-                                 ((9, 17, 33), 600), ((25, 4, 40), 40)])
+                                 ((9, 17, 33), 600), ((25, 4, 40), 40),
+                                 # grids that give a lane 2, 4 and 8 voxels
+                                 ((9, 130, 129), 40), ((19, 130, 129), 40), ((21, 161, 176), 40)])
 @pytest.mark.parametrize("iso", [False, True])
 @pytest.mark.parametrize("back", [False, True])
 def test_rendering(eng, cuda_ready, n, N, iso, back):
