@@ -1574,11 +1574,20 @@ int tuning_get(const Tuning &t, int key) {
          : key == 8 ? t.deriv_wide_rows : key == 9 ? t.deriv_block_warps : -1;
 }
 
-size_t derivs_workspace_bytes(int K, int n_atoms, int n_angles, int order, const Tuning &t) {
-  DerivCfg c = deriv_cfg(K, n_atoms, n_angles, order, t);
+// Workspace of a launch under the split c.
+static size_t derivs_bytes(const DerivCfg &c, int n_atoms) {
   size_t b = align_up((size_t)c.nchunks * c.qn * (size_t)n_atoms * sizeof(float));
   b += align_up(kSumSqBlocks * sizeof(double)) + align_up(sizeof(double));
   return b;
+}
+
+// The query names no operator: the larger of the point-sampled and the
+// pixel-integrated kernels' splits (either can have more chunks: the second never
+// shares a pair among lanes, but gives a warp four atoms up to longer series).
+size_t derivs_workspace_bytes(int K, int n_atoms, int n_angles, int order, const Tuning &t) {
+  const size_t point = derivs_bytes(deriv_cfg(K, n_atoms, n_angles, order, t, true), n_atoms);
+  const size_t pixel = derivs_bytes(deriv_cfg(K, n_atoms, n_angles, order, t, false), n_atoms);
+  return point > pixel ? point : pixel;
 }
 
 struct DerivArgs {
@@ -1640,11 +1649,9 @@ int launch_derivs(const Atoms &at, const Geom &g, const DerivIn &in,
   const int K = g.K;
   if (at.n <= 0) return kOk;
   if (in.order < 1 || in.order > 2) return kErrArg;
-  // the pixel-integrated kernel walks whole pairs per lane (no cell split);
-  // its chunking never needs more workspace than the split one
-  DerivCfg c = deriv_cfg(K, at.n, g.n_angles, in.order, t, !in.psf);
-  if (ws == nullptr || ws_bytes < derivs_workspace_bytes(K, at.n, g.n_angles, in.order, t))
-    return kErrWorkspace;
+  // (the pixel-integrated kernels do not share a pair's cells out by rs)
+  const DerivCfg c = deriv_cfg(K, at.n, g.n_angles, in.order, t, !in.psf);
+  if (ws == nullptr || ws_bytes < derivs_bytes(c, at.n)) return kErrWorkspace;
   char *wp = static_cast<char *>(ws);
   float *part = reinterpret_cast<float *>(wp);
   wp += align_up((size_t)c.nchunks * c.qn * (size_t)at.n * sizeof(float));
