@@ -52,27 +52,39 @@ def _stream_handle(device):
     return ctypes.c_void_p(_raw_stream(device))
 
 
-def _host_f32(a):
-    """A host array or CPU tensor as a flat float32 numpy array."""
+def _on_host(a):
+    """Whether an array's values lie in host memory (an object with
+    ``__cuda_array_interface__`` is a device array, as a CUDA tensor is)."""
     if isinstance(a, torch.Tensor):
-        a = a.detach().to(torch.float32).numpy()
-    return np.asarray(a, dtype=np.float32).reshape(-1)
+        return not a.is_cuda
+    return not hasattr(a, "__cuda_array_interface__")
+
+
+def _host_f32(a):
+    """A host array, CPU tensor or sequence as a float32 numpy array."""
+    if not isinstance(a, torch.Tensor):
+        try:
+            return np.asarray(a, dtype=np.float32)
+        except (TypeError, ValueError):
+            a = torch.as_tensor(a)      # (sequences of tensors)
+    return a.detach().to(device="cpu", dtype=torch.float32).numpy()
 
 
 def to_device_packed(arrays, device):
-    """Float32 device copies of host arrays of any shape, moved with one copy
-    (a small host-to-device copy costs 17 us whatever its size): flat views of
-    one buffer, each starting at a multiple of 16 bytes."""
-    flat = [_host_f32(a) for a in arrays]
+    """Float32 device copies of host arrays, moved with one copy (a small
+    host-to-device copy costs 17 us whatever its size): views of one buffer, each
+    from a multiple of 16 bytes on."""
+    host_arrays = [_host_f32(a) for a in arrays]
     off, n = [], 0
-    for t in flat:
+    for t in host_arrays:
         off.append(n)
         n += (t.size + 3) // 4 * 4
     host = np.zeros(n, dtype=np.float32)
-    for o, t in zip(off, flat):
-        host[o:o + t.size] = t
+    for o, t in zip(off, host_arrays):
+        host[o:o + t.size] = t.reshape(-1)
     buf = torch.from_numpy(host).to(device)
-    return [buf[o:o + t.size] for o, t in zip(off, flat)]
+    flat = [buf[o:o + t.size] for o, t in zip(off, host_arrays)]
+    return [f if t.ndim == 1 else f.view(t.shape) for f, t in zip(flat, host_arrays)]
 
 
 def morton_order(x):
@@ -101,15 +113,8 @@ class DeviceAtoms:
     def __init__(self, I, x, r, device=None, order=None):
         device = torch.device(device or "cuda")
         _require_cuda(device)
-        on_host = not any(isinstance(a, torch.Tensor) and a.is_cuda for a in (I, x, r))
-        if on_host:
-            # host arrays travel together
-            xs, rs = np.shape(x), np.shape(r)
-            I, x, r = to_device_packed((I, x, r), device)
-            if x.shape != xs:
-                x = x.reshape(xs)
-            if r.shape != rs:
-                r = r.reshape(rs)
+        if _on_host(I) and _on_host(x) and _on_host(r):
+            I, x, r = to_device_packed((I, x, r), device)   # host arrays travel together
         else:
             I, x, r = (torch.as_tensor(a).to(device=device, dtype=torch.float32)
                        for a in (I, x, r))

@@ -20,7 +20,7 @@ def volproj(atoms, coords, device=None, psf=False):
         ys = [torch.as_tensor(np.asarray(c, dtype=np.float32).reshape(-1) if not isinstance(c, torch.Tensor)
                               else c.float().reshape(-1)).to(dev).contiguous() for c in coords]
     else:
-        ys = engine.to_device_packed([np.asarray(c, dtype=np.float32) for c in coords], dev)
+        ys = engine.to_device_packed([np.asarray(c, dtype=np.float32).reshape(-1) for c in coords], dev)
     shape = tuple(int(y.numel()) for y in ys)
     u = torch.empty(shape, dtype=torch.float32, device=dev)
     n = (ctypes.c_int * 3)(*(list(shape) + [1] * (3 - dim)))
