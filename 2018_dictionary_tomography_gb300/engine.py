@@ -72,8 +72,9 @@ def _host_f32(a):
 
 def to_device_packed(arrays, device):
     """Float32 device copies of host arrays, moved with one copy (a small
-    host-to-device copy costs 17 us whatever its size): views of one buffer, each
-    from a multiple of 16 bytes on."""
+    host-to-device copy costs 17 us whatever its size).  They share one buffer,
+    each from a multiple of 16 bytes on, but not a version counter: autograd
+    takes an in-place change of one for a change of that one alone."""
     host_arrays = [_host_f32(a) for a in arrays]
     off, n = [], 0
     for t in host_arrays:
@@ -83,7 +84,7 @@ def to_device_packed(arrays, device):
     for o, t in zip(off, host_arrays):
         host[o:o + t.size] = t.reshape(-1)
     buf = torch.from_numpy(host).to(device)
-    flat = [buf[o:o + t.size] for o, t in zip(off, host_arrays)]
+    flat = [buf[o:o + t.size].data for o, t in zip(off, host_arrays)]
     return [f if t.ndim == 1 else f.view(t.shape) for f, t in zip(flat, host_arrays)]
 
 

@@ -1,4 +1,5 @@
-"""DeviceAtoms from each kind of array: values and shapes."""
+"""DeviceAtoms from each kind of array: values and shapes, and no ties between the
+three device arrays."""
 import numpy as np
 import pytest
 import torch
@@ -41,3 +42,17 @@ def test_arrays_of_every_kind(eng, cuda_ready, kind, dim, iso):
     assert torch.equal(at.I.cpu(), torch.from_numpy(I).float())
     assert torch.equal(at.x.cpu(), torch.from_numpy(x).float())
     assert torch.equal(at.r.cpu(), torch.from_numpy(r[:, 0] if iso else r).float())
+
+
+@pytest.mark.parametrize("iso", [False, True])
+def test_one_arrays_change_is_its_own(eng, cuda_ready, iso):
+    """An array saved for a backward pass stays valid when another one changes."""
+    I, x, r = make_atoms(3, 5, 1, iso=iso)
+    at = eng.DeviceAtoms(I, x, r)
+    y = (at.I.requires_grad_() ** 2).sum()
+    with torch.no_grad():
+        at.x += 1.0
+        at.r *= 2.0
+    y.backward()
+    assert torch.equal(at.I.grad, 2 * at.I.detach())
+    assert torch.allclose(at.x.cpu(), torch.from_numpy(x).float() + 1)
