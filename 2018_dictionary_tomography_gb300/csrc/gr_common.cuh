@@ -425,9 +425,11 @@ __device__ __forceinline__ void psf_setup(const Atoms &at, int j, const Geom &g,
     const DetAxis &ax = g.ax[k];
     const float c = (p.qh[k] - ax.first) * ax.inv_step;
     // (no cell beyond rr + s counts; the slack covers how far an axis accepted as
-    // uniform, to 1e-4 of a step a cell, strays from first + k / inv_step, and
-    // rounding.  A whole cell of slack doubled the cells looked at.)
-    const float h = (q.rr + s) * ax.inv_step + fmaf(1e-4f, (float)ax.n, 0.01f);
+    // uniform, to 1e-4 of a step a cell, strays from first + k / inv_step, and the
+    // rounding of the centre, which counts on a detector far from the origin.  A
+    // whole cell of slack doubled the cells looked at.)
+    const float h = fmaf(q.rr + s + 1.2e-7f * (fabsf(p.qh[k]) + fabsf(ax.first)), ax.inv_step,
+                         fmaf(1e-4f, (float)ax.n, 0.01f));
     const float lo = ceilf(c - h), hi = floorf(c + h);
     const bool fin = ok && (lo == lo) && (hi == hi) && fabsf(c) < 1e8f && h < 1e8f;
     q.lo[k] = fin ? max(0, (int)lo) : 1;
