@@ -548,13 +548,6 @@ __device__ __forceinline__ void pair_add(float &s, float &c, float t, float d) {
   s = h;
   c += d + e;
 }
-__device__ __forceinline__ void pair_warp_sum(float &s, float &c) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float t = __shfl_xor_sync(0xffffffffu, s, o), d = __shfl_xor_sync(0xffffffffu, c, o);
-    pair_add(s, c, t, d);
-  }
-}
 
 __device__ __forceinline__ double warp_sum_d(double v) {
 #pragma unroll

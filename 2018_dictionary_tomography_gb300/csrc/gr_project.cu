@@ -443,23 +443,19 @@ __global__ void __launch_bounds__(NW * 32, 32 / NW)
       lcmp += (fabsf(lsum) >= fabsf(l)) ? ((lsum - tt) + l) : ((l - tt) + lsum);
       lsum = tt;
     }
-    if (out.loss_part) {
-      // the block's sum as an FP32 pair (exact two-sums, about 46 bits), FP64
-      // from the item's partial on: 12 conversions and adds an item would
-      // hold the SM's FP64 pipe, at 16 cycles each, longer than its memory
-      s_loss[tid] = make_float2(lsum, lcmp);
-      __syncthreads();
-      if (warp == 0) {
-#pragma unroll
-        for (int w = 1; w < NW; ++w)
-          pair_add(lsum, lcmp, s_loss[32 * w + lane].x, s_loss[32 * w + lane].y);
-        pair_warp_sum(lsum, lcmp);
-        if (lane == 0) out.loss_part[item] = (double)lsum + (double)lcmp;
-      }
-    }
+    if (out.loss_part) s_loss[tid] = make_float2(lsum, lcmp);
     if (tid == 0) s_item = ahead;
-    __syncthreads();  // sV, s_count and s_loss are reused
+    __syncthreads();  // sV and s_count are reused
     take = s_item;
+    if (out.loss_part && warp == 0) {
+      // a column's cells as an FP32 pair, the columns in FP64 (the other warps go
+      // on: s_loss and s_item are written again behind the next item's barriers)
+#pragma unroll
+      for (int w = 1; w < NW; ++w)
+        pair_add(lsum, lcmp, s_loss[32 * w + lane].x, s_loss[32 * w + lane].y);
+      const double d = warp_sum_d((double)lsum + (double)lcmp);
+      if (lane == 0) out.loss_part[item] = d;
+    }
   }
 
   if (loss_out && out.loss_part) {
@@ -964,9 +960,9 @@ __global__ void __launch_bounds__(kPsfTileWarps * 32, 8)
 #pragma unroll
     for (int w = 1; w < kPsfTileWarps; ++w)
       pair_add(lsum, lcmp, s_loss[32 * w + lane].x, s_loss[32 * w + lane].y);
-    pair_warp_sum(lsum, lcmp);
+    const double d = warp_sum_d((double)lsum + (double)lcmp);
     if (lane == 0) {
-      out.loss_part[item] = (double)lsum + (double)lcmp;
+      out.loss_part[item] = d;
       if (loss_out) {
         __threadfence();
         s_last = atomicAdd(done, 1) == n_items - 1;
