@@ -459,27 +459,33 @@ __device__ __forceinline__ int psf_cell_kind(const PsfPair<K> &q, const float *d
 }
 
 // A row of the 3D quadrature: its 11 points two to a register pair (1..10, then
-// 11), exponent e(d) = c + d (u + g d) in powers of two.
+// 11).  The form m(d) = t + d (u + G11 d) is scaled by -30 log2 e once (with the
+// factor in each coefficient, a fused operation a pair less, every coefficient
+// is rounded once more).
 struct PsfRow {
   F2 d[5];
-  float last, g;
-  F2 g2;
-  __device__ __forceinline__ PsfRow(float base, float step, float G11) {
+  float last, g, l2amp;
+  F2 g2, amp;
+  __device__ __forceinline__ PsfRow(float base, float step, float G11, float l2a) {
 #pragma unroll
     for (int i = 0; i < 5; ++i)
       d[i] = f2_fma(f2((float)(2 * i + 1), (float)(2 * i + 2)), f2(step, step), f2(base, base));
     last = fmaf(11.f, step, base);
-    g = G11 * kNegThirtyLog2e;
+    g = G11;
     g2 = f2(g, g);
+    l2amp = l2a;
+    amp = f2(l2a, l2a);
   }
   // weights of points 2i + 1 and 2i + 2, and of point 11
-  __device__ __forceinline__ F2 pair(int i, F2 u, F2 c) const {
+  __device__ __forceinline__ F2 pair(int i, F2 u, F2 t) const {
+    const F2 m = f2_fma(d[i], f2_fma(g2, d[i], u), t);
     float x, y;
-    f2_get(f2_fma(d[i], f2_fma(g2, d[i], u), c), x, y);
+    f2_get(f2_fma(m, f2(kNegThirtyLog2e, kNegThirtyLog2e), amp), x, y);
     return f2(ex2_approx(x), ex2_approx(y));
   }
-  __device__ __forceinline__ float end(float u, float c) const {
-    return ex2_approx(fmaf(last, fmaf(g, last, u), c));
+  __device__ __forceinline__ float end(float u, float t) const {
+    const float m = fmaf(last, fmaf(g, last, u), t);
+    return ex2_approx(fmaf(m, kNegThirtyLog2e, l2amp));
   }
 };
 
@@ -499,18 +505,17 @@ __device__ __forceinline__ float psf_quadrature(const Pair<K> &p, const float *b
     }
     return sum * (10.f * step[0] / 11.f);
   } else {
-    const PsfRow row(base[1], step[1], p.G[2]);
-    const float g0 = p.G[0] * kNegThirtyLog2e, g1 = 2.f * p.G[1] * kNegThirtyLog2e;
+    const PsfRow row(base[1], step[1], p.G[2], p.l2amp);
     F2 sum = f2(0.f, 0.f);
     float sum1 = 0.f;
 #pragma unroll 1
     for (int t = 1; t <= 11; ++t) {
       const float d0 = fmaf((float)t, step[0], base[0]);
-      const float c = fmaf(g0 * d0, d0, p.l2amp), u = g1 * d0;
-      const F2 cp = f2(c, c), up = f2(u, u);
+      const float t0 = p.G[0] * d0 * d0, u = 2.f * p.G[1] * d0;
+      const F2 tp = f2(t0, t0), up = f2(u, u);
 #pragma unroll
-      for (int i = 0; i < 5; ++i) sum = f2_add(sum, row.pair(i, up, cp));
-      sum1 += row.end(u, c);
+      for (int i = 0; i < 5; ++i) sum = f2_add(sum, row.pair(i, up, tp));
+      sum1 += row.end(u, t0);
     }
     float s0, s1;
     f2_get(sum, s0, s1);

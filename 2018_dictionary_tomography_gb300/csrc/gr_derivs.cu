@@ -1141,24 +1141,23 @@ __global__ void __launch_bounds__(32 * kPsfWarps, ORDER == 1 ? 4 : 2)
         float M[NM];
 #pragma unroll
         for (int i = 0; i < NM; ++i) M[i] = 0.f;
-        const PsfRow row(base[1], step[1], p.G[2]);
-        const float g0 = p.G[0] * kNegThirtyLog2e, g1 = 2.f * p.G[1] * kNegThirtyLog2e;
+        const PsfRow row(base[1], step[1], p.G[2], l2n);
 #pragma unroll 1
         for (int t = 1; t <= 11; ++t) {
           const float d0 = fmaf((float)t, step[0], base[0]);
-          const float c0 = fmaf(g0 * d0, d0, l2n), u = g1 * d0;
-          const F2 cp = f2(c0, c0), up = f2(u, u);
+          const float t0 = p.G[0] * d0 * d0, u = 2.f * p.G[1] * d0;
+          const F2 tp = f2(t0, t0), up = f2(u, u);
           F2 S2[DEG + 1];
 #pragma unroll
           for (int v = 0; v < 5; ++v) {
-            F2 w = row.pair(v, up, cp);
+            F2 w = row.pair(v, up, tp);
 #pragma unroll
             for (int i = 0; i <= DEG; ++i) {
               S2[i] = v == 0 ? w : f2_add(S2[i], w);
               if (i < DEG) w = f2_mul(w, row.d[v]);
             }
           }
-          float w = row.end(u, c0);
+          float w = row.end(u, t0);
           float S[DEG + 1];
 #pragma unroll
           for (int i = 0; i <= DEG; ++i) {
