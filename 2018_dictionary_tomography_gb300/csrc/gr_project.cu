@@ -479,16 +479,25 @@ __global__ void __launch_bounds__(NW * 32, 32 / NW)
 // the bitmap is written once: no clear, and no global atomics (whose latency
 // and contention bounded the launch before).  Instruction issue bounds it (89 % of
 // the slots, 500 a warp of pairs): four divisions by the tile's sides were a
-// fifth of them (8192 atoms x 20000: 3.05 ms, 2.46 with shifts).
+// fifth of them (8192 atoms x 20000: 3.05 ms, 2.46 with shifts).  In a range a
+// thread goes through its tiles there only (all of them in every range: 2.3 ms
+// for one atom across 2048^2 cells, 1024 cells wide 600 atoms x 60: 272 us; 10 and
+// 89 us so).  Where atoms and angles give few blocks, the ranges are dealt to
+// blocks of their own (kBinFewBlocks, two an SM: one narrow atom x 2048^2 31 ->
+// 3.6 us, 5000 x 1024^2 16.5 -> 5.6 us; from there on a block takes all ranges, so
+// that a pair is set up once).
 // counters (nullable): zeroed, for the projection that follows.
+// Each block takes the ranges z, z + gridDim.z, ... of its atoms and angle.
 constexpr int kBinTiles = 512;
+constexpr int kBinOwnTiles = 32;
+constexpr int kBinFewBlocks = 304;
 __global__ void __launch_bounds__(256)
     gr_bin3d_kernel(Atoms at, Geom g, TileCfg tc, uint32_t *bitmap, int W, Proj3Rec *rec,
                     int *counters, uint32_t *flag, int *list, int *n_list) {
   __shared__ uint32_t sw[kBinTiles][8];
   const int tid = threadIdx.x, a = blockIdx.y, w0 = 8 * blockIdx.x;
   const int j = 32 * w0 + tid;
-  if (counters && blockIdx.x == 0 && a == 0 && tid < 4) counters[tid] = 0;
+  if (counters && blockIdx.x == 0 && a == 0 && blockIdx.z == 0 && tid < 4) counters[tid] = 0;
   int r_lo = 1, r_hi = 0, c_lo = 1, c_hi = 0;
   if (j < at.n) {
     Frame<2> f;
@@ -501,21 +510,45 @@ __global__ void __launch_bounds__(256)
       r_hi = p.hi[0] >> sh;
       c_lo = p.lo[1] / kTileDim1;
       c_hi = p.hi[1] / kTileDim1;
-      if (rec) rec[(size_t)a * at.n + j] = proj3_record(p);
+      if (rec && blockIdx.z == 0) rec[(size_t)a * at.n + j] = proj3_record(p);
     }
   }
   const uint32_t bit = 1u << (j & 31);
   const int nw = min(8, W - w0);
-  for (int t0 = 0; t0 < tc.ntiles; t0 += kBinTiles) {
+  const int first = kBinTiles * blockIdx.z, stride = kBinTiles * gridDim.z;
+  for (int t0 = first; t0 < tc.ntiles; t0 += stride) {
     const int nt = min(kBinTiles, tc.ntiles - t0);
-    if (t0 > 0) __syncthreads();
+    if (t0 > first) __syncthreads();
     for (int e = tid; e < nt * 8; e += 256) (&sw[0][0])[e] = 0u;
+    // the thread's tiles among these: rows of tiles r_a .. r_b, the first and
+    // last of which may lie in the range only in part
+    int r_a = r_lo, r_b = r_hi;
+    if (nt < tc.ntiles) {
+      r_a = max(r_a, tile_div(t0, tc.nt1, tc.inv_nt1));
+      r_b = min(r_b, tile_div(t0 + nt - 1, tc.nt1, tc.inv_nt1));
+    }
+    const int width = c_hi - c_lo + 1, own = max(r_b - r_a + 1, 0) * width;
     __syncthreads();
-    for (int r = r_lo; r <= r_hi; ++r)
-      for (int c = c_lo; c <= c_hi; ++c) {
-        const int t = r * tc.nt1 + c - t0;
-        if (t >= 0 && t < nt) atomicOr(&sw[t][tid >> 5], bit);
-      }
+    auto set = [&](int r, int c, uint32_t b) {
+      const int t = r * tc.nt1 + c - t0;
+      if (t >= 0 && t < nt) atomicOr(&sw[t][tid >> 5], b);
+    };
+    // a lane sets its own atom's tiles; where a few wide supports would keep the
+    // others waiting (an atom's tiles shared out cost some four times as much a
+    // tile), the lanes set theirs together
+    uint32_t wide = __ballot_sync(0xffffffffu, own > kBinOwnTiles);
+    if (wide && __reduce_add_sync(0xffffffffu, own) >= 8 * __reduce_max_sync(0xffffffffu, own))
+      wide = 0u;
+    if (!(wide >> (tid & 31) & 1u))
+      for (int r = r_a; r <= r_b; ++r)
+        for (int c = c_lo; c <= c_hi; ++c) set(r, c, bit);
+    while (wide) {
+      const int src = __ffs(wide) - 1;
+      wide &= wide - 1;
+      const int n = __shfl_sync(0xffffffffu, own, src), w = __shfl_sync(0xffffffffu, width, src);
+      const int ra = __shfl_sync(0xffffffffu, r_a, src), ca = __shfl_sync(0xffffffffu, c_lo, src);
+      for (int e = tid & 31; e < n; e += 32) set(ra + e / w, ca + e % w, 1u << src);
+    }
     __syncthreads();
     const size_t base = (size_t)a * tc.ntiles + t0;
     for (int e0 = 0; e0 < nt * 8; e0 += 256) {
@@ -1017,6 +1050,13 @@ __global__ void __launch_bounds__(kLossThreads)
   if (threadIdx.x == 0) out[0] = sh[0];
 }
 
+static dim3 bin3d_grid(int W, int n_angles, int ntiles) {
+  const long long blocks = (long long)((W + 7) / 8) * n_angles;
+  const int ranges = (ntiles + kBinTiles - 1) / kBinTiles;
+  const long long z = blocks < kBinFewBlocks ? (kBinFewBlocks + blocks - 1) / blocks : 1;
+  return dim3((W + 7) / 8, n_angles, (unsigned)(z < ranges ? z : ranges));
+}
+
 // Tiling of the point-sampled 3D projection (Tuning::proj_form, key 3):
 // 1: 16-row tiles (more resident warps), 2: 32-row tiles (fewer atoms cut
 // by tile edges).
@@ -1228,7 +1268,7 @@ int launch_project(const Atoms &at, const Geom &g, const ProjOut &o_in,
       if (oc.loss_part) oc.loss_part += i0;
       uint32_t *bm = bitmap + i0 * W;
       if (W > 0 && !record) {
-        gr_bin3d_kernel<<<dim3((W + 7) / 8, gr.n_angles), 256, 0, stream>>>(
+        gr_bin3d_kernel<<<bin3d_grid(W, gr.n_angles, tc.ntiles), 256, 0, stream>>>(
             at, gr, tc, bm, W, rec, skip ? nullptr : next_item,
             skip ? flag : nullptr, item_list, next_item + 2);
         note_launches(1);
