@@ -1063,9 +1063,14 @@ static dim3 bin3d_grid(int W, int n_angles, int ntiles) {
 static int proj_rows(int form) { return form == 2 ? kTileDim0 : 16; }
 
 // Loss partials of up to this many items are summed by the projection's last
-// block (sum_partials_block: a chain of n / 512 FP64 adds, 2 us for 16384);
-// above it gr_loss_finalize_kernel does it (6 to 9 us and a launch).
-constexpr size_t kFusedLossItems = 16384;
+// block (sum_partials_block), more by gr_loss_finalize_kernel (7 us and a launch).
+// With a block per item each block has a fence and an atomic to end with, and a
+// block's short life pays for them; the persistent 3D blocks do it once.  Fused
+// and separate, whole forward (us): 2D, 4 atoms x 510 cells: 3280 items 17.9 and
+// 20.6, 6400: 24.7 and 24.0, 16384: 43.0 and 34.8; pixel-integrated 3D: 2550:
+// 25.8 and 28.9, 5100: 37.4 and 37.4, 10200: 63.3 and 59.8; 3D, 20 atoms x 70^2:
+// 7695: 31.7 and 33.4, 10350: 39.3 and 39.2, 13500: 47.6 and 45.9.
+constexpr size_t kFusedLossItems = 5120, kFusedLossItems3D = 10240;
 
 template <int NW>
 static void launch_project3d(size_t items, const Atoms &at, const Geom &g, const TileCfg &tc,
@@ -1253,7 +1258,7 @@ int launch_project(const Atoms &at, const Geom &g, const ProjOut &o_in,
       range = g.n_angles;
     }
     const size_t cells = (size_t)D0 * D1;
-    fused_loss = loss_out != nullptr && items <= kFusedLossItems && range == (size_t)g.n_angles;
+    fused_loss = loss_out != nullptr && items <= kFusedLossItems3D && range == (size_t)g.n_angles;
     double *lo = fused_loss ? loss_out : nullptr;
     for (size_t a0 = 0; a0 < (size_t)g.n_angles; a0 += range) {
       Geom gr = g;
