@@ -878,26 +878,27 @@ __global__ void __launch_bounds__(32, QUAD ? 28 : 32)
 // "total mass" cells zero derivatives).  The pair's sums
 //   Sa = sum alpha A_cell, Ta = sum alpha BC_cell, Ub = sum beta A_cell A_cell^T
 // feed the same chain-rule assembly as the point-sampled kernel.
-// A block's 32 pairs: the sums over an atom's pairs, in angle order.
+// A block's 32 pairs: the sums over an atom's pairs, in angle order, as FP32 pairs
+// (a Hessian's 28 or 66 values in FP64 held the SM's FP64 pipe for half of the time
+// of 2154 x 736 narrow pairs: 243 and 119 us).
 template <int QN>
 __device__ __forceinline__ void psf_close(const float (*vals)[QN + 1], int n_atoms,
                                           const DerivCfg &cfg, int chunk, int wa, float *part) {
   for (int e = threadIdx.x; e < cfg.ag * QN; e += blockDim.x) {
     const int t = e / QN, q = e - t * QN;
     if (wa * cfg.ag + t >= n_atoms) continue;
-    double v = 0.0;
-    for (int k = 0; k < cfg.sg; ++k) v += (double)vals[t + k * cfg.ag][q];
-    part[((size_t)chunk * cfg.qn + q) * n_atoms + wa * cfg.ag + t] = (float)v;
+    float v = 0.f, c = 0.f;
+    for (int k = 0; k < cfg.sg; ++k) pair_add(v, c, vals[t + k * cfg.ag][q], 0.f);
+    part[((size_t)chunk * cfg.qn + q) * n_atoms + wa * cfg.ag + t] = v + c;
   }
 }
 
 // 2D: a block takes 32 (atom, angle) pairs at a time (as a warp of the other
-// kernels does), four lanes each, which share the pair's few cells (11 points
+// kernels does), L lanes each, which share the pair's few cells (11 points
 // each); a pair's first lane assembles, and the block adds its pairs' values per
 // atom.
-constexpr int kPsfLanes = 4;
-template <int ORDER>
-__global__ void __launch_bounds__(32 * kPsfLanes)
+template <int ORDER, int L>
+__global__ void __launch_bounds__(32 * L)
     gr_psf_deriv1d_kernel(Atoms at, Geom g, DerivIn in, DerivCfg cfg, float *part, float s) {
   constexpr int K = 1;
   constexpr int P = n_par<K>();
@@ -909,8 +910,8 @@ __global__ void __launch_bounds__(32 * kPsfLanes)
   constexpr int NT = ORDER > 1 ? NPSI * (NPSI + 1) / 2 : 1;   // upper triangles
   __shared__ float vals[32][QN + 1];
   const int gw = blockIdx.x;
-  const int pr = threadIdx.x / kPsfLanes, gl = threadIdx.x % kPsfLanes;
-  const unsigned gmask = ((1u << kPsfLanes) - 1u) << ((threadIdx.x & 31) & ~(kPsfLanes - 1));
+  const int pr = threadIdx.x / L, gl = threadIdx.x % L;
+  const unsigned gmask = ((1u << L) - 1u) << ((threadIdx.x & 31) & ~(L - 1));
   const int warps_atoms = (at.n + cfg.ag - 1) / cfg.ag;
   const int chunk = gw / warps_atoms, wa = gw - chunk * warps_atoms;
   const int j = wa * cfg.ag + (pr % cfg.ag);   // slot
@@ -943,7 +944,7 @@ __global__ void __launch_bounds__(32 * kPsfLanes)
     for (int k = 0; k < NPSI; ++k) Sa[k] = 0.f;
 #pragma unroll
     for (int k = 0; k < NT; ++k) Tt[k] = Ut[k] = 0.f;
-    for (int k0 = q.lo[0] + gl; k0 <= q.hi[0]; k0 += kPsfLanes) {
+    for (int k0 = q.lo[0] + gl; k0 <= q.hi[0]; k0 += L) {
       float dc[K], base[K], step[K];
       dc[0] = (__ldg(g.ax[0].coords + k0) - p.qh[0]) - p.ql[0];
       const int kind = psf_cell_kind<K>(q, dc, s, base, step);
@@ -1007,7 +1008,7 @@ __global__ void __launch_bounds__(32 * kPsfLanes)
     }
     __syncwarp(gmask);
 #pragma unroll
-    for (int o = kPsfLanes / 2; o > 0; o >>= 1) {
+    for (int o = L / 2; o > 0; o >>= 1) {
       fa += __shfl_xor_sync(gmask, fa, o);
 #pragma unroll
       for (int k = 0; k < NPSI; ++k) Sa[k] += __shfl_xor_sync(gmask, Sa[k], o);
@@ -1049,15 +1050,16 @@ __global__ void __launch_bounds__(32 * kPsfLanes)
   psf_close<QN>(vals, at.n, cfg, chunk, wa, part);
 }
 
-// 3D: a block takes 32 (atom, angle) pairs at a time, a warp eight of them.  The
+// 3D: a block takes 32 (atom, angle) pairs at a time, a warp PW of them.  The
 // warp's lanes look over a pair's cell box and queue the cells it reaches; 32
 // queued cells at a time, of as many pairs as that takes, are summed over their
-// 121 points, two to a register pair (this bounds it), and reduced pair by pair
-// into shared memory.  A lane per pair then assembles, and the block adds its
-// pairs' values per atom.  128 atoms x 401 x 64^2, gradient: 163 us with a lane
+// 121 points, two to a register pair (this bounds it), and reduced into shared
+// memory.  A lane per pair sets up and assembles, and the block adds its pairs'
+// values per atom.  128 atoms x 401 x 64^2, gradient: 163 us with a lane
 // per pair, which walked some 40 cells in series on 10 warps an SM; 143 us with
-// eight lanes a pair, 12 of 32 lanes at work; with the queue 66 us.
-constexpr int kPsfWarps = 4, kPsfPairs = 8;
+// eight lanes a pair, 12 of 32 lanes at work; with the queue and PW = 8 69 us.
+// Narrow supports are set-up and assembly above all, of which PW = 8 does four
+// times the instructions (start_psf).
 
 struct PsfWalk {
   float4 a, b;        // qh0 ql0 qh1 ql1; G00 G01 G11 log2 n
@@ -1066,10 +1068,11 @@ struct PsfWalk {
   int lo0, lo1, bw, ncell;
 };
 
-template <int ORDER>
-__global__ void __launch_bounds__(32 * kPsfWarps, ORDER == 1 ? 4 : 2)
+template <int ORDER, int PW>
+__global__ void __launch_bounds__(1024 / PW, (ORDER == 1 ? 16 : 8) * PW / 32)
     gr_psf_deriv_kernel(Atoms at, Geom g, DerivIn in, DerivCfg cfg, float *part, float s) {
   constexpr int K = 2;
+  constexpr int NW = 32 / PW;
   constexpr int P = n_par<K>();
   constexpr int NPSI = n_psi<K>();
   constexpr int DEG = ORDER == 1 ? 2 : 4;
@@ -1079,21 +1082,21 @@ __global__ void __launch_bounds__(32 * kPsfWarps, ORDER == 1 ? 4 : 2)
   constexpr int NT = ORDER > 1 ? NPSI * (NPSI + 1) / 2 : 0;   // upper triangles
   // a cell's sums: f, first order, second order against alpha and against beta
   constexpr int NV = (1 + NPSI + 2 * NT + 7) / 8 * 8;
-  __shared__ PsfWalk s_walk[kPsfWarps][kPsfPairs];
-  __shared__ int2 s_queue[kPsfWarps][64];
-  __shared__ float s_sum[kPsfWarps][kPsfPairs][NV + 1];
-  __shared__ float vals[kPsfWarps * kPsfPairs][QN + 1];
+  __shared__ PsfWalk s_walk[NW][PW];
+  __shared__ int2 s_queue[NW][64];
+  __shared__ float s_sum[NW][PW][NV + 1];
+  __shared__ float vals[32][QN + 1];
   const int gw = blockIdx.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   PsfWalk *walk = s_walk[warp];
   int2 *queue = s_queue[warp];
   float(*sum)[NV + 1] = s_sum[warp];
-  const int pr = warp * kPsfPairs + (lane & (kPsfPairs - 1));
+  const int pr = warp * PW + (lane & (PW - 1));
   const int warps_atoms = (at.n + cfg.ag - 1) / cfg.ag;
   const int chunk = gw / warps_atoms, wa = gw - chunk * warps_atoms;
   const int j = wa * cfg.ag + (pr % cfg.ag);   // slot
   const int sub = pr / cfg.ag;
-  const bool valid = lane < kPsfPairs && j < at.n;
+  const bool valid = lane < PW && j < at.n;
   const int jj = valid ? (at.order ? at.order[j] : j) : 0;  // atom of the slot
   const float I = at.I[jj];
   const int a_lo = chunk * cfg.ch;
@@ -1112,7 +1115,7 @@ __global__ void __launch_bounds__(32 * kPsfWarps, ORDER == 1 ? 4 : 2)
   auto add_cells = [&](int n) {
     const bool on = lane < n;
     const int2 it = queue[on ? lane : n - 1];
-    const int slot = it.x & (kPsfPairs - 1), k0 = it.x >> 3, k1 = it.y;
+    const int slot = it.x & (PW - 1), k0 = it.x >> 5, k1 = it.y;
     const float4 wa4 = walk[slot].a, wb4 = walk[slot].b;
     const float Ij = walk[slot].I;
     float V[NV];
@@ -1211,9 +1214,26 @@ __global__ void __launch_bounds__(32 * kPsfWarps, ORDER == 1 ? 4 : 2)
         }
       }
     }
-    // pair by pair, eight values at a time: halve the values held over three
-    // exchanges, then sum the four lanes that hold the same one
+    // into the pairs' sums: pair by pair, eight values at a time, the values held
+    // halved over three exchanges, then the four lanes that hold the same one
+    // summed.  A Hessian's many values of more pairs than a pair has cells: the
+    // pairs' cells in turn, each lane its own values.
     const int first = __shfl_sync(0xffffffffu, slot, 0), last = __shfl_sync(0xffffffffu, slot, 31);
+    if (ORDER > 1 && last - first > 1) {
+      const unsigned same = __match_any_sync(0xffffffffu, on ? slot : -1 - lane);
+      const int rank = __popc(same & ((1u << lane) - 1u));
+      const int turns = __reduce_max_sync(0xffffffffu, rank) + 1;
+      if (turns <= last - first) {
+        for (int k = 0; k < turns; ++k) {
+          if (on && rank == k) {
+#pragma unroll
+            for (int i = 0; i < 1 + NPSI + 2 * NT; ++i) sum[slot][i] += V[i];
+          }
+          __syncwarp();
+        }
+        return;
+      }
+    }
     for (int sl = first; sl <= last; ++sl) {
       const bool mine = on && slot == sl;
       if (!__any_sync(0xffffffffu, mine)) continue;
@@ -1246,7 +1266,7 @@ __global__ void __launch_bounds__(32 * kPsfWarps, ORDER == 1 ? 4 : 2)
     Frame<K> fr;
     Pair<K> p;
     int ncell = 0;
-    for (int i = lane; i < kPsfPairs * (NV + 1); i += 32) (&sum[0][0])[i] = 0.f;
+    for (int i = lane; i < PW * (NV + 1); i += 32) (&sum[0][0])[i] = 0.f;
     if (on) {
       load_frame<K>(g.frames, a, fr);
       const bool ok = pair_setup<K>(at, jj, fr, g, p);
@@ -1267,7 +1287,7 @@ __global__ void __launch_bounds__(32 * kPsfWarps, ORDER == 1 ? 4 : 2)
     }
     __syncwarp();
     int queued = 0;
-    for (int sl = 0; sl < kPsfPairs; ++sl) {
+    for (int sl = 0; sl < PW; ++sl) {
       const int nc = __shfl_sync(0xffffffffu, ncell, sl);
       if (nc == 0) continue;
       const PsfWalk w = walk[sl];
@@ -1289,7 +1309,7 @@ __global__ void __launch_bounds__(32 * kPsfWarps, ORDER == 1 ? 4 : 2)
           hit = psf_cell_kind<K>(q, dc, s, base, step) != 0;
         }
         const unsigned m = __ballot_sync(0xffffffffu, hit);
-        if (hit) queue[queued + __popc(m & ((1u << lane) - 1u))] = make_int2(k0 << 3 | sl, k1);
+        if (hit) queue[queued + __popc(m & ((1u << lane) - 1u))] = make_int2(k0 << 5 | sl, k1);
         queued += __popc(m);
         __syncwarp();
         if (queued >= 32) {
@@ -1324,7 +1344,7 @@ __global__ void __launch_bounds__(32 * kPsfWarps, ORDER == 1 ? 4 : 2)
     __syncwarp();
   }
 
-  if (lane < kPsfPairs) {
+  if (lane < PW) {
     vals[pr][0] = f;
 #pragma unroll
     for (int i = 0; i < P; ++i) vals[pr][1 + i] = gacc[i].get();
@@ -1642,6 +1662,39 @@ static void start_hess(const DerivArgs &d) {
   }
 }
 
+// Pixel-integrated derivatives.  2D, lanes a pair: as many as keep the blocks'
+// warps to 32 an SM (gradients; Hessians 16), since wide supports want lanes and
+// narrow ones are mostly set-up and assembly, which L lanes do once for 32 / L
+// pairs (us with 4, 2 and 1; gradients, 200 atoms x 100 angles x 467 cells, r = 4:
+// 25, 31, 46; 500 x 130 x 300, r = 4: 38, 41, 43, x 64, r = 30: 15, 13.5, 11.4; 2154
+// x 736 x 75, r = 30: 152, 104, 72; Hessians there: 282, 183, 119).  3D, pairs a
+// warp: all 32 from 2.5 full waves of such blocks on, for the same reason (8 and 32
+// a warp; gradients, 128 x 401 x 64^2, r = 8: 116, 150; 300 x 401, r = 20: 100, 104;
+// 1412 x 907, r = 35: 780, 643; Hessians 233, 296; 229, 214; 1849, 1512).
+constexpr int kPsfSms = 152;
+template <int ORDER>
+static void start_psf(const DerivArgs &d, float s) {
+  auto go = [&](auto kernel, int threads) {
+    kernel<<<d.warps, threads, 0, d.stream>>>(d.at, d.g, d.in, d.cfg, d.part, s);
+  };
+  if (d.g.K == 1) {
+    const long long room = kPsfSms * (ORDER == 1 ? 32 : 16);
+    if (4ll * d.warps <= room) go(gr_psf_deriv1d_kernel<ORDER, 4>, 128);
+    else if (2ll * d.warps <= room) go(gr_psf_deriv1d_kernel<ORDER, 2>, 64);
+    else go(gr_psf_deriv1d_kernel<ORDER, 1>, 32);
+  } else if (d.warps < kPsfSms * (ORDER == 1 ? 40 : 20)) {
+    go(gr_psf_deriv_kernel<ORDER, 8>, 128);
+  } else {
+    go(gr_psf_deriv_kernel<ORDER, 32>, 32);
+  }
+}
+template <int ORDER>
+static int preload_psf() {
+  return preload_fn(gr_psf_deriv1d_kernel<ORDER, 1>) + preload_fn(gr_psf_deriv1d_kernel<ORDER, 2>) +
+         preload_fn(gr_psf_deriv1d_kernel<ORDER, 4>) + preload_fn(gr_psf_deriv_kernel<ORDER, 8>) +
+         preload_fn(gr_psf_deriv_kernel<ORDER, 32>);
+}
+
 int launch_derivs(const Atoms &at, const Geom &g, const DerivIn &in,
                   const DerivOut &out, void *ws, size_t ws_bytes,
                   cudaStream_t stream, const Tuning &t) {
@@ -1669,14 +1722,9 @@ int launch_derivs(const Atoms &at, const Geom &g, const DerivIn &in,
   const float s = 0.5f / g.ax[0].inv_step;  // cell half-width (pixel-integrated operator)
   timer_mark(2, 0, stream);
   if (in.psf) {
-    constexpr int T1 = 32 * kPsfLanes, T2 = 32 * kPsfWarps;
-    if (K == 1) {
-      if (in.order == 1) gr_psf_deriv1d_kernel<1><<<warps, T1, 0, stream>>>(at, g, in, c, part, s);
-      else gr_psf_deriv1d_kernel<2><<<warps, T1, 0, stream>>>(at, g, in, c, part, s);
-    } else {
-      if (in.order == 1) gr_psf_deriv_kernel<1><<<warps, T2, 0, stream>>>(at, g, in, c, part, s);
-      else gr_psf_deriv_kernel<2><<<warps, T2, 0, stream>>>(at, g, in, c, part, s);
-    }
+    const DerivArgs d{at, g, in, c, part, warps, false, stream};
+    if (in.order == 1) start_psf<1>(d, s);
+    else start_psf<2>(d, s);
   } else {
     // at most one angle per lane: a lane's angles a_lo + sub + k sg lie
     // below a_lo + ch
@@ -1765,8 +1813,8 @@ int preload_derivs() {
          preload_fn(gr_grad_kernel<2, true, true, false>) + preload_fn(gr_grad_kernel<2, false, true, false>) +
          preload_fn(gr_grad_kernel<2, true, true, true>) + preload_fn(gr_grad_kernel<2, false, true, true>) +
          preload_fn(gr_grad_kernel<2, true, false, true>) + preload_fn(gr_grad_kernel<2, false, false, true>) +
-         preload_fn(gr_psf_deriv1d_kernel<1>) + preload_fn(gr_psf_deriv1d_kernel<2>) +
-         preload_fn(gr_psf_deriv_kernel<1>) + preload_fn(gr_psf_deriv_kernel<2>) +
+         
+         preload_psf<1>() + preload_psf<2>() +
          preload_fn(gr_deriv_finalize_kernel<1>) + preload_fn(gr_deriv_finalize_kernel<2>) +
          preload_fn(gr_sumsq_kernel) + preload_fn(gr_sumsq_finalize_kernel) +
          preload_fn(gr_batch_deriv_kernel) + preload_fn(gr_batch_finalize_kernel);

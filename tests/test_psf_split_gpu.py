@@ -1,0 +1,42 @@
+"""The pixel-integrated derivatives in each form of their dispatch: 4, 2 and 1 lanes a
+pair in 2D, 8 and 32 pairs a warp in 3D, at the largest number of blocks of one form and
+one more, with supports of one cell and of many.  Tolerance: the repository's FP32 bar,
+1e-5 of the oracle (gradients per parameter entry, Hessians per atom normwise)."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import gauss_oracle as go
+from problems import (atom_normwise_relerr, engine_atoms, engine_geometry, entry_relerr,
+                      make_atoms, make_geometry, relerr)
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-5
+SMS = 152
+# blocks: of 4 atoms for gradients, of one for Hessians (up to 32 or 8 angles)
+LINES = {("2d", 1): (SMS * 8, SMS * 16), ("2d", 2): (SMS * 4, SMS * 8),
+         ("2p5d", 1): (SMS * 40 - 1,), ("2p5d", 2): (SMS * 20 - 1,)}
+
+
+@pytest.mark.parametrize("kind,order,blocks", [(k, o, b + more) for (k, o), bs in LINES.items()
+                                               for b in bs for more in (0, 1)])
+@pytest.mark.parametrize("D,rdiag", [(24, (3, 6)), (9, (0.6, 1.0)), (33, (20, 40))])
+def test_forms(eng, cuda_ready, kind, order, blocks, D, rdiag):
+    N, A = blocks * (4 if order == 1 else 1), 3
+    g = make_geometry(kind, A, D)
+    I, x, r = make_atoms(2 if kind == "2d" else 3, N, N + D, rdiag=rdiag, roff=0.2 * rdiag[0])
+    C = (go.psf_radproj(I[:1] * 1.1, x[:1], r[:1], g) + 0.001).astype(np.float32).astype(np.float64)
+    f, G, H = eng.atom_derivs(engine_atoms(I, x, r), engine_geometry(g), "l2_atom",
+                              torch.from_numpy(C).float(), order=order, psf=True)
+    pick = np.unique(np.concatenate([np.linspace(0, N - 1, 24).astype(int), [1, 2, 3, N - 2]]))
+    out = [go.psf_atom_derivs("l2", I[j], x[j], r[j], g, C, 2) for j in pick]
+    assert relerr(f.cpu().numpy()[pick], np.array([o[0] for o in out])) < TOL
+    assert entry_relerr(G.cpu().numpy()[pick], np.array([o[1] for o in out])) < TOL
+    if order == 2:
+        # (the same atoms alone, in the form for few blocks)
+        few = eng.atom_derivs(engine_atoms(I[pick], x[pick], r[pick]), engine_geometry(g), "l2_atom",
+                              torch.from_numpy(C).float(), order=2, psf=True)[2]
+        assert relerr(H.cpu().numpy()[pick], few.cpu().numpy()) < TOL
+    if order == 2 and rdiag[0] < 20:
+        # (Hessians of supports inside one cell cancel beyond FP32 atom by atom)
+        assert atom_normwise_relerr(H.cpu().numpy()[pick], np.array([o[2] for o in out])) < TOL
