@@ -118,7 +118,17 @@ DerivCfg deriv_cfg(int K, int n_atoms, int n_angles, int order, const Tuning &t,
 // cells of a lane loaded together (even)
 template <int K>
 __host__ __device__ constexpr int walk_cells_of() { return 6; }
-// lanes of a group (8 where a warp has four pairs)
+// Where all pairs of a warp have boxes of at most this many cells along each axis, a
+// lane walks its own pair, two cells at a time: groups would give most of their lanes
+// nothing and pay for the exchange of 16 or 32 sums (us, own lane up to 0, 4, 5, 6, 8,
+// 10, 12, 16 cells: 3364 atoms x 751 x 41^2, r = 30: 432, 307, 307, 307, 307, 307, 307,
+// 307; 7599 x 63 x 24^2, 5 cells: 123, 129, 126, 113, 101, 100, 100, 100; 1000 x 100 x
+// 128^2, r = 7: -, -, -, -, 82, 82, 84, 92; 2D, up to 0, 8, 12, 16, 24, 32, 48, 64 cells:
+// 7293 x 106 x 55: 54, 44, 43, 43, 43, 43, 43, 43; 2150 x 153 x 467, r = 8: 37, -, -, -,
+// 37, 37, 39, 40).
+template <int K>
+__host__ __device__ constexpr int walk_narrow_of() { return K == 1 ? 24 : 8; }
+// lanes of a group (8 where a warp has four pairs; in 2D 4 where it has eight)
 template <int K>
 __host__ __device__ constexpr int walk_lanes_of() { return K == 1 ? 2 : 4; }
 template <int K>
@@ -408,7 +418,16 @@ __device__ __forceinline__ void hess_body(const Atoms &at, const Geom &g, const 
       sm.pair[lane].box = make_int4(1, 0, 1, 0);
     }
     __syncwarp();
-    for (int s0 = 0; s0 < npairs; s0 += NG) {
+    const bool narrow =
+        cfg.rs == 1 && __all_sync(0xffffffffu, !mine || (p.hi[0] - p.lo[0] < walk_narrow_of<K>() &&
+                                                         p.hi[K - 1] - p.lo[K - 1] < walk_narrow_of<K>()));
+    if (narrow) {
+      float v[NV];
+      walk_pair<K, 1, 2, FK>(sm.pair[lane], g, in, a, 0, v);
+#pragma unroll
+      for (int k = 0; k < NV; ++k) sm.sum[lane][k] = v[k];
+    }
+    for (int s0 = narrow ? npairs : 0; s0 < npairs; s0 += NG) {
       const int s = s0 + lane / GL, gl = lane % GL;
       float v[NV];
       walk_pair<K, GL, R, FK>(sm.pair[s < 32 ? s : 31], g, in, a0 + s / cfg.ag, gl, v);
@@ -1654,6 +1673,12 @@ static void start_hess(const DerivArgs &d) {
     if (l2atom) start_one<K, 8, kFieldL2Atom>(d);
     else if (beta) start_one<K, 8, kFieldBeta>(d);
     else start_one<K, 8, kFieldPlain>(d);
+  } else if (K == 1 && d.cfg.rs == 4) {
+    // (64 atoms x 180 x 512, supports of 230 cells, with the closing sums: 23.3 us by
+    // two lanes a pair, half of the warp idle, 17.3 by four)
+    if (l2atom) start_one<K, 4, kFieldL2Atom>(d);
+    else if (beta) start_one<K, 4, kFieldBeta>(d);
+    else start_one<K, 4, kFieldPlain>(d);
   } else {
     constexpr int GL = walk_lanes_of<K>();
     if (l2atom) start_one<K, GL, kFieldL2Atom>(d);
@@ -1768,6 +1793,9 @@ __global__ void __launch_bounds__(128, hess_min_warps(1, true) / 4)
   if (B.cfg.rs == 8)
     hess_body<1, true, 8, walk_cells_of<1>(), kFieldPlain>(
         B.cur, B.g, B.din, B.cfg, B.part, warp0, w);
+  else if (B.cfg.rs == 4)
+    hess_body<1, true, 4, walk_cells_of<1>(), kFieldPlain>(
+        B.cur, B.g, B.din, B.cfg, B.part, warp0, w);
   else
     hess_body<1, true, walk_lanes_of<1>(), walk_cells_of<1>(), kFieldPlain>(
         B.cur, B.g, B.din, B.cfg, B.part, warp0, w);
@@ -1803,6 +1831,7 @@ static int preload_one() {
 template <int K>
 static int preload_walk() {
   return preload_one<K, walk_lanes_of<K>()>() + preload_one<K, 8>() +
+         (K == 1 ? preload_one<K, 4>() : 0) +
          preload_fn(gr_hess_kernel<K, false, walk_lanes_of<K>(), walk_cells_of<K>(), kFieldAny>) +
          preload_fn(gr_grad_kernel<K, true, false, false>) +
          preload_fn(gr_grad_kernel<K, false, false, false>);
