@@ -1069,8 +1069,9 @@ static int proj_rows(int form) { return form == 2 ? kTileDim0 : 16; }
 // and separate, whole forward (us): 2D, 4 atoms x 510 cells: 3280 items 17.9 and
 // 20.6, 6400: 24.7 and 24.0, 16384: 43.0 and 34.8; pixel-integrated 3D: 2550:
 // 25.8 and 28.9, 5100: 37.4 and 37.4, 10200: 63.3 and 59.8; 3D, 20 atoms x 70^2:
-// 7695: 31.7 and 33.4, 10350: 39.3 and 39.2, 13500: 47.6 and 45.9.
-constexpr size_t kFusedLossItems = 5120, kFusedLossItems3D = 10240;
+// 7695: 31.7 and 33.4, 10350: 39.3 and 39.2, 13500: 47.6 and 45.9 (a launch less
+// is 2 us less on the host, too).
+constexpr size_t kFusedLossItems = 5120, kFusedLossItems3D = 12288;
 
 template <int NW>
 static void launch_project3d(size_t items, const Atoms &at, const Geom &g, const TileCfg &tc,

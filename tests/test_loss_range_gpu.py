@@ -30,7 +30,7 @@ def test_loss_of_large_residuals(eng, cuda_ready, kind, form, psf):
 
 @pytest.mark.parametrize("kind,D,psf,line", [("2d", (32, None), False, 5120), ("2d", (32, None), True, 5120),
                                              ("2p5d", (16, 32), True, 5120),
-                                             ("2p5d", (16, 32), False, 10240)])
+                                             ("2p5d", (16, 32), False, 12288)])
 @pytest.mark.parametrize("more", [0, 1])
 def test_loss_on_both_sides_of_the_fused_line(eng, cuda_ready, kind, D, psf, line, more):
     """A tile an angle: the most items that the projection's last block sums, and one more."""
