@@ -27,6 +27,8 @@
 // summed in FP64 in chunk order by gr_deriv_finalize_kernel, which also applies
 // the isotropic chain rule.  No float atomics anywhere: results are bitwise
 // reproducible.
+#include <type_traits>
+
 #include "gr_assembly.cuh"
 
 namespace gr {
@@ -1382,7 +1384,9 @@ __global__ void __launch_bounds__(1024 / PW, (ORDER == 1 ? 16 : 8) * PW / 32)
 // pipes (16 cycles per warp instruction each).  Where an atom has fewer than
 // 64 values, S threads share one, each summing a contiguous range of chunks in
 // chunk order (a dependent FP64 add takes 64 cycles), and the ranges are added
-// in order; a thread loads kFinBatch partials before it adds any.  8192 atoms x
+// in order; a thread loads kFinBatch partials before it adds any.  Ranges of less
+// than kFinBatch chunks gain nothing (fin_shares), and an atom whose values fill half
+// of the threads has half of them (fin_threads: 6298 atoms x 1 chunk 5.4 -> 3.0 us, 3.3 before ranges).  8192 atoms x
 // 625 chunks: 357 -> 244 us (conversions and adds on the FP64 pipe), 1000 x 126:
 // 21.7 -> 13.7 us, 64 x 60: 10.2 -> 5.9 us (one thread per value with four loads
 // in flight before).
@@ -1390,6 +1394,16 @@ constexpr int kFinAtoms = 4;
 constexpr int kFinPer = 64;            // threads per atom
 constexpr int kFinThreads = kFinPer * kFinAtoms;
 constexpr int kFinBatch = 8;
+// threads that share a value of an atom
+__host__ __device__ __forceinline__ int fin_shares(const DerivCfg &cfg) {
+  int S = 1;
+  while (2 * S * cfg.qn <= kFinPer && S < 8 && cfg.nchunks >= 2 * S * kFinBatch) S *= 2;
+  return S;
+}
+// threads of a block
+__host__ __device__ __forceinline__ int fin_threads(const DerivCfg &cfg) {
+  return fin_shares(cfg) * cfg.qn <= kFinPer / 2 ? kFinThreads / 2 : kFinThreads;
+}
 // Gradients as float32 arrays per parameter kind (gr_atom_grads); q = 0 is the
 // value, 1 the intensity.
 template <int D>
@@ -1412,32 +1426,38 @@ __device__ __forceinline__ void finalize_body(const float *part, const DerivCfg 
   __shared__ double ps[kFinPer][kFinAtoms];   // ranges of shared values
   const int tx = threadIdx.x % kFinAtoms, ty = threadIdx.x / kFinAtoms;
   const int slot = block * kFinAtoms + tx;
-  int S = 1;
-  while (2 * S * cfg.qn <= kFinPer && S < 8) S *= 2;
-  // sum of value q over chunks [lo, hi)
-  auto range = [&](int q, int lo, int hi) -> double {
-    const float *src = part + (size_t)q * n + slot;
+  const int S = fin_shares(cfg), per = (int)blockDim.x / kFinAtoms;
+  for (int e = ty; slot < n && e < cfg.qn * S; e += per) {
+    // value q over the s-th of S ranges of chunks
+    const int sh = 31 - __clz(S), q = e >> sh, s = e & (S - 1);
+    int c = (int)((unsigned)cfg.nchunks * s >> sh);   // (8 times the chunks: 32 bits)
+    const int hi = (int)((unsigned)cfg.nchunks * (s + 1) >> sh);
     const size_t step = (size_t)cfg.qn * n;
+    const float *src = part + (size_t)q * n + slot + c * step;
     double t = 0.0;
-    int c = lo;
-    for (; c + kFinBatch <= hi; c += kFinBatch) {
-      float v[kFinBatch];
+    auto add = [&](auto batch) {
+      constexpr int B = decltype(batch)::value;
+      float v[B];
 #pragma unroll
-      for (int i = 0; i < kFinBatch; ++i) v[i] = __ldcs(src + (c + i) * step);
+      for (int i = 0; i < B; ++i) v[i] = __ldcs(src + i * step);
 #pragma unroll
-      for (int i = 0; i < kFinBatch; ++i) t += (double)v[i];
+      for (int i = 0; i < B; ++i) t += (double)v[i];
+      c += B;
+      src += B * step;
+    };
+    while (c + kFinBatch <= hi) add(std::integral_constant<int, kFinBatch>());
+    if (c + 4 <= hi) add(std::integral_constant<int, 4>());
+    if (c < hi) {
+      float v[3];
+#pragma unroll
+      for (int i = 0; i < 3; ++i) v[i] = c + i < hi ? __ldcs(src + i * step) : 0.f;
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+        if (c + i < hi) t += (double)v[i];
     }
-    for (; c < hi; ++c) t += (double)__ldcs(src + c * step);
-    return t;
-  };
-  if (S == 1) {
-    if (slot < n)
-      for (int q = ty; q < cfg.qn; q += kFinPer) vs[q][tx] = range(q, 0, cfg.nchunks);
-  } else {
-    const int q = ty / S, s = ty - q * S;
-    if (slot < n && q < cfg.qn)
-      ps[ty][tx] = range(q, (int)((long long)cfg.nchunks * s / S),
-                         (int)((long long)cfg.nchunks * (s + 1) / S));
+    (S == 1 ? vs[q] : ps[e])[tx] = t;
+  }
+  if (S > 1) {
     __syncthreads();
     if (slot < n && ty < cfg.qn) {
       double t = ps[ty * S][tx];
@@ -1762,10 +1782,10 @@ int launch_derivs(const Atoms &at, const Geom &g, const DerivIn &in,
   timer_mark(2, 1, stream);
   const int fblocks = (at.n + kFinAtoms - 1) / kFinAtoms;
   if (K == 1)
-    gr_deriv_finalize_kernel<1><<<fblocks, kFinThreads, 0, stream>>>(
+    gr_deriv_finalize_kernel<1><<<fblocks, fin_threads(c), 0, stream>>>(
         part, c, at.n, in.order, at.r_iso, out, fe, at.order);
   else
-    gr_deriv_finalize_kernel<2><<<fblocks, kFinThreads, 0, stream>>>(
+    gr_deriv_finalize_kernel<2><<<fblocks, fin_threads(c), 0, stream>>>(
         part, c, at.n, in.order, at.r_iso, out, fe, at.order);
   note_launches(2);
   return cudaGetLastError() == cudaSuccess ? kOk : kErrLaunch;
