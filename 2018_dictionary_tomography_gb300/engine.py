@@ -73,19 +73,26 @@ def _host_f32(a):
 def to_device_packed(arrays, device):
     """Float32 device copies of host arrays, moved with one copy (a small
     host-to-device copy costs 17 us whatever its size).  They share one buffer,
-    each from a multiple of 16 bytes on, but not a version counter: autograd
-    takes an in-place change of one for a change of that one alone."""
+    each from a multiple of 16 bytes on, but no version counter (unsafe_split):
+    autograd takes an in-place change of one for a change of that one alone."""
     host_arrays = [_host_f32(a) for a in arrays]
-    off, n = [], 0
+    sizes, off, n = [], [], 0
     for t in host_arrays:
         off.append(n)
-        n += (t.size + 3) // 4 * 4
+        pad = -t.size % 4
+        sizes += (t.size, pad) if pad else (t.size,)
+        n += t.size + pad
     host = np.zeros(n, dtype=np.float32)
     for o, t in zip(off, host_arrays):
-        host[o:o + t.size] = t.reshape(-1)
-    buf = torch.from_numpy(host).to(device)
-    flat = [buf[o:o + t.size].data for o, t in zip(off, host_arrays)]
-    return [f if t.ndim == 1 else f.view(t.shape) for f, t in zip(flat, host_arrays)]
+        host[o:o + t.size] = t if t.ndim == 1 else t.reshape(-1)
+    parts = iter(torch.unsafe_split_with_sizes(torch.from_numpy(host).to(device), sizes))
+    out = []
+    for t in host_arrays:
+        d = next(parts)
+        out.append(d if t.ndim == 1 else d.view(t.shape))
+        if t.size % 4:
+            next(parts)
+    return out
 
 
 def morton_order(x):
