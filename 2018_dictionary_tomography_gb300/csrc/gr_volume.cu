@@ -219,41 +219,49 @@ __global__ void __launch_bounds__(kVolThreads)
 }
 
 // ---- 3D, point values -------------------------------------------------------
-// A block of 256 threads owns V0 x 16 x 16 voxels (V0 = 8 on large grids), a warp
-// V0 x 4 x 8 of them: a lane a column of V0 voxels along axis 0, its sums in registers.  The block
-// finds the atoms that meet its voxels, kAtoms at a time (a thread each, so an
-// atom is set up once per 2048 voxels), and stages them in index order; each
-// warp ballots them against its own voxels, 32 at a time, and adds those left.
+// A block of 256 threads owns V0 x 16 x 16 voxels (W0 = 1; V0 = 8 on large grids) or
+// 4 x 8 x 8 (W0 = 4, V0 = 1), a warp V0 x 4 x 8 of them: a lane a column of V0 voxels
+// along axis 0, its sums in registers.  The block finds the atoms that meet its
+// voxels, kAtoms at a time (a thread each, so an atom is set up once per 2048 voxels),
+// and stages them in index order; each warp ballots them against its own voxels, 32 at
+// a time, and adds those left; with a voxel a lane it takes all 32 where kVolMost of
+// them are left (a loop of known ends hides the latency of the staged values).
 // Voxels sum their atoms in index order, as above.
 // What bounds it: the scan of all atoms by every block (1000 atoms on 128 x 124
 // x 120 voxels: 13.2 us; with 256 voxels a block, one per thread, 65.7 us: eight
-// times the scans, and every listed atom evaluated at every voxel of the tile).
-constexpr int kVol1 = 16, kVol2 = 16;
-template <int V0>
+// times the scans, and every listed atom evaluated at every voxel of the tile), on
+// small grids the latency of a lane's chain of atoms (4000 atoms on 31^3, r = 1.2 and
+// 8: 1 x 16 x 16 tiles 289 and 27 us, 4 x 8 x 8 158 and 29).
+constexpr int kVolMost = 12;
+template <int V0, int W0>
 __global__ void __launch_bounds__(kVolThreads)
     gr_volproj3_kernel(Atoms at, VolGrid vg, float *u) {
   constexpr int kAtoms = kVolThreads;
   constexpr int NWarp = kVolThreads / 32;
+  constexpr int W1 = W0 == 1 ? 4 : 2, W2 = NWarp / W0 / W1;   // warps along axes 1, 2
+  constexpr int T0 = V0 * W0, T1 = 4 * W1, T2 = 8 * W2;       // the tile
   // centre, r (r00 r11 r22 r01 r12 r02), intensity; half-extents of the support
   __shared__ float4 sX[kAtoms], sR[kAtoms], sQ[kAtoms];
   __shared__ float2 sE[kAtoms];
+  __shared__ float sE0[W0 > 1 ? kAtoms : 1];
   __shared__ int wcount[NWarp];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int nt1 = (vg.n[1] + kVol1 - 1) / kVol1, nt2 = (vg.n[2] + kVol2 - 1) / kVol2;
+  const int nt1 = (vg.n[1] + T1 - 1) / T1, nt2 = (vg.n[2] + T2 - 1) / T2;
   int b = blockIdx.x;
   const int b2 = b % nt2;
   b /= nt2;
   const int b1 = b % nt1, b0 = b / nt1;
-  const int o0 = b0 * V0, o1 = b1 * kVol1, o2 = b2 * kVol2;
-  // the warp's voxels: 4 x 8 columns of the tile's 16 x 16
-  const int w1 = o1 + 4 * (warp >> 1), w2 = o2 + 8 * (warp & 1);
+  const int o0 = b0 * T0, o1 = b1 * T1, o2 = b2 * T2;
+  // the warp's voxels: 4 x 8 columns of V0
+  const int w0 = o0 + V0 * (warp / (W1 * W2));
+  const int w1 = o1 + 4 * (warp / W2 % W1), w2 = o2 + 8 * (warp % W2);
   const int i1 = w1 + (lane >> 3), i2 = w2 + (lane & 7);
   const bool inside = i1 < vg.n[1] && i2 < vg.n[2];
-  const int n0 = min(V0, vg.n[0] - o0);
+  const int n0 = min(V0, vg.n[0] - w0);
   float y0[V0], acc[V0];
 #pragma unroll
   for (int k = 0; k < V0; ++k) {
-    y0[k] = vg.y[0][min(o0 + k, vg.n[0] - 1)];
+    y0[k] = vg.y[0][min(w0 + k, vg.n[0] - 1)];
     acc[k] = 0.f;
   }
   const float y1 = vg.y[1][min(i1, vg.n[1] - 1)], y2 = vg.y[2][min(i2, vg.n[2] - 1)];
@@ -265,9 +273,10 @@ __global__ void __launch_bounds__(kVolThreads)
     hi = fmaxf(p, q);
   };
   float blo[3], bhi[3], wlo[3], whi[3];
-  box(0, o0, V0, blo[0], bhi[0]);
-  box(1, o1, kVol1, blo[1], bhi[1]);
-  box(2, o2, kVol2, blo[2], bhi[2]);
+  box(0, o0, T0, blo[0], bhi[0]);
+  box(1, o1, T1, blo[1], bhi[1]);
+  box(2, o2, T2, blo[2], bhi[2]);
+  box(0, w0, V0, wlo[0], whi[0]);
   box(1, w1, 4, wlo[1], whi[1]);
   box(2, w2, 8, wlo[2], whi[2]);
   constexpr float kNorm = 3.0901936161855166f;  // sqrt(30 / pi)
@@ -309,10 +318,10 @@ __global__ void __launch_bounds__(kVolThreads)
       sR[pos] = make_float4(M[0][0], M[0][1], M[0][2], 0.f);
       sQ[pos] = make_float4(M[1][1], M[1][2], M[2][2], 0.f);
       sE[pos] = make_float2(e[1], e[2]);
+      if constexpr (W0 > 1) sE0[pos] = e[0];
     }
     __syncthreads();
     for (int k0 = 0; k0 < total; k0 += 32) {
-      // (axis 0 is the tile's own for every warp)
       const int k = k0 + lane;
       bool mine = false;
       if (k < total) {
@@ -320,11 +329,12 @@ __global__ void __launch_bounds__(kVolThreads)
         const float2 E = sE[k];
         mine = X.y + E.x >= wlo[1] && X.y - E.x <= whi[1] && X.z + E.y >= wlo[2] &&
                X.z - E.y <= whi[2];
+        // (with one warp along axis 0 the tile's test there was its own)
+        if constexpr (W0 > 1)
+          mine = mine && X.x + sE0[k] >= wlo[0] && X.x - sE0[k] <= whi[0];
       }
       unsigned m = __ballot_sync(0xffffffffu, mine);
-      while (m) {
-        const int q = k0 + __ffs(m) - 1;
-        m &= m - 1;
+      auto add = [&](int q) {
         const float4 X = sX[q], R = sR[q], Q = sQ[q];
         const float Y1 = y1 - X.y, Y2 = y2 - X.z;
         const float t = fmaf(R.y, Y1, R.z * Y2);
@@ -336,6 +346,16 @@ __global__ void __launch_bounds__(kVolThreads)
           const float nn = fmaf(a, a, cd);
           if (nn <= 1.f) acc[k2] = fmaf(X.w, ex2_approx(nn * kNegThirtyLog2e), acc[k2]);
         }
+      };
+      if (V0 == 1 && __popc(m) >= kVolMost) {
+        const int end = min(k0 + 32, total);
+#pragma unroll 8
+        for (int q = k0; q < end; ++q) add(q);
+        continue;
+      }
+      while (m) {
+        add(k0 + __ffs(m) - 1);
+        m &= m - 1;
       }
     }
     __syncthreads();
@@ -343,12 +363,14 @@ __global__ void __launch_bounds__(kVolThreads)
   if (inside)
 #pragma unroll
     for (int k = 0; k < V0; ++k)
-      if (k < n0) u[((size_t)(o0 + k) * vg.n[1] + i1) * vg.n[2] + i2] = acc[k];
+      if (k < n0) u[((size_t)(w0 + k) * vg.n[1] + i1) * vg.n[2] + i2] = acc[k];
 }
 
-// 3D point values: the most voxels a lane (of 8, 4, 2, 1 along axis 0) that still
+// 3D point values: the most voxels a lane (of 8, 4, 2 along axis 0) that still
 // gives two blocks an SM: a block scans all atoms, so few blocks of many voxels
-// leave the SMs idle (16 blocks for 32^3 voxels).
+// leave the SMs idle (16 blocks for 32^3 voxels).  Smaller grids: a voxel a lane in
+// compact tiles, which fewer atoms meet (48^3, 4000 atoms, r = 2.4: 111 us in tiles of
+// 2 x 16 x 16, 95 in 4 x 8 x 8; 64^3: 119 and 137).
 constexpr int kVolBlocks = 304;
 int launch_volproj(const Atoms &at, int dim, const int *n, const float *const *y,
                    float *u, int psf, float s, cudaStream_t stream) {
@@ -364,12 +386,14 @@ int launch_volproj(const Atoms &at, int dim, const int *n, const float *const *y
     else gr_volproj_kernel<2, false><<<blocks, kVolThreads, 0, stream>>>(at, vg, t0, t1, 1, s, u);
   } else {
     if (!psf) {
-      const int nb12 = ((vg.n[1] + kVol1 - 1) / kVol1) * ((vg.n[2] + kVol2 - 1) / kVol2);
-      auto nb = [&](int v) { return ((vg.n[0] + v - 1) / v) * nb12; };
-      if (nb(8) >= kVolBlocks) gr_volproj3_kernel<8><<<nb(8), kVolThreads, 0, stream>>>(at, vg, u);
-      else if (nb(4) >= kVolBlocks) gr_volproj3_kernel<4><<<nb(4), kVolThreads, 0, stream>>>(at, vg, u);
-      else if (nb(2) >= kVolBlocks) gr_volproj3_kernel<2><<<nb(2), kVolThreads, 0, stream>>>(at, vg, u);
-      else gr_volproj3_kernel<1><<<nb(1), kVolThreads, 0, stream>>>(at, vg, u);
+      auto nb = [&](int t0, int t1, int t2) {
+        return ((vg.n[0] + t0 - 1) / t0) * ((vg.n[1] + t1 - 1) / t1) * ((vg.n[2] + t2 - 1) / t2);
+      };
+      const int b8 = nb(8, 16, 16), b4 = nb(4, 16, 16), b2 = nb(2, 16, 16), b1 = nb(4, 8, 8);
+      if (b8 >= kVolBlocks) gr_volproj3_kernel<8, 1><<<b8, kVolThreads, 0, stream>>>(at, vg, u);
+      else if (b4 >= kVolBlocks) gr_volproj3_kernel<4, 1><<<b4, kVolThreads, 0, stream>>>(at, vg, u);
+      else if (b2 >= kVolBlocks) gr_volproj3_kernel<2, 1><<<b2, kVolThreads, 0, stream>>>(at, vg, u);
+      else gr_volproj3_kernel<1, 4><<<b1, kVolThreads, 0, stream>>>(at, vg, u);
       note_launches(1);
       return cudaGetLastError() == cudaSuccess ? kOk : kErrLaunch;
     }
@@ -383,9 +407,9 @@ int launch_volproj(const Atoms &at, int dim, const int *n, const float *const *y
 }
 
 int preload_volume() {
-  return preload_fn(gr_volproj_kernel<2, false>) + preload_fn(gr_volproj3_kernel<8>) +
-         preload_fn(gr_volproj3_kernel<4>) + preload_fn(gr_volproj3_kernel<2>) +
-         preload_fn(gr_volproj3_kernel<1>) +
+  return preload_fn(gr_volproj_kernel<2, false>) + preload_fn(gr_volproj3_kernel<8, 1>) +
+         preload_fn(gr_volproj3_kernel<4, 1>) + preload_fn(gr_volproj3_kernel<2, 1>) +
+         preload_fn(gr_volproj3_kernel<1, 4>) +
          preload_fn(gr_volproj_kernel<2, true>) + preload_fn(gr_volproj_kernel<3, true>);
 }
 
