@@ -1153,16 +1153,29 @@ size_t project_min_bytes(int K, int n_atoms, int n_angles, int D0, int D1, const
 
 // 3D pair records: setting a pair up again in each of the 1.3 to 2.5 tiles it
 // touches took 40 % of the projection (8.4 of 20.9 ms on 8192 atoms x 20000
-// orientations), so the binning writes each pair's 32-byte record once.  Problems whose records pass
-// kRecBytes run in ranges of angles, each binned and projected in turn.
+// orientations), so the binning writes each pair's 32-byte record once.  Problems
+// whose records pass kRecBytes run in ranges of angles, each binned and projected in
+// turn.  A range must fill the GPU many times over: 8192 atoms x 2000 x 128^2 in
+// ranges of 512, 4096, 16384 and 64000 items 7.9, 3.1, 2.25 and 2.01 ms, without
+// records 2.18; 20000 x 60 x 64^2 in 15 ranges of 32 items 2.45 ms, without 0.26.  So
+// ranges of fewer than kRangeItems are not taken: then no records.
 constexpr size_t kRecBytes = (size_t)512 << 20;
+constexpr size_t kRangeItems = 32768;
+
+// Angles whose records `bytes` hold and that are taken at a time (0: no records).
+static size_t record_range(size_t bytes, int n_atoms, int n_angles, int ntiles) {
+  const size_t row = (size_t)n_atoms * sizeof(Proj3Rec), range = row > 0 ? bytes / row : 0;
+  if (range >= (size_t)n_angles) return n_angles;
+  return range * ntiles >= kRangeItems ? range : 0;
+}
 
 size_t project_workspace_bytes(int K, int n_atoms, int n_angles, int D0, int D1,
                                const Tuning &t) {
   size_t bytes = project_min_bytes(K, n_atoms, n_angles, D0, D1, t);
   if (K == 2) {
-    const size_t row = (size_t)n_atoms * sizeof(Proj3Rec), all = row * (size_t)n_angles;
-    bytes += align_up(all <= kRecBytes ? all : (row <= kRecBytes ? kRecBytes / row * row : row));
+    const int ntiles = make_tiles(2, D0, D1, proj_rows(t.proj_form)).ntiles;
+    bytes += align_up(record_range(kRecBytes, n_atoms, n_angles, ntiles) * n_atoms *
+                      sizeof(Proj3Rec));
   }
   return bytes;
 }
@@ -1249,11 +1262,9 @@ int launch_project(const Atoms &at, const Geom &g, const ProjOut &o_in,
   if (point3) {
     // records: as many angles at a time as the workspace holds; a skipping
     // forward (one list of items) takes all angles at once or none
-    const size_t row = (size_t)at.n * sizeof(Proj3Rec);
     const size_t base = align_up(need);
     Proj3Rec *rec = reinterpret_cast<Proj3Rec *>(static_cast<char *>(ws) + base);
-    size_t range = row > 0 && ws_bytes > base ? (ws_bytes - base) / row : 0;
-    if (range > (size_t)g.n_angles) range = g.n_angles;
+    size_t range = ws_bytes > base ? record_range(ws_bytes - base, at.n, g.n_angles, tc.ntiles) : 0;
     if (range == 0 || record || (skip && range < (size_t)g.n_angles)) {
       rec = nullptr;
       range = g.n_angles;

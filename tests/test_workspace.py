@@ -104,3 +104,59 @@ def test_queried_workspace_is_not_passed(eng, cuda_ready, N, A, order, psf, mode
     out = [derivs({"inner": "ip", "l2_atom": "l2"}[mode], I[j], x[j], r[j], g, C, 2) for j in pick]
     assert relerr(f.cpu().numpy()[pick], np.array([o[0] for o in out])) < TOL
     assert entry_relerr(G.cpu().numpy()[pick], np.array([o[1] for o in out])) < TOL
+
+
+@pytest.mark.parametrize("n,A,D", [(8192, 20000, 128), (1000000, 64, 64), (40, 60, 32), (8192, 2049, 16)])
+def test_records_are_asked_for_where_they_are_used_without_gpu(n, A, D):
+    """Up to 512 MB of records of all angles, or of ranges of 32768 items and more."""
+    lib = LIB.load()
+    at, g = host_problem(2, n, A, D)
+    at0, g0 = host_problem(2, n, A, D)
+    tiles = -(-D // 16) * -(-D // 32)
+    rng = min(A, (512 << 20) // (32 * n))
+    want = rng * n * 32 if rng == A or rng * tiles >= 32768 else 0
+    have = lib.gr_workspace_bytes(LIB.GR_OP_PROJECT, ctypes.byref(at), ctypes.byref(g))
+    least = 256 + 4 * (A * tiles * (-(-n // 32) + 1)) + 12 * A * tiles + 2048   # all but the records
+    assert want <= have - least + 4096 and have <= want + least + 4096, (have, want, least)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("angles", [0, 1, 7, 59, 60])
+def test_few_records_do_not_split_a_projection(eng, cuda_ready, angles):
+    """Room for the records of some angles, too few for the GPU at a time: one launch each of
+    binning and projection, the same bits."""
+    lib = LIB.load()
+    g = make_geometry("2p5d", 60, 64)
+    I, x, r = make_atoms(3, 500, 3, rdiag=(4, 20))
+    atoms, geom = engine_atoms(I, x, r), engine_geometry(g)
+    want = eng.radproj(atoms, geom)
+    full = eng.workspace_bytes(LIB.GR_OP_PROJECT, atoms, geom)
+    size = full - (60 - angles) * 500 * 32
+    ws = torch.empty(full, dtype=torch.uint8, device="cuda")
+    R = torch.empty_like(want)
+    before = eng.launch_count()
+    LIB.check(lib.gr_radproj(ctypes.byref(atoms.struct), ctypes.byref(geom.struct), R.data_ptr(),
+                             ws.data_ptr(), size, eng._stream_handle(geom.device)), "gr_radproj")
+    assert eng.launch_count() - before == 2
+    assert torch.equal(R, want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("angles,launches", [(32767, 2), (32768, 4), (39999, 4), (40000, 2)])
+def test_ranges_of_angles(eng, cuda_ready, angles, launches):
+    """A tile an angle: ranges are taken from 32768 items on, and give the same bits."""
+    lib = LIB.load()
+    A, n = 40000, 9
+    g = make_geometry("2p5d", A, 16, 32)
+    I, x, r = make_atoms(3, n, 3)
+    atoms, geom = engine_atoms(I, x, r), engine_geometry(g)
+    want = eng.radproj(atoms, geom)
+    full = eng.workspace_bytes(LIB.GR_OP_PROJECT, atoms, geom)
+    ws = torch.empty(full, dtype=torch.uint8, device="cuda")
+    R = torch.empty_like(want)
+    before = eng.launch_count()
+    LIB.check(lib.gr_radproj(ctypes.byref(atoms.struct), ctypes.byref(geom.struct), R.data_ptr(),
+                             ws.data_ptr(), full - (A - angles) * n * 32,
+                             eng._stream_handle(geom.device)), "gr_radproj")
+    assert eng.launch_count() - before == launches
+    assert torch.equal(R, want)
