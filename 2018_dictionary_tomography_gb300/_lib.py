@@ -12,7 +12,7 @@ from . import build_ext
 GR_OK = 0
 GR_FIT_NONE, GR_FIT_L2, GR_FIT_KL = 0, 1, 2
 GR_MODE_FIELD, GR_MODE_L2_ATOM, GR_MODE_INNER = 0, 1, 2
-GR_OP_PROJECT, GR_OP_DERIVS_1, GR_OP_DERIVS_2, GR_OP_ATOM_STEP = 0, 1, 2, 3
+GR_OP_PROJECT, GR_OP_DERIVS_1, GR_OP_DERIVS_2, GR_OP_ATOM_STEP, GR_OP_PSF_PROJECT = 0, 1, 2, 3, 4
 
 
 class GrAtoms(ctypes.Structure):

@@ -140,6 +140,8 @@ static size_t workspace_bytes_impl(int op, const gr_atoms *atoms, const gr_geome
   const int D1 = g.K == 2 ? g.ax[1].n : 1;
   if (op == GR_OP_PROJECT)
     return project_workspace_bytes(g.K, at.n, g.n_angles, g.ax[0].n, D1, t);
+  if (op == GR_OP_PSF_PROJECT)
+    return project_min_bytes(g.K, at.n, g.n_angles, g.ax[0].n, D1, t);
   if (op == GR_OP_DERIVS_1 || op == GR_OP_DERIVS_2)
     return derivs_workspace_bytes(g.K, at.n, g.n_angles, op == GR_OP_DERIVS_1 ? 1 : 2, t);
   if (op == GR_OP_ATOM_STEP) return align_up((size_t)g.n_angles * sizeof(double));

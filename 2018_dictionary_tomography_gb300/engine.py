@@ -240,6 +240,10 @@ def _ws_for(op, atoms, geom, plan=None):
     return workspace(n, geom.device), n
 
 
+def _project_op(psf):
+    return _lib.GR_OP_PSF_PROJECT if psf else _lib.GR_OP_PROJECT
+
+
 def _fn(name, psf, plan):
     """The entry point for a call: psf variant, or the plan-taking variant
     (bound to the plan's handle)."""
@@ -260,7 +264,7 @@ def radproj(atoms, geom, out=None, psf=False, plan=None):
         out = torch.empty(geom.shape, dtype=torch.float32, device=geom.device)
     if tuple(out.shape) != tuple(geom.shape) or out.dtype != torch.float32 or not out.is_contiguous():
         raise ValueError("output must be a contiguous float32 tensor of shape %s" % (geom.shape,))
-    ws, n = _ws_for(_lib.GR_OP_PROJECT, atoms, geom, plan)
+    ws, n = _ws_for(_project_op(psf), atoms, geom, plan)
     fn = _fn("radproj", psf, plan)
     st = fn(ctypes.byref(atoms.struct), ctypes.byref(geom.struct),
             out.data_ptr(), ws.data_ptr(), n, _stream_handle(geom.device))
@@ -286,7 +290,7 @@ def fit_forward(atoms, geom, data, fit="l2", background=0.0, want_R=False,
     alpha = torch.empty(geom.shape, dtype=torch.float32, device=dev) if want_fields else None
     beta = (torch.empty(geom.shape, dtype=torch.float32, device=dev)
             if (want_fields and fit == "kl") else None)
-    ws, n = _ws_for(_lib.GR_OP_PROJECT, atoms, geom, plan)
+    ws, n = _ws_for(_project_op(psf), atoms, geom, plan)
     p = lambda t: None if t is None else t.data_ptr()
     fn = _fn("fit_forward", psf, plan)
     st = fn(
@@ -672,7 +676,7 @@ class FitStep:
         self.loss_h = _packed_view(self.out_h, olay["loss"])
         self.g_h = _packed_view(self.out_h, olay["g"])
         self.H_h = _packed_view(self.out_h, olay["H"]) if self.order > 1 else None
-        nb = max(workspace_bytes(_lib.GR_OP_PROJECT, self.atoms, geom),
+        nb = max(workspace_bytes(_project_op(self.psf), self.atoms, geom),
                  workspace_bytes(_lib.GR_OP_DERIVS_2 if self.order > 1 else _lib.GR_OP_DERIVS_1,
                                  self.atoms, geom))
         self.ws = torch.empty(max(nb, 256), dtype=torch.uint8, device=dev)

@@ -83,7 +83,13 @@ typedef struct {
 
 enum { GR_FIT_NONE = 0, GR_FIT_L2 = 1, GR_FIT_KL = 2 };
 enum { GR_MODE_FIELD = 0, GR_MODE_L2_ATOM = 1, GR_MODE_INNER = 2 };
-enum { GR_OP_PROJECT = 0, GR_OP_DERIVS_1 = 1, GR_OP_DERIVS_2 = 2, GR_OP_ATOM_STEP = 3 };
+enum {
+  GR_OP_PROJECT = 0,
+  GR_OP_DERIVS_1 = 1,
+  GR_OP_DERIVS_2 = 2,
+  GR_OP_ATOM_STEP = 3,
+  GR_OP_PSF_PROJECT = 4   /* gr_psf_radproj, gr_psf_fit_forward: no pair records */
+};
 
 /* Library version (major*10000 + minor*100 + patch). */
 int gr_version(void);
@@ -104,6 +110,8 @@ const char *gr_status_string(int status);
  * (256-byte aligned) and may reuse it across calls on the same stream.  For a
  * 3D projection it includes up to 512 MB of 32-byte (atom, angle) records; a
  * launch given less works through the angles in ranges, or without records.
+ * The pixel-integrated forwards take GR_OP_PSF_PROJECT (GR_OP_PROJECT is enough
+ * too).
  */
 size_t gr_workspace_bytes(int op, const gr_atoms *atoms, const gr_geometry *geom);
 

@@ -160,3 +160,34 @@ def test_ranges_of_angles(eng, cuda_ready, angles, launches):
                              eng._stream_handle(geom.device)), "gr_radproj")
     assert eng.launch_count() - before == launches
     assert torch.equal(R, want)
+
+
+def test_pixel_integrated_forward_asks_for_no_records_without_gpu():
+    lib = LIB.load()
+    at, g = host_problem(2, 8192, 2000, 64)
+    size = lambda op: lib.gr_workspace_bytes(op, ctypes.byref(at), ctypes.byref(g))
+    assert size(LIB.GR_OP_PROJECT) - size(LIB.GR_OP_PSF_PROJECT) > 8192 * 2000 * 32 - 4096
+    at1, g1 = host_problem(1, 8192, 2000, 64)
+    both = [lib.gr_workspace_bytes(op, ctypes.byref(at1), ctypes.byref(g1))
+            for op in (LIB.GR_OP_PROJECT, LIB.GR_OP_PSF_PROJECT)]
+    assert both[0] == both[1]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["2d", "2p5d"])
+def test_pixel_integrated_forward_in_its_own_workspace(eng, cuda_ready, kind):
+    """Projection, fit and a fit step hold no more than the query for them."""
+    g = make_geometry(kind, 70, 40)
+    I, x, r = make_atoms(2 if kind == "2d" else 3, 300, 3)
+    atoms, geom = engine_atoms(I, x, r), engine_geometry(g)
+    s = torch.cuda.Stream()
+    with torch.cuda.stream(s):
+        R = eng.radproj(atoms, geom, psf=True)
+        eng.fit_forward(atoms, geom, R, "l2", psf=True)
+        need = eng.workspace_bytes(LIB.GR_OP_PSF_PROJECT, atoms, geom)
+        assert eng.workspace(0, geom.device).numel() == need
+    s.synchronize()
+    assert relerr(R.cpu().numpy(), go.psf_radproj(I, x, r, g)) < TOL
+    derivs = eng.workspace_bytes(LIB.GR_OP_DERIVS_1, atoms, geom)
+    step = eng.FitStep(geom, 300, order=1, psf=True)
+    assert step.ws.numel() == max(need, derivs)
