@@ -20,7 +20,7 @@ struct TileCfg {
   int t0, t1;     // tile extent along detector axes 0 and 1
   int nt0, nt1;   // tiles along each axis
   int ntiles;
-  uint32_t inv_ntiles, inv_nt1;   // floor(2^32 / .), for tile_div
+  uint32_t inv_ntiles, inv_nt1, inv_angles;   // floor(2^32 / .), for tile_div
 };
 
 // n / d, inv = floor(2^32 / d) (2^32 - 1 for d = 1): the product is at most
@@ -109,7 +109,8 @@ extern Tuning g_tuning;
 int tuning_set(Tuning &t, int key, int value);
 int tuning_get(const Tuning &t, int key);
 
-TileCfg make_tiles(int K, int D0, int D1, int rows);
+// (n_angles: for launches that go through the angles tile by tile)
+TileCfg make_tiles(int K, int D0, int D1, int rows, int n_angles = 1);
 // (angle, tile) items of a forward that can skip items no atom meets (the
 // point-sampled 3D projection under t's tiling; 0 for the others)
 size_t project_skip_items(const Geom &g, int psf, const Tuning &t = g_tuning);

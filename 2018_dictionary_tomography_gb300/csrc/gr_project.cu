@@ -604,7 +604,7 @@ __device__ __forceinline__ void project1d_body(const Atoms &at, const Geom &g, c
   __shared__ int wsum[NW];
   __shared__ float parts[NW][2][32 * CPL];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int a = item / tc.ntiles, t = item - a * tc.ntiles;
+  const int a = tile_div(item, tc.ntiles, tc.inv_ntiles), t = item - a * tc.ntiles;
   const int D0 = g.ax[0].n;
   int cell[CPL];
   float pc[CPL], acc[CPL], cmp[CPL];
@@ -631,9 +631,17 @@ __device__ __forceinline__ void project1d_body(const Atoms &at, const Geom &g, c
     }
     if (lane == 31) wsum[warp] = incl;
     __syncthreads();
+    int any = 0;
 #pragma unroll
-    for (int w = 0; w < NW; ++w)
+    for (int w = 0; w < NW; ++w) {
+      any += wsum[w];
       if (w < warp) incl += wsum[w];
+    }
+    if (any == 0) {     // (a tile without atoms: nothing to list)
+      wb += T;
+      if (wb < W) __syncthreads();
+      continue;
+    }
     // the words that fit form a prefix (incl never decreases); one word
     // always fits (a word holds at most 32 <= LT atoms)
     const bool take = incl <= LT;
@@ -744,10 +752,12 @@ __device__ __forceinline__ void project1d_body(const Atoms &at, const Geom &g, c
 // short ones (in angle order, the SMs idled for a third of the launch on 2150
 // atoms x 153 angles x 15 tiles: 51.1 us, 41.1 us; pixel-integrated, 128
 // x 401 x 8 tiles: 64.8 and 62.5 us).
+template <int K>
 __device__ __forceinline__ int centre_out(int b, int n_angles, const TileCfg &tc) {
-  const int rank = b / n_angles, a = b - rank * n_angles;
-  const int k0 = rank / tc.nt1, k1 = rank - k0 * tc.nt1;
   auto at = [](int k, int n) { return (k & 1) ? n / 2 - (k + 1) / 2 : n / 2 + k / 2; };
+  const int rank = tile_div(b, n_angles, tc.inv_angles), a = b - rank * n_angles;
+  if constexpr (K == 1) return a * tc.ntiles + at(rank, tc.ntiles);
+  const int k0 = tile_div(rank, tc.nt1, tc.inv_nt1), k1 = rank - k0 * tc.nt1;
   return a * tc.ntiles + at(k0, tc.nt0) * tc.nt1 + at(k1, tc.nt1);
 }
 
@@ -757,7 +767,7 @@ __global__ void __launch_bounds__(NW * 32)
                         int W, ProjOut out, double *loss_out, int *done,
                         const float4 *__restrict__ pairs) {
   project1d_body<KAHAN, NW, CPL, LM>(at, g, tc, bitmap, W, out, loss_out, done, pairs,
-                                     centre_out(blockIdx.x, g.n_angles, tc), gridDim.x);
+                                     centre_out<1>(blockIdx.x, g.n_angles, tc), gridDim.x);
 }
 
 // ---- pixel-integrated operator: binning and projection -------------------
@@ -788,12 +798,12 @@ __global__ void __launch_bounds__(128) gr_psf_bin_kernel(Atoms at, Geom g, TileC
   }
 }
 
-// A block per (angle, tile): its atoms, in index order, go round its four
+// A block per (angle, tile): its atoms, in index order, go round its NW
 // warps.  A warp's lanes look over an atom's cell box clipped to the tile and
 // queue the cells it reaches; 32 queued cells at a time, of as many atoms as
 // that takes, get their value by the quadrature rule (121 exponentials, what
 // bounds it) and go into the warp's own compensated sums in shared memory,
-// those of one cell in atom order; a cell then adds the four sums in warp order
+// those of one cell in atom order; a cell then adds the warps' sums in warp order
 // (deterministic).  128 atoms x 401 x 64^2: 138 us with a warp per tile of 32 x
 // 32 cells, 109 us with four, 15 of 32 lanes at work; with the queue 65 us.
 struct PsfStage {
@@ -802,25 +812,32 @@ struct PsfStage {
   int4 box;      // first and last cell along each axis, clipped to the tile
 };
 constexpr int kPsfTileWarps = 4;
+// 2D: many tiles of few atoms take a warp each (latency: 32 tiles an SM in flight, not 8;
+// 1 and 4 warps: 4 atoms x 1500 x 435 cells, 21000 tiles, 31 and 55 us; 64 x 800 x 300, 8000
+// tiles, 67 and 75; 256 there 214 and 191, x 1500 x 435 193 and 208; 16 x 400 x 300, 4000
+// tiles, 33 and 29).
+static int psf_tile_warps(int K, size_t items, int n_atoms) {
+  return K == 1 && items >= 6144 && items >= 64 * (size_t)n_atoms ? 1 : kPsfTileWarps;
+}
 constexpr int kPsfList = 256;  // atoms listed at a time (8 bitmap words)
 static_assert(kTileDim0 <= 32 && kTileDim1 <= 32, "a queued cell's row and column: 5 bits each");
 
 // words a warp's staging and sums take (rows x cols cells)
 __host__ __device__ constexpr int psf_warp_words(int cells) { return 2 * cells + 32 * 16; }
 
-template <int K>
-__global__ void __launch_bounds__(kPsfTileWarps * 32, 8)
+template <int K, int NW>
+__global__ void __launch_bounds__(NW * 32, 32 / NW)
     gr_psf_project_kernel(Atoms at, Geom g, TileCfg tc, const uint32_t *bitmap, int W,
                           float s, ProjOut out, double *loss_out, int *done) {
   extern __shared__ __align__(16) float smem[];
   __shared__ int list[kPsfList];
   __shared__ float pc0[kTileDim0], pc1[kTileDim1];
-  __shared__ float2 s_loss[kPsfTileWarps * 32];
-  __shared__ uint32_t s_queue[kPsfTileWarps][64];
+  __shared__ float2 s_loss[NW * 32];
+  __shared__ uint32_t s_queue[NW][64];
   __shared__ int s_last;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   uint32_t *queue = s_queue[warp];
-  const int item = centre_out(blockIdx.x, g.n_angles, tc), n_items = g.n_angles * tc.ntiles;
+  const int item = centre_out<K>(blockIdx.x, g.n_angles, tc), n_items = g.n_angles * tc.ntiles;
   const int cells = tc.t0 * tc.t1;
   float *acc = smem + (size_t)warp * psf_warp_words(cells);
   float *cmp = acc + cells;
@@ -857,11 +874,11 @@ __global__ void __launch_bounds__(kPsfTileWarps * 32, 8)
       }
     }
     __syncthreads();
-    const int mine = (total - warp + kPsfTileWarps - 1) / kPsfTileWarps;   // entries warp, warp + 4, ..
+    const int mine = (total - warp + NW - 1) / NW;   // entries warp, warp + 4, ..
     for (int bs = 0; bs < mine; bs += 32) {
       const int nb = min(32, mine - bs);
       if (lane < nb) {
-        const int j = list[warp + kPsfTileWarps * (bs + lane)];
+        const int j = list[warp + NW * (bs + lane)];
         Frame<K> f;
         load_frame<K>(g.frames, a, f);
         Pair<K> p;
@@ -955,14 +972,14 @@ __global__ void __launch_bounds__(kPsfTileWarps * 32, 8)
   }
   __syncthreads();
   float lsum = 0.f, lcmp = 0.f;
-  for (int e = tid; e < cells; e += kPsfTileWarps * 32) {
+  for (int e = tid; e < cells; e += NW * 32) {
     const int lr = e / tc.t1, lc = e - lr * tc.t1;
     const int row = r0 + lr, col = c0 + lc;
     if (row >= D0 || col >= D1) continue;
     // the warps' sums in warp order
     float sv = 0.f, cv = 0.f;
 #pragma unroll
-    for (int w = 0; w < kPsfTileWarps; ++w) {
+    for (int w = 0; w < NW; ++w) {
       const float *aw = smem + (size_t)w * psf_warp_words(cells);
       pair_add(sv, cv, aw[e], aw[cells + e]);
     }
@@ -991,7 +1008,7 @@ __global__ void __launch_bounds__(kPsfTileWarps * 32, 8)
   __syncthreads();
   if (warp == 0) {
 #pragma unroll
-    for (int w = 1; w < kPsfTileWarps; ++w)
+    for (int w = 1; w < NW; ++w)
       pair_add(lsum, lcmp, s_loss[32 * w + lane].x, s_loss[32 * w + lane].y);
     const double d = warp_sum_d((double)lsum + (double)lcmp);
     if (lane == 0) {
@@ -1007,7 +1024,7 @@ __global__ void __launch_bounds__(kPsfTileWarps * 32, 8)
   if (!s_last) return;
   // the last block to finish sums the items' partials in item order
   __threadfence();
-  sum_partials_block<kPsfTileWarps>(out.loss_part, n_items, loss_out);
+  sum_partials_block<NW>(out.loss_part, n_items, loss_out);
 }
 
 // Fixed-order FP64 sum of n loss partials over many blocks (one block's FP64
@@ -1100,7 +1117,7 @@ static void launch_project3d(size_t items, const Atoms &at, const Geom &g, const
 }
 
 // rows: the tile's rows (3D) or cells (2D)
-TileCfg make_tiles(int K, int D0, int D1, int rows) {
+TileCfg make_tiles(int K, int D0, int D1, int rows, int n_angles) {
   TileCfg tc;
   if (K == 1) {
     tc.t0 = rows;
@@ -1117,6 +1134,7 @@ TileCfg make_tiles(int K, int D0, int D1, int rows) {
   auto inv = [](int d) { return d > 1 ? (uint32_t)((1ull << 32) / (unsigned)d) : 0xffffffffu; };
   tc.inv_ntiles = inv(tc.ntiles);
   tc.inv_nt1 = inv(tc.nt1);
+  tc.inv_angles = inv(n_angles);
   return tc;
 }
 
@@ -1192,7 +1210,8 @@ int launch_project(const Atoms &at, const Geom &g, const ProjOut &o_in,
   const bool wide4 = K == 1 && !o_in.psf && form == 3;
   TileCfg tc = make_tiles(K, D0, D1,
                           K == 1 ? (wide4 ? 4 * kTile1D : wide2d ? 2 * kTile1D : kTile1D)
-                                 : proj_rows(form));
+                                 : proj_rows(form),
+                          g.n_angles);
   const int W = (at.n + 31) / 32;
   const size_t items = (size_t)g.n_angles * tc.ntiles;
   const size_t need = project_min_bytes(K, at.n, g.n_angles, D0, D1, t);
@@ -1255,7 +1274,6 @@ int launch_project(const Atoms &at, const Geom &g, const ProjOut &o_in,
   }
   // below the 48 KB that needs no opt-in, so no function attribute is set (safe
   // under capture)
-  const size_t smem = (size_t)kPsfTileWarps * psf_warp_words(tc.t0 * tc.t1) * sizeof(float);
   static_assert(kPsfTileWarps * psf_warp_words(kTileDim0 * kTileDim1) * sizeof(float) <= 42 * 1024,
                 "smem");
   bool fused_loss = false;
@@ -1306,12 +1324,15 @@ int launch_project(const Atoms &at, const Geom &g, const ProjOut &o_in,
     if (o.psf) {
       fused_loss = loss_out != nullptr && items <= kFusedLossItems;
       double *lo = fused_loss ? loss_out : nullptr;
-      if (K == 1)
-        gr_psf_project_kernel<1><<<(unsigned)items, kPsfTileWarps * 32, smem, stream>>>(
-            at, g, tc, bitmap, W, psf_s, o, lo, next_item + 1);
-      else
-        gr_psf_project_kernel<2><<<(unsigned)items, kPsfTileWarps * 32, smem, stream>>>(
-            at, g, tc, bitmap, W, psf_s, o, lo, next_item + 1);
+      const int nw = psf_tile_warps(K, items, at.n);
+      const size_t smem = (size_t)nw * psf_warp_words(tc.t0 * tc.t1) * sizeof(float);
+      auto go = [&](auto kernel) {
+        kernel<<<(unsigned)items, nw * 32, smem, stream>>>(at, g, tc, bitmap, W, psf_s, o, lo,
+                                                           next_item + 1);
+      };
+      if (K == 2) go(gr_psf_project_kernel<2, kPsfTileWarps>);
+      else if (nw == 1) go(gr_psf_project_kernel<1, 1>);
+      else go(gr_psf_project_kernel<1, kPsfTileWarps>);
     } else {
       // one block per (angle, tile) item; for up to kFusedLossItems tiles the
       // last block also sums the loss partials (no separate finalize launch)
@@ -1410,7 +1431,8 @@ int preload_project() {
          preload_fn(gr_project1d_kernel<true, kProjWarps, 2>) +
          preload_fn(gr_project1d_kernel<true, 8, 4, 2>) +
          preload_fn(gr_project1d_kernel<true, kProjWarps, 4>) +
-         preload_fn(gr_psf_project_kernel<1>) + preload_fn(gr_psf_project_kernel<2>) +
+         preload_fn(gr_psf_project_kernel<1, 1>) + preload_fn(gr_psf_project_kernel<1, kPsfTileWarps>) +
+         preload_fn(gr_psf_project_kernel<2, kPsfTileWarps>) +
          preload_fn(gr_loss_finalize_kernel) + preload_fn(gr_batch_bin_kernel) +
          preload_fn(gr_batch_project_kernel);
 }

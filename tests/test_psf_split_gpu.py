@@ -40,3 +40,20 @@ def test_forms(eng, cuda_ready, kind, order, blocks, D, rdiag):
     if order == 2 and rdiag[0] < 20:
         # (Hessians of supports inside one cell cancel beyond FP32 atom by atom)
         assert atom_normwise_relerr(H.cpu().numpy()[pick], np.array([o[2] for o in out])) < TOL
+
+
+@pytest.mark.parametrize("N,A,D", [(3, 3071, 64), (3, 3072, 64), (40, 6143, 20), (40, 6144, 20),
+                                   (97, 3103, 50), (97, 3104, 50), (300, 6144, 33)])
+def test_forward_with_one_warp_a_tile(eng, cuda_ready, N, A, D):
+    """2D: the least tiles of the one-warp form for few atoms and for 97, and one angle less."""
+    g = make_geometry("2d", A, D)
+    I, x, r = make_atoms(2, N, N + D, rdiag=(2, 8), roff=0.5)
+    atoms, geom = engine_atoms(I, x, r), engine_geometry(g)
+    ref = go.psf_radproj(I, x, r, g)
+    R = eng.radproj(atoms, geom, psf=True)
+    assert relerr(R.cpu().numpy(), ref) < TOL
+    data = torch.from_numpy(1.1 * ref + 0.01 * ref.max()).float().cuda()
+    fw = eng.fit_forward(atoms, geom, data, "l2", psf=True)
+    assert torch.equal(fw["alpha"], R - data)
+    want = 0.5 * (fw["alpha"].double() ** 2).sum().item()
+    assert abs(float(fw["loss"]) - want) < 1e-6 * want
