@@ -820,6 +820,10 @@ static int psf_tile_warps(int K, size_t items, int n_atoms) {
   return K == 1 && items >= 6144 && items >= 64 * (size_t)n_atoms ? 1 : kPsfTileWarps;
 }
 constexpr int kPsfList = 256;  // atoms listed at a time (8 bitmap words)
+// 2D: an atom that meets at least this many of a tile's 32 cells takes a lane a cell
+// (us, queued and so: 32 atoms x 647 x 811, r = 0.9: 170, 93; 256 x 400 x 300, r = 3: 109,
+// 82; 16 there, a third of the atoms so wide: 30.6, 30.4).
+constexpr int kPsfWide1 = 20;
 static_assert(kTileDim0 <= 32 && kTileDim1 <= 32, "a queued cell's row and column: 5 bits each");
 
 // words a warp's staging and sums take (rows x cols cells)
@@ -928,6 +932,26 @@ __global__ void __launch_bounds__(NW * 32, 32 / NW)
           __syncwarp();
         }
       };
+      // 2D: an atom's value at the lane's cell of the tile
+      auto direct = [&](int s2, const int4 &box) {
+        const int lr = lane;
+        if (lr < box.x - r0 || lr > box.y - r0) return;
+        const float4 qa = stage[s2].a, qb = stage[s2].b, qc = stage[s2].c;
+        Pair<K> p;
+        p.G[0] = qb.x;
+        p.l2amp = qb.w;
+        PsfPair<K> q;
+        q.rr = qc.y;
+        float dc[K], base[K], step[K];
+        dc[0] = (pc0[lr] - qa.x) - qa.y;
+        const int kind = psf_cell_kind<K>(q, dc, s, base, step);
+        if (kind == 0) return;
+        float v = qc.z;
+        if (kind == 2) v = qc.x * psf_quadrature<K>(p, base, step);
+        const float s0 = acc[lr], tt = s0 + v;
+        cmp[lr] += (fabsf(s0) >= fabsf(v)) ? ((s0 - tt) + v) : ((v - tt) + s0);
+        acc[lr] = tt;
+      };
       int queued = 0;
       for (int s2 = 0; s2 < nb; ++s2) {
         const int4 box = stage[s2].box;
@@ -937,6 +961,13 @@ __global__ void __launch_bounds__(NW * 32, 32 / NW)
         q.rr = stage[s2].c.y;
         const int bw = box.w - box.z + 1;
         const int ncell = (box.y - box.x + 1) * bw;
+        if constexpr (K == 1) {
+          if (ncell >= kPsfWide1) {
+            // most of a 2D tile: its cells at once, a lane each, no queue
+            direct(s2, box);
+            continue;
+          }
+        }
         const float inv_bw = 1.f / (float)bw;
         for (int e0 = 0; e0 < ncell; e0 += 32) {
           const int e = e0 + lane;
