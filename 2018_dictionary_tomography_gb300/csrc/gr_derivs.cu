@@ -1082,6 +1082,10 @@ __global__ void __launch_bounds__(32 * L)
 // Narrow supports are set-up and assembly above all, of which PW = 8 does four
 // times the instructions (start_psf).
 
+// PW = 32: pairs whose boxes all have at most this many cells are looked over by their
+// own lanes, 32 pairs at a time, not one after the other (2366 atoms x 572 x 29^2, one or
+// two cells a pair: gradient 410 -> 216 us; 1412 x 907 x 78^2, r = 35: 644 -> 414).
+constexpr int kPsfNarrow = 16;
 struct PsfWalk {
   float4 a, b;        // qh0 ql0 qh1 ql1; G00 G01 G11 log2 n
   float rr, total, I;
@@ -1237,10 +1241,18 @@ __global__ void __launch_bounds__(1024 / PW, (ORDER == 1 ? 16 : 8) * PW / 32)
     }
     // into the pairs' sums: pair by pair, eight values at a time, the values held
     // halved over three exchanges, then the four lanes that hold the same one
-    // summed.  A Hessian's many values of more pairs than a pair has cells: the
-    // pairs' cells in turn, each lane its own values.
-    const int first = __shfl_sync(0xffffffffu, slot, 0), last = __shfl_sync(0xffffffffu, slot, 31);
-    if (ORDER > 1 && last - first > 1) {
+    // summed.  More pairs than a pair has cells: the pairs' cells in turn, each lane
+    // its own values (gradients with PW = 8 lose by the test, 116 and 122 us on
+    // 128 x 401 x 64^2).
+    int first, last;
+    if constexpr (PW >= 16) {   // (the pairs of a batch may come in any order)
+      first = __reduce_min_sync(0xffffffffu, slot);
+      last = __reduce_max_sync(0xffffffffu, slot);
+    } else {
+      first = __shfl_sync(0xffffffffu, slot, 0);
+      last = __shfl_sync(0xffffffffu, slot, 31);
+    }
+    if ((ORDER > 1 || PW >= 16) && last - first > 1) {
       const unsigned same = __match_any_sync(0xffffffffu, on ? slot : -1 - lane);
       const int rank = __popc(same & ((1u << lane) - 1u));
       const int turns = __reduce_max_sync(0xffffffffu, rank) + 1;
@@ -1308,7 +1320,45 @@ __global__ void __launch_bounds__(1024 / PW, (ORDER == 1 ? 16 : 8) * PW / 32)
     }
     __syncwarp();
     int queued = 0;
-    for (int sl = 0; sl < PW; ++sl) {
+    // the queued cells of all lanes, 32 at a time
+    auto push = [&](bool hit, int2 cell) {
+      const unsigned m = __ballot_sync(0xffffffffu, hit);
+      if (hit) queue[queued + __popc(m & ((1u << lane) - 1u))] = cell;
+      queued += __popc(m);
+      __syncwarp();
+      if (queued >= 32) {
+        add_cells(32);
+        queued -= 32;
+        const int2 left = queue[32 + lane];
+        __syncwarp();
+        if (lane < queued) queue[lane] = left;
+        __syncwarp();
+      }
+    };
+    // narrow supports: a lane looks over its own pair's few cells
+    const bool narrow = PW >= 16 && __reduce_max_sync(0xffffffffu, ncell) <= kPsfNarrow;
+    if (narrow) {
+      const int most = __reduce_max_sync(0xffffffffu, ncell);
+      const PsfWalk w = walk[lane & (PW - 1)];
+      PsfPair<K> q;
+      q.rr = w.rr;
+      int k0 = w.lo0, k1 = w.lo1;
+      for (int e = 0; e < most; ++e) {
+        bool hit = false;
+        if (e < ncell) {
+          float dc[K], base[K], step[K];
+          dc[0] = (__ldg(g.ax[0].coords + k0) - w.a.x) - w.a.y;
+          dc[1] = (__ldg(g.ax[1].coords + k1) - w.a.z) - w.a.w;
+          hit = psf_cell_kind<K>(q, dc, s, base, step) != 0;
+        }
+        push(hit, make_int2(k0 << 5 | lane, k1));
+        if (++k1 == w.lo1 + w.bw) {
+          k1 = w.lo1;
+          ++k0;
+        }
+      }
+    }
+    for (int sl = narrow ? PW : 0; sl < PW; ++sl) {
       const int nc = __shfl_sync(0xffffffffu, ncell, sl);
       if (nc == 0) continue;
       const PsfWalk w = walk[sl];
@@ -1329,18 +1379,7 @@ __global__ void __launch_bounds__(1024 / PW, (ORDER == 1 ? 16 : 8) * PW / 32)
           dc[1] = (__ldg(g.ax[1].coords + k1) - w.a.z) - w.a.w;
           hit = psf_cell_kind<K>(q, dc, s, base, step) != 0;
         }
-        const unsigned m = __ballot_sync(0xffffffffu, hit);
-        if (hit) queue[queued + __popc(m & ((1u << lane) - 1u))] = make_int2(k0 << 5 | sl, k1);
-        queued += __popc(m);
-        __syncwarp();
-        if (queued >= 32) {
-          add_cells(32);
-          queued -= 32;
-          const int2 left = queue[32 + lane];
-          __syncwarp();
-          if (lane < queued) queue[lane] = left;
-          __syncwarp();
-        }
+        push(hit, make_int2(k0 << 5 | sl, k1));
       }
     }
     if (queued) add_cells(queued);
@@ -1713,9 +1752,11 @@ static void start_hess(const DerivArgs &d) {
 // pairs (us with 4, 2 and 1; gradients, 200 atoms x 100 angles x 467 cells, r = 4:
 // 25, 31, 46; 500 x 130 x 300, r = 4: 38, 41, 43, x 64, r = 30: 15, 13.5, 11.4; 2154
 // x 736 x 75, r = 30: 152, 104, 72; Hessians there: 282, 183, 119).  3D, pairs a
-// warp: all 32 from 2.5 full waves of such blocks on, for the same reason (8 and 32
-// a warp; gradients, 128 x 401 x 64^2, r = 8: 116, 150; 300 x 401, r = 20: 100, 104;
-// 1412 x 907, r = 35: 780, 643; Hessians 233, 296; 229, 214; 1849, 1512).
+// warp: all 32 from 2.5 full waves of such blocks on, for the same reason; wide
+// supports lose a tenth by their last wave (us, 8 and 32 a warp; gradients, 300 x 401 x
+// 64^2, 25 blocks an SM, r = 8 and 20: 246, 295 and 104, 90; 600 x 401, 50 blocks, r = 8
+// and 30: 476, 520 and 160, 89; 1412 x 907 x 78^2, r = 12 and 35: 1894, 1835 and 804, 414;
+// Hessians 497, 535 and 229, 172; 961, 978 and 366, 197; 3866, 3654 and 1845, 975).
 constexpr int kPsfSms = 152;
 template <int ORDER>
 static void start_psf(const DerivArgs &d, float s) {
