@@ -1424,7 +1424,7 @@ __global__ void __launch_bounds__(1024 / PW, (ORDER == 1 ? 16 : 8) * PW / 32)
 // 64 values, S threads share one, each summing a contiguous range of chunks in
 // chunk order (a dependent FP64 add takes 64 cycles), and the ranges are added
 // in order; a thread loads kFinBatch partials before it adds any.  Ranges of less
-// than kFinBatch chunks gain nothing (fin_shares), and an atom whose values fill half
+// than kFinBatch / 2 chunks gain nothing (fin_shares), and an atom whose values fill half
 // of the threads has half of them (fin_threads: 6298 atoms x 1 chunk 5.4 -> 3.0 us, 3.3 before ranges).  8192 atoms x
 // 625 chunks: 357 -> 244 us (conversions and adds on the FP64 pipe), 1000 x 126:
 // 21.7 -> 13.7 us, 64 x 60: 10.2 -> 5.9 us (one thread per value with four loads
@@ -1436,7 +1436,7 @@ constexpr int kFinBatch = 8;
 // threads that share a value of an atom
 __host__ __device__ __forceinline__ int fin_shares(const DerivCfg &cfg) {
   int S = 1;
-  while (2 * S * cfg.qn <= kFinPer && S < 8 && cfg.nchunks >= 2 * S * kFinBatch) S *= 2;
+  while (2 * S * cfg.qn <= kFinPer && S < 8 && cfg.nchunks >= S * kFinBatch) S *= 2;
   return S;
 }
 // threads of a block
