@@ -1082,8 +1082,8 @@ __global__ void __launch_bounds__(32 * L)
 // Narrow supports are set-up and assembly above all, of which PW = 8 does four
 // times the instructions (start_psf).
 
-// PW = 32: pairs whose boxes all have at most this many cells are looked over by their
-// own lanes, 32 pairs at a time, not one after the other (2366 atoms x 572 x 29^2, one or
+// From PW = 16 on: pairs whose boxes all have at most this many cells are looked over by their
+// own lanes, all at a time, not one after the other (2366 atoms x 572 x 29^2, one or
 // two cells a pair: gradient 410 -> 216 us; 1412 x 907 x 78^2, r = 35: 644 -> 414).
 constexpr int kPsfNarrow = 16;
 struct PsfWalk {
@@ -1752,11 +1752,13 @@ static void start_hess(const DerivArgs &d) {
 // pairs (us with 4, 2 and 1; gradients, 200 atoms x 100 angles x 467 cells, r = 4:
 // 25, 31, 46; 500 x 130 x 300, r = 4: 38, 41, 43, x 64, r = 30: 15, 13.5, 11.4; 2154
 // x 736 x 75, r = 30: 152, 104, 72; Hessians there: 282, 183, 119).  3D, pairs a
-// warp: all 32 from 2.5 full waves of such blocks on, for the same reason; wide
-// supports lose a tenth by their last wave (us, 8 and 32 a warp; gradients, 300 x 401 x
-// 64^2, 25 blocks an SM, r = 8 and 20: 246, 295 and 104, 90; 600 x 401, 50 blocks, r = 8
-// and 30: 476, 520 and 160, 89; 1412 x 907 x 78^2, r = 12 and 35: 1894, 1835 and 804, 414;
-// Hessians 497, 535 and 229, 172; 961, 978 and 366, 197; 3866, 3654 and 1845, 975).
+// warp: all 32 from some four full waves of such blocks on, half from one, for the same
+// reason; wide supports lose up to a tenth by their last wave (us, 8, 16 and 32 a warp;
+// gradients, 128 x 401 x 64^2, 11 blocks an SM, r = 8 and 20: 122, 145, 161 and 52, 50,
+// 54; 300 x 401, 25 blocks: 246, 265, 295 and 104, 89, 90; 600 x 401, 50 blocks, r = 8 and
+// 30: 476, 493, 520 and 160, 101, 89; 1412 x 907 x 78^2, 265 blocks, r = 12 and 35: 1894,
+// 1869, 1835 and 804, 510, 414; Hessians 234, 247, 306 and 110, 92, 103; 497, 501, 535 and
+// 229, 185, 172; 961, 949, 978 and 366, 242, 197; 3866, 3652, 3654 and 1845, 1231, 975).
 constexpr int kPsfSms = 152;
 template <int ORDER>
 static void start_psf(const DerivArgs &d, float s) {
@@ -1764,12 +1766,16 @@ static void start_psf(const DerivArgs &d, float s) {
     kernel<<<d.warps, threads, 0, d.stream>>>(d.at, d.g, d.in, d.cfg, d.part, s);
   };
   if (d.g.K == 1) {
-    const long long room = kPsfSms * (ORDER == 1 ? 32 : 16);
-    if (4ll * d.warps <= room) go(gr_psf_deriv1d_kernel<ORDER, 4>, 128);
-    else if (2ll * d.warps <= room) go(gr_psf_deriv1d_kernel<ORDER, 2>, 64);
+    // lanes that the pairs of short series leave idle count as free
+    const long long room = kPsfSms * 32 * (ORDER == 1 ? 32 : 16);
+    const long long pairs = (long long)d.at.n * d.g.n_angles, slots = 32ll * d.warps;
+    if (4 * pairs <= room || 4 * pairs <= slots) go(gr_psf_deriv1d_kernel<ORDER, 4>, 128);
+    else if (2 * pairs <= room || 2 * pairs <= slots) go(gr_psf_deriv1d_kernel<ORDER, 2>, 64);
     else go(gr_psf_deriv1d_kernel<ORDER, 1>, 32);
-  } else if (d.warps < kPsfSms * (ORDER == 1 ? 40 : 20)) {
+  } else if (d.warps < kPsfSms * (ORDER == 1 ? 20 : 10)) {
     go(gr_psf_deriv_kernel<ORDER, 8>, 128);
+  } else if (d.warps < kPsfSms * (ORDER == 1 ? 60 : 40)) {
+    go(gr_psf_deriv_kernel<ORDER, 16>, 64);
   } else {
     go(gr_psf_deriv_kernel<ORDER, 32>, 32);
   }
@@ -1778,7 +1784,7 @@ template <int ORDER>
 static int preload_psf() {
   return preload_fn(gr_psf_deriv1d_kernel<ORDER, 1>) + preload_fn(gr_psf_deriv1d_kernel<ORDER, 2>) +
          preload_fn(gr_psf_deriv1d_kernel<ORDER, 4>) + preload_fn(gr_psf_deriv_kernel<ORDER, 8>) +
-         preload_fn(gr_psf_deriv_kernel<ORDER, 32>);
+         preload_fn(gr_psf_deriv_kernel<ORDER, 16>) + preload_fn(gr_psf_deriv_kernel<ORDER, 32>);
 }
 
 int launch_derivs(const Atoms &at, const Geom &g, const DerivIn &in,
