@@ -1,6 +1,6 @@
 // Chain-rule assembly of per-atom gradients and Hessians from psi-space
-// sums, shared by the point-sampled (gr_derivs.cu) and pixel-integrated
-// (gr_psf.cu) derivative kernels.  See gr_derivs.cu for the derivation.
+// sums, shared by the point-sampled and pixel-integrated derivative kernels.
+// See gr_derivs.cu for the derivation.
 #pragma once
 #include "gr_kernels.cuh"
 

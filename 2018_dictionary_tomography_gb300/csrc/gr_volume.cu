@@ -68,6 +68,7 @@ __device__ __forceinline__ float psf_voxel(float Iv, const float *X, const float
 template <int D, bool PSF>
 __global__ void __launch_bounds__(kVolThreads)
     gr_volproj_kernel(Atoms at, VolGrid vg, int t0, int t1, int t2, float s, float *u) {
+  static_assert(D == 2 || PSF, "3D point values: gr_volproj3_kernel");
   __shared__ float sI[kVolThreads], sx[3][kVolThreads], sr[6][kVolThreads];
   __shared__ int wcount[kVolThreads / 32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -179,19 +180,12 @@ __global__ void __launch_bounds__(kVolThreads)
     __syncthreads();
     if (inside) {
       for (int k = 0; k < total; ++k) {
-        const float Y0 = yv[0] - sx[0][k], Y1 = yv[1] - sx[1][k];
-        float nn;
-        if (D == 2) {
+        if constexpr (!PSF) {
+          const float Y0 = yv[0] - sx[0][k], Y1 = yv[1] - sx[1][k];
           const float a = sr[0][k] * Y0 + sr[2][k] * Y1, c = sr[1][k] * Y1;
-          nn = a * a + c * c;
-        } else {
-          const float Y2 = yv[2] - sx[2][k];
-          const float a = sr[0][k] * Y0 + sr[3][k] * Y1 + sr[5][k] * Y2;
-          const float c = sr[1][k] * Y1 + sr[4][k] * Y2;
-          const float d = sr[2][k] * Y2;
-          nn = a * a + c * c + d * d;
+          const float nn = a * a + c * c;
+          if (nn <= 1.f) acc += sI[k] * ex2_approx(nn * kNegThirtyLog2e);
         }
-        if (!PSF && nn <= 1.f) acc += sI[k] * ex2_approx(nn * kNegThirtyLog2e);
         if (PSF) {
           float Mk[3][3] = {{sr[0][k], D == 2 ? sr[2][k] : sr[3][k], D == 2 ? 0.f : sr[5][k]},
                             {0.f, sr[1][k], D == 2 ? 0.f : sr[4][k]},
