@@ -93,8 +93,7 @@ def autotune_derivs(atoms, geom, field, beta_field=None, beta_const=1.0, order=1
     for cand in cands:
         w, m = cand[0], cand[1]
         g = cand[2] if len(cand) > 2 else plan.get(2)
-        wide = cand[3] if len(cand) > 3 else 0
-        plan.set(0, w).set(1, m).set(2, g).set(8, wide)
+        plan.set(0, w).set(1, m).set(2, g)
         run = lambda: engine.atom_derivs(atoms, geom, "field", field, beta_field, beta_const,
                                          order, psf=psf, plan=None if psf else plan)
         if psf:
@@ -115,12 +114,12 @@ def autotune_derivs(atoms, geom, field, beta_field=None, beta_const=1.0, order=1
         # split timed alone on an idle GPU that wins by a hair need not win
         # among concurrent fits
         if best is None or ms < best[3] * (1.0 - MARGIN):
-            best = (w, m, g, ms, wide)
+            best = (w, m, g, ms)
     if best is None:
         return None
-    plan.set(0, best[0]).set(1, best[1]).set(2, best[2]).set(8, best[4])
+    plan.set(0, best[0]).set(1, best[1]).set(2, best[2])
     _cache[key] = plan
-    return best[:4]
+    return best
 
 
 def plan_for(atoms, geom, order, psf=False):
@@ -145,7 +144,7 @@ _req_plans = {}
 # (the derivatives keep the default split: splits into fewer warps won alone on
 # an idle GPU but lost among concurrent fits, 1.655 s against 1.624 s untuned on
 # the 512-request stream)
-DERIV_CANDIDATES = ((131072, 1, 1),)
+DERIV_SPLIT = (131072, 1, 1)
 PROJ_CANDIDATES = (1, 2)          # 3D: tiles of 16 or 32 rows
 PROJ_CANDIDATES_2D = (1, 2, 3)    # 2D: tiles of 32, 64 or 128 cells
 
@@ -165,8 +164,8 @@ def plans_for_request(req, order=2):
 
 def tune_request_classes(requests, device, reps=3, order=2):
     """Tune each shape class among ``requests`` once, on its first request:
-    the projection's tiling and the derivative split, each timed under a plan
-    of its own.  Returns the number of classes tuned."""
+    the projection's tiling, timed under a plan of its own; the derivatives get
+    a plan with DERIV_SPLIT.  Returns the number of classes tuned."""
     from .geometry import DeviceGeometry
     done = 0
     for req in requests:
@@ -186,11 +185,11 @@ def tune_request_classes(requests, device, reps=3, order=2):
             if best_p is None or ms < best_p[1] * (1.0 - MARGIN):
                 best_p = (form, ms)
         pp.set(3, best_p[0])
-        fw = engine.fit_forward(atoms, geom, data, req.fit, req.background, plan=pp)
-        autotune_derivs(atoms, geom, fw["alpha"], fw["beta"],
-                        1.0 if req.fit == "l2" else 0.0, order=order, reps=reps,
-                        candidates=DERIV_CANDIDATES)
-        _req_plans[key] = (pp, plan_for(atoms, geom, order))
+        dp = engine.Plan(_lib.GR_OP_DERIVS_1 if order == 1 else _lib.GR_OP_DERIVS_2, atoms, geom)
+        for tune_key, value in enumerate(DERIV_SPLIT):
+            dp.set(tune_key, value)
+        _cache[shape_key(atoms, geom, order)] = dp
+        _req_plans[key] = (pp, dp)
         done += 1
     torch.cuda.synchronize(device)
     return done
