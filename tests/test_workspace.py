@@ -175,11 +175,12 @@ def test_pixel_integrated_forward_asks_for_no_records_without_gpu():
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("kind", ["2d", "2p5d"])
-def test_pixel_integrated_forward_in_its_own_workspace(eng, cuda_ready, kind):
+def test_pixel_integrated_forward_in_its_own_workspace(eng, cuda_ready, monkeypatch, kind):
     """Projection, fit and a fit step hold no more than the query for them."""
     g = make_geometry(kind, 70, 40)
     I, x, r = make_atoms(2 if kind == "2d" else 3, 300, 3)
     atoms, geom = engine_atoms(I, x, r), engine_geometry(g)
+    monkeypatch.setattr(eng, "_workspaces", {})    # (a stream's handle may be an older one's)
     s = torch.cuda.Stream()
     with torch.cuda.stream(s):
         R = eng.radproj(atoms, geom, psf=True)
