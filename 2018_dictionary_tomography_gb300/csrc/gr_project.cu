@@ -259,7 +259,18 @@ __global__ void __launch_bounds__(NW * 32, 32 / NW)
   // persistent blocks: the first item is the block's own, the others come from
   // a counter (asked for an item ahead), so heavy tiles do not hold the others
   // idle; what an item computes does not depend on which block takes it
-  int take = blockIdx.x;
+  int take = blockIdx.x, done = -1;
+  // the loss of the item done before: a column's cells as an FP32 pair, the columns in
+  // FP64, by the first warp while it waits for the next item's data (s_loss is written
+  // again behind that item's first barrier)
+  auto close_loss = [&]() {
+    if (!out.loss_part || done < 0 || warp != 0) return;
+    float ls = s_loss[lane].x, lc = s_loss[lane].y;
+#pragma unroll
+    for (int w = 1; w < NW; ++w) pair_add(ls, lc, s_loss[32 * w + lane].x, s_loss[32 * w + lane].y);
+    const double d = warp_sum_d((double)ls + (double)lc);
+    if (lane == 0) out.loss_part[done] = d;
+  };
   while (take < n_take) {
     int ahead = 0;
     if (tid == 0) ahead = (int)gridDim.x + atomicAdd(next_item, 1);
@@ -287,6 +298,7 @@ __global__ void __launch_bounds__(NW * 32, 32 / NW)
       for (int r = 0; r < 4; ++r, src += D1)
         if (r < nr) dv[r] = __ldg(src);
     }
+    close_loss();
     float v[4] = {0.f, 0.f, 0.f, 0.f};
     mine = __reduce_add_sync(0xffffffffu, mine);
     if (lane == 0) s_count[warp] = mine;
@@ -447,16 +459,9 @@ __global__ void __launch_bounds__(NW * 32, 32 / NW)
     if (tid == 0) s_item = ahead;
     __syncthreads();  // sV and s_count are reused
     take = s_item;
-    if (out.loss_part && warp == 0) {
-      // a column's cells as an FP32 pair, the columns in FP64 (the other warps go
-      // on: s_loss and s_item are written again behind the next item's barriers)
-#pragma unroll
-      for (int w = 1; w < NW; ++w)
-        pair_add(lsum, lcmp, s_loss[32 * w + lane].x, s_loss[32 * w + lane].y);
-      const double d = warp_sum_d((double)lsum + (double)lcmp);
-      if (lane == 0) out.loss_part[item] = d;
-    }
+    done = item;
   }
+  close_loss();
 
   if (loss_out && out.loss_part) {
     // the last block to finish sums the items' partials in item order (a flag of
