@@ -1485,16 +1485,22 @@ __device__ __forceinline__ void finalize_body(const float *part, const DerivCfg 
       src += B * step;
     };
     while (c + kFinBatch <= hi) add(std::integral_constant<int, kFinBatch>());
-    if (c + 4 <= hi) add(std::integral_constant<int, 4>());
-    if (c < hi) {
-      float v[3];
+    if constexpr (K == 2) {
+      // (66 values an atom keep the loads coming: 2936 x 5 chunks 7.5 us, 9.2 as below)
+      for (; c < hi; ++c, src += step) t += (double)__ldcs(src);
+    } else {
+      if (c + 4 <= hi) add(std::integral_constant<int, 4>());
+      if (c < hi) {
+        float v[3];
 #pragma unroll
-      for (int i = 0; i < 3; ++i) v[i] = c + i < hi ? __ldcs(src + i * step) : 0.f;
+        for (int i = 0; i < 3; ++i) v[i] = c + i < hi ? __ldcs(src + i * step) : 0.f;
 #pragma unroll
-      for (int i = 0; i < 3; ++i)
-        if (c + i < hi) t += (double)v[i];
+        for (int i = 0; i < 3; ++i)
+          if (c + i < hi) t += (double)v[i];
+      }
     }
-    (S == 1 ? vs[q] : ps[e])[tx] = t;
+    if (S == 1) vs[q][tx] = t;
+    else ps[e][tx] = t;
   }
   if (S > 1) {
     __syncthreads();
