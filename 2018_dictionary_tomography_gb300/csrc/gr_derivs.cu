@@ -53,10 +53,13 @@ __host__ __device__ constexpr int hess_min_warps(int K, bool one) {
 // atom per warp for Hessians and for long angle series, else four (so each
 // lane still has a few angles to amortise the warp's closing reduction).  A 3D
 // gradient has a cheap closing reduction for one atom, so there a series is long
-// from two angles per lane on (fewer would leave lanes idle): 4096 atoms x 121 x
-// 256^2: 63.7 us and 4.1 to sum the chunks, against 71.8 and 6.6 with four; 1000
-// x 1001 x 95^2: 89.4 + 4.5 against 98.0 + 13.7.  (The pixel-integrated kernel
-// keeps the longer line: 66 us with four, 76 with one at 128 x 401 x 64^2.)
+// from 64 angles on if rounding it up to a warp's 32 angles leaves few more lanes
+// idle than rounding to eight, or if pairs are shared among lanes anyway (us, one and
+// four atoms a warp, 8192 atoms x 64^2: 32 angles 33.7, 33.7; 33: 51.7, 40.6; 48: 53.4,
+// 46.8; 64: 56.5, 57.8; 65: 74.8, 64.2; 80: 77.3, 71.0; 96: 78.7, 82.4; 97: 97.7, 86.2; 128:
+// 101.2, 106.4; 300: 237, 240; 700: 508, 538; 100 atoms, shared: 64: 8.6, 10.1; 65: 9.4,
+// 10.7; 300: 11.6, 12.7).  (The pixel-integrated kernel keeps the longer line: 66 us
+// with four, 76 with one at 128 x 401 x 64^2.)
 // deriv_split_lanes: problems with few (atom, angle) pairs give a warp 32 / rs
 // of them, rs the largest power of two up to 8 with pairs * rs <=
 // deriv_split_lanes, so that the pairs spread over more warps (a 3D gradient's
@@ -70,11 +73,14 @@ __host__ __device__ constexpr int hess_min_warps(int K, bool one) {
 DerivCfg deriv_cfg(int K, int n_atoms, int n_angles, int order, const Tuning &t, bool split) {
   DerivCfg c;
   c.ag = next_pow2(n_atoms < 1 ? 1 : n_atoms);
-  const int ag_cap = t.deriv_atoms_per_warp > 0 ? t.deriv_atoms_per_warp
-                     : (order > 1 || n_angles >= (K == 2 && split ? 64 : 1024)) ? 1 : 4;
+  const long long pairs = (long long)(n_atoms < 1 ? 1 : n_atoms) * (n_angles < 1 ? 1 : n_angles);
+  bool one_atom = order > 1 || n_angles >= 1024;
+  if (K == 2 && split && n_angles >= 64)
+    one_atom = one_atom || 2 * pairs <= (long long)t.deriv_split_lanes ||
+               32 * ((n_angles + 31) / 32) <= 8 * ((n_angles + 7) / 8) * 17 / 16;
+  const int ag_cap = t.deriv_atoms_per_warp > 0 ? t.deriv_atoms_per_warp : one_atom ? 1 : 4;
   if (c.ag > ag_cap) c.ag = ag_cap;
   c.sg = 32 / c.ag;
-  const long long pairs = (long long)(n_atoms < 1 ? 1 : n_atoms) * (n_angles < 1 ? 1 : n_angles);
   c.rs = 1;
   while (split && t.deriv_split_lanes > 0 && c.rs < 8 && c.rs < c.sg &&
          pairs * c.rs * 2 <= (long long)t.deriv_split_lanes)

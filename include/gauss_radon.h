@@ -296,9 +296,9 @@ unsigned long long gr_launch_count(void);
  * GR_TUNE_DERIV_MIN_ANGLES: at least this many angles per lane group in a
  * chunk (default 1); GR_TUNE_DERIV_ATOMS_PER_WARP: atoms sharing a warp, a
  * power of two up to 32, the other lanes taking further angles of the same
- * atoms (default 0: automatic, one atom per warp for Hessians, for
- * point-sampled 3D gradients of 64 or more angles and for series of 1024 or
- * more, else four).  GR_TUNE_PROJ_TILING: tiles of the
+ * atoms (default 0: automatic, one atom per warp for Hessians, for series of
+ * 1024 or more angles and for point-sampled 3D gradients of 64 or more that
+ * fill warps of 32, else four).  GR_TUNE_PROJ_TILING: tiles of the
  * point-sampled 3D projection, 1 = 16 x 32 cells (default), 2 = 32 x 32
  * (fewer atoms cut by tile edges), 3 = as 1; of the 2D
  * projection, 32, 64 and 128 cells (one, two or four per lane: wide

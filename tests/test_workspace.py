@@ -28,13 +28,16 @@ def partials_bytes(kdet, n, A, order, atoms_per_warp, split):
 
 def schedules(kdet, n, A, order):
     """(point-sampled, pixel-integrated) partials: one atom a warp for Hessians and
-    long series, else four; a 3D point-sampled series is long from 64 angles."""
+    long series, else four; a 3D point-sampled series is long from 64 angles where they fill
+    warps of 32 about as well as eights, or pairs are shared."""
     ag = 1
     while ag < min(n, 4):
         ag *= 2
-    long_split = 64 if kdet == 2 else 1024
-    point = partials_bytes(kdet, n, A, order, 1 if order == 2 or A >= long_split else ag, True)
-    pixel = partials_bytes(kdet, n, A, order, 1 if order == 2 or A >= 1024 else ag, False)
+    one = order == 2 or A >= 1024
+    fits = -(-A // 32) * 32 <= -(-A // 8) * 8 * 17 // 16
+    one_point = one or (kdet == 2 and A >= 64 and (2 * n * A <= 65536 or fits))
+    point = partials_bytes(kdet, n, A, order, 1 if one_point else ag, True)
+    pixel = partials_bytes(kdet, n, A, order, 1 if one else ag, False)
     return point, pixel
 
 
