@@ -113,16 +113,16 @@ DerivCfg deriv_cfg(int K, int n_atoms, int n_angles, int order, const Tuning &t,
 // combined and handed back to the pair's lane, which does the chain-rule
 // assembly.  The groups walk rows (3D) in step, so that their loads share
 // sectors, and two cells at a time in packed FP32 pairs.
-// What bounds it: issue (58 % of the slots) and the 128 registers of the 3D
-// assembly (16 warps an SM; 168 registers and 12 warps: 363 against 301 us, 96
-// registers 310 us with four rows a lane).  A lane walking its pair alone, as
-// before, waited on 32 lines of the field per load with 12 warps an SM and 124
+// What bounds it: issue (51 % of the slots in 3D, 60 % in 2D) and the 128 registers
+// of the 3D assembly (16 warps an SM; 168 registers and 12 warps: 363 against 301 us,
+// 96 registers 310 us with four rows a lane).  A lane walking a wide pair alone
+// waited on 32 lines of the field per load with 12 warps an SM and 124
 // registers of moment sums; a group's lane keeps 20.  2936 atoms x 148 x 493^2
 // (3D, 120 cells a pair): 401 -> 277 us; 146 x 61 x 301 x 275: 18.7 -> 15.5 us;
-// 2150 x 153 x 467 (2D): 85.5 -> 58.6 us; 512 x 180 x 256 (9 cells a pair): 10.6
-// -> 11.8 us.  Cells a lane loads together: 2D, 2 lanes: 4, 6, 8: 60.0, 58.6,
-// 56.8 us there, 11.5, 11.8, 11.8 us on the small one; 3D, 4 lanes: 2, 4, 6, 8:
-// 397, 301, 277, 290 us.  4 lanes in 2D: 61.9 and 11.2 us.
+// 2150 x 153 x 467 (2D): 85.5 -> 58.6 us.  Cells a lane loads together: 2D, 2 lanes:
+// 4, 6, 8: 60.0, 58.6, 56.8 us there, 11.5, 11.8, 11.8 us on 512 x 180 x 256 (9 cells a
+// pair); 3D, 4 lanes: 2, 4, 6, 8: 397, 301, 277, 290 us.  4 lanes in 2D: 61.9 and 11.2
+// us.  Narrow pairs: walk_narrow_of.
 // cells of a lane loaded together (even)
 template <int K>
 __host__ __device__ constexpr int walk_cells_of() { return 6; }

@@ -96,7 +96,7 @@ __device__ __forceinline__ float kl_term(float f, float g) {
 // A cell therefore adds its atoms in index order with an exact two-sum and a
 // running compensation, whatever the tiling: results are bitwise reproducible
 // and the same under every tile height.
-// What bounds it: instruction issue (75 % of the slots on 8192 atoms x 2048
+// What bounds it: instruction issue (77 % of the slots on 8192 atoms x 2000
 // orientations; DRAM under 10 %).  Per (atom, angle) pair of 22 in-support
 // cells it issues 60 warp instructions: the visits 28, the masks' walk 15, the
 // staging the rest.  One warp walking an atom's whole box over sums in shared
@@ -106,9 +106,10 @@ __device__ __forceinline__ float kl_term(float f, float g) {
 // 2 x 2 to 8 x 4 cells they gave the fewest warp steps times instructions for
 // footprints of 20 to 140 cells; packed FP32 pairs do both rows at once.
 // 8192 atoms x 20000 x 128^2 cells: binning + projection 23.6 -> 15.1 ms; 1000
-// atoms x 1001 x 95^2: 185 -> 128 us; 2936 atoms x 148 x 493^2: 309 -> 278 us
-// (there 127 us are the 73408 items' own loads and stores: 2.1 us an item and
-// block, latency).  64 registers, 8 blocks an SM; 48 registers: 5 to 10 % slower.
+// atoms x 1001 x 95^2: 185 -> 128 us; 2936 atoms x 148 x 493^2: 309 -> 260 us
+// (there about half is the 73408 items' own work, some 600 warp instructions each;
+// forwards of few atoms over many items are all that: 20 atoms x 600 x 200^2 105 us,
+// 82 with a warp an item).  64 registers, 8 blocks an SM; 48 registers: 5 to 10 % slower.
 struct Proj3Rec {
   float4 a;   // (-qh0, -ql0, -qh1, -ql1): the centre's negative, as a float pair
   float4 b;   // (G00, 2 G01, G11, log2 amplitude)
@@ -482,7 +483,7 @@ __global__ void __launch_bounds__(NW * 32, 32 / NW)
 // angle, writes their records (rec, nullable) and gathers the tiles' words in
 // shared memory, a range of kBinTiles tiles at a time, so that every word of
 // the bitmap is written once: no clear, and no global atomics (whose latency
-// and contention bounded the launch before).  Instruction issue bounds it (89 % of
+// and contention bounded the launch before).  Instruction issue bounds it (91 % of
 // the slots, 500 a warp of pairs): four divisions by the tile's sides were a
 // fifth of them (8192 atoms x 20000: 3.05 ms, 2.46 with shifts).  In a range a
 // thread goes through its tiles there only (all of them in every range: 2.3 ms
@@ -588,7 +589,7 @@ __global__ void __launch_bounds__(256)
 // so tiles crossed by many atoms take fewer passes and barriers (2150 atoms x
 // 153 angles: 87.9 us with one atom per thread, 82.6 with two, 79.5 with
 // four; 512 atoms: 20.6, 20.7, 21.1 us).
-// What bounds it: issue (78 % of the slots), some 17 instructions a cell and
+// What bounds it: issue (81 % of the slots), some 17 instructions a cell and
 // atom: one 16-byte record, the form, the exponential and the compensated sum,
 // without a branch (with the support box in a second record and tests of it and
 // of the form: 75 us where this takes 51.1; with the form's test alone as a
@@ -810,7 +811,8 @@ __global__ void __launch_bounds__(128) gr_psf_bin_kernel(Atoms at, Geom g, TileC
 // bounds it) and go into the warp's own compensated sums in shared memory,
 // those of one cell in atom order; a cell then adds the warps' sums in warp order
 // (deterministic).  128 atoms x 401 x 64^2: 138 us with a warp per tile of 32 x
-// 32 cells, 109 us with four, 15 of 32 lanes at work; with the queue 65 us.
+// 32 cells, 109 us with four, 15 of 32 lanes at work; with the queue 69 us (issue, 68 %
+// of the slots).
 struct PsfStage {
   float4 a, b;   // qh0 ql0 qh1 ql1; G00 G01 G11 log2 amplitude
   float4 c;      // sign of I, rr, total mass

@@ -111,7 +111,8 @@ const char *gr_status_string(int status);
  * 3D projection it includes up to 512 MB of 32-byte (atom, angle) records; a
  * launch given less works through the angles in ranges, or without records.
  * The pixel-integrated forwards take GR_OP_PSF_PROJECT (GR_OP_PROJECT is enough
- * too).
+ * too); GR_OP_DERIVS_1 and _2 cover the point-sampled and the pixel-integrated
+ * derivatives.
  */
 size_t gr_workspace_bytes(int op, const gr_atoms *atoms, const gr_geometry *geom);
 
