@@ -249,7 +249,10 @@ __global__ void __launch_bounds__(NW * 32, 32 / NW)
   const int D0 = g.ax[0].n, D1 = g.ax[1].n;
   // the lane's subtile and cells
   const int grp = lane >> 1;
-  const int band = 4 * (warp >> 2) + (grp >> 2), cpair = 4 * (warp & 3) + (grp & 3);
+  // (a warp's columns differ from block to block: a warp beyond the detector's last
+  // column has no walk, and should not be the same scheduler's in every block)
+  const int wcol = (warp + (int)blockIdx.x) & 3;
+  const int band = 4 * (warp >> 2) + (grp >> 2), cpair = 4 * wcol + (grp & 3);
   const int row_in = 4 * band + 2 * (lane & 1), col_in = 2 * cpair;
   const int n_take = LIST ? *n_list : n_items;
   if (tid < kWords) {
@@ -397,8 +400,9 @@ __global__ void __launch_bounds__(NW * 32, 32 / NW)
           const char *pa = reinterpret_cast<const char *>(sA);
           const char *pb = reinterpret_cast<const char *>(sB);
           const uint32_t *pm = &sMask[0][16 * band + cpair];
-          uint32_t m = *pm;
-          int left = nwords - 1;
+          const bool off = c0 + 8 * wcol >= D1;
+          uint32_t m = off ? 0u : *pm;
+          int left = off ? 0 : nwords - 1;
           int base = 16;
           while (m != 0u || left > 0) {
             if (m == 0u) {
