@@ -976,6 +976,7 @@ __global__ void __launch_bounds__(NW * 32, 32 / NW)
           if (ncell >= kPsfWide1) {
             // most of a 2D tile: its cells at once, a lane each, no queue
             direct(s2, box);
+            __syncwarp();  // (a queued cell's sum may be another lane's next)
             continue;
           }
         }
