@@ -18,7 +18,7 @@ SMS = 152
 LINES = {("2d", 1): ((SMS * 8, 32), (SMS * 16, 32), (1000, 2), (3000, 4)),
          ("2d", 2): ((SMS * 4, 32), (SMS * 8, 32), (1500, 8), (1500, 9), (1500, 16), (1500, 17)),
          ("2p5d", 1): ((SMS * 20 - 1, 3), (SMS * 60 - 1, 3)),
-         ("2p5d", 2): ((SMS * 10 - 1, 3), (SMS * 40 - 1, 3))}
+         ("2p5d", 2): ((SMS * 20 - 1, 3), (SMS * 40 - 1, 3))}
 
 
 @pytest.mark.parametrize("kind,order,blocks,A", [(k, o, b + more, A) for (k, o), bs in LINES.items()
