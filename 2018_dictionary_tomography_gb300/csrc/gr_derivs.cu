@@ -1765,14 +1765,15 @@ static void start_hess(const DerivArgs &d) {
 // 25, 31, 46; 500 x 130 x 300, r = 4: 38, 41, 43, x 64, r = 30: 15, 13.5, 11.4; 2154
 // x 736 x 75, r = 30: 152, 104, 72; Hessians there: 282, 183, 119).  3D, pairs a
 // warp: all 32 from some four full waves of such blocks on, half from 20 blocks an SM
-// on, for the same reason; wide supports lose a tenth by their last wave, more in fewer
-// blocks (us, 8, 16 and 32 a warp; gradients, 128 x 401 x 64^2, 11 blocks an SM, r = 8
-// and 20: 122, 145, 161 and 52, 50,
-// 54; 300 x 401, 25 blocks: 246, 265, 295 and 104, 89, 90; 600 x 401, 50 blocks, r = 8 and
-// 30: 476, 493, 520 and 160, 101, 89; 1412 x 907 x 78^2, 265 blocks, r = 12 and 35: 1894,
-// 1869, 1835 and 804, 510, 414; Hessians 234, 247, 306 and 110, 92, 103; 497, 501, 535 and
-// 229, 185, 172; 961, 949, 978 and 366, 242, 197; 3866, 3652, 3654 and 1845, 1231, 975; 651 x
-// 86 x 57^2, whole detectors, 13 blocks: 1900, 2406, -).
+// on, for the same reason; wide supports lose by their last wave, a tenth or, in few
+// blocks, a fifth, and narrow ones gain as much there, so the line of the Hessians keeps
+// the long calls from losing (us, 8, 16 and 32 a warp; gradients, 128 x 401 x 64^2, 11
+// blocks an SM, r = 8 and 20: 122, 145, 161 and 52, 50, 54; 300 x 401, 25 blocks: 246,
+// 265, 295 and 104, 89, 90; 600 x 401, 50 blocks, r = 8 and 30: 476, 493, 520 and 160,
+// 101, 89; 1412 x 907 x 78^2, 265 blocks, r = 12 and 35: 1894, 1869, 1835 and 804, 510,
+// 414; Hessians 234, 247, 306 and 110, 92, 103; 497, 501, 535 and 229, 185, 172; 961, 949,
+// 978 and 366, 242, 197; 3866, 3652, 3654 and 1845, 1231, 975; with 8 and 16 alone, 651 x
+// 86 x 57^2, whole detectors, 13 blocks: 1939, 2335, of six-parameter atoms 2473, 2856).
 constexpr int kPsfSms = 152;
 template <int ORDER>
 static void start_psf(const DerivArgs &d, float s) {
